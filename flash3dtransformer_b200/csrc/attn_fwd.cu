@@ -8,24 +8,30 @@
 // those buckets attend to each other with softmax(Q K^T / sqrt(D)) V; LSE is the natural-log row normaliser.
 // Buckets that no scope lists are left untouched.
 //
-// Kernel shape: one CTA = NQ tiles of 128 query rows of one (scope, head, batch row) that share one stream of K/V
-// tiles (the library instantiates NQ = 1; the scope's query tiles must be a multiple of NQ); 32 + 128 * NQ threads:
-//   warp 0        one elected thread is both the TMA producer and the MMA issuer.  It loads the Q tiles once and K/V
-//                 tiles of 64 keys through a 4-stage ring (3-D tensor maps over [token, head, dim], swizzle width =
-//                 min(128, 2*D) bytes), issues S_t = Q_t K^T (M=128, N=64) and O_t += P_t V (A operand P read from
-//                 tensor memory, V as MN-major B operand) for every query tile t and commits mbarriers.  A ring stage
-//                 is refilled without a barrier of its own: when the softmax warps of every tile have delivered P of
-//                 key tile j, they had all seen O complete up to tile j-1, so the MMAs that read stage (j-1) % 4 are
-//                 done and key tile j+3 may land there.
-//   warps 1..4NQ  softmax, four warps per query tile, one thread per query row; S is read with tcgen05.ld, the
-//                 running maximum and sum are kept in the base-2 domain, P is written as bf16 with tcgen05.st, O is
-//                 rescaled in tensor memory only when the row maximum moved, and the epilogue normalises and stores O
-//                 and LSE
-// Per query tile, tensor memory holds S (64 columns), P (32) and O (D) side by side: because P does not overwrite S,
-// the next key tile's Q K^T is issued as soon as the softmax threads have pulled S into registers, so the tensor pipe
-// computes S(j+1) while the warps exponentiate tile j.  At D = 32 the kernel is bound by the special-function unit
-// (one ex2 per score against 4*D = 128 tensor FLOPs) and by instruction issue of the softmax warps, not by the tensor
-// pipe; three of every sixteen exponentials are therefore computed on the FMA pipe (poly_exp2_pair).
+// Kernel shape: one CTA = 128 query rows of one (scope, head, batch row), 160 threads; four CTAs per SM up to D = 64, two
+// at D = 128:
+//   warp 0        one elected thread is both the TMA producer and the MMA issuer.  Keys come in tiles of 32 through a ring of
+//                 four stages (3-D tensor maps over [token, head, dim], swizzle width = min(128, 2*D) bytes).  In turn i it
+//                 waits for P of key tile i, issues O += P V (A operand P from tensor memory, V as MN-major B operand) and
+//                 behind it S(i + 2) = Q K^T over the columns that P(i) occupies (products of one thread run in order), and
+//                 commits both with one barrier.  A stage of the ring therefore holds V(i) and K(i + 2), and needs no barrier
+//                 of its own to be refilled: P(i) comes from threads that have seen the commit of turn i - 2.
+//   warps 1..4    softmax, one thread per query row: S is read with tcgen05.ld, P is written with tcgen05.st over the first
+//                 half of the same columns; the epilogue normalises and stores O and LSE
+// Two score buffers (2 x 32 columns) and O (D columns) share 128 tensor-memory columns (256 at D = 128).  With the scores of
+// two tiles in flight the softmax threads hand over P and go on with the next tile without waiting for a product, one
+// barrier wait per tile instead of two (the wait for S(j + 1) is also the wait for O to be complete up to tile j - 1), and
+// D = 64 / 128 fit four / two CTAs on an SM where 64-key tiles with separate P columns fit two / one.
+//
+// What bounds it.  One exponential per score against 4*D tensor FLOPs: the special-function unit (16 per clock per SM) needs
+// 512 cycles for 128 x 64 scores; three of every sixteen exponentials go to the FMA pipe (poly_exp2_pair), which leaves 416.
+// The softmax loop alone, with every barrier satisfied and no products, takes 485 cycles there (four warps per scheduler),
+// the kernel 550 including the start of its CTAs.  The loop takes no row maximum (SoftmaxRow::run): a 3-input maximum
+// occupies the ALU and the FMA pipe together, and the scan was a tenth of the loop.
+// Measured (B200, bf16, window 4096, TFLOP/s, before with 64-key tiles and one score buffer -> now): D = 16 248 -> 261,
+// D = 32 490 -> 510, D = 64 626-662 -> 813-844, D = 128 737-790 -> 972.
+// The issuing thread's code is on the critical path: unrolled by four it costs 8 % (instruction cache), as `lane == 0`
+// instead of elect.sync 20 % (the compiler then serialises every uniform operand).
 #include "f3d_common.cuh"
 #include "tc_sm100.cuh"
 #include "../../include/f3d_b200.h"
@@ -35,8 +41,6 @@ namespace f3d {
 int *status_word(int device);
 
 constexpr int kBQ = 128;      // query rows per tile
-constexpr int kBKV = 64;      // keys per tile
-constexpr int kKvStages = 4;
 
 struct AttnFwdArgs {
   __nv_bfloat16 *O; float *lse; const uint32_t *scopes;
@@ -104,272 +108,316 @@ __device__ __forceinline__ void poly_exp2_pair(uint64_t x2, float &e0, float &e1
   e1 = __int_as_float(__float_as_int(p1) + (n1 << 23));
 }
 
-template <int D, int BKV, int NQ> struct AttnCfg {
+template <int D> struct AttnCfg {
+  static constexpr int BKV = 32;                    // keys per tile
   static constexpr int DCH = D < 64 ? D : 64;       // columns per swizzled row
   static constexpr int NDCH = D / DCH;
   static constexpr int RB = DCH * 2;                // bytes per swizzled row
   static constexpr uint64_t SWZ = RB == 128 ? tc::kSwizzle128 : (RB == 64 ? tc::kSwizzle64 : tc::kSwizzle32);
-  static constexpr int kQBytes = kBQ * D * 2;       // one Q tile
+  static constexpr int kQBytes = kBQ * D * 2;
   static constexpr int kTileBytes = BKV * D * 2;    // one K or V tile
-  static constexpr int kStageBytes = 2 * kTileBytes;
-  static constexpr int kSmem = NQ * kQBytes + kKvStages * kStageBytes + 512 + 1024;
-  static constexpr int kThreads = 32 + 128 * NQ;
-  // Tensor memory columns of one query tile: S (fp32 scores, BKV), P (bf16 probabilities, two per column, BKV / 2),
-  // O (fp32, D).  P has columns of its own so that the next tile's S = Q K^T can be issued as soon as the softmax
-  // warps have read S, while they are still computing P.
-  static constexpr uint32_t kPCol = BKV;
-  static constexpr uint32_t kOCol = BKV + BKV / 2;
-  static constexpr uint32_t kTileCols = (kOCol + D) <= 128 ? 128u : 256u;
-  static constexpr uint32_t kTmemCols = kTileCols * NQ;
-  static constexpr int kMinCtas = (512 / (int)kTmemCols) < 4 ? (512 / (int)kTmemCols) : 4;
-  static_assert(kTmemCols <= 512, "tensor memory holds 512 columns");
+  static constexpr int R = 4;                       // ring stages: V of key tile i and K of key tile i + 2
+  static constexpr int kSmem = kQBytes + R * 2 * kTileBytes + 256 + 1024;
+  static constexpr int kThreads = 160;
+  static constexpr uint32_t kOCol = 2 * BKV;        // S0 (P0 over its first 16 columns), S1, O
+  static constexpr uint32_t kTmemCols = kOCol + D <= 128 ? 128 : 256;
+  static constexpr int kMinCtas = 512 / kTmemCols;
+  // pairs of a tile whose exponentials go to the FMA pipe: every fifth, spread out so that both pipes work on every row
+  // (an eighth to three eighths of the pairs measure within 2 % of one another)
+  static constexpr int kPoly = 0x4210;
 };
 
-// POLY8 != 0: of the sixteen pairs of scores of a half tile, pairs 4, 9 and 14 take their exponential from poly_exp2_pair
-// (FMA pipe) and the rest from ex2.approx (special-function unit), so that both pipes work on every row.  Share and
-// placement are measured choices (D = 32, W = 4096): none 439, two adjacent pairs of every eight 476, every fourth pair
-// 484, every fifth pair 497 TFLOP/s; larger shares cost more issue slots than the special-function slots they free.
-template <int D, int BKV, int NQ, int POLY8, bool F16>
-__global__ void __launch_bounds__((AttnCfg<D, BKV, NQ>::kThreads), (AttnCfg<D, BKV, NQ>::kMinCtas))
+// One pair of scores: x = s * c - m on packed fp32 pairs, the exponentials on the special-function unit or (pairs in POLY)
+// on the FMA pipe, the row sum of the unrounded probabilities, the packed 16-bit result.
+template <int POLY, bool F16, bool GUARD>
+__device__ __forceinline__ void exp_pair(const uint32_t (&r)[32], int i, uint64_t c2, uint64_t m2, uint64_t &sum2, uint32_t (&p)[16], float &poly_mx) {
+  const uint64_t xx = fma2(pack2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1])), c2, m2);
+  float e0, e1, x0, x1;
+  unpack2(xx, x0, x1);
+  if ((POLY >> i) & 1) {
+    if (GUARD) poly_mx = max3(poly_mx, x0, x1);
+    poly_exp2_pair(xx, e0, e1);
+  } else {
+    e0 = fast_exp2(x0); e1 = fast_exp2(x1);
+  }
+  sum2 = add2(sum2, pack2(e0, e1));
+  p[i] = pack_p2<F16>(e0, e1);
+}
+
+__device__ __forceinline__ float row_max32(const uint32_t (&r)[32]) {
+  float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+  for (int k = 0; k < 16; ++k) mx[k & 3] = max3(mx[k & 3], __uint_as_float(r[2 * k]), __uint_as_float(r[2 * k + 1]));
+  return fmaxf(max3(mx[0], mx[1], mx[2]), mx[3]);
+}
+
+__device__ __forceinline__ float sum4(uint64_t a, uint64_t b) {
+  float s0, s1, s2, s3;
+  unpack2(a, s0, s1);
+  unpack2(b, s2, s3);
+  return (s0 + s1) + (s2 + s3);
+}
+
+// Softmax state of one query row (one thread).
+template <int D, bool F16> struct SoftmaxRow {
+  using C = AttnCfg<D>;
+  uint32_t tmem, tmem_o, s_full, p_full;            // scores and O in this warp's lanes; barrier addresses
+  float m_run, l_run, alpha, poly_mx;
+  uint64_t c2;
+  bool ok, moved, bad;
+
+  __device__ __forceinline__ void wait_s(int j, const tc::WaitCtx &wc) {
+    ok = ok && tc::mbar_wait(s_full + 8u * ((uint32_t)j & 1u), (uint32_t)(j >> 1) & 1u, wc, 205);
+    tc::tc_fence_after_sync();
+  }
+  __device__ __forceinline__ void rescale_o() {
+#pragma unroll
+    for (int c = 0; c < D; c += 16) {
+      uint32_t o[16];
+      tc::tmem_ld_32x32b_x16(tmem_o + c, o);
+      tc::tmem_ld_wait();
+#pragma unroll
+      for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+      tc::tmem_st_32x32b_x16(tmem_o + c, o);
+    }
+  }
+  // key tile j, whose scores are in r: publishes P, fetches the scores of tile j + 1 into rn, returns the row sum.  The
+  // wait for those scores is also the wait for O: their product was committed together with P V of tile j - 1.
+  template <bool GUARD, bool FIRST>
+  __device__ __forceinline__ float tile(int j, const uint32_t (&r)[32], uint32_t (&rn)[32], const tc::WaitCtx &wc) {
+    const uint32_t b = (uint32_t)j & 1u;
+    if (FIRST && moved) {
+      wait_s(j + 1, wc);
+      rescale_o();
+    }
+    const uint64_t m2 = pack2(-m_run, -m_run);
+    uint64_t sa = pack2(0.f, 0.f), sb = sa;
+    uint32_t p[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) exp_pair<C::kPoly, F16, GUARD>(r, i, c2, m2, (i & 1) ? sb : sa, p, poly_mx);
+    wait_s(j + 1, wc);
+    tc::tmem_ld_32x32b_x32(tmem + (b ^ 1u) * C::BKV, rn);
+    tc::tmem_st_32x32b_x16(tmem + b * C::BKV, p);
+    tc::tmem_ld_wait();
+    tc::tmem_st_wait();
+    tc::tc_fence_before_sync();
+    tc::mbar_arrive(p_full + 8u * b);
+    return sum4(sa, sb);
+  }
+
+  // The usual loop takes no maximum.  The reference m_run is the maximum of the first key tile; it moves by the exponent of
+  // the row sum whenever that sum shows that scores have outgrown it, which leaves P, 16-bit floating point, and the fp32
+  // sums as exact as any other reference.  What it cannot follow is a jump by more than 2^kJump within two tiles: such a
+  // row marks itself bad and the CTA starts over with the maximum of every tile taken (`careful`).
+  __device__ __forceinline__ void run(int n, uint32_t (&ra)[32], uint32_t (&rb)[32], float scale_log2, const tc::WaitCtx &wc) {
+    constexpr float kMoveAt = 4096.f, kJump = F16 ? 16384.f : 1.2676506e30f;
+    m_run = row_max32(ra) * scale_log2;
+    for (int j = 0; j < n && ok; j += 2) {
+      float s = tile<true, true>(j, ra, rb, wc);
+      s += tile<true, false>(j + 1, rb, ra, wc);
+      l_run += s;
+      moved = __any_sync(0xFFFFFFFFu, !(s <= kMoveAt));
+      if (moved) {
+        bad = bad || !(s < kJump);
+        const float up = s > kMoveAt ? (float)((__float_as_int(s) >> 23) - 127) : 0.f;
+        alpha = fast_exp2(-up);
+        m_run += up;
+        l_run *= alpha;
+      }
+    }
+    bad = bad || !(poly_mx < 100.f);
+  }
+  // The same with the maximum of every tile, for fp16 (whose P overflows past 65504) and for rows that `run` gave up on.
+  // The reference still moves only when a maximum exceeds it by more than kMaxSlack (base-2 units), so that O is almost
+  // never rescaled after the first tiles.
+  __device__ __forceinline__ void run_careful(int n, uint32_t (&ra)[32], uint32_t (&rb)[32], float scale_log2, const tc::WaitCtx &wc) {
+    for (int j = 0; j < n && ok; j += 2) {
+      follow(row_max32(ra) * scale_log2, j > 0);
+      l_run += tile<false, true>(j, ra, rb, wc);
+      follow(row_max32(rb) * scale_log2, true);
+      l_run += tile<false, true>(j + 1, rb, ra, wc);
+    }
+  }
+  __device__ __forceinline__ void follow(float mx, bool have_o) {
+    constexpr float kMaxSlack = 8.f;
+    moved = __any_sync(0xFFFFFFFFu, mx > m_run + kMaxSlack);
+    if (moved) {
+      const float m_new = mx > m_run + kMaxSlack ? mx : m_run;
+      alpha = fast_exp2(m_run - m_new);                                    // 1 for rows that keep their reference
+      m_run = m_new;
+      l_run *= alpha;
+    }
+    moved = moved && have_o;
+  }
+};
+
+template <int D, bool F16>
+__global__ void __launch_bounds__(AttnCfg<D>::kThreads, AttnCfg<D>::kMinCtas)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                const __grid_constant__ CUtensorMap map_v, AttnFwdArgs a) {
-  using C = AttnCfg<D, BKV, NQ>;
+                   const __grid_constant__ CUtensorMap map_v, AttnFwdArgs a) {
+  using C = AttnCfg<D>;
+  constexpr int R = C::R, BKV = C::BKV;
   extern __shared__ unsigned char smem_raw[];
   unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  unsigned char *sq = smem;
-  unsigned char *skv = smem + NQ * C::kQBytes;
-  uint64_t *bars = reinterpret_cast<uint64_t *>(skv + kKvStages * C::kStageBytes);
-  uint64_t *q_full = bars, *kv_full = bars + 1;
-  uint64_t *s_full = kv_full + kKvStages, *p_full = s_full + NQ, *o_full = p_full + NQ, *s_free = o_full + NQ;
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(s_free + NQ);
+  unsigned char *sq = smem, *sk = smem + C::kQBytes, *sv = sk + R * C::kTileBytes;
+  uint64_t *bars = reinterpret_cast<uint64_t *>(sv + R * C::kTileBytes);
+  uint64_t *kv_full = bars, *s_full = bars + R, *p_full = s_full + 2, *q_full = p_full + 2;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(q_full + 1);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // which group of NQ query tiles: tiles of a scope are numbered in scope order, bucket slot major
   const int tiles_per_scope = a.k * a.q_blocks_per_bucket;
-  const int groups_per_scope = tiles_per_scope / NQ;
-  const int scope = blockIdx.x / groups_per_scope;
-  const int tile0 = (blockIdx.x % groups_per_scope) * NQ;
+  const int scope = blockIdx.x / tiles_per_scope, qt = blockIdx.x % tiles_per_scope;
   const int head = blockIdx.y, brow = blockIdx.z;
   const uint32_t *my_scope = a.scopes + (size_t)scope * a.k;
-  const int tiles_per_bucket = a.bucket / BKV;
-  const int num_tiles = a.k * tiles_per_bucket;
-  auto q_token = [&](int t) -> int {                    // first query token of tile t of this CTA (inside batch row)
-    const int ti = tile0 + t;
-    return (int)my_scope[ti / a.q_blocks_per_bucket] * a.bucket + (ti % a.q_blocks_per_bucket) * kBQ;
+  const int n = a.k * a.q_blocks_per_bucket * (128 / BKV);        // key tiles, a multiple of four
+  const int row0 = brow * a.L;
+
+  auto load_tile = [&](unsigned char *dst, const CUtensorMap *map, uint64_t *bar, int tok) {
+#pragma unroll
+    for (int c = 0; c < C::NDCH; ++c) tc::tma_load_3d(dst + c * BKV * C::RB, map, bar, c * C::DCH, head, tok);
   };
-
-  if (threadIdx.x == 0) {
-    tc::mbar_init(q_full, 1);
-    for (int s = 0; s < kKvStages; ++s) tc::mbar_init(&kv_full[s], 1);
-    for (int t = 0; t < NQ; ++t) {
-      tc::mbar_init(&s_full[t], 1); tc::mbar_init(&p_full[t], 128); tc::mbar_init(&o_full[t], 1); tc::mbar_init(&s_free[t], 128);
-    }
-    *abort_flag = 0;
-    tc::mbar_fence_init();
-  }
-  if (warp == 0) { tc::tmem_alloc(tmem_slot, C::kTmemCols); tc::tmem_relinquish(); }
-  tc::tc_fence_before_sync();
-  __syncthreads();
-  tc::tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
+  uint32_t tmem_base = 0;
   tc::WaitCtx wc{abort_flag, a.status};
-
-  if (warp == 0) {
-    if (tc::elect_one()) {
-      tc::tma_prefetch_desc(&map_q); tc::tma_prefetch_desc(&map_k); tc::tma_prefetch_desc(&map_v);
-      tc::mbar_expect_tx(q_full, NQ * C::kQBytes);
+  SoftmaxRow<D, F16> sm;
+  sm.ok = sm.bad = false;
+  for (int pass = 0; pass < 2; ++pass) {
+    // One thread fills the ring and issues the products.  It sets the barriers up itself, so that its first loads are under
+    // way before the CTA has its tensor memory.  Stage i of the ring holds V of key tile i and K of key tile i + 2; the first
+    // four key tiles always lie in one bucket.
+    if (warp == 0 && tc::elect_one()) {
+      if (pass) for (uint64_t *bar = bars; bar <= q_full; ++bar) tc::mbar_inval(bar);
+      *abort_flag = 0;
+      for (int s = 0; s < R; ++s) tc::mbar_init(&kv_full[s], 1);
+      for (int b = 0; b < 2; ++b) { tc::mbar_init(&s_full[b], 1); tc::mbar_init(&p_full[b], 128); }
+      tc::mbar_init(q_full, 1);
+      tc::mbar_fence_init();
+      const int q_tok = (int)my_scope[qt / a.q_blocks_per_bucket] * a.bucket + (qt % a.q_blocks_per_bucket) * kBQ;
+      const int tok0 = row0 + (int)my_scope[0] * a.bucket;
+      tc::mbar_expect_tx(q_full, C::kQBytes + 2 * C::kTileBytes);
 #pragma unroll
-      for (int t = 0; t < NQ; ++t)
-#pragma unroll
-        for (int c = 0; c < C::NDCH; ++c)
-          tc::tma_load_3d(sq + t * C::kQBytes + c * kBQ * C::RB, &map_q, q_full, c * C::DCH, head, brow * a.L + q_token(t));
-      auto load_kv = [&](int j) {
-        const int s = j % kKvStages;
-        const int key_tok = (int)my_scope[j / tiles_per_bucket] * a.bucket + (j % tiles_per_bucket) * BKV;
-        unsigned char *sk = skv + s * C::kStageBytes, *sv = sk + C::kTileBytes;
-        tc::mbar_expect_tx(&kv_full[s], C::kStageBytes);
-#pragma unroll
-        for (int c = 0; c < C::NDCH; ++c) {
-          tc::tma_load_3d(sk + c * BKV * C::RB, &map_k, &kv_full[s], c * C::DCH, head, brow * a.L + key_tok);
-          tc::tma_load_3d(sv + c * BKV * C::RB, &map_v, &kv_full[s], c * C::DCH, head, brow * a.L + key_tok);
-        }
-      };
-      for (int j = 0; j < kKvStages && j < num_tiles; ++j) load_kv(j);
-
-      constexpr uint32_t idesc_s = tc::make_idesc_f16(kBQ, BKV, !F16, false, false);
-      constexpr uint32_t idesc_o = tc::make_idesc_f16(kBQ, C::DCH, !F16, false, true);    // B (= V) is MN-major
-      const uint32_t q_addr = tc::smem_u32(sq);
-      // S_t = Q_t K^T of key tile j: K-major operands, 8-row groups are 8*RB bytes apart
-      auto issue_s = [&](int t, int j) {
-        const uint32_t k_addr = tc::smem_u32(skv + (j % kKvStages) * C::kStageBytes);
-        const uint32_t s_tmem = tmem_base + t * C::kTileCols;
-#pragma unroll
-        for (int c = 0; c < C::NDCH; ++c) {
-#pragma unroll
-          for (int kk = 0; kk < C::DCH / 16; ++kk) {
-            uint64_t ad = tc::make_smem_desc(q_addr + t * C::kQBytes + c * kBQ * C::RB + kk * 32, 16, 8 * C::RB, C::SWZ);
-            uint64_t bd = tc::make_smem_desc(k_addr + c * BKV * C::RB + kk * 32, 16, 8 * C::RB, C::SWZ);
-            tc::mma_f16_ss(s_tmem, ad, bd, idesc_s, (c | kk) != 0 ? 1u : 0u);
-          }
-        }
-        tc::mma_commit(&s_full[t]);
-      };
-      bool ok = tc::mbar_wait(q_full, 0, wc, 202) && tc::mbar_wait(&kv_full[0], 0, wc, 203);
-      if (ok) {
-        tc::tc_fence_after_sync();
-#pragma unroll
-        for (int t = 0; t < NQ; ++t) issue_s(t, 0);
+      for (int c = 0; c < C::NDCH; ++c) tc::tma_load_3d(sq + c * kBQ * C::RB, &map_q, q_full, c * C::DCH, head, row0 + q_tok);
+      for (int i = 0; i < 2; ++i) load_tile(sk + (R - 2 + i) * C::kTileBytes, &map_k, q_full, tok0 + i * BKV);
+      for (int i = 0; i < 2; ++i) {
+        tc::mbar_expect_tx(&kv_full[i], 2 * C::kTileBytes);
+        load_tile(sv + i * C::kTileBytes, &map_v, &kv_full[i], tok0 + i * BKV);
+        load_tile(sk + i * C::kTileBytes, &map_k, &kv_full[i], tok0 + (i + 2) * BKV);
       }
-      for (int j = 0; j < num_tiles && ok; ++j) {
-        const int s = j % kKvStages;
-        if (j + 1 < num_tiles) {
-          if (!tc::mbar_wait(&kv_full[(j + 1) % kKvStages], (uint32_t)((j + 1) / kKvStages) & 1u, wc, 203)) { ok = false; break; }
-#pragma unroll
-          for (int t = 0; t < NQ; ++t) {
-            // the next scores may overwrite S once every softmax thread of the tile has read key tile j
-            if (!tc::mbar_wait(&s_free[t], (uint32_t)j & 1u, wc, 208)) { ok = false; break; }
-            tc::tc_fence_after_sync();
-            issue_s(t, j + 1);
+    }
+    if (pass == 0 && warp == 1) { tc::tmem_alloc(tmem_slot, C::kTmemCols); tc::tmem_relinquish(); }
+    tc::tc_fence_before_sync();
+    __syncthreads();
+    tc::tc_fence_after_sync();
+    tmem_base = *tmem_slot;
+    if (warp == 0) {
+      if (tc::elect_one()) {
+        // position of a stream of key tiles: row inside its bucket, first token of the bucket and of the next one (the scope
+        // table's entry is fetched a bucket ahead)
+        struct Stream {
+          const uint32_t *scope; int bucket, k, slot, row, base, next;
+          __device__ __forceinline__ void init(const uint32_t *sc, int bk, int kk, int from) {
+            scope = sc; bucket = bk; k = kk; slot = 0; row = from - BKV;
+            base = (int)sc[0] * bk;
+            next = kk > 1 ? (int)sc[1] * bk : 0;
+            take();
           }
-          if (!ok) break;
-        }
-        const uint32_t v_addr = tc::smem_u32(skv + s * C::kStageBytes) + C::kTileBytes;
-#pragma unroll
-        for (int t = 0; t < NQ; ++t) {
-          // O_t += P_t V once the softmax warps of the tile have written P
-          if (!tc::mbar_wait(&p_full[t], (uint32_t)j & 1u, wc, 204)) { ok = false; break; }
-          tc::tc_fence_after_sync();
-          const uint32_t p_tmem = tmem_base + t * C::kTileCols + C::kPCol, o_tmem = tmem_base + t * C::kTileCols + C::kOCol;
-#pragma unroll
-          for (int c = 0; c < C::NDCH; ++c) {
-#pragma unroll
-            for (int kk = 0; kk < BKV / 16; ++kk) {
-              // 16 keys per MMA: V rows kk*16.. ; P columns kk*8.. (two bf16 per 32-bit column)
-              uint64_t bd = tc::make_smem_desc(v_addr + c * BKV * C::RB + kk * 16 * C::RB, 16, 8 * C::RB, C::SWZ);
-              tc::mma_f16_ts(o_tmem + c * C::DCH, p_tmem + kk * 8, bd, idesc_o, (j | kk) != 0 ? 1u : 0u);
+          __device__ __forceinline__ int take() {
+            const int t = base + row;
+            row += BKV;
+            if (row == bucket) {
+              row = 0;
+              base = next;
+              ++slot;
+              if (slot + 1 < k) next = (int)scope[slot + 1] * bucket;
             }
+            return t;
           }
-          tc::mma_commit(&o_full[t]);
-        }
-        if (!ok) break;
-        // every tile has delivered P(j), so every tile had seen O complete up to key tile j-1: stage (j-1) % 4 is free
-        if (j >= 1 && j + kKvStages - 1 < num_tiles) load_kv(j + kKvStages - 1);
-      }
-    }
-  } else {
-    const int t = (warp - 1) >> 2;                               // query tile of this warp
-    const int q = warp & 3;                                      // tensor-memory lane quarter this warp may access
-    const int row = q * 32 + lane;                               // query row inside the tile = tensor-memory lane
-    const int q_tok = q_token(t);
-    const uint32_t lane_off = (uint32_t)(q * 32) << 16;
-    const uint32_t tile_tmem = tmem_base + t * C::kTileCols + lane_off;
-    const uint32_t s_tmem = tile_tmem, p_tmem = tile_tmem + C::kPCol, o_tmem = tile_tmem + C::kOCol;
-    uint64_t *my_s_full = &s_full[t], *my_s_free = &s_free[t], *my_p_full = &p_full[t], *my_o_full = &o_full[t];
-    float m_run = -INFINITY, l_run = 0.f;
-    const uint64_t c2 = pack2(a.scale_log2, a.scale_log2);
-    bool ok = true;
-    for (int j = 0; j < num_tiles && ok; ++j) {
-      if (!tc::mbar_wait(my_s_full, (uint32_t)j & 1u, wc, 205)) { ok = false; break; }
-      tc::tc_fence_after_sync();
-      uint32_t r0[32], r1[32];
-      tc::tmem_ld_32x32b_x32(s_tmem, r0);
-      tc::tmem_ld_32x32b_x32(s_tmem + 32, r1);
-      tc::tmem_ld_wait();
-      // the scores are in registers: the next key tile's Q K^T may be issued over them
-      tc::tc_fence_before_sync();
-      tc::mbar_arrive(my_s_free);
-      // four independent chains of 3-input maxima instead of one 32 deep
-      float mxa = -INFINITY, mxb = -INFINITY, mxc = -INFINITY, mxd = -INFINITY;
+        } ks, vs;
+        ks.init(my_scope, a.bucket, a.k, 4 * BKV);
+        vs.init(my_scope, a.bucket, a.k, 2 * BKV);
+        auto load_stage = [&](int i) {
+          const int s = i % R;
+          const bool has_k = i + 2 < n;
+          tc::mbar_expect_tx(&kv_full[s], has_k ? 2 * C::kTileBytes : C::kTileBytes);
+          load_tile(sv + s * C::kTileBytes, &map_v, &kv_full[s], row0 + vs.take());
+          if (has_k) load_tile(sk + s * C::kTileBytes, &map_k, &kv_full[s], row0 + ks.take());
+        };
+        constexpr uint32_t idesc_s = tc::make_idesc_f16(kBQ, BKV, !F16, false, false);
+        constexpr uint32_t idesc_o = tc::make_idesc_f16(kBQ, C::DCH, !F16, false, true);       // B (= V) is MN-major
+        const uint64_t qd = tc::make_smem_desc(tc::smem_u32(sq), 16, 8 * C::RB, C::SWZ);
+        const uint64_t kd = tc::make_smem_desc(tc::smem_u32(sk), 16, 8 * C::RB, C::SWZ);
+        const uint64_t vd = tc::make_smem_desc(tc::smem_u32(sv), 16, 8 * C::RB, C::SWZ);
+        auto issue_s = [&](int slot, uint32_t b) {
+          const uint64_t kds = kd + (uint32_t)(slot * (C::kTileBytes >> 4));
 #pragma unroll
-      for (int i = 0; i < 32; i += 4) {
-        mxa = max3(mxa, __uint_as_float(r0[i]), __uint_as_float(r1[i]));
-        mxb = max3(mxb, __uint_as_float(r0[i + 1]), __uint_as_float(r1[i + 1]));
-        mxc = max3(mxc, __uint_as_float(r0[i + 2]), __uint_as_float(r1[i + 2]));
-        mxd = max3(mxd, __uint_as_float(r0[i + 3]), __uint_as_float(r1[i + 3]));
-      }
-      const float mx = fmaxf(max3(mxa, mxb, mxc), mxd) * a.scale_log2;
-      // The reference point m_run of the exponentials follows the row maximum lazily: it moves only when the tile's
-      // maximum exceeds it by more than kMaxSlack (base-2 units), so probabilities stay below 2^kMaxSlack, which bf16 /
-      // fp16 and the fp32 sums hold without loss, and the result O / l does not depend on the choice.  On typical
-      // rows the maximum settles within the first tile or two; afterwards no thread of the warp rescales anything:
-      // no exponential for alpha, no round trip of O through tensor memory.
-      constexpr float kMaxSlack = 8.f;
-      float alpha = 1.f;
-      const bool moved = __any_sync(0xFFFFFFFFu, mx > m_run + kMaxSlack);       // first tile: m_run = -inf
-      if (moved) {
-        const float m_new = mx > m_run + kMaxSlack ? mx : m_run;
-        alpha = fast_exp2(m_run - m_new);                 // 1 for rows that keep their reference, 0 on the first tile
-        m_run = m_new;
-      }
-      // x = s * c - m and the row sum run on packed fp32 pairs; the sum adds the unrounded probabilities (the
-      // bf16 rounding of P is unbiased, so the normaliser stays consistent with what the MMA reads)
-      const uint64_t m2 = pack2(-m_run, -m_run);
-      uint64_t sum2 = pack2(0.f, 0.f);
-      uint32_t p[16];
+          for (int c = 0; c < C::NDCH; ++c)
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const uint64_t xx = fma2(pack2(__uint_as_float(r0[2 * i]), __uint_as_float(r0[2 * i + 1])), c2, m2);
-        float e0, e1;
-        if (POLY8 != 0 && (i % 5) == 4) {
-          poly_exp2_pair(xx, e0, e1);
-        } else {
-          float x0, x1;
-          unpack2(xx, x0, x1);
-          e0 = fast_exp2(x0); e1 = fast_exp2(x1);
-        }
-        sum2 = add2(sum2, pack2(e0, e1));
-        p[i] = pack_p2<F16>(e0, e1);
-      }
-      if (j > 0) {
-        // P of the previous tile has been consumed and O is complete up to it: P may be overwritten, O rescaled
-        if (!tc::mbar_wait(my_o_full, (uint32_t)(j - 1) & 1u, wc, 206)) { ok = false; break; }
+            for (int kk = 0; kk < C::DCH / 16; ++kk)
+              tc::mma_f16_ss(tmem_base + b * BKV, qd + (uint32_t)(c * (kBQ * C::RB >> 4) + 2 * kk), kds + (uint32_t)(c * (BKV * C::RB >> 4) + 2 * kk),
+                             idesc_s, (c | kk) != 0);
+        };
+        for (int i = 2; i < R - 2; ++i) load_stage(i);
+        bool ok = tc::mbar_wait(q_full, 0, wc, 202);
         tc::tc_fence_after_sync();
-      }
-      tc::tmem_st_32x32b_x16(p_tmem, p);
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const uint64_t xx = fma2(pack2(__uint_as_float(r1[2 * i]), __uint_as_float(r1[2 * i + 1])), c2, m2);
-        float e0, e1;
-        if (POLY8 != 0 && (i % 5) == 4) {
-          poly_exp2_pair(xx, e0, e1);
-        } else {
-          float x0, x1;
-          unpack2(xx, x0, x1);
-          e0 = fast_exp2(x0); e1 = fast_exp2(x1);
+        for (uint32_t b = 0; b < 2 && ok; ++b) {
+          issue_s(R - 2 + b, b);
+          tc::mma_commit(&s_full[b]);
         }
-        sum2 = add2(sum2, pack2(e0, e1));
-        p[i] = pack_p2<F16>(e0, e1);
-      }
-      tc::tmem_st_32x32b_x16(p_tmem + 16, p);
-      float sum, sum_hi;
-      unpack2(sum2, sum, sum_hi);
-      sum += sum_hi;
-      l_run = l_run * alpha + sum;
-      if (j > 0 && moved) {
+        for (int i = 0; i < n && ok; ++i) {
+          const uint32_t b = (uint32_t)i & 1u;
+          const int slot = i % R;
+          // the two stages that carried K of tiles 0 and 1 have had no turn of their own yet
+          if (!tc::mbar_wait(&kv_full[slot], (uint32_t)(i / R) & 1u, wc, 203)) { ok = false; break; }
+          if (!tc::mbar_wait(&p_full[b], (uint32_t)(i >> 1) & 1u, wc, 204)) { ok = false; break; }
+          tc::tc_fence_after_sync();
+          const uint64_t vds = vd + (uint32_t)(slot * (C::kTileBytes >> 4));
 #pragma unroll
-        for (int c = 0; c < D; c += 16) {
-          uint32_t o[16];
-          tc::tmem_ld_32x32b_x16(o_tmem + c, o);
-          tc::tmem_ld_wait();
+          for (int c = 0; c < C::NDCH; ++c)
 #pragma unroll
-          for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-          tc::tmem_st_32x32b_x16(o_tmem + c, o);
+            for (int kk = 0; kk < BKV / 16; ++kk)                 // 16 keys per MMA: V rows kk * 16.., P columns kk * 8..
+              tc::mma_f16_ts(tmem_base + C::kOCol + c * C::DCH, tmem_base + b * BKV + kk * 8,
+                             vds + (uint32_t)(c * (BKV * C::RB >> 4) + kk * C::RB), idesc_o, (i | kk) != 0);
+          // the next scores of this buffer overwrite P behind the product that reads it: MMAs of one thread run in order
+          if (i + 2 < n) issue_s(slot, b);
+          tc::mma_commit(&s_full[b]);
+          // P of tile i was written by threads that had seen the commit behind tile i - 2: its stage may be filled again
+          if (i + R - 2 < n) load_stage(i + R - 2);
         }
       }
-      tc::tmem_st_wait();
-      tc::tc_fence_before_sync();
-      tc::mbar_arrive(my_p_full);
-    }
-    if (ok && tc::mbar_wait(my_o_full, (uint32_t)(num_tiles - 1) & 1u, wc, 207) && q_tok + row < a.L) {
-      tc::tc_fence_after_sync();
-      const float inv = 1.f / l_run;
+    } else {
+    sm.tmem = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);    // the tensor-memory lanes this warp may access
+    sm.tmem_o = sm.tmem + C::kOCol;
+    sm.s_full = tc::smem_u32(s_full);
+    sm.p_full = tc::smem_u32(p_full);
+    sm.c2 = pack2(a.scale_log2, a.scale_log2);
+    sm.m_run = sm.poly_mx = -INFINITY;
+    sm.l_run = 0.f;
+    sm.alpha = 1.f;
+    sm.moved = sm.bad = false;
+    sm.ok = true;
+    uint32_t ra[32], rb[32];
+    sm.wait_s(0, wc);
+    tc::tmem_ld_32x32b_x32(sm.tmem, ra);
+    tc::tmem_ld_wait();
+    if (pass == 0) sm.run(n, ra, rb, a.scale_log2, wc);
+    else sm.run_careful(n, ra, rb, a.scale_log2, wc);
+    sm.wait_s(n + 1, wc);                                         // every product has been committed
+    if (pass == 0 && sm.moved) sm.rescale_o();            // a reference that moved behind the last tile
+  }
+  if (pass == 1 || !__syncthreads_or(sm.ok && sm.bad)) break;
+  }
+
+  if (warp != 0) {
+    const int row = (warp & 3) * 32 + lane;                      // query row inside the tile = tensor-memory lane
+    const int q_tok = (int)my_scope[qt / a.q_blocks_per_bucket] * a.bucket + (qt % a.q_blocks_per_bucket) * kBQ;
+    if (sm.ok && q_tok + row < a.L) {
+      const float inv = 1.f / sm.l_run;
       const size_t tok = (size_t)brow * a.L + q_tok + row;
       __nv_bfloat16 *op = a.O + (tok * a.H + head) * D;
 #pragma unroll
       for (int c = 0; c < D; c += 16) {
         uint32_t o[16];
-        tc::tmem_ld_32x32b_x16(o_tmem + c, o);
+        tc::tmem_ld_32x32b_x16(sm.tmem_o + c, o);
         tc::tmem_ld_wait();
         uint4 w[2];
         uint32_t *h2 = reinterpret_cast<uint32_t *>(w);
@@ -378,7 +426,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         *reinterpret_cast<uint4 *>(op + c) = w[0];
         *reinterpret_cast<uint4 *>(op + c + 8) = w[1];
       }
-      a.lse[tok * a.H + head] = (m_run + log2f(l_run)) * 0.6931471805599453f;
+      a.lse[tok * a.H + head] = (sm.m_run + log2f(sm.l_run)) * 0.6931471805599453f;
     }
   }
 
@@ -388,37 +436,33 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     for (int i = 0; i < 2000; ++i) __nanosleep(1000);
     __syncthreads();
   }
-  if (warp == 0) { tc::tc_fence_after_sync(); tc::tmem_dealloc(tmem_base, C::kTmemCols); }
+  if (warp == 1) { tc::tc_fence_after_sync(); tc::tmem_dealloc(tmem_base, C::kTmemCols); }
 }
 
-template <int D, int BKV, int NQ, int POLY8, bool F16>
+template <int D, bool F16>
 static int launch_attn_fwd(const void *Q, const void *K, const void *V, AttnFwdArgs a, int device, cudaStream_t st) {
-  using C = AttnCfg<D, BKV, NQ>;
-  auto kern = attn_fwd_kernel<D, BKV, NQ, POLY8, F16>;
+  using C = AttnCfg<D>;
+  auto kern = attn_fwd_kernel<D, F16>;
   const int dt = F16 ? 1 : 0;
   F3D_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(kern), device, C::kSmem));
   CUtensorMap mq, mk, mv;
   const uint64_t rows = (uint64_t)a.B * a.L;
   const uint64_t s1 = (uint64_t)D * 2, s2 = (uint64_t)a.H * D * 2;
   F3D_TRY(encode_tmap_3d(&mq, dt, Q, D, a.H, rows, s1, s2, C::DCH, 1, kBQ, C::RB));
-  F3D_TRY(encode_tmap_3d(&mk, dt, K, D, a.H, rows, s1, s2, C::DCH, 1, BKV, C::RB));
-  F3D_TRY(encode_tmap_3d(&mv, dt, V, D, a.H, rows, s1, s2, C::DCH, 1, BKV, C::RB));
-  dim3 grid(a.num_scopes * (a.k * a.q_blocks_per_bucket / NQ), a.H, a.B);
+  F3D_TRY(encode_tmap_3d(&mk, dt, K, D, a.H, rows, s1, s2, C::DCH, 1, C::BKV, C::RB));
+  F3D_TRY(encode_tmap_3d(&mv, dt, V, D, a.H, rows, s1, s2, C::DCH, 1, C::BKV, C::RB));
+  dim3 grid(a.num_scopes * a.k * a.q_blocks_per_bucket, a.H, a.B);
   kern<<<grid, C::kThreads, C::kSmem, st>>>(mq, mk, mv, a);
   return check_launch("buck_swin_fwd");
 }
 
-// Head sizes up to 32 are bound by the special-function unit: three of every sixteen exponentials go to the FMA pipe
-// (measured at D = 32, window 4096, with adjacent pairs: 0 / 12.5 / 25 / 37.5 / 50 % -> 439 / 448 / 462 / 446 / 413
-// TFLOP/s; spread out as every fifth pair, 18.75 %: 497).  One query tile per CTA:
-// two and four tiles per CTA sharing the K/V stream measured 2 % and 4 % slower (their exponential phases line up).
 template <bool F16>
 static int launch_attn_fwd_any(int D, const void *Q, const void *K, const void *V, AttnFwdArgs a, int device, cudaStream_t st) {
   switch (D) {
-    case 16: return launch_attn_fwd<16, 64, 1, 2, F16>(Q, K, V, a, device, st);
-    case 32: return launch_attn_fwd<32, 64, 1, 2, F16>(Q, K, V, a, device, st);
-    case 64: return launch_attn_fwd<64, 64, 1, 0, F16>(Q, K, V, a, device, st);
-    default: return launch_attn_fwd<128, 64, 1, 0, F16>(Q, K, V, a, device, st);
+    case 16: return launch_attn_fwd<16, F16>(Q, K, V, a, device, st);
+    case 32: return launch_attn_fwd<32, F16>(Q, K, V, a, device, st);
+    case 64: return launch_attn_fwd<64, F16>(Q, K, V, a, device, st);
+    default: return launch_attn_fwd<128, F16>(Q, K, V, a, device, st);
   }
 }
 

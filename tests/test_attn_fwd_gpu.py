@@ -76,6 +76,37 @@ def test_scaled_inputs(cuda_device, mul):
     assert ((lse - ref_lse).abs() / ref_lse.abs().clamp(min=1)).max().item() <= 2e-2
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("d", [16, 32, 64, 128])
+@pytest.mark.parametrize("steps", ["first", "middle", "last", "ramp"])
+def test_growing_scores(cuda_device, d, dtype, steps):
+    """Rows whose later keys outgrow the reference taken from the first ones: a jump in the first, a middle or the last pair
+    of 32-key tiles (past what the loop without a row maximum can follow: the careful pass) and a ramp it follows by moving
+    its reference."""
+    from flash3dtransformer_b200.lib import pshattn
+    dev = cuda_device
+    l, h, bucket = 512, 2, 256
+    g = torch.Generator().manual_seed(11)
+    q, k, v = (torch.randn(1, l, h, d, generator=g).to(dtype) for _ in range(3))
+    big = 60.0 if dtype == torch.bfloat16 else 12.0
+    gain = torch.ones(bucket)
+    if steps == "ramp":
+        gain = torch.linspace(1.0, 8.0, bucket)
+    else:
+        at = {"first": 40, "middle": 140, "last": bucket - 3}[steps]
+        gain[at] = big
+    k = (k.float() * gain.repeat(l // bucket)[None, :, None, None]).to(dtype)
+    sc = torch.arange(l // bucket, dtype=torch.int64).reshape(-1, 1)
+    o = torch.zeros(1, l, h, d, dtype=dtype, device=dev)
+    lse = torch.zeros(1, l, h, dtype=torch.float32, device=dev)
+    pshattn.buck_swin_fwd(q.to(dev), k.to(dev), v.to(dev), o, lse, sc.to(torch.uint32).to(dev), bucket)
+    pshattn.device_status()
+    ref_o, ref_lse = ao.buck_swin_fwd(q, k, v, sc, bucket)
+    assert torch.isfinite(o.float()).all() and torch.isfinite(lse).all()
+    assert (o.float().cpu() - ref_o).abs().max().item() <= 3e-2
+    assert ((lse.cpu() - ref_lse).abs() / ref_lse.abs().clamp(min=1)).max().item() <= 1e-4
+
+
 def test_errors(cuda_device):
     from flash3dtransformer_b200.lib import pshattn
     dev = cuda_device
