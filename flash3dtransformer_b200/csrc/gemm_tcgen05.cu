@@ -477,7 +477,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         // stage 32 rows x 32 columns (64 bytes per row) in the layout the 64-byte-swizzled TMA store reads:
         // 16-byte chunk j of row r sits at chunk j ^ ((r >> 1) & 3)
         unsigned char *ob = my_out + obuf * 32 * 64;
-        if (lane == 0) tc::tma_wait_read<1>();    // the store issued two tasks ago has drained this buffer
+        if (tc::elect_one()) tc::tma_wait_read<1>();    // the store issued two tasks ago has drained this buffer
         __syncwarp();
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -489,7 +489,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         }
         tc::fence_proxy_async();
         __syncwarp();
-        if (lane == 0) {
+        if (tc::elect_one()) {
           const int sp = g.nsplit == 1 ? 0 : oc0 / g.split_n;     // which output matrix (no division without splits)
           tc::tma_store_3d(&map_c, ob, oc0 - sp * g.split_n, m0 + q * 32, sp);
           tc::tma_commit();
@@ -532,7 +532,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&acc_empty[acc]);
     }
-    if (lane == 0) tc::tma_wait_all<0>();
+    if (tc::elect_one()) tc::tma_wait_all<0>();
   }
 
   __syncthreads();
