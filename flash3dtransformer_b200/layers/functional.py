@@ -7,6 +7,7 @@ attention, pooling and unpooling run the native kernels.
 """
 from __future__ import annotations
 
+import weakref
 from typing import Optional
 
 import torch
@@ -17,16 +18,22 @@ from ..lib import pshattn
 _BF16_CACHE = {}
 
 
+def _forget(cache, key, p):
+    """A reference to p that drops the cache's entry when p goes (ids are reused, and a model's 16-bit weights should not
+    outlive it)."""
+    return weakref.ref(p, lambda _: cache.pop(key, None))
+
+
 def bf16_weight(p: torch.Tensor) -> torch.Tensor:
     """bf16 copy of a parameter, refreshed when the parameter is modified in place (optimizer step)."""
     if p.dtype == torch.bfloat16:
         return p.detach()
     key = id(p)
     hit = _BF16_CACHE.get(key)
-    if hit is not None and hit[0] == p._version and hit[1].device == p.device and hit[2] is p:
+    if hit is not None and hit[0] == p._version and hit[1].device == p.device and hit[2]() is p:
         return hit[1]
     w = p.detach().to(torch.bfloat16).contiguous()
-    _BF16_CACHE[key] = (p._version, w, p)
+    _BF16_CACHE[key] = (p._version, w, _forget(_BF16_CACHE, key, p))
     return w
 
 
@@ -52,7 +59,7 @@ def folded_layernorm(weight, bias, gamma, beta):
     key = (id(weight), id(gamma))
     ver = (weight._version, gamma._version, beta._version, bias._version if bias is not None else -1, weight.device)
     hit = _FOLD_CACHE.get(key)
-    if hit is not None and hit[0] == ver and hit[4] is weight:
+    if hit is not None and hit[0] == ver and hit[4]() is weight:
         return hit[1], hit[2], hit[3]
     with torch.no_grad():
         w32 = weight.detach().float()
@@ -62,7 +69,7 @@ def folded_layernorm(weight, bias, gamma, beta):
         if bias is not None:
             bf = bf + bias.detach().float()
         bf = bf.contiguous()
-    _FOLD_CACHE[key] = (ver, wf, s, bf, weight)
+    _FOLD_CACHE[key] = (ver, wf, s, bf, _forget(_FOLD_CACHE, key, weight))
     return wf, s, bf
 
 

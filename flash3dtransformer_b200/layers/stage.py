@@ -12,11 +12,14 @@ from typing import List
 import torch
 import torch.cuda.nvtx as nvtx
 from torch import nn
+from torch.nn.modules import module as nn_module
 
 from . import buck_swin, elem_wise
 from . import functional as F3
+from ..lib import _cabi, pshattn
 from ..psh import bucket_scope
 from ..psh import dev_context as f3ddev
+from ..psh import swin_attn as sa
 
 
 @dataclass(slots=True)
@@ -94,6 +97,116 @@ class XFMR(nn.Module):
         return out
 
 
+class BlockStack:
+    """Runs a list of XFMR blocks through one native call (f3d_xfmr_stack_bf16) where nothing but their forward is asked
+    for: no autograd, no NVTX ranges, no hooks, the layer types of this package.  `run` returns None otherwise and the
+    caller goes block by block; both give the same bits.
+
+    What the call needs (pointers to the 16-bit weights, the folded LayerNorms, the scope tables) is laid out once per
+    number of rows and stays valid as long as the blocks hold the same modules and unmodified parameters."""
+
+    MAX_SIGNATURES = 32
+    ENABLED = True
+
+    def __init__(self):
+        self._key, self._plans, self._keep = None, {}, ()
+
+    def __reduce__(self):          # copies and pickles of a model start without a plan
+        return (BlockStack, ())
+
+    @staticmethod
+    def _state(blocks):
+        """(identity and version of everything the plan is made from, parameters per block), or None if a block is not
+        the plain one."""
+        key, params = [], []
+        for b in blocks:
+            if type(b) is not XFMR:
+                return None, None
+            m = b._modules
+            norm, bwa, mlp = m["norm"], m["bwa"], m["mlp"]
+            if type(norm) is not nn.LayerNorm or type(bwa) is not buck_swin.BucketSwinAttentionModule or type(mlp) is not elem_wise.MLP:
+                return None, None
+            qkv, proj, inner = bwa._modules["qkv"], bwa._modules["proj"], mlp._modules["mlp"]
+            if type(inner) is not elem_wise.LayerNormMLP or inner.activation != "swiglu" or type(qkv) is not nn.Linear or type(proj) is not nn.Linear:
+                return None, None
+            for mod in (b, bwa, mlp, inner):
+                if mod._forward_hooks or mod._forward_pre_hooks:
+                    return None, None
+            n, q, o, i = norm._parameters, qkv._parameters, proj._parameters, inner._parameters
+            ps = (n["weight"], n["bias"], q["weight"], q["bias"], o["weight"], o["bias"], i["layer_norm_weight"], i["layer_norm_bias"],
+                  i["fc1_weight"], i["fc1_bias"], i["fc2_weight"], i["fc2_bias"])
+            for p in ps:
+                if p is None:
+                    key.append(None)
+                else:
+                    key += (id(p), p._version, p.data_ptr())
+            key += (id(b.swin_plan), norm.eps, inner.eps, bwa.num_heads, bwa.attn.buck_size)
+            params.append(ps)
+        return key, params
+
+    def _build(self, blocks, params, n, c, device):
+        """The argument array of the native call for n rows, and what its pointers need kept alive; None where the blocks
+        have to run one by one."""
+        arr, keep = (_cabi.XfmrBlock * len(blocks))(), []
+        hidden = heads = 0
+
+        def ptr(t):
+            keep.append(t)
+            return t.data_ptr()
+
+        for a, b, ps in zip(arr, blocks, params):
+            nw, nb, qw, qb, ow, ob, lw, lb, w1, b1, w2, b2 = ps
+            if (nw is None or nb is None or tuple(b.norm.normalized_shape) != (c,) or b.set_chnn != c or any(p is not None and p.device != device for p in ps)):
+                return None
+            fold = XFMR.FOLD_MIN_CHANNELS <= c <= 2048
+            a.norm_w, a.norm_b, a.ln2_w, a.ln2_b = (ptr(F3._fp32_param(p)) for p in (nw, nb, lw, lb))
+            if fold:
+                w, col, bias = F3.folded_layernorm(qw, qb, nw, nb)
+                a.qkv_w, a.qkv_colsum, a.qkv_b = ptr(w), ptr(col), ptr(bias)
+                w, col, bias = F3.folded_layernorm(w1, b1, lw, lb)
+                a.fc1_w, a.fc1_colsum, a.fc1_b = ptr(w), ptr(col), ptr(bias)
+            else:
+                a.qkv_w, a.fc1_w = ptr(F3.bf16_weight(qw)), ptr(F3.bf16_weight(w1))
+                a.qkv_b = ptr(F3._fp32_bias(qb)) if qb is not None else None
+                a.fc1_b = ptr(F3._fp32_bias(b1)) if b1 is not None else None
+            a.proj_w, a.fc2_w = ptr(F3.bf16_weight(ow)), ptr(F3.bf16_weight(w2))
+            a.proj_b = ptr(F3._fp32_bias(ob)) if ob is not None else None
+            a.fc2_b = ptr(F3._fp32_bias(b2)) if b2 is not None else None
+            scopes = b.swin_plan.gen_scopes_from_plan(n, device)
+            a.scopes = ptr(scopes)
+            a.norm_eps, a.ln2_eps = b.norm.eps, b.mlp.mlp.eps
+            a.heads, a.hidden = b.bwa.num_heads, w2.shape[1]
+            a.num_scopes, a.scope_size, a.bucket = scopes.shape[0], scopes.shape[1], b.bwa.attn.buck_size
+            hidden, heads = max(hidden, a.hidden), max(heads, a.heads)
+        return arr, int(_cabi.load().f3d_xfmr_stack_scratch(n, c, hidden)), heads, tuple(keep)
+
+    def run(self, blocks, x):
+        if (not self.ENABLED or not x.is_cuda or torch.is_grad_enabled() or x.dim() != 2 or x.shape[1] % 8 or x.shape[0] == 0 or not len(blocks)
+                or f3ddev.get_nvtx() or nn_module._has_any_global_hook()):
+            return None
+        key, params = self._state(blocks)
+        if key is None:
+            return None
+        n, c = x.shape
+        if key != self._key or len(self._plans) >= self.MAX_SIGNATURES:
+            self._key, self._plans = key, {}
+        plans = self._plans
+        sig = (n, c, x.device, XFMR.FOLD_MIN_CHANNELS)
+        if sig not in plans:
+            plans[sig] = self._build(blocks, params, n, c, x.device)
+        plan = plans[sig]
+        if plan is None:
+            return None
+        feat = (x if x.dtype == torch.bfloat16 else x.to(torch.bfloat16)).contiguous()
+        out = torch.empty_like(feat)
+        lse = sa.lse_rows(1, n, plan[2], x.device)
+        scratch = torch.empty(plan[1], dtype=torch.uint8, device=x.device)
+        st = _cabi.load().f3d_xfmr_stack_bf16(plan[0], len(blocks), feat.data_ptr(), out.data_ptr(), lse.data_ptr(), scratch.data_ptr(),
+                                              plan[1], n, c, pshattn._dev_index(x.device), pshattn._stream(x.device))
+        _cabi.check(st, "xfmr_stack")
+        return out
+
+
 class Stage(nn.Module):
     """Encoder blocks -> middle submodule -> decoder blocks, all with the (coord, feat, sep) signature."""
     NVTX_SCOPE = "Stage"
@@ -111,16 +224,23 @@ class Stage(nn.Module):
         self.encoder_blocks = nn.ModuleList([block(s) for s in encoder_specs])
         self.middle = submodule
         self.decoder_blocks = nn.ModuleList([block(s) for s in decoder_specs])
+        self._encoder_stack, self._decoder_stack = BlockStack(), BlockStack()
+
+    @staticmethod
+    def _run(stack, blocks, coord, x, sep):
+        out = stack.run(blocks, x)
+        if out is None:
+            for blk in blocks:
+                x = blk(coord, x, sep)
+            out = x
+        return out
 
     def forward(self, reduced_coord, reduced_feat, reduced_sep):
         if f3ddev.get_nvtx():
             nvtx.range_push(self.NVTX_SCOPE)
-        x = reduced_feat
-        for blk in self.encoder_blocks:
-            x = blk(reduced_coord, x, reduced_sep)
+        x = self._run(self._encoder_stack, self.encoder_blocks, reduced_coord, reduced_feat, reduced_sep)
         x = self.middle(reduced_coord, x, reduced_sep)
-        for blk in self.decoder_blocks:
-            x = blk(reduced_coord, x, reduced_sep)
+        x = self._run(self._decoder_stack, self.decoder_blocks, reduced_coord, x, reduced_sep)
         if f3ddev.get_nvtx():
             nvtx.range_pop()
         return x

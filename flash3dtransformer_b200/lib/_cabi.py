@@ -13,6 +13,15 @@ LIB_PATH = Path(__file__).resolve().parent / "libf3d_b200.so"
 
 _u32, _vp, _int, _f32 = c_uint32, c_void_p, c_int, c_float
 
+
+class XfmrBlock(ctypes.Structure):
+    """f3d_xfmr_block of include/f3d_b200.h."""
+    _fields_ = [(n, c_void_p) for n in ("norm_w", "norm_b", "qkv_w", "qkv_b", "proj_w", "proj_b", "ln2_w", "ln2_b", "fc1_w",
+                                        "fc1_b", "fc2_w", "fc2_b", "qkv_colsum", "fc1_colsum", "scopes")] + [
+                (n, c_float) for n in ("norm_eps", "ln2_eps")] + [
+                (n, c_int) for n in ("heads", "hidden", "num_scopes", "scope_size", "bucket")]
+
+
 # name -> (restype, argtypes); mirrors include/f3d_b200.h declaration by declaration
 PROTOTYPES = {
     "f3d_last_error": (c_char_p, []),
@@ -42,6 +51,8 @@ PROTOTYPES = {
     "f3d_buck_swin_fwd_dtype": (_int, [_vp, _vp, _vp, _vp, _vp, _vp, _int, _int, _int, _int, _int, _int, _u32, _int, _int, _vp]),
     "f3d_linear_fused": (_int, [_vp, _vp, _vp, _vp, _vp, _int, _int, _int, _int, _int, _int, _vp, _vp, _f32, _vp, _int, _vp]),
     "f3d_row_stats_bf16": (_int, [_vp, _vp, _u32, _u32, _int, _vp]),
+    "f3d_xfmr_stack_bf16": (_int, [ctypes.POINTER(XfmrBlock), _int, _vp, _vp, _vp, _vp, c_uint64, _u32, _u32, _int, _vp]),
+    "f3d_xfmr_stack_scratch": (c_uint64, [_u32, _u32, _u32]),
     "f3d_gemm_sm_bf16": (_int, [_vp, _vp, _vp, _int, _int, _int, _int, _vp]),
     "f3d_buck_swin_fwd": (_int, [_vp, _vp, _vp, _vp, _vp, _vp, _int, _int, _int, _int, _int, _int, _u32, _int, _vp]),
     "f3d_layernorm_bf16": (_int, [_vp, _vp, _vp, _vp, _u32, _u32, _f32, _int, _int, _vp]),

@@ -8,6 +8,11 @@ import torch
 from . import plan as f3dplan
 
 
+def lse_rows(b: int, l: int, h: int, device) -> torch.Tensor:
+    """Log-sum-exp rows that nobody reads: inside plan.level_buffers() one buffer per shape."""
+    return f3dplan.pooled(("lse", b, l, h, str(device)), lambda: torch.empty(b, l, h, dtype=torch.float32, device=device))
+
+
 @dataclass(slots=True)
 class BuckSwinFwdBuffers:
     O: torch.Tensor
@@ -17,9 +22,7 @@ class BuckSwinFwdBuffers:
     def create_buckswin_fwd_buff(Q: torch.Tensor):
         b, l, h, _ = Q.shape
         if f3dplan.enabled():
-            # inference inside plan.level_buffers(): the log-sum-exp rows are scratch nobody reads; one buffer per shape
-            lse = f3dplan.pooled(("lse", b, l, h, str(Q.device)), lambda: torch.empty(b, l, h, dtype=torch.float32, device=Q.device))
-            return BuckSwinFwdBuffers(torch.empty_like(Q), lse)
+            return BuckSwinFwdBuffers(torch.empty_like(Q), lse_rows(b, l, h, Q.device))
         return BuckSwinFwdBuffers(torch.empty_like(Q), torch.zeros(b, l, h, dtype=torch.float32, device=Q.device))
 
 

@@ -239,6 +239,24 @@ int f3d_linear_fused(const void *A, const void *W, const void *bias, const void 
  * of f3d_linear_fused for rows that no GEMM of this library produced.  C a multiple of 8, <= 2048. */
 int f3d_row_stats_bf16(const void *x, void *stats, uint32_t rows, uint32_t C, int device, void *stream);
 
+/* One transformer block of f3d_xfmr_stack_bf16 (the reference's XFMR, flash3dxfmr/layers/stage.py:90-101): weights bf16
+ * [out, in], biases, LayerNorm parameters and column sums fp32.  With qkv_colsum and fc1_colsum (both or neither) the two
+ * LayerNorms are folded into the projections behind them as in f3d_linear_fused (qkv_w / fc1_w then hold the scaled weights,
+ * qkv_b / fc1_b the folded biases).  fc1 is the SwiGLU projection [2 * hidden, C]; scopes is u32 [num_scopes, scope_size]. */
+typedef struct f3d_xfmr_block {
+  const void *norm_w, *norm_b, *qkv_w, *qkv_b, *proj_w, *proj_b, *ln2_w, *ln2_b, *fc1_w, *fc1_b, *fc2_w, *fc2_b;
+  const void *qkv_colsum, *fc1_colsum, *scopes;
+  float norm_eps, ln2_eps;
+  int heads, hidden, num_scopes, scope_size, bucket;
+} f3d_xfmr_block;
+
+/* out = the `count` blocks applied to x, both bf16 [rows, channels]; forward only.  The kernels of the operator entry points
+ * issued by one call.  lse: fp32 [rows, most heads of a block], overwritten; scratch: at least f3d_xfmr_stack_scratch bytes of device memory, 256-byte aligned. */
+int f3d_xfmr_stack_bf16(const f3d_xfmr_block *blocks, int count, const void *x, void *out, void *lse,
+                        void *scratch, uint64_t scratch_bytes, uint32_t rows, uint32_t channels, int device, void *stream);
+/* scratch bytes for the widest hidden layer among the blocks */
+uint64_t f3d_xfmr_stack_scratch(uint32_t rows, uint32_t channels, uint32_t hidden);
+
 /* replaces f3d::gemm_sm_bf16 (src/psh/gemm_dispatcher.cu:26-80; binding src/f3d_frontend.cu:135): O[M,N] = A[M,K] . B[K,N],
  * bf16 in/out, fp32 accumulation; synchronises the stream like the reference (:77).  Any M; N, K multiples of 8. */
 int f3d_gemm_sm_bf16(const void *A, const void *B, void *O, int M, int N, int K, int device, void *stream);
