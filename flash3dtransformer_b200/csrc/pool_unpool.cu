@@ -216,10 +216,13 @@ __global__ void __launch_bounds__(kPoolThreads) pool_reduce_bwd_kernel(const T *
 template <typename T>
 __global__ void __launch_bounds__(kPoolThreads) unpool_add_kernel(const T *__restrict__ res, const T *__restrict__ down,
                                                                   T *__restrict__ up, GatherArgs a, uint32_t covered_rows,
-                                                                  uint32_t up_rows, uint32_t gather_blocks) {
+                                                                  uint32_t up_rows, uint32_t zero_blocks) {
   constexpr int N = Chunk<T>::N;
-  if (blockIdx.x >= gather_blocks) {
-    uint64_t gid = (uint64_t)(blockIdx.x - gather_blocks) * kPoolThreads + threadIdx.x;
+  // The blocks that clear the tail come first in the grid.  The mark of an unfilled slot (rows of the pooled input + 3) is
+  // out of range for the pooling, but not for a residual padded by more than three rows: what the gather blocks store
+  // there, as the reference does, has to come behind the zeros.
+  if (blockIdx.x < zero_blocks) {
+    uint64_t gid = (uint64_t)blockIdx.x * kPoolThreads + threadIdx.x;
     uint64_t row = covered_rows + gid / a.chunks_per_row;
     uint32_t ch = (uint32_t)(gid % a.chunks_per_row);
     if (row < up_rows) {
@@ -230,7 +233,7 @@ __global__ void __launch_bounds__(kPoolThreads) unpool_add_kernel(const T *__res
     }
     return;
   }
-  uint64_t gid = (uint64_t)blockIdx.x * kPoolThreads + threadIdx.x;
+  uint64_t gid = (uint64_t)(blockIdx.x - zero_blocks) * kPoolThreads + threadIdx.x;
   uint32_t row = (uint32_t)(gid / a.chunks_per_row), ch = (uint32_t)(gid % a.chunks_per_row);
   if (row >= a.ind_rows) return;
   float d[N];
@@ -364,7 +367,7 @@ extern "C" int f3d_additive_unpool_fwd(
   if (gb + zb > 0) {
     F3D_DISPATCH_DT(feat_dtype, unpool_add_kernel<T><<<gb + zb, kPoolThreads, 0, st>>>(
         static_cast<const T *>(res_feat), static_cast<const T *>(down_feat), static_cast<T *>(up_add_feat), a, covered_rows,
-        up_rows, gb));
+        up_rows, zb));
   }
   F3D_TRY(check_launch("additive_unpool_fwd"));
   return maybe_sync(st, "additive_unpool_fwd");
