@@ -18,20 +18,22 @@ class SubbuckReduceFunction(Function):
         """Returns (reduced_feat, SubbuckBuffers); only reduced_feat is differentiable."""
         max_n = f3dbatch.max_inslen_from_seps(seps)
         feat = input_feat.contiguous()
-        sb = f3dsubbuck.SubbuckBuffers.create_subbuck_buff(coords, feat, seps, subbuck_size, out_alignment=out_alignment)
+        sb = f3dsubbuck.SubbuckBuffers.create_subbuck_buff(coords, feat, seps, subbuck_size, out_alignment=out_alignment, fill=False)
         pshattn.batch_subbuck_reduce(coords, feat, seps, max_n, subbuck_size, NUM_VOX, sb.bbox_min, sb.bbox_max,
                                      sb.subbuck_id, sb.subbuck_off, sb.reduced_sep, sb.reduced_coord, sb.reduced_feat,
                                      sb.unpool_ind, 1, reduction_op)
         ctx.save_for_backward(feat, sb.unpool_ind)
         ctx.subbuck_size = subbuck_size
         ctx.reduction_op = reduction_op
+        ctx.pooled_rows = sb.pooled_rows
         sb.remove_unused_buffers()
         return sb.reduced_feat, sb
 
     @staticmethod
     def backward(ctx, grad_reduced_feat, grad_buffers=None):
         input_feat, unpool_ind = ctx.saved_tensors
-        grad_input = torch.zeros_like(input_feat)
+        # the kernel writes every row of a scene; rows behind the last one (tail padding) have no gradient
+        grad_input = f3dsubbuck.zero_tail(torch.empty_like(input_feat), ctx.pooled_rows)
         pshattn.batch_subbuck_reduce_backward(grad_reduced_feat.contiguous(), input_feat, unpool_ind, grad_input,
                                               ctx.subbuck_size, ctx.reduction_op)
         return None, grad_input, None, None, None, None

@@ -202,7 +202,7 @@ class BlockStack:
         lse = sa.lse_rows(1, n, plan[2], x.device)
         scratch = torch.empty(plan[1], dtype=torch.uint8, device=x.device)
         st = _cabi.load().f3d_xfmr_stack_bf16(plan[0], len(blocks), feat.data_ptr(), out.data_ptr(), lse.data_ptr(), scratch.data_ptr(),
-                                              plan[1], n, c, pshattn._dev_index(x.device), pshattn._stream(x.device))
+                                              plan[1], n, c, x.get_device(), pshattn._stream(x.get_device()))
         _cabi.check(st, "xfmr_stack")
         return out
 

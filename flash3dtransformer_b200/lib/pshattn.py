@@ -21,14 +21,20 @@ _FEAT_DTYPES = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}
 
 
 # ------------------------------------------------------------------------------------------------ helpers
-def _require(cond: bool, msg: str) -> None:
-    if not cond:
-        raise RuntimeError(msg)
-
-
-def _check_tensors(tensors, names) -> torch.device:
-    """assert_contiguous + assert_same_device of src/common/runtime.h:36-70.  (The checks run on every operator call of
-    a forward pass, so the passing case is kept to plain comparisons; the messages are built only on failure.)"""
+def _check_tensors(tensors, names) -> int:
+    """assert_contiguous + assert_same_device of src/common/runtime.h:36-70; returns the device index.  (The checks run on
+    every operator call of a forward pass, so the passing case is kept to plain comparisons; the messages are built only on
+    failure.)"""
+    try:
+        dev = tensors[0].get_device()
+        if dev >= 0:
+            for t in tensors:
+                if t.get_device() != dev or not t.is_contiguous():
+                    break
+            else:
+                return dev
+    except AttributeError:
+        pass
     dev = None
     for t, n in zip(tensors, names):
         if not isinstance(t, torch.Tensor):
@@ -41,32 +47,31 @@ def _check_tensors(tensors, names) -> torch.device:
             dev = t.device
         elif t.device != dev:
             raise RuntimeError(f"Tensor {n} is on {t.device}, expected {dev}")
-    return dev
+    return tensors[0].get_device()
 
 
 def _check_dtype(tensors, names, dtype) -> None:
     """assert_dtype of src/common/runtime.h:72-86."""
+    for t in tensors:
+        if t.dtype != dtype:
+            break
+    else:
+        return
     for t, n in zip(tensors, names):
         if t.dtype != dtype:
             raise RuntimeError(f"Tensor {n} has dtype {t.dtype}, expected {dtype}")
 
 
-def _ptr(t: torch.Tensor) -> ctypes.c_void_p:
-    return ctypes.c_void_p(t.data_ptr())
+def _ptr(t: torch.Tensor) -> int:
+    return t.data_ptr()
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 
-def _stream(dev: torch.device) -> ctypes.c_void_p:
+def _stream(dev: int) -> int:
     """cudaStream_t of torch's current stream on the device."""
-    if _raw_stream is not None:
-        return ctypes.c_void_p(_raw_stream(dev.index if dev.index is not None else torch.cuda.current_device()))
-    return ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
-
-
-def _dev_index(dev: torch.device) -> int:
-    return dev.index if dev.index is not None else torch.cuda.current_device()
+    return _raw_stream(dev) if _raw_stream is not None else torch.cuda.current_stream(dev).cuda_stream
 
 
 # ------------------------------------------------------------------------------- DeviceManagerSingleton
@@ -138,21 +143,25 @@ def batch_psh_scatter_pad_hash(coord, bucket_id, bucket_counter, bucket_offset, 
                  ["bucket_counter", "bucket_offset", "batch_sep", "cumsum_counter"], torch.uint32)
     _check_dtype([bucket_id], ["bucket_id"], torch.uint16)
     _check_dtype([probe_offsets], ["probe_offsets"], torch.int16)
-    _require(coord.dim() == 2 and coord.shape[1] == 3, f"coord must be [N,3], got {tuple(coord.shape)}")
-    _require(scatter_coord.dim() == 2 and scatter_coord.shape[1] == 3, "scatter_coord must be [pad_to,3]")
+    if not (coord.dim() == 2 and coord.shape[1] == 3):
+        raise RuntimeError(f"coord must be [N,3], got {tuple(coord.shape)}")
+    if not (scatter_coord.dim() == 2 and scatter_coord.shape[1] == 3):
+        raise RuntimeError("scatter_coord must be [pad_to,3]")
     total_n = coord.shape[0]
     batch = batch_sep.shape[0]
-    _require(bucket_id.numel() >= total_n and bucket_offset.numel() >= total_n,
-             "bucket_id / bucket_offset are shorter than coord")
-    _require(bucket_counter.numel() == batch * num_bucket and cumsum_counter.numel() == batch * num_bucket,
-             f"bucket_counter / cumsum_counter must be [{batch},{num_bucket}]")
-    _require(probe_offsets.numel() == 128 * 3, "probe_offsets must be [128,3]")
-    _require(bbox_min.numel() == 3 and bbox_max.numel() == 3, "bbox_min / bbox_max must have 3 elements")
+    if not (bucket_id.numel() >= total_n and bucket_offset.numel() >= total_n):
+        raise RuntimeError("bucket_id / bucket_offset are shorter than coord")
+    if not (bucket_counter.numel() == batch * num_bucket and cumsum_counter.numel() == batch * num_bucket):
+        raise RuntimeError(f"bucket_counter / cumsum_counter must be [{batch},{num_bucket}]")
+    if probe_offsets.numel() != 128 * 3:
+        raise RuntimeError("probe_offsets must be [128,3]")
+    if not (bbox_min.numel() == 3 and bbox_max.numel() == 3):
+        raise RuntimeError("bbox_min / bbox_max must have 3 elements")
     st = _cabi.load().f3d_batch_psh_scatter_pad_hash(
         _ptr(coord), _ptr(bucket_id), _ptr(bucket_counter), _ptr(bucket_offset), _ptr(batch_sep),
         total_n, batch, int(instance_max_N), int(num_bucket), int(bucket_divisor), int(bucket_size), int(num_vox),
         _ptr(bbox_min), _ptr(bbox_max), _ptr(probe_offsets), _ptr(cumsum_counter), _ptr(scatter_coord),
-        scatter_coord.shape[0], float(pad_num), int(hash_type), _dev_index(dev), _stream(dev))
+        scatter_coord.shape[0], float(pad_num), int(hash_type), dev, _stream(dev))
     _cabi.check(st, "batch_psh_scatter_pad_hash")
 
 
@@ -189,20 +198,21 @@ def batch_bucket_sanitizer_cpu(bucket_id, bucket_counter, bucket_offset, offset_
     names = ["bucket_id", "bucket_counter", "bucket_offset", "offset_check_table", "bucket_residual", "batch_sep",
              "offset_maxcnt"]
     for t, n in zip(tensors, names):
-        _require(isinstance(t, torch.Tensor), f"{n} must be a torch.Tensor")
+        if not isinstance(t, torch.Tensor):
+            raise RuntimeError(f"{n} must be a torch.Tensor")
     _check_dtype([bucket_id], ["bucket_id"], torch.uint16)
     _check_dtype([bucket_counter, bucket_offset, bucket_residual, batch_sep, offset_maxcnt],
                  ["bucket_counter", "bucket_offset", "bucket_residual", "batch_sep", "offset_maxcnt"], torch.uint32)
     _check_dtype([offset_check_table], ["offset_check_table"], torch.int8)
     batch_size, num_bucket = int(batch_size), int(num_bucket)
-    _require(offset_check_table.dim() == 3 and offset_check_table.shape[0] == batch_size
-             and offset_check_table.shape[1] == num_bucket,
-             f"offset_check_table must be [{batch_size},{num_bucket},max_count], got {tuple(offset_check_table.shape)}")
-    _require(bucket_counter.numel() == batch_size * num_bucket and bucket_residual.numel() == batch_size * num_bucket,
-             f"bucket_counter / bucket_residual must be [{batch_size},{num_bucket}]")
-    _require(batch_sep.numel() >= batch_size and offset_maxcnt.numel() >= batch_size,
-             "batch_sep / offset_maxcnt are shorter than batch_size")
-    _require(bucket_offset.numel() >= bucket_id.numel(), "bucket_offset is shorter than bucket_id")
+    if not (offset_check_table.dim() == 3 and offset_check_table.shape[0] == batch_size and offset_check_table.shape[1] == num_bucket):
+        raise RuntimeError(f"offset_check_table must be [{batch_size},{num_bucket},max_count], got {tuple(offset_check_table.shape)}")
+    if not (bucket_counter.numel() == batch_size * num_bucket and bucket_residual.numel() == batch_size * num_bucket):
+        raise RuntimeError(f"bucket_counter / bucket_residual must be [{batch_size},{num_bucket}]")
+    if not (batch_sep.numel() >= batch_size and offset_maxcnt.numel() >= batch_size):
+        raise RuntimeError("batch_sep / offset_maxcnt are shorter than batch_size")
+    if bucket_offset.numel() < bucket_id.numel():
+        raise RuntimeError("bucket_offset is shorter than bucket_id")
     host = [t.detach().cpu().contiguous() for t in tensors]
     # the two in/out buffers are private host copies even for CPU inputs, so a failed check changes nothing
     table, residual = host[3].clone(), host[4].clone()
@@ -216,7 +226,8 @@ def batch_bucket_sanitizer_cpu(bucket_id, bucket_counter, bucket_offset, offset_
 
 # ------------------------------------------------------------------------------------- pooling / unpooling
 def _feat_code(t: torch.Tensor, name: str) -> int:
-    _require(t.dtype in _FEAT_DTYPES, f"Tensor {name} has dtype {t.dtype}; bfloat16, float16 and float32 are supported")
+    if t.dtype not in _FEAT_DTYPES:
+        raise RuntimeError(f"Tensor {name} has dtype {t.dtype}; bfloat16, float16 and float32 are supported")
     return _FEAT_DTYPES[t.dtype]
 
 
@@ -236,26 +247,30 @@ def batch_subbuck_reduce(scattered_coord, scattered_feat, batch_sep, instance_ma
     _check_dtype([batch_sep, subbuck_id, reduced_batch_sep, unpool_ind],
                  ["batch_sep", "subbuck_id", "reduced_batch_sep", "unpool_ind"], torch.uint32)
     _check_dtype([subbuck_off], ["subbuck_off"], torch.uint16)
-    _require(scattered_feat.shape[1] == reduced_feat.shape[1],
-             f"Input feature dim({scattered_feat.shape[1]}) != output feature dim({reduced_feat.shape[1]}).")
-    _require(reduced_coord.shape[0] == reduced_feat.shape[0],
-             f"Reduced coordinate length({reduced_coord.shape[0]}) != reduced feature length({reduced_feat.shape[0]}).")
-    _require(scattered_coord.shape[1] == 3 and reduced_coord.shape[1] == 3,
-             f"Input coordinates dim({scattered_coord.shape[1]}) or reduced coordinates dim({reduced_coord.shape[1]}) "
-             "are NOT 3D.")
-    _require(0 <= int(red_op) <= 3, f"Unsupported reduction operation id-{red_op}")
-    _require(unpool_ind.dim() == 2 and unpool_ind.shape[1] == subbuck_size,
-             f"Unpool_ind last dimension({unpool_ind.shape[-1]}) != subbucket_size({subbuck_size})")
+    if scattered_feat.shape[1] != reduced_feat.shape[1]:
+        raise RuntimeError(f"Input feature dim({scattered_feat.shape[1]}) != output feature dim({reduced_feat.shape[1]}).")
+    if reduced_coord.shape[0] != reduced_feat.shape[0]:
+        raise RuntimeError(f"Reduced coordinate length({reduced_coord.shape[0]}) != reduced feature length({reduced_feat.shape[0]}).")
+    if not (scattered_coord.shape[1] == 3 and reduced_coord.shape[1] == 3):
+        raise RuntimeError(f"Input coordinates dim({scattered_coord.shape[1]}) or reduced coordinates dim({reduced_coord.shape[1]}) "
+                           "are NOT 3D.")
+    if not (0 <= int(red_op) <= 3):
+        raise RuntimeError(f"Unsupported reduction operation id-{red_op}")
+    if not (unpool_ind.dim() == 2 and unpool_ind.shape[1] == subbuck_size):
+        raise RuntimeError(f"Unpool_ind last dimension({unpool_ind.shape[-1]}) != subbucket_size({subbuck_size})")
     total_n = scattered_coord.shape[0]
-    _require(scattered_feat.shape[0] >= total_n, "scattered_feat has fewer rows than scattered_coord")
-    _require(subbuck_id.numel() >= total_n and subbuck_off.numel() >= total_n, "subbuck_id / subbuck_off too short")
-    _require(reduced_batch_sep.shape[0] == batch_sep.shape[0], "reduced_batch_sep and batch_sep differ in length")
+    if scattered_feat.shape[0] < total_n:
+        raise RuntimeError("scattered_feat has fewer rows than scattered_coord")
+    if not (subbuck_id.numel() >= total_n and subbuck_off.numel() >= total_n):
+        raise RuntimeError("subbuck_id / subbuck_off too short")
+    if reduced_batch_sep.shape[0] != batch_sep.shape[0]:
+        raise RuntimeError("reduced_batch_sep and batch_sep differ in length")
     st = _cabi.load().f3d_batch_subbuck_reduce(
         _ptr(scattered_coord), _ptr(scattered_feat), _ptr(batch_sep), total_n, batch_sep.shape[0],
         int(instance_max_N), int(subbuck_size), int(num_vox), _ptr(bbox_min), _ptr(bbox_max), _ptr(subbuck_id),
         _ptr(subbuck_off), _ptr(reduced_batch_sep), _ptr(reduced_coord), _ptr(reduced_feat), _ptr(unpool_ind),
         unpool_ind.shape[0], reduced_feat.shape[0], scattered_feat.shape[1], code, int(hash_type), int(red_op),
-        _dev_index(dev), _stream(dev))
+        dev, _stream(dev))
     _cabi.check(st, "batch_subbuck_reduce")
 
 
@@ -267,15 +282,19 @@ def batch_subbuck_reduce_backward(grad_red_feat, input_feat, unpool_ind, grad_in
     code = _feat_code(input_feat, "input_feat")
     _check_dtype([grad_red_feat, grad_input_feat], ["grad_red_feat", "grad_input_feat"], input_feat.dtype)
     _check_dtype([unpool_ind], ["unpool_ind"], torch.uint32)
-    _require(unpool_ind.dim() == 2 and unpool_ind.shape[1] == subbuck_size,
-             f"Unpool_ind last dimension({unpool_ind.shape[-1]}) != subbucket_size({subbuck_size})")
-    _require(grad_red_feat.shape[0] >= unpool_ind.shape[0], "grad_red_feat has fewer rows than unpool_ind")
-    _require(grad_red_feat.shape[1] == input_feat.shape[1] == grad_input_feat.shape[1], "feature dims differ")
-    _require(grad_input_feat.shape[0] == input_feat.shape[0], "grad_input_feat and input_feat differ in length")
-    _require(0 <= int(reduction_op) <= 3, f"Unsupported reduction_op={reduction_op}")
+    if not (unpool_ind.dim() == 2 and unpool_ind.shape[1] == subbuck_size):
+        raise RuntimeError(f"Unpool_ind last dimension({unpool_ind.shape[-1]}) != subbucket_size({subbuck_size})")
+    if grad_red_feat.shape[0] < unpool_ind.shape[0]:
+        raise RuntimeError("grad_red_feat has fewer rows than unpool_ind")
+    if not (grad_red_feat.shape[1] == input_feat.shape[1] == grad_input_feat.shape[1]):
+        raise RuntimeError("feature dims differ")
+    if grad_input_feat.shape[0] != input_feat.shape[0]:
+        raise RuntimeError("grad_input_feat and input_feat differ in length")
+    if not (0 <= int(reduction_op) <= 3):
+        raise RuntimeError(f"Unsupported reduction_op={reduction_op}")
     st = _cabi.load().f3d_batch_subbuck_reduce_backward(
         _ptr(grad_red_feat), _ptr(input_feat), _ptr(unpool_ind), _ptr(grad_input_feat), input_feat.shape[0],
-        unpool_ind.shape[0], input_feat.shape[1], code, int(subbuck_size), int(reduction_op), _dev_index(dev),
+        unpool_ind.shape[0], input_feat.shape[1], code, int(subbuck_size), int(reduction_op), dev,
         _stream(dev))
     _cabi.check(st, "batch_subbuck_reduce_backward")
 
@@ -289,16 +308,19 @@ def additive_unpool_fwd(res_feat, down_feat, up_add_feat, unpool_ind, subbuck_si
     code = _feat_code(res_feat, "res_feat")
     _check_dtype([down_feat, up_add_feat], ["down_feat", "up_add_feat"], res_feat.dtype)
     _check_dtype([unpool_ind], ["unpool_ind"], torch.uint32)
-    _require(unpool_ind.dim() == 2 and unpool_ind.shape[1] == subbuck_size,
-             f"Unpool_ind last dimension({unpool_ind.shape[-1]}) != subbucket_size({subbuck_size})")
-    _require(res_feat.shape == up_add_feat.shape, "res_feat and up_add_feat differ in shape")
-    _require(down_feat.shape[0] >= unpool_ind.shape[0], "down_feat has fewer rows than unpool_ind")
-    _require(down_feat.shape[1] == res_feat.shape[1], "feature dims differ")
+    if not (unpool_ind.dim() == 2 and unpool_ind.shape[1] == subbuck_size):
+        raise RuntimeError(f"Unpool_ind last dimension({unpool_ind.shape[-1]}) != subbucket_size({subbuck_size})")
+    if res_feat.shape != up_add_feat.shape:
+        raise RuntimeError("res_feat and up_add_feat differ in shape")
+    if down_feat.shape[0] < unpool_ind.shape[0]:
+        raise RuntimeError("down_feat has fewer rows than unpool_ind")
+    if down_feat.shape[1] != res_feat.shape[1]:
+        raise RuntimeError("feature dims differ")
     up_rows = res_feat.shape[0]
     st = _cabi.load().f3d_additive_unpool_fwd(
         _ptr(res_feat), _ptr(down_feat), _ptr(up_add_feat), _ptr(unpool_ind), up_rows, unpool_ind.shape[0],
         up_rows if covered_rows is None else int(covered_rows), res_feat.shape[1], code, int(subbuck_size),
-        _dev_index(dev), _stream(dev))
+        dev, _stream(dev))
     _cabi.check(st, "additive_unpool_fwd")
 
 
@@ -309,13 +331,15 @@ def additive_unpool_bwd(grad_res, grad_down, grad_up_added, unpool_ind, subbuck_
     code = _feat_code(grad_up_added, "grad_up_added")
     _check_dtype([grad_res, grad_down], ["grad_res", "grad_down"], grad_up_added.dtype)
     _check_dtype([unpool_ind], ["unpool_ind"], torch.uint32)
-    _require(unpool_ind.dim() == 2 and unpool_ind.shape[1] == subbuck_size,
-             f"Unpool_ind last dimension({unpool_ind.shape[-1]}) != subbucket_size({subbuck_size})")
-    _require(grad_res.shape == grad_up_added.shape, "grad_res and grad_up_added differ in shape")
-    _require(grad_down.shape[0] >= unpool_ind.shape[0], "grad_down has fewer rows than unpool_ind")
+    if not (unpool_ind.dim() == 2 and unpool_ind.shape[1] == subbuck_size):
+        raise RuntimeError(f"Unpool_ind last dimension({unpool_ind.shape[-1]}) != subbucket_size({subbuck_size})")
+    if grad_res.shape != grad_up_added.shape:
+        raise RuntimeError("grad_res and grad_up_added differ in shape")
+    if grad_down.shape[0] < unpool_ind.shape[0]:
+        raise RuntimeError("grad_down has fewer rows than unpool_ind")
     st = _cabi.load().f3d_additive_unpool_bwd(
         _ptr(grad_res), _ptr(grad_down), _ptr(grad_up_added), _ptr(unpool_ind), grad_up_added.shape[0],
-        unpool_ind.shape[0], grad_up_added.shape[1], code, int(subbuck_size), _dev_index(dev), _stream(dev))
+        unpool_ind.shape[0], grad_up_added.shape[1], code, int(subbuck_size), dev, _stream(dev))
     _cabi.check(st, "additive_unpool_bwd")
 
 
@@ -325,7 +349,8 @@ EPI_NONE, EPI_GELU, EPI_SWIGLU = 0, 1, 2
 
 def device_status(device=None) -> None:
     """Raise if a kernel of this library abandoned a bounded wait on `device` since the last check."""
-    idx = torch.cuda.current_device() if device is None else _dev_index(torch.device(device))
+    idx = None if device is None else torch.device(device).index
+    idx = torch.cuda.current_device() if idx is None else idx
     _cabi.check(_cabi.load().f3d_device_status(idx), "device_status")
 
 
@@ -333,12 +358,15 @@ def gemm_sm_bf16(A, B, O) -> None:
     """f3d::gemm_sm_bf16 (src/psh/gemm_dispatcher.cu:26-80): O[M,N] = A[M,K] @ B[K,N], bf16."""
     dev = _check_tensors([A, B, O], ["A", "B", "O"])
     _check_dtype([A, B, O], ["A", "B", "O"], torch.bfloat16)
-    _require(A.dim() == 2 and B.dim() == 2 and O.dim() == 2, "A, B, O must be matrices")
+    if not (A.dim() == 2 and B.dim() == 2 and O.dim() == 2):
+        raise RuntimeError("A, B, O must be matrices")
     m, k = A.shape
-    _require(B.shape[0] == k, f"A is [{m},{k}] but B is {tuple(B.shape)}")
+    if B.shape[0] != k:
+        raise RuntimeError(f"A is [{m},{k}] but B is {tuple(B.shape)}")
     n = B.shape[1]
-    _require(tuple(O.shape) == (m, n), f"O must be [{m},{n}], got {tuple(O.shape)}")
-    _cabi.check(_cabi.load().f3d_gemm_sm_bf16(_ptr(A), _ptr(B), _ptr(O), m, n, k, _dev_index(dev), _stream(dev)),
+    if tuple(O.shape) != (m, n):
+        raise RuntimeError(f"O must be [{m},{n}], got {tuple(O.shape)}")
+    _cabi.check(_cabi.load().f3d_gemm_sm_bf16(_ptr(A), _ptr(B), _ptr(O), m, n, k, dev, _stream(dev)),
                 "gemm_sm_bf16")
 
 
@@ -352,25 +380,30 @@ def linear_bf16(x, weight, bias, out, residual=None, nsplit=1, epilogue=EPI_NONE
     if residual is not None:
         tensors.append(residual); names.append("residual")
     dev = _check_tensors(tensors, names)
-    _require(x.dtype in (torch.bfloat16, torch.float16), f"Tensor x has dtype {x.dtype}; bfloat16 and float16 are supported")
+    if x.dtype not in (torch.bfloat16, torch.float16):
+        raise RuntimeError(f"Tensor x has dtype {x.dtype}; bfloat16 and float16 are supported")
     _check_dtype(tensors, names, x.dtype)
     m, k = x.shape
     n = weight.shape[0]
-    _require(weight.shape[1] == k, f"weight must be [N,{k}], got {tuple(weight.shape)}")
+    if weight.shape[1] != k:
+        raise RuntimeError(f"weight must be [N,{k}], got {tuple(weight.shape)}")
     out_n = n // 2 if epilogue == EPI_SWIGLU else n
-    _require(out.numel() == m * out_n, f"out must hold {m}x{out_n} elements, got {out.numel()}")
-    bptr = ctypes.c_void_p(0)
+    if out.numel() != m * out_n:
+        raise RuntimeError(f"out must hold {m}x{out_n} elements, got {out.numel()}")
+    bptr = None
     if bias is not None:
         _check_tensors([bias], ["bias"])
         _check_dtype([bias], ["bias"], torch.float32)
-        _require(bias.numel() == n, f"bias must have {n} elements")
+        if bias.numel() != n:
+            raise RuntimeError(f"bias must have {n} elements")
         bptr = _ptr(bias)
-    rptr = ctypes.c_void_p(0)
+    rptr = None
     if residual is not None:
-        _require(tuple(residual.shape) == (m, out_n), f"residual must be [{m},{out_n}]")
+        if tuple(residual.shape) != (m, out_n):
+            raise RuntimeError(f"residual must be [{m},{out_n}]")
         rptr = _ptr(residual)
     st = _cabi.load().f3d_linear_dtype(_ptr(x), _ptr(weight), bptr, rptr, _ptr(out), m, n, k, int(nsplit), int(epilogue),
-                                       _FEAT_DTYPES[x.dtype], _dev_index(dev), _stream(dev))
+                                       _FEAT_DTYPES[x.dtype], dev, _stream(dev))
     _cabi.check(st, "linear_bf16")
 
 
@@ -383,31 +416,38 @@ def linear_fused(x, weight, bias, out, residual=None, nsplit=1, epilogue=EPI_NON
     LayerNorm weight, `ln_colsum` fp32 [N] its row sums, `bias` fp32 [N] with the LayerNorm bias folded in) and / or the
     row sums of the output written to `stats_out` fp32 [M, 2] for the LayerNorm that follows.  See f3d_linear_fused."""
     tensors, names = [x, weight, out], ["x", "weight", "out"]
-    for t, n in ((residual, "residual"),):
-        if t is not None:
-            tensors.append(t); names.append(n)
+    if residual is not None:
+        tensors.append(residual); names.append("residual")
     dev = _check_tensors(tensors, names)
-    _require(x.dtype in (torch.bfloat16, torch.float16), f"Tensor x has dtype {x.dtype}; bfloat16 and float16 are supported")
+    if x.dtype not in (torch.bfloat16, torch.float16):
+        raise RuntimeError(f"Tensor x has dtype {x.dtype}; bfloat16 and float16 are supported")
     _check_dtype(tensors, names, x.dtype)
     m, k = x.shape
     n = weight.shape[0]
-    _require(weight.shape[1] == k, f"weight must be [N,{k}], got {tuple(weight.shape)}")
+    if weight.shape[1] != k:
+        raise RuntimeError(f"weight must be [N,{k}], got {tuple(weight.shape)}")
     out_n = n // 2 if epilogue == EPI_SWIGLU else n
-    _require(out.numel() == m * out_n, f"out must hold {m}x{out_n} elements, got {out.numel()}")
-    _require(residual is None or tuple(residual.shape) == (m, out_n), f"residual must be [{m},{out_n}]")
+    if out.numel() != m * out_n:
+        raise RuntimeError(f"out must hold {m}x{out_n} elements, got {out.numel()}")
+    if not (residual is None or tuple(residual.shape) == (m, out_n)):
+        raise RuntimeError(f"residual must be [{m},{out_n}]")
     f32 = [t for t in (bias, ln_stats, ln_colsum, stats_out) if t is not None]
     if f32:
         _check_tensors(f32, ["fp32 side input"] * len(f32))
         _check_dtype(f32, ["fp32 side input"] * len(f32), torch.float32)
-    _require(bias is None or bias.numel() == n, f"bias must have {n} elements")
+    if not (bias is None or bias.numel() == n):
+        raise RuntimeError(f"bias must have {n} elements")
     if ln_stats is not None:
-        _require(ln_colsum is not None and bias is not None, "a folded LayerNorm needs ln_colsum and the folded bias")
-        _require(ln_stats.numel() == 2 * m and ln_colsum.numel() == n, f"ln_stats must be [{m},2] and ln_colsum [{n}]")
-    _require(stats_out is None or stats_out.numel() == 2 * m, f"stats_out must be [{m},2]")
-    opt = lambda t: _ptr(t) if t is not None else ctypes.c_void_p(0)
+        if not (ln_colsum is not None and bias is not None):
+            raise RuntimeError("a folded LayerNorm needs ln_colsum and the folded bias")
+        if not (ln_stats.numel() == 2 * m and ln_colsum.numel() == n):
+            raise RuntimeError(f"ln_stats must be [{m},2] and ln_colsum [{n}]")
+    if not (stats_out is None or stats_out.numel() == 2 * m):
+        raise RuntimeError(f"stats_out must be [{m},2]")
+    opt = lambda t: _ptr(t) if t is not None else None
     st = _cabi.load().f3d_linear_fused(_ptr(x), _ptr(weight), opt(bias), opt(residual), _ptr(out), m, n, k, int(nsplit),
                                        int(epilogue), _FEAT_DTYPES[x.dtype], opt(ln_stats), opt(ln_colsum), float(ln_eps),
-                                       opt(stats_out), _dev_index(dev), _stream(dev))
+                                       opt(stats_out), dev, _stream(dev))
     _cabi.check(st, "linear_fused")
 
 
@@ -416,8 +456,9 @@ def row_stats_bf16(x, stats) -> None:
     dev = _check_tensors([x, stats], ["x", "stats"])
     _check_dtype([x], ["x"], torch.bfloat16)
     _check_dtype([stats], ["stats"], torch.float32)
-    _require(x.dim() == 2 and stats.numel() == 2 * x.shape[0], "x must be [rows, C] and stats [rows, 2]")
-    st = _cabi.load().f3d_row_stats_bf16(_ptr(x), _ptr(stats), x.shape[0], x.shape[1], _dev_index(dev), _stream(dev))
+    if not (x.dim() == 2 and stats.numel() == 2 * x.shape[0]):
+        raise RuntimeError("x must be [rows, C] and stats [rows, 2]")
+    st = _cabi.load().f3d_row_stats_bf16(_ptr(x), _ptr(stats), x.shape[0], x.shape[1], dev, _stream(dev))
     _cabi.check(st, "row_stats_bf16")
 
 
@@ -435,13 +476,16 @@ def linear_wgrad_bf16(grad_out, x, grad_weight, grad_bias=None) -> None:
     dev = _check_tensors(ts, names)
     _check_dtype([grad_out, x], ["grad_out", "x"], torch.bfloat16)
     _check_dtype(ts[2:], names[2:], torch.float32)
-    _require(grad_out.dim() == 2 and x.dim() == 2 and grad_out.shape[0] == x.shape[0], "grad_out must be [M, N] and x [M, K]")
+    if not (grad_out.dim() == 2 and x.dim() == 2 and grad_out.shape[0] == x.shape[0]):
+        raise RuntimeError("grad_out must be [M, N] and x [M, K]")
     m, n = grad_out.shape
     k = x.shape[1]
-    _require(tuple(grad_weight.shape) == (n, k), f"grad_weight must be [{n},{k}]")
-    _require(grad_bias is None or grad_bias.numel() == n, f"grad_bias must have {n} elements")
+    if tuple(grad_weight.shape) != (n, k):
+        raise RuntimeError(f"grad_weight must be [{n},{k}]")
+    if not (grad_bias is None or grad_bias.numel() == n):
+        raise RuntimeError(f"grad_bias must have {n} elements")
     st = _cabi.load().f3d_linear_wgrad_bf16(_ptr(grad_out), _ptr(x), _ptr(grad_weight), _ptr(grad_bias) if grad_bias is not None else None,
-                                            m, n, k, _dev_index(dev), _stream(dev))
+                                            m, n, k, dev, _stream(dev))
     _cabi.check(st, "linear_wgrad_bf16")
 
 
@@ -453,32 +497,39 @@ def linear_ksplit_bf16(x, weight, out, bias=None, residual=None) -> None:
         tensors.append(residual); names.append("residual")
     dev = _check_tensors(tensors, names)
     _check_dtype(tensors, names, torch.bfloat16)
-    _require(x.dim() == 3 and weight.dim() == 3 and x.shape[0] == weight.shape[0] and x.shape[2] == weight.shape[2],
-             f"x must be [S, M, K] and weight [S, N, K], got {tuple(x.shape)} and {tuple(weight.shape)}")
+    if not (x.dim() == 3 and weight.dim() == 3 and x.shape[0] == weight.shape[0] and x.shape[2] == weight.shape[2]):
+        raise RuntimeError(f"x must be [S, M, K] and weight [S, N, K], got {tuple(x.shape)} and {tuple(weight.shape)}")
     s, m, k = x.shape
     n = weight.shape[1]
-    _require(tuple(out.shape) == (m, n), f"out must be [{m},{n}]")
-    _require(residual is None or tuple(residual.shape) == (m, n), f"residual must be [{m},{n}]")
-    bptr = ctypes.c_void_p(0)
+    if tuple(out.shape) != (m, n):
+        raise RuntimeError(f"out must be [{m},{n}]")
+    if not (residual is None or tuple(residual.shape) == (m, n)):
+        raise RuntimeError(f"residual must be [{m},{n}]")
+    bptr = None
     if bias is not None:
         _check_tensors([bias], ["bias"])
         _check_dtype([bias], ["bias"], torch.float32)
-        _require(bias.numel() == n, f"bias must have {n} elements")
+        if bias.numel() != n:
+            raise RuntimeError(f"bias must have {n} elements")
         bptr = _ptr(bias)
     st = _cabi.load().f3d_linear_ksplit_bf16(_ptr(x), _ptr(weight), bptr, _ptr(residual) if residual is not None else None,
-                                             _ptr(out), m, n, k, s, _dev_index(dev), _stream(dev))
+                                             _ptr(out), m, n, k, s, dev, _stream(dev))
     _cabi.check(st, "linear_ksplit_bf16")
 
 
 # --------------------------------------------------------------------------------------- bucketed attention
 def _check_qkv(tensors, names, dtypes=(torch.bfloat16,)):
     dev = _check_tensors(tensors, names)
-    _require(tensors[0].dtype in dtypes, f"Tensor {names[0]} has dtype {tensors[0].dtype}; supported: {', '.join(str(d) for d in dtypes)}")
-    _check_dtype(tensors, names, tensors[0].dtype)
-    shape = tuple(tensors[0].shape)
-    _require(len(shape) == 4, f"Expect {names[0]} with four axes [B, L, H, D], but got shape={shape}")
+    first = tensors[0]
+    if first.dtype not in dtypes:
+        raise RuntimeError(f"Tensor {names[0]} has dtype {first.dtype}; supported: {', '.join(str(d) for d in dtypes)}")
+    _check_dtype(tensors, names, first.dtype)
+    shape = first.shape
+    if len(shape) != 4:
+        raise RuntimeError(f"Expect {names[0]} with four axes [B, L, H, D], but got shape={tuple(shape)}")
     for t, n in zip(tensors, names):
-        _require(tuple(t.shape) == shape, f"{n} has shape {tuple(t.shape)}, expected {shape}")
+        if t.shape != shape:
+            raise RuntimeError(f"{n} has shape {tuple(t.shape)}, expected {tuple(shape)}")
     return dev, shape
 
 
@@ -490,11 +541,13 @@ def buck_swin_fwd(Q, K, V, O, L, Scope_buckets, bucket_size) -> None:
     _check_tensors([L, Scope_buckets], ["L", "Scope_buckets"])
     _check_dtype([L], ["L"], torch.float32)
     _check_dtype([Scope_buckets], ["Scope_buckets"], torch.uint32)
-    _require(tuple(L.shape) == (b, l, h), f"L must be [{b},{l},{h}], got {tuple(L.shape)}")
-    _require(Scope_buckets.dim() == 2, "Scope_buckets must be [num_scopes, scope_size]")
+    if L.shape != (b, l, h):
+        raise RuntimeError(f"L must be [{b},{l},{h}], got {tuple(L.shape)}")
+    if Scope_buckets.dim() != 2:
+        raise RuntimeError("Scope_buckets must be [num_scopes, scope_size]")
     st = _cabi.load().f3d_buck_swin_fwd_dtype(_ptr(Q), _ptr(K), _ptr(V), _ptr(O), _ptr(L), _ptr(Scope_buckets), b, l, h, d,
                                               Scope_buckets.shape[0], Scope_buckets.shape[1], int(bucket_size),
-                                              _FEAT_DTYPES[Q.dtype], _dev_index(dev), _stream(dev))
+                                              _FEAT_DTYPES[Q.dtype], dev, _stream(dev))
     _cabi.check(st, "buck_swin_fwd")
 
 
@@ -504,10 +557,12 @@ def layernorm_bf16(x, weight, bias, out, eps=1e-5, gelu=False) -> None:
     dev = _check_tensors([x, weight, bias, out], ["x", "weight", "bias", "out"])
     _check_dtype([x, out], ["x", "out"], torch.bfloat16)
     _check_dtype([weight, bias], ["weight", "bias"], torch.float32)
-    _require(x.dim() == 2 and x.shape == out.shape, "x and out must be [rows, C] of equal shape")
-    _require(weight.numel() == x.shape[1] and bias.numel() == x.shape[1], "weight / bias must have C elements")
+    if not (x.dim() == 2 and x.shape == out.shape):
+        raise RuntimeError("x and out must be [rows, C] of equal shape")
+    if not (weight.numel() == x.shape[1] and bias.numel() == x.shape[1]):
+        raise RuntimeError("weight / bias must have C elements")
     st = _cabi.load().f3d_layernorm_bf16(_ptr(x), _ptr(weight), _ptr(bias), _ptr(out), x.shape[0], x.shape[1], float(eps),
-                                         1 if gelu else 0, _dev_index(dev), _stream(dev))
+                                         1 if gelu else 0, dev, _stream(dev))
     _cabi.check(st, "layernorm_bf16")
 
 
@@ -517,10 +572,12 @@ def layernorm_bwd_bf16(x, grad_out, weight, grad_x, grad_weight, grad_bias, eps=
     dev = _check_tensors([x, grad_out, weight, grad_x, grad_weight, grad_bias], ["x", "grad_out", "weight", "grad_x", "grad_weight", "grad_bias"])
     _check_dtype([x, grad_out, grad_x], ["x", "grad_out", "grad_x"], torch.bfloat16)
     _check_dtype([weight, grad_weight, grad_bias], ["weight", "grad_weight", "grad_bias"], torch.float32)
-    _require(x.dim() == 2 and x.shape == grad_out.shape == grad_x.shape, "x, grad_out and grad_x must be [rows, C] of equal shape")
-    _require(weight.numel() == x.shape[1] == grad_weight.numel() == grad_bias.numel(), "weight, grad_weight, grad_bias must be [C]")
+    if not (x.dim() == 2 and x.shape == grad_out.shape == grad_x.shape):
+        raise RuntimeError("x, grad_out and grad_x must be [rows, C] of equal shape")
+    if not (weight.numel() == x.shape[1] == grad_weight.numel() == grad_bias.numel()):
+        raise RuntimeError("weight, grad_weight, grad_bias must be [C]")
     st = _cabi.load().f3d_layernorm_bwd_bf16(_ptr(x), _ptr(grad_out), _ptr(weight), _ptr(grad_x), _ptr(grad_weight), _ptr(grad_bias),
-                                             x.shape[0], x.shape[1], float(eps), _dev_index(dev), _stream(dev))
+                                             x.shape[0], x.shape[1], float(eps), dev, _stream(dev))
     _cabi.check(st, "layernorm_bwd_bf16")
 
 
@@ -529,10 +586,12 @@ def swiglu_bwd_bf16(pre_act, grad_out, grad_pre_act) -> None:
     Not part of the reference's operator module (its MLP backward is TransformerEngine's)."""
     dev = _check_tensors([pre_act, grad_out, grad_pre_act], ["pre_act", "grad_out", "grad_pre_act"])
     _check_dtype([pre_act, grad_out, grad_pre_act], ["pre_act", "grad_out", "grad_pre_act"], torch.bfloat16)
-    _require(pre_act.dim() == 2 and grad_out.dim() == 2 and pre_act.shape == grad_pre_act.shape, "pre_act and grad_pre_act must be [rows, 2F]")
-    _require(pre_act.shape[0] == grad_out.shape[0] and pre_act.shape[1] == 2 * grad_out.shape[1], "grad_out must be [rows, F]")
+    if not (pre_act.dim() == 2 and grad_out.dim() == 2 and pre_act.shape == grad_pre_act.shape):
+        raise RuntimeError("pre_act and grad_pre_act must be [rows, 2F]")
+    if not (pre_act.shape[0] == grad_out.shape[0] and pre_act.shape[1] == 2 * grad_out.shape[1]):
+        raise RuntimeError("grad_out must be [rows, F]")
     st = _cabi.load().f3d_swiglu_bwd_bf16(_ptr(pre_act), _ptr(grad_out), _ptr(grad_pre_act), pre_act.shape[0], grad_out.shape[1],
-                                          _dev_index(dev), _stream(dev))
+                                          dev, _stream(dev))
     _cabi.check(st, "swiglu_bwd_bf16")
 
 
@@ -541,9 +600,10 @@ def gelu_bwd_bf16(pre_act, grad_out, grad_pre_act, tanh_form: bool = False) -> N
     of the GEMM's GELU epilogue.  Not part of the reference's operator module (its GELU backward is torch autograd's)."""
     dev = _check_tensors([pre_act, grad_out, grad_pre_act], ["pre_act", "grad_out", "grad_pre_act"])
     _check_dtype([pre_act, grad_out, grad_pre_act], ["pre_act", "grad_out", "grad_pre_act"], torch.bfloat16)
-    _require(pre_act.shape == grad_out.shape == grad_pre_act.shape, "pre_act, grad_out and grad_pre_act must have one shape")
+    if not (pre_act.shape == grad_out.shape == grad_pre_act.shape):
+        raise RuntimeError("pre_act, grad_out and grad_pre_act must have one shape")
     st = _cabi.load().f3d_gelu_bwd_bf16(_ptr(pre_act), _ptr(grad_out), _ptr(grad_pre_act), pre_act.numel(), int(bool(tanh_form)),
-                                        _dev_index(dev), _stream(dev))
+                                        dev, _stream(dev))
     _cabi.check(st, "gelu_bwd_bf16")
 
 
@@ -552,8 +612,9 @@ def colsum_bf16(x, out) -> None:
     dev = _check_tensors([x, out], ["x", "out"])
     _check_dtype([x], ["x"], torch.bfloat16)
     _check_dtype([out], ["out"], torch.float32)
-    _require(x.dim() == 2 and out.numel() == x.shape[1], "x must be [rows, C] and out [C]")
-    st = _cabi.load().f3d_colsum_bf16(_ptr(x), _ptr(out), x.shape[0], x.shape[1], _dev_index(dev), _stream(dev))
+    if not (x.dim() == 2 and out.numel() == x.shape[1]):
+        raise RuntimeError("x must be [rows, C] and out [C]")
+    st = _cabi.load().f3d_colsum_bf16(_ptr(x), _ptr(out), x.shape[0], x.shape[1], dev, _stream(dev))
     _cabi.check(st, "colsum_bf16")
 
 
@@ -564,11 +625,14 @@ def coord_embed_bf16(coords, weight, bias, out) -> None:
     _check_dtype([coords], ["coords"], torch.float16)
     _check_dtype([weight, bias], ["weight", "bias"], torch.float32)
     _check_dtype([out], ["out"], torch.bfloat16)
-    _require(coords.dim() == 2 and coords.shape[1] == 3, "coords must be [rows, 3]")
-    _require(weight.dim() == 2 and weight.shape[1] == 3 and bias.numel() == weight.shape[0], "weight must be [C, 3], bias [C]")
-    _require(out.dim() == 2 and out.shape[0] == coords.shape[0] and out.shape[1] == weight.shape[0], "out must be [rows, C]")
+    if not (coords.dim() == 2 and coords.shape[1] == 3):
+        raise RuntimeError("coords must be [rows, 3]")
+    if not (weight.dim() == 2 and weight.shape[1] == 3 and bias.numel() == weight.shape[0]):
+        raise RuntimeError("weight must be [C, 3], bias [C]")
+    if not (out.dim() == 2 and out.shape[0] == coords.shape[0] and out.shape[1] == weight.shape[0]):
+        raise RuntimeError("out must be [rows, C]")
     st = _cabi.load().f3d_coord_embed_bf16(_ptr(coords), _ptr(weight), _ptr(bias), _ptr(out), coords.shape[0], weight.shape[0],
-                                           _dev_index(dev), _stream(dev))
+                                           dev, _stream(dev))
     _cabi.check(st, "coord_embed_bf16")
 
 
@@ -580,12 +644,14 @@ def coord_embed_bwd(coords, grad_out, grad_weight, grad_bias=None) -> None:
     _check_dtype([coords], ["coords"], torch.float16)
     _check_dtype([grad_out], ["grad_out"], torch.bfloat16)
     _check_dtype(ts[2:], ["grad_weight", "grad_bias"][:len(ts) - 2], torch.float32)
-    _require(coords.dim() == 2 and coords.shape[1] == 3 and grad_out.dim() == 2 and grad_out.shape[0] == coords.shape[0],
-             "coords must be [rows, 3] and grad_out [rows, C]")
-    _require(tuple(grad_weight.shape) == (grad_out.shape[1], 3), "grad_weight must be [C, 3]")
-    _require(grad_bias is None or grad_bias.numel() == grad_out.shape[1], "grad_bias must be [C]")
+    if not (coords.dim() == 2 and coords.shape[1] == 3 and grad_out.dim() == 2 and grad_out.shape[0] == coords.shape[0]):
+        raise RuntimeError("coords must be [rows, 3] and grad_out [rows, C]")
+    if tuple(grad_weight.shape) != (grad_out.shape[1], 3):
+        raise RuntimeError("grad_weight must be [C, 3]")
+    if not (grad_bias is None or grad_bias.numel() == grad_out.shape[1]):
+        raise RuntimeError("grad_bias must be [C]")
     st = _cabi.load().f3d_coord_embed_bwd(_ptr(coords), _ptr(grad_out), _ptr(grad_weight), _ptr(grad_bias) if grad_bias is not None else None,
-                                          coords.shape[0], grad_out.shape[1], _dev_index(dev), _stream(dev))
+                                          coords.shape[0], grad_out.shape[1], dev, _stream(dev))
     _cabi.check(st, "coord_embed_bwd")
 
 
@@ -596,14 +662,24 @@ def collate_points_f32(records, coords, extra=None) -> None:
     dev = _check_tensors(ts, ["records", "coords", "extra"][:len(ts)])
     _check_dtype([records], ["records"], torch.float32)
     _check_dtype([coords], ["coords"], torch.float16)
-    _require(records.dim() == 2 and tuple(coords.shape) == (records.shape[0], 3), "records must be [rows, dim], coords [rows, 3]")
+    if not (records.dim() == 2 and tuple(coords.shape) == (records.shape[0], 3)):
+        raise RuntimeError("records must be [rows, dim], coords [rows, 3]")
     if extra is not None:
         _check_dtype([extra], ["extra"], torch.float32)
-        _require(records.shape[1] > 3 and tuple(extra.shape) == (records.shape[0], records.shape[1] - 3),
-                 "extra must be [rows, dim - 3]")
+        if not (records.shape[1] > 3 and tuple(extra.shape) == (records.shape[0], records.shape[1] - 3)):
+            raise RuntimeError("extra must be [rows, dim - 3]")
     st = _cabi.load().f3d_collate_points_f32(_ptr(records), _ptr(coords), _ptr(extra) if extra is not None else None,
-                                             records.shape[0], records.shape[1], _dev_index(dev), _stream(dev))
+                                             records.shape[0], records.shape[1], dev, _stream(dev))
     _cabi.check(st, "collate_points_f32")
+
+
+def bbox_f16(coords, bbox_min, bbox_max) -> None:
+    """bbox_min / bbox_max fp16 [3] = the bounding box of fp16 coords [rows, 3], rows > 0."""
+    dev = _check_tensors([coords, bbox_min, bbox_max], ["coords", "bbox_min", "bbox_max"])
+    _check_dtype([coords, bbox_min, bbox_max], ["coords", "bbox_min", "bbox_max"], torch.float16)
+    if coords.dim() != 2 or coords.shape[1] != 3 or bbox_min.numel() != 3 or bbox_max.numel() != 3:
+        raise RuntimeError("coords must be [rows, 3], the box 3 + 3 values")
+    _cabi.check(_cabi.load().f3d_bbox_f16(_ptr(coords), _ptr(bbox_min), _ptr(bbox_max), coords.shape[0], dev, _stream(dev)), "bbox_f16")
 
 
 def scatter_index(bucket_id, bucket_offset, cumsum_counter, batch_sep, out2in, in2out=None) -> None:
@@ -616,13 +692,17 @@ def scatter_index(bucket_id, bucket_offset, cumsum_counter, batch_sep, out2in, i
     _check_dtype([bucket_id], ["bucket_id"], torch.uint16)
     _check_dtype(ts[1:], ["bucket_offset", "cumsum_counter", "batch_sep", "out2in", "in2out"][:len(ts) - 1], torch.uint32)
     n = bucket_id.numel()
-    _require(bucket_offset.numel() == n, "bucket_offset must have one entry per point")
-    _require(cumsum_counter.dim() == 2 and cumsum_counter.shape[0] == batch_sep.numel(), "cumsum_counter must be [B, num_bucket]")
-    _require(out2in.numel() >= n, "out2in must hold at least one entry per point")
-    _require(in2out is None or in2out.numel() == n, "in2out must have one entry per point")
+    if bucket_offset.numel() != n:
+        raise RuntimeError("bucket_offset must have one entry per point")
+    if not (cumsum_counter.dim() == 2 and cumsum_counter.shape[0] == batch_sep.numel()):
+        raise RuntimeError("cumsum_counter must be [B, num_bucket]")
+    if out2in.numel() < n:
+        raise RuntimeError("out2in must hold at least one entry per point")
+    if not (in2out is None or in2out.numel() == n):
+        raise RuntimeError("in2out must have one entry per point")
     st = _cabi.load().f3d_scatter_index(_ptr(bucket_id), _ptr(bucket_offset), _ptr(cumsum_counter), _ptr(batch_sep), _ptr(out2in),
                                         _ptr(in2out) if in2out is not None else None, n, batch_sep.numel(),
-                                        cumsum_counter.shape[1], out2in.numel(), _dev_index(dev), _stream(dev))
+                                        cumsum_counter.shape[1], out2in.numel(), dev, _stream(dev))
     _cabi.check(st, "scatter_index")
 
 
@@ -630,11 +710,12 @@ def gather_rows(src, index, out) -> None:
     """out[i] = src[index[i]] over rows of any element type; rows whose index is not a row of src are zero."""
     dev = _check_tensors([src, index, out], ["src", "index", "out"])
     _check_dtype([index], ["index"], torch.uint32)
-    _require(src.dim() == 2 and out.dim() == 2 and src.shape[1] == out.shape[1] and src.dtype == out.dtype,
-             "src and out must be [rows, C] of one dtype and width")
-    _require(index.numel() == out.shape[0], "index must have one entry per row of out")
+    if not (src.dim() == 2 and out.dim() == 2 and src.shape[1] == out.shape[1] and src.dtype == out.dtype):
+        raise RuntimeError("src and out must be [rows, C] of one dtype and width")
+    if index.numel() != out.shape[0]:
+        raise RuntimeError("index must have one entry per row of out")
     st = _cabi.load().f3d_gather_rows(_ptr(src), _ptr(index), _ptr(out), out.shape[0], src.shape[0],
-                                      src.shape[1] * src.element_size(), _dev_index(dev), _stream(dev))
+                                      src.shape[1] * src.element_size(), dev, _stream(dev))
     _cabi.check(st, "gather_rows")
 
 
@@ -662,20 +743,20 @@ def batch_psh_scatter_pad_hash_noalloc(coord, bucket_id, bucket_counter, bucket_
                  ["bucket_counter", "bucket_offset", "batch_sep", "cumsum_counter"], torch.uint32)
     _check_dtype([bucket_id], ["bucket_id"], torch.uint16)
     _check_dtype([probe_offsets], ["probe_offsets"], torch.int16)
-    _require(coord.dim() == 2 and coord.shape[1] == 3 and scatter_coord.dim() == 2 and scatter_coord.shape[1] == 3,
-             "coord and scatter_coord must be [rows, 3]")
+    if not (coord.dim() == 2 and coord.shape[1] == 3 and scatter_coord.dim() == 2 and scatter_coord.shape[1] == 3):
+        raise RuntimeError("coord and scatter_coord must be [rows, 3]")
     total_n, batch = coord.shape[0], batch_sep.shape[0]
-    _require(bucket_id.numel() >= total_n and bucket_offset.numel() >= total_n,
-             "bucket_id / bucket_offset are shorter than coord")
-    _require(bucket_counter.numel() == batch * num_bucket and cumsum_counter.numel() == batch * num_bucket,
-             f"bucket_counter / cumsum_counter must be [{batch},{num_bucket}]")
-    _require(probe_offsets.numel() == 128 * 3 and bbox_min.numel() == 3 and bbox_max.numel() == 3,
-             "probe_offsets must be [128,3] and the bounding box 3 + 3 values")
+    if not (bucket_id.numel() >= total_n and bucket_offset.numel() >= total_n):
+        raise RuntimeError("bucket_id / bucket_offset are shorter than coord")
+    if not (bucket_counter.numel() == batch * num_bucket and cumsum_counter.numel() == batch * num_bucket):
+        raise RuntimeError(f"bucket_counter / cumsum_counter must be [{batch},{num_bucket}]")
+    if not (probe_offsets.numel() == 128 * 3 and bbox_min.numel() == 3 and bbox_max.numel() == 3):
+        raise RuntimeError("probe_offsets must be [128,3] and the bounding box 3 + 3 values")
     st = _cabi.load().f3d_batch_psh_scatter_pad_hash_noalloc(
         _ptr(coord), _ptr(bucket_id), _ptr(bucket_counter), _ptr(bucket_offset), _ptr(batch_sep),
         total_n, batch, int(instance_max_N), int(num_bucket), int(bucket_divisor), int(bucket_size), int(num_vox),
         _ptr(bbox_min), _ptr(bbox_max), _ptr(probe_offsets), _ptr(cumsum_counter), _ptr(scatter_coord),
-        scatter_coord.shape[0], float(pad_num), int(hash_type), _dev_index(dev), _stream(dev))
+        scatter_coord.shape[0], float(pad_num), int(hash_type), dev, _stream(dev))
     _cabi.check(st, "batch_psh_scatter_pad_hash_noalloc")
 
 
@@ -686,9 +767,11 @@ def buck_swin_bwd(Q, K, V, O, dO, LSE, Delta, dQ, dK, dV, Scope_buckets, bucket_
     _check_tensors([LSE, Delta, Scope_buckets], ["LSE", "Delta", "Scope_buckets"])
     _check_dtype([LSE, Delta], ["LSE", "Delta"], torch.float32)
     _check_dtype([Scope_buckets], ["Scope_buckets"], torch.uint32)
-    _require(tuple(LSE.shape) == (b, l, h) and tuple(Delta.shape) == (b, l, h), f"LSE and Delta must be [{b},{l},{h}]")
-    _require(Scope_buckets.dim() == 2, "Scope_buckets must be [num_scopes, scope_size]")
+    if LSE.shape != (b, l, h) or Delta.shape != (b, l, h):
+        raise RuntimeError(f"LSE and Delta must be [{b},{l},{h}]")
+    if Scope_buckets.dim() != 2:
+        raise RuntimeError("Scope_buckets must be [num_scopes, scope_size]")
     st = _cabi.load().f3d_buck_swin_bwd(_ptr(Q), _ptr(K), _ptr(V), _ptr(O), _ptr(dO), _ptr(LSE), _ptr(Delta), _ptr(dQ),
                                         _ptr(dK), _ptr(dV), _ptr(Scope_buckets), b, l, h, d, Scope_buckets.shape[0],
-                                        Scope_buckets.shape[1], int(bucket_size), _dev_index(dev), _stream(dev))
+                                        Scope_buckets.shape[1], int(bucket_size), dev, _stream(dev))
     _cabi.check(st, "buck_swin_bwd")

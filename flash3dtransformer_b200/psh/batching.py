@@ -32,6 +32,17 @@ def host_seps(seps: torch.Tensor) -> torch.Tensor:
     return cached
 
 
+def planned(seps: torch.Tensor, key, make):
+    """make() once per separator tensor and key: what the host derives from the scene sizes of a batch (bucket counts, row
+    plans of the pooling levels) is laid out when the batch is first seen and travels with its separators."""
+    plans = getattr(seps, "_f3d_plans", None)
+    if plans is None:
+        plans = seps._f3d_plans = {}
+    if key not in plans:
+        plans[key] = make()
+    return plans[key]
+
+
 def attach_host_seps(seps_dev: torch.Tensor, seps_cpu: torch.Tensor) -> torch.Tensor:
     seps_dev._f3d_host = seps_cpu.to(torch.int64)
     return seps_dev
@@ -44,7 +55,7 @@ def sep2sizes(seps: torch.Tensor) -> torch.Tensor:
 
 
 def max_inslen_from_seps(seps: torch.Tensor) -> int:
-    return int(sep2sizes(host_seps(seps)).max())
+    return planned(seps, "max", lambda: int(sep2sizes(host_seps(seps)).max()))
 
 
 def bulk_to(ts: List[torch.Tensor], dest):

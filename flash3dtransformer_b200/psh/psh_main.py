@@ -28,6 +28,10 @@ NUM_VOX = 0xFFFF
 def bucket_plan(seps: torch.Tensor, bucket_size: int, mean_n=None):
     """(mean scene size, largest scene, num_buck, divisor) as psh_main.py:97-104 computes them.  `mean_n` overrides
     the local mean scene size (a scene-sharded run passes the mean over all ranks' scenes)."""
+    return f3dbatch.planned(seps, ("psh", bucket_size, mean_n), lambda: _bucket_plan(seps, bucket_size, mean_n))
+
+
+def _bucket_plan(seps, bucket_size, mean_n):
     sizes = f3dbatch.sep2sizes(f3dbatch.host_seps(seps))
     if mean_n is None:
         mean_n = float(sizes.to(torch.float32).mean()) if sizes.numel() else 0.0
@@ -47,10 +51,11 @@ class BucketScatterBuffers:
     scattered_coord: torch.Tensor
 
     @staticmethod
-    def create_buffers(coords: torch.Tensor, seps: torch.Tensor, bucket_size: int, pad_to: int, num_buck=None):
+    def create_buffers(coords: torch.Tensor, seps: torch.Tensor, bucket_size: int, pad_to: int, num_buck=None, fill=True):
         """Allocate every output of the scatter: ids u16 (ones), counters u32 (zeros), offsets u32 (empty),
         cumsum u32 (zeros), probe table i16 [128,3], scattered coords fp16 [pad_to, D] filled with NaN so that a
-        row the kernel misses shows up in the reference's "no NaN" check (tests/test_psh.py:117-120)."""
+        row the kernel misses shows up in the reference's "no NaN" check (tests/test_psh.py:117-120).  `fill` False leaves
+        them as allocated: for callers that run the kernels next, which write every element of every output."""
         total_n, d = coords.shape
         dev = coords.device
         if num_buck is None:
@@ -66,6 +71,14 @@ class BucketScatterBuffers:
                 bucket_cumsum=torch.empty(b, num_buck, dtype=torch.uint32, device=dev),
                 probe_offs=f3dbuck.generate_probe_offsets(dev, row_major=True),
                 scattered_coord=torch.empty((pad_to, d), dtype=torch.float16, device=dev)))
+        if not fill:
+            return BucketScatterBuffers(
+                bucket_id=torch.empty(total_n, dtype=torch.uint16, device=dev),
+                bucket_cntr=torch.empty(b, num_buck, dtype=torch.uint32, device=dev),
+                bucket_offs=torch.empty(total_n, dtype=torch.uint32, device=dev),
+                bucket_cumsum=torch.empty(b, num_buck, dtype=torch.uint32, device=dev),
+                probe_offs=f3dbuck.generate_probe_offsets(dev, row_major=True),
+                scattered_coord=torch.empty((pad_to, d), dtype=torch.float16, device=dev))
         return BucketScatterBuffers(
             bucket_id=torch.ones(total_n, dtype=torch.uint16, device=dev),
             bucket_cntr=torch.zeros(b, num_buck, dtype=torch.uint32, device=dev),
@@ -88,9 +101,9 @@ def batch_bucket_scatter(coords: torch.Tensor, seps: torch.Tensor, bucket_size: 
     """
     f3ddev.init_dev(coords.get_device())
     _, max_n, num_buck, divisor = bucket_plan(seps, bucket_size, mean_n)
-    buffers = BucketScatterBuffers.create_buffers(coords, seps, bucket_size, pad_to, num_buck)
+    buffers = BucketScatterBuffers.create_buffers(coords, seps, bucket_size, pad_to, num_buck, fill=coords.shape[0] == 0)
     if bbox is None:
-        bbox_min, bbox_max = torch.aminmax(coords, dim=0)
+        bbox_min, bbox_max = bounding_box(coords)
     else:
         bbox_min, bbox_max = bbox
     if scene_base is not None:
@@ -100,6 +113,15 @@ def batch_bucket_scatter(coords: torch.Tensor, seps: torch.Tensor, bucket_size: 
         bucket_size, NUM_VOX, bbox_min.contiguous(), bbox_max.contiguous(), buffers.probe_offs,
         buffers.bucket_cumsum, buffers.scattered_coord, 0.0, hash_op)
     return buffers.scattered_coord, buffers
+
+
+def bounding_box(coords: torch.Tensor):
+    """(min, max) fp16 [3] over all rows."""
+    if coords.dtype != torch.float16 or coords.dim() != 2 or coords.shape[1] != 3 or coords.shape[0] == 0 or not coords.is_contiguous():
+        return torch.aminmax(coords, dim=0)
+    bbox_min, bbox_max = torch.empty(2, 3, dtype=torch.float16, device=coords.device).unbind(0)
+    pshattn.bbox_f16(coords, bbox_min, bbox_max)
+    return bbox_min, bbox_max
 
 
 def scatter_index(buffers: BucketScatterBuffers, seps: torch.Tensor, pad_to: int, inverse: bool = True):
