@@ -47,6 +47,7 @@ struct AttnFwdArgs {
   int B, L, H, num_scopes, k, bucket, q_blocks_per_bucket;   // q_blocks_per_bucket = bucket / 128
   float scale_log2;          // log2(e) / sqrt(D)
   int *status;
+  int splits;                // CTAs (one cluster) that share the keys of a query tile: 1, 2 or 4
 };
 
 __device__ __forceinline__ float fast_exp2(float x) {
@@ -122,6 +123,7 @@ template <int D> struct AttnCfg {
   static constexpr uint32_t kOCol = 2 * BKV;        // S0 (P0 over its first 16 columns), S1, O
   static constexpr uint32_t kTmemCols = kOCol + D <= 128 ? 128 : 256;
   static constexpr int kMinCtas = 512 / kTmemCols;
+  static_assert(kBQ * (D + 2 * 4) * 4 <= kQBytes + R * 2 * kTileBytes, "room for the parts of a split tile");
   // pairs of a tile whose exponentials go to the FMA pipe: every fifth, spread out so that both pipes work on every row
   // (an eighth to three eighths of the pairs measure within 2 % of one another)
   static constexpr int kPoly = 0x4210;
@@ -267,10 +269,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tiles_per_scope = a.k * a.q_blocks_per_bucket;
-  const int scope = blockIdx.x / tiles_per_scope, qt = blockIdx.x % tiles_per_scope;
+  const int part = blockIdx.x % a.splits, tile = blockIdx.x / a.splits;      // the parts of a tile are one cluster
+  const int scope = tile / tiles_per_scope, qt = tile % tiles_per_scope;
   const int head = blockIdx.y, brow = blockIdx.z;
   const uint32_t *my_scope = a.scopes + (size_t)scope * a.k;
-  const int n = a.k * a.q_blocks_per_bucket * (128 / BKV);        // key tiles, a multiple of four
+// this CTA's keys: groups of 128 (always inside one bucket), [g0, g1) of the scope's; key tiles are a multiple of four
+  const int g0 = tiles_per_scope * part / a.splits, g1 = tiles_per_scope * (part + 1) / a.splits;
+  const int n = (g1 - g0) * (128 / BKV);
+  const int slot0 = g0 / a.q_blocks_per_bucket, at0 = (g0 % a.q_blocks_per_bucket) * 128;
   const int row0 = brow * a.L;
 
   auto load_tile = [&](unsigned char *dst, const CUtensorMap *map, uint64_t *bar, int tok) {
@@ -293,7 +299,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       tc::mbar_init(q_full, 1);
       tc::mbar_fence_init();
       const int q_tok = (int)my_scope[qt / a.q_blocks_per_bucket] * a.bucket + (qt % a.q_blocks_per_bucket) * kBQ;
-      const int tok0 = row0 + (int)my_scope[0] * a.bucket;
+      const int tok0 = row0 + (int)my_scope[slot0] * a.bucket + at0;
       tc::mbar_expect_tx(q_full, C::kQBytes + 2 * C::kTileBytes);
 #pragma unroll
       for (int c = 0; c < C::NDCH; ++c) tc::tma_load_3d(sq + c * kBQ * C::RB, &map_q, q_full, c * C::DCH, head, row0 + q_tok);
@@ -315,10 +321,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         // table's entry is fetched a bucket ahead)
         struct Stream {
           const uint32_t *scope; int bucket, k, slot, row, base, next;
-          __device__ __forceinline__ void init(const uint32_t *sc, int bk, int kk, int from) {
-            scope = sc; bucket = bk; k = kk; slot = 0; row = from - BKV;
-            base = (int)sc[0] * bk;
-            next = kk > 1 ? (int)sc[1] * bk : 0;
+          __device__ __forceinline__ void init(const uint32_t *sc, int bk, int kk, int slot0, int from) {
+            scope = sc; bucket = bk; k = kk; slot = slot0; row = from - BKV;
+            base = (int)sc[slot] * bk;
+            next = slot + 1 < kk ? (int)sc[slot + 1] * bk : 0;
             take();
           }
           __device__ __forceinline__ int take() {
@@ -333,8 +339,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             return t;
           }
         } ks, vs;
-        ks.init(my_scope, a.bucket, a.k, 4 * BKV);
-        vs.init(my_scope, a.bucket, a.k, 2 * BKV);
+        ks.init(my_scope, a.bucket, a.k, slot0, at0 + 4 * BKV);
+        vs.init(my_scope, a.bucket, a.k, slot0, at0 + 2 * BKV);
         auto load_stage = [&](int i) {
           const int s = i % R;
           const bool has_k = i + 2 < n;
@@ -407,12 +413,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   if (pass == 1 || !__syncthreads_or(sm.ok && sm.bad)) break;
   }
 
-  if (warp != 0) {
-    const int row = (warp & 3) * 32 + lane;                      // query row inside the tile = tensor-memory lane
-    const int q_tok = (int)my_scope[qt / a.q_blocks_per_bucket] * a.bucket + (qt % a.q_blocks_per_bucket) * kBQ;
-    if (sm.ok && q_tok + row < a.L) {
+  const int row = (warp & 3) * 32 + lane;                        // query row inside the tile = tensor-memory lane
+  const int q_tok = (int)my_scope[qt / a.q_blocks_per_bucket] * a.bucket + (qt % a.q_blocks_per_bucket) * kBQ;
+  const size_t tok = (size_t)row0 + q_tok + row;
+  if (a.splits == 1) {
+    if (warp != 0 && sm.ok && q_tok + row < a.L) {
       const float inv = 1.f / sm.l_run;
-      const size_t tok = (size_t)brow * a.L + q_tok + row;
       __nv_bfloat16 *op = a.O + (tok * a.H + head) * D;
 #pragma unroll
       for (int c = 0; c < D; c += 16) {
@@ -427,6 +433,49 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         *reinterpret_cast<uint4 *>(op + c + 8) = w[1];
       }
       a.lse[tok * a.H + head] = (sm.m_run + log2f(sm.l_run)) * 0.6931471805599453f;
+    }
+  } else {
+    // The parts of a tile meet in shared memory: CTA p of the cluster receives columns [p D / splits, (p + 1) D / splits) of
+    // every part's O with its reference and sum, over the operands nobody needs any more, and writes them.
+    const int cols = D / a.splits, stride = cols + 2;             // floats per row of a part: O, reference, sum
+    const uint32_t xbuf = tc::smem_u32(sq) + (uint32_t)((part * kBQ + row) * stride) * 4u;
+    tc::cluster_sync();                                           // every CTA of the cluster is done with its operands
+    if (warp != 0) {
+#pragma unroll
+      for (int c = 0; c < D; c += 16) {
+        uint32_t o[16];
+        tc::tmem_ld_32x32b_x16(sm.tmem_o + c, o);
+        tc::tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 16; i += 2) {
+          const int col = c + i, p = col / cols;
+          tc::sts_cluster64(tc::mapa(xbuf, p) + (uint32_t)(col - p * cols) * 4u, o[i], o[i + 1]);
+        }
+      }
+      for (int p = 0; p < a.splits; ++p) tc::sts_cluster64(tc::mapa(xbuf, p) + (uint32_t)cols * 4u, __float_as_uint(sm.m_run), __float_as_uint(sm.l_run));
+    }
+    tc::cluster_sync();
+    if (warp != 0 && sm.ok && q_tok + row < a.L) {
+      const float *mine = reinterpret_cast<const float *>(sq) + row * stride;
+      const int step = kBQ * stride;
+      float m = -INFINITY, l = 0.f, w[4];
+      for (int p = 0; p < a.splits; ++p) m = fmaxf(m, mine[p * step + cols]);
+      for (int p = 0; p < a.splits; ++p) {
+        w[p & 3] = fast_exp2(mine[p * step + cols] - m);
+        l = fmaf(w[p & 3], mine[p * step + cols + 1], l);
+      }
+      const float inv = 1.f / l;
+      __nv_bfloat16 *op = a.O + (tok * a.H + head) * D + part * cols;
+      for (int c = 0; c < cols; c += 2) {
+        float x = 0.f, y = 0.f;
+        for (int p = 0; p < a.splits; ++p) {
+          const float2 v = *reinterpret_cast<const float2 *>(mine + p * step + c);
+          x = fmaf(w[p & 3], v.x, x);
+          y = fmaf(w[p & 3], v.y, y);
+        }
+        *reinterpret_cast<uint32_t *>(op + c) = pack_p2<F16>(x * inv, y * inv);
+      }
+      if (part == 0) a.lse[tok * a.H + head] = (m + log2f(l)) * 0.6931471805599453f;
     }
   }
 
@@ -451,8 +500,30 @@ static int launch_attn_fwd(const void *Q, const void *K, const void *V, AttnFwdA
   F3D_TRY(encode_tmap_3d(&mq, dt, Q, D, a.H, rows, s1, s2, C::DCH, 1, kBQ, C::RB));
   F3D_TRY(encode_tmap_3d(&mk, dt, K, D, a.H, rows, s1, s2, C::DCH, 1, C::BKV, C::RB));
   F3D_TRY(encode_tmap_3d(&mv, dt, V, D, a.H, rows, s1, s2, C::DCH, 1, C::BKV, C::RB));
-  dim3 grid(a.num_scopes * a.k * a.q_blocks_per_bucket, a.H, a.B);
-  kern<<<grid, C::kThreads, C::kSmem, st>>>(mq, mk, mv, a);
+  // A query tile is a chain of key tiles, 0.4 us each on an SM that has little else to do.  Where the tiles are so few that
+  // the SMs would hold less than half of the CTAs they have room for, the keys of a tile are shared out to two or four CTAs
+  // of a cluster; a part keeps at least 512 keys, below which joining the parts costs what the split saves.
+  const long long tiles = (long long)a.num_scopes * a.k * a.q_blocks_per_bucket;
+  const long long room = (long long)sm_count(device) * C::kMinCtas;
+  a.splits = 1;
+  while (a.splits < 4 && tiles * a.H * a.B * a.splits * 2 <= room && a.k * a.q_blocks_per_bucket / (2 * a.splits) >= 4) a.splits *= 2;
+  dim3 grid((unsigned)(tiles * a.splits), a.H, a.B);
+  if (a.splits == 1) {
+    kern<<<grid, C::kThreads, C::kSmem, st>>>(mq, mk, mv, a);
+    return check_launch("buck_swin_fwd");
+  }
+  cudaLaunchAttribute cluster[1];
+  cluster[0].id = cudaLaunchAttributeClusterDimension;
+  cluster[0].val.clusterDim.x = (unsigned)a.splits;
+  cluster[0].val.clusterDim.y = cluster[0].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(C::kThreads);
+  cfg.dynamicSmemBytes = C::kSmem;
+  cfg.stream = st;
+  cfg.attrs = cluster;
+  cfg.numAttrs = 1;
+  F3D_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, mq, mk, mv, a));
   return check_launch("buck_swin_fwd");
 }
 
@@ -486,7 +557,7 @@ static int buck_swin_fwd_impl(const void *Q, const void *K, const void *V, void 
   F3D_TRY(maybe_sync(st, "buck_swin_fwd"));
   AttnFwdArgs a{static_cast<__nv_bfloat16 *>(O), static_cast<float *>(LSE), static_cast<const uint32_t *>(scope_buckets),
                 B, L, H, num_scopes, scope_size, (int)bucket_size, (int)bucket_size / kBQ,
-                1.4426950408889634f / sqrtf((float)D), status_word(device)};
+                1.4426950408889634f / sqrtf((float)D), status_word(device), 1};
   if (!a.status) return F3D_ERR_CUDA;
   F3D_TRY(dtype == 1 ? launch_attn_fwd_any<true>(D, Q, K, V, a, device, st) : launch_attn_fwd_any<false>(D, Q, K, V, a, device, st));
   return maybe_sync(st, "buck_swin_fwd");

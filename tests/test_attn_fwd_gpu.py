@@ -78,14 +78,14 @@ def test_scaled_inputs(cuda_device, mul):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("d", [16, 32, 64, 128])
-@pytest.mark.parametrize("steps", ["first", "middle", "last", "ramp"])
-def test_growing_scores(cuda_device, d, dtype, steps):
+@pytest.mark.parametrize("steps,bucket", [("first", 256), ("middle", 256), ("last", 256), ("ramp", 256), ("middle", 1024), ("ramp", 2048)])
+def test_growing_scores(cuda_device, d, dtype, steps, bucket):
     """Rows whose later keys outgrow the reference taken from the first ones: a jump in the first, a middle or the last pair
     of 32-key tiles (past what the loop without a row maximum can follow: the careful pass) and a ramp it follows by moving
-    its reference."""
+    its reference; in the larger buckets the keys of a query tile are shared out to two and four CTAs."""
     from flash3dtransformer_b200.lib import pshattn
     dev = cuda_device
-    l, h, bucket = 512, 2, 256
+    l, h = 2 * bucket, 2
     g = torch.Generator().manual_seed(11)
     q, k, v = (torch.randn(1, l, h, d, generator=g).to(dtype) for _ in range(3))
     big = 60.0 if dtype == torch.bfloat16 else 12.0
