@@ -41,13 +41,18 @@ namespace f3d {
 int *status_word(int device);
 
 constexpr int kBQ = 128;      // query rows per tile
+constexpr int kShortWindow = 8;     // query tiles of a scope up to which a CTA takes two (W = 1024)
+
+// How query tiles map to CTAs: one each; two of a scope one after the other (kTwoTiles); one shared by a cluster (kSplit).
+// Builds of their own: the issuing thread's code is on the critical path, and what the plain mapping does not need costs it 2 %.
+enum AttnMode : int { kPlain = 0, kTwoTiles = 1, kSplit = 2 };
 
 struct AttnFwdArgs {
   __nv_bfloat16 *O; float *lse; const uint32_t *scopes;
   int B, L, H, num_scopes, k, bucket, q_blocks_per_bucket;   // q_blocks_per_bucket = bucket / 128
   float scale_log2;          // log2(e) / sqrt(D)
   int *status;
-  int splits;                // CTAs (one cluster) that share the keys of a query tile: 1, 2 or 4
+  int splits;                // kSplit: CTAs (one cluster) that share the keys of a query tile, 2 or 4
 };
 
 __device__ __forceinline__ float fast_exp2(float x) {
@@ -118,12 +123,14 @@ template <int D> struct AttnCfg {
   static constexpr int kQBytes = kBQ * D * 2;
   static constexpr int kTileBytes = BKV * D * 2;    // one K or V tile
   static constexpr int R = 4;                       // ring stages: V of key tile i and K of key tile i + 2
-  static constexpr int kSmem = kQBytes + R * 2 * kTileBytes + 256 + 1024;
+  template <int MODE> static constexpr int q_bufs() { return MODE == kTwoTiles ? 2 : 1; }
+  template <int MODE> static constexpr int smem() { return q_bufs<MODE>() * kQBytes + R * 2 * kTileBytes + 256 + 1024; }
   static constexpr int kThreads = 160;
   static constexpr uint32_t kOCol = 2 * BKV;        // S0 (P0 over its first 16 columns), S1, O
   static constexpr uint32_t kTmemCols = kOCol + D <= 128 ? 128 : 256;
   static constexpr int kMinCtas = 512 / kTmemCols;
-  static_assert(kBQ * (D + 2 * 4) * 4 <= kQBytes + R * 2 * kTileBytes, "room for the parts of a split tile");
+  // parts of a split tile: 128 rows of O, reference and sum
+  static_assert(kBQ * (D + 4) * 4 <= kQBytes + R * 2 * kTileBytes, "room for the parts of a split tile");
   // pairs of a tile whose exponentials go to the FMA pipe: every fifth, spread out so that both pipes work on every row
   // (an eighth to three eighths of the pairs measure within 2 % of one another)
   static constexpr int kPoly = 0x4210;
@@ -211,12 +218,12 @@ template <int D, bool F16> struct SoftmaxRow {
   // the row sum whenever that sum shows that scores have outgrown it, which leaves P, 16-bit floating point, and the fp32
   // sums as exact as any other reference.  What it cannot follow is a jump by more than 2^kJump within two tiles: such a
   // row marks itself bad and the CTA starts over with the maximum of every tile taken (`careful`).
-  __device__ __forceinline__ void run(int n, uint32_t (&ra)[32], uint32_t (&rb)[32], float scale_log2, const tc::WaitCtx &wc) {
+  __device__ __forceinline__ void run(int j0, int n, uint32_t (&ra)[32], uint32_t (&rb)[32], float scale_log2, const tc::WaitCtx &wc) {
     constexpr float kMoveAt = 4096.f, kJump = F16 ? 16384.f : 1.2676506e30f;
     m_run = row_max32(ra) * scale_log2;
     for (int j = 0; j < n && ok; j += 2) {
-      float s = tile<true, true>(j, ra, rb, wc);
-      s += tile<true, false>(j + 1, rb, ra, wc);
+      float s = tile<true, true>(j0 + j, ra, rb, wc);
+      s += tile<true, false>(j0 + j + 1, rb, ra, wc);
       l_run += s;
       moved = __any_sync(0xFFFFFFFFu, !(s <= kMoveAt));
       if (moved) {
@@ -232,12 +239,12 @@ template <int D, bool F16> struct SoftmaxRow {
   // The same with the maximum of every tile, for fp16 (whose P overflows past 65504) and for rows that `run` gave up on.
   // The reference still moves only when a maximum exceeds it by more than kMaxSlack (base-2 units), so that O is almost
   // never rescaled after the first tiles.
-  __device__ __forceinline__ void run_careful(int n, uint32_t (&ra)[32], uint32_t (&rb)[32], float scale_log2, const tc::WaitCtx &wc) {
+  __device__ __forceinline__ void run_careful(int j0, int n, uint32_t (&ra)[32], uint32_t (&rb)[32], float scale_log2, const tc::WaitCtx &wc) {
     for (int j = 0; j < n && ok; j += 2) {
       follow(row_max32(ra) * scale_log2, j > 0);
-      l_run += tile<false, true>(j, ra, rb, wc);
+      l_run += tile<false, true>(j0 + j, ra, rb, wc);
       follow(row_max32(rb) * scale_log2, true);
-      l_run += tile<false, true>(j + 1, rb, ra, wc);
+      l_run += tile<false, true>(j0 + j + 1, rb, ra, wc);
     }
   }
   __device__ __forceinline__ void follow(float mx, bool have_o) {
@@ -253,7 +260,7 @@ template <int D, bool F16> struct SoftmaxRow {
   }
 };
 
-template <int D, bool F16>
+template <int D, bool F16, int MODE>
 __global__ void __launch_bounds__(AttnCfg<D>::kThreads, AttnCfg<D>::kMinCtas)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                    const __grid_constant__ CUtensorMap map_v, AttnFwdArgs a) {
@@ -261,22 +268,26 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   constexpr int R = C::R, BKV = C::BKV;
   extern __shared__ unsigned char smem_raw[];
   unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  unsigned char *sq = smem, *sk = smem + C::kQBytes, *sv = sk + R * C::kTileBytes;
+  unsigned char *sq = smem, *sk = smem + C::template q_bufs<MODE>() * C::kQBytes, *sv = sk + R * C::kTileBytes;
   uint64_t *bars = reinterpret_cast<uint64_t *>(sv + R * C::kTileBytes);
-  uint64_t *kv_full = bars, *s_full = bars + R, *p_full = s_full + 2, *q_full = p_full + 2;
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(q_full + 1);
+  uint64_t *kv_full = bars, *s_full = bars + R, *p_full = s_full + 2, *q_full = p_full + 2 /*[2]*/;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(q_full + 2);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tiles_per_scope = a.k * a.q_blocks_per_bucket;
-  const int part = blockIdx.x % a.splits, tile = blockIdx.x / a.splits;      // the parts of a tile are one cluster
-  const int scope = tile / tiles_per_scope, qt = tile % tiles_per_scope;
+  constexpr bool SPLIT = MODE == kSplit;
+  constexpr int nq = MODE == kTwoTiles ? 2 : 1;
+  const int part = SPLIT ? blockIdx.x % a.splits : 0;            // the parts of a query tile are one cluster
+  const int unit = SPLIT ? blockIdx.x / a.splits : blockIdx.x, units_per_scope = tiles_per_scope / nq;
+  const int scope = unit / units_per_scope, qt = unit % units_per_scope * nq;
   const int head = blockIdx.y, brow = blockIdx.z;
   const uint32_t *my_scope = a.scopes + (size_t)scope * a.k;
 // this CTA's keys: groups of 128 (always inside one bucket), [g0, g1) of the scope's; key tiles are a multiple of four
-  const int g0 = tiles_per_scope * part / a.splits, g1 = tiles_per_scope * (part + 1) / a.splits;
+  const int g0 = SPLIT ? tiles_per_scope * part / a.splits : 0, g1 = SPLIT ? tiles_per_scope * (part + 1) / a.splits : tiles_per_scope;
   const int n = (g1 - g0) * (128 / BKV);
-  const int slot0 = g0 / a.q_blocks_per_bucket, at0 = (g0 % a.q_blocks_per_bucket) * 128;
+  const int slot0 = SPLIT ? g0 / a.q_blocks_per_bucket : 0, at0 = SPLIT ? (g0 % a.q_blocks_per_bucket) * 128 : 0;
+  auto q_token = [&](int t) { return (int)my_scope[t / a.q_blocks_per_bucket] * a.bucket + (t % a.q_blocks_per_bucket) * kBQ; };
   const int row0 = brow * a.L;
 
   auto load_tile = [&](unsigned char *dst, const CUtensorMap *map, uint64_t *bar, int tok) {
@@ -287,18 +298,40 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   tc::WaitCtx wc{abort_flag, a.status};
   SoftmaxRow<D, F16> sm;
   sm.ok = sm.bad = false;
+  const int row = (warp & 3) * 32 + lane;                        // query row inside the tile = tensor-memory lane
+  // normalised O and LSE of query tile qt + c
+  auto store = [&](int c) {
+    const int q_tok = q_token(qt + c);
+    if (!sm.ok || q_tok + row >= a.L) return;
+    const size_t tok = (size_t)row0 + q_tok + row;
+    const float inv = 1.f / sm.l_run;
+    __nv_bfloat16 *op = a.O + (tok * a.H + head) * D;
+#pragma unroll
+    for (int ch = 0; ch < D; ch += 16) {
+      uint32_t o[16];
+      tc::tmem_ld_32x32b_x16(sm.tmem_o + ch, o);
+      tc::tmem_ld_wait();
+      uint4 w[2];
+      uint32_t *h2 = reinterpret_cast<uint32_t *>(w);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) h2[i] = pack_p2<F16>(__uint_as_float(o[2 * i]) * inv, __uint_as_float(o[2 * i + 1]) * inv);
+      *reinterpret_cast<uint4 *>(op + ch) = w[0];
+      *reinterpret_cast<uint4 *>(op + ch + 8) = w[1];
+    }
+    a.lse[tok * a.H + head] = (sm.m_run + log2f(sm.l_run)) * 0.6931471805599453f;
+  };
   for (int pass = 0; pass < 2; ++pass) {
     // One thread fills the ring and issues the products.  It sets the barriers up itself, so that its first loads are under
     // way before the CTA has its tensor memory.  Stage i of the ring holds V of key tile i and K of key tile i + 2; the first
     // four key tiles always lie in one bucket.
     if (warp == 0 && tc::elect_one()) {
-      if (pass) for (uint64_t *bar = bars; bar <= q_full; ++bar) tc::mbar_inval(bar);
+      if (pass) for (uint64_t *bar = bars; bar <= q_full + 1; ++bar) tc::mbar_inval(bar);
       *abort_flag = 0;
       for (int s = 0; s < R; ++s) tc::mbar_init(&kv_full[s], 1);
       for (int b = 0; b < 2; ++b) { tc::mbar_init(&s_full[b], 1); tc::mbar_init(&p_full[b], 128); }
-      tc::mbar_init(q_full, 1);
+      tc::mbar_init(&q_full[0], 1); tc::mbar_init(&q_full[1], 1);
       tc::mbar_fence_init();
-      const int q_tok = (int)my_scope[qt / a.q_blocks_per_bucket] * a.bucket + (qt % a.q_blocks_per_bucket) * kBQ;
+      const int q_tok = q_token(qt);
       const int tok0 = row0 + (int)my_scope[slot0] * a.bucket + at0;
       tc::mbar_expect_tx(q_full, C::kQBytes + 2 * C::kTileBytes);
 #pragma unroll
@@ -324,26 +357,28 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
           __device__ __forceinline__ void init(const uint32_t *sc, int bk, int kk, int slot0, int from) {
             scope = sc; bucket = bk; k = kk; slot = slot0; row = from - BKV;
             base = (int)sc[slot] * bk;
-            next = slot + 1 < kk ? (int)sc[slot + 1] * bk : 0;
+            next = (int)sc[slot + 1 == kk ? 0 : slot + 1] * bk;
             take();
           }
           __device__ __forceinline__ int take() {
             const int t = base + row;
             row += BKV;
-            if (row == bucket) {
+            if (row == bucket) {                                  // behind the last bucket the next query tile starts over
               row = 0;
               base = next;
-              ++slot;
-              if (slot + 1 < k) next = (int)scope[slot + 1] * bucket;
+              if (++slot == k) slot = 0;
+              if (k > 1) next = (int)scope[slot + 1 == k ? 0 : slot + 1] * bucket;
             }
             return t;
           }
         } ks, vs;
         ks.init(my_scope, a.bucket, a.k, slot0, at0 + 4 * BKV);
         vs.init(my_scope, a.bucket, a.k, slot0, at0 + 2 * BKV);
+        constexpr bool two = nq > 1;
+        const int total = nq * n;
         auto load_stage = [&](int i) {
           const int s = i % R;
-          const bool has_k = i + 2 < n;
+          const bool has_k = i + 2 < total;
           tc::mbar_expect_tx(&kv_full[s], has_k ? 2 * C::kTileBytes : C::kTileBytes);
           load_tile(sv + s * C::kTileBytes, &map_v, &kv_full[s], row0 + vs.take());
           if (has_k) load_tile(sk + s * C::kTileBytes, &map_k, &kv_full[s], row0 + ks.take());
@@ -353,23 +388,30 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         const uint64_t qd = tc::make_smem_desc(tc::smem_u32(sq), 16, 8 * C::RB, C::SWZ);
         const uint64_t kd = tc::make_smem_desc(tc::smem_u32(sk), 16, 8 * C::RB, C::SWZ);
         const uint64_t vd = tc::make_smem_desc(tc::smem_u32(sv), 16, 8 * C::RB, C::SWZ);
-        auto issue_s = [&](int slot, uint32_t b) {
+        auto issue_s = [&](int slot, uint32_t b, bool second) {
+          const uint64_t qds = two && second ? qd + (uint32_t)(C::kQBytes >> 4) : qd;
           const uint64_t kds = kd + (uint32_t)(slot * (C::kTileBytes >> 4));
 #pragma unroll
           for (int c = 0; c < C::NDCH; ++c)
 #pragma unroll
             for (int kk = 0; kk < C::DCH / 16; ++kk)
-              tc::mma_f16_ss(tmem_base + b * BKV, qd + (uint32_t)(c * (kBQ * C::RB >> 4) + 2 * kk), kds + (uint32_t)(c * (BKV * C::RB >> 4) + 2 * kk),
+              tc::mma_f16_ss(tmem_base + b * BKV, qds + (uint32_t)(c * (kBQ * C::RB >> 4) + 2 * kk), kds + (uint32_t)(c * (BKV * C::RB >> 4) + 2 * kk),
                              idesc_s, (c | kk) != 0);
         };
         for (int i = 2; i < R - 2; ++i) load_stage(i);
-        bool ok = tc::mbar_wait(q_full, 0, wc, 202);
+        int rem = 0;                                              // key tile inside its query tile
+        bool second = false;                                      // kTwoTiles: of the second query tile
+        if (two) {
+          tc::mbar_expect_tx(&q_full[1], C::kQBytes);
+          tc::tma_load_3d(sq + C::kQBytes, &map_q, &q_full[1], 0, head, row0 + q_token(qt + 1));
+        }
+        bool ok = tc::mbar_wait(&q_full[0], 0, wc, 202);
         tc::tc_fence_after_sync();
         for (uint32_t b = 0; b < 2 && ok; ++b) {
-          issue_s(R - 2 + b, b);
+          issue_s(R - 2 + b, b, false);
           tc::mma_commit(&s_full[b]);
         }
-        for (int i = 0; i < n && ok; ++i) {
+        for (int i = 0; i < total && ok; ++i) {
           const uint32_t b = (uint32_t)i & 1u;
           const int slot = i % R;
           // the two stages that carried K of tiles 0 and 1 have had no turn of their own yet
@@ -382,12 +424,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 #pragma unroll
             for (int kk = 0; kk < BKV / 16; ++kk)                 // 16 keys per MMA: V rows kk * 16.., P columns kk * 8..
               tc::mma_f16_ts(tmem_base + C::kOCol + c * C::DCH, tmem_base + b * BKV + kk * 8,
-                             vds + (uint32_t)(c * (BKV * C::RB >> 4) + kk * C::RB), idesc_o, (i | kk) != 0);
+                             vds + (uint32_t)(c * (BKV * C::RB >> 4) + kk * C::RB), idesc_o, ((two ? rem : i) | kk) != 0);
           // the next scores of this buffer overwrite P behind the product that reads it: MMAs of one thread run in order
-          if (i + 2 < n) issue_s(slot, b);
+          if (i + 2 < total) {
+            if (two && rem + 2 == n) {
+              second = true;
+              if (!tc::mbar_wait(&q_full[1], 0u, wc, 202)) { ok = false; break; }
+            }
+            issue_s(slot, b, second);
+          }
           tc::mma_commit(&s_full[b]);
           // P of tile i was written by threads that had seen the commit behind tile i - 2: its stage may be filled again
-          if (i + R - 2 < n) load_stage(i + R - 2);
+          if (i + R - 2 < total) load_stage(i + R - 2);
+          if (two && ++rem == n) rem = 0;
         }
       }
     } else {
@@ -396,86 +445,72 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     sm.s_full = tc::smem_u32(s_full);
     sm.p_full = tc::smem_u32(p_full);
     sm.c2 = pack2(a.scale_log2, a.scale_log2);
-    sm.m_run = sm.poly_mx = -INFINITY;
-    sm.l_run = 0.f;
-    sm.alpha = 1.f;
-    sm.moved = sm.bad = false;
+    sm.poly_mx = -INFINITY;
+    sm.bad = false;
     sm.ok = true;
     uint32_t ra[32], rb[32];
     sm.wait_s(0, wc);
     tc::tmem_ld_32x32b_x32(sm.tmem, ra);
     tc::tmem_ld_wait();
-    if (pass == 0) sm.run(n, ra, rb, a.scale_log2, wc);
-    else sm.run_careful(n, ra, rb, a.scale_log2, wc);
-    sm.wait_s(n + 1, wc);                                         // every product has been committed
-    if (pass == 0 && sm.moved) sm.rescale_o();            // a reference that moved behind the last tile
-  }
+    for (int c = 0; c < nq && sm.ok; ++c) {
+      sm.m_run = -INFINITY;
+      sm.l_run = 0.f;
+      sm.alpha = 1.f;
+      sm.moved = false;
+      if (pass == 0) sm.run(c * n, n, ra, rb, a.scale_log2, wc);
+      else sm.run_careful(c * n, n, ra, rb, a.scale_log2, wc);
+      sm.wait_s((c + 1) * n + 1, wc);                             // behind the last product of this query tile
+      if (pass == 0 && sm.moved) sm.rescale_o();                  // a reference that moved behind the last tile
+      if (!SPLIT) store(c);
+    }
+    }
   if (pass == 1 || !__syncthreads_or(sm.ok && sm.bad)) break;
   }
 
-  const int row = (warp & 3) * 32 + lane;                        // query row inside the tile = tensor-memory lane
-  const int q_tok = (int)my_scope[qt / a.q_blocks_per_bucket] * a.bucket + (qt % a.q_blocks_per_bucket) * kBQ;
-  const size_t tok = (size_t)row0 + q_tok + row;
-  if (a.splits == 1) {
-    if (warp != 0 && sm.ok && q_tok + row < a.L) {
-      const float inv = 1.f / sm.l_run;
-      __nv_bfloat16 *op = a.O + (tok * a.H + head) * D;
-#pragma unroll
-      for (int c = 0; c < D; c += 16) {
-        uint32_t o[16];
-        tc::tmem_ld_32x32b_x16(sm.tmem_o + c, o);
-        tc::tmem_ld_wait();
-        uint4 w[2];
-        uint32_t *h2 = reinterpret_cast<uint32_t *>(w);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) h2[i] = pack_p2<F16>(__uint_as_float(o[2 * i]) * inv, __uint_as_float(o[2 * i + 1]) * inv);
-        *reinterpret_cast<uint4 *>(op + c) = w[0];
-        *reinterpret_cast<uint4 *>(op + c + 8) = w[1];
-      }
-      a.lse[tok * a.H + head] = (sm.m_run + log2f(sm.l_run)) * 0.6931471805599453f;
-    }
-  } else {
-    // The parts of a tile meet in shared memory: CTA p of the cluster receives columns [p D / splits, (p + 1) D / splits) of
-    // every part's O with its reference and sum, over the operands nobody needs any more, and writes them.
-    const int cols = D / a.splits, stride = cols + 2;             // floats per row of a part: O, reference, sum
-    const uint32_t xbuf = tc::smem_u32(sq) + (uint32_t)((part * kBQ + row) * stride) * 4u;
+  if (SPLIT) {
+    // The parts of a query tile meet in shared memory: CTA p of the cluster receives every part's O, reference and sum of
+    // `share` of the rows, over the operands nobody needs any more, and writes those rows.
+    constexpr int kStride = D + 4;                                // floats per row of a part
+    const int share = kBQ / a.splits;
     tc::cluster_sync();                                           // every CTA of the cluster is done with its operands
     if (warp != 0) {
+      const int owner = row / share;
+      const uint32_t dst = tc::mapa(tc::smem_u32(sq), owner) + (uint32_t)((part * share + row - owner * share) * kStride) * 4u;
 #pragma unroll
       for (int c = 0; c < D; c += 16) {
         uint32_t o[16];
         tc::tmem_ld_32x32b_x16(sm.tmem_o + c, o);
         tc::tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < 16; i += 2) {
-          const int col = c + i, p = col / cols;
-          tc::sts_cluster64(tc::mapa(xbuf, p) + (uint32_t)(col - p * cols) * 4u, o[i], o[i + 1]);
-        }
+        for (int i = 0; i < 16; i += 4) tc::sts_cluster128(dst + (uint32_t)(c + i) * 4u, make_uint4(o[i], o[i + 1], o[i + 2], o[i + 3]));
       }
-      for (int p = 0; p < a.splits; ++p) tc::sts_cluster64(tc::mapa(xbuf, p) + (uint32_t)cols * 4u, __float_as_uint(sm.m_run), __float_as_uint(sm.l_run));
+      tc::sts_cluster128(dst + (uint32_t)D * 4u, make_uint4(__float_as_uint(sm.m_run), __float_as_uint(sm.l_run), 0u, 0u));
     }
     tc::cluster_sync();
-    if (warp != 0 && sm.ok && q_tok + row < a.L) {
-      const float *mine = reinterpret_cast<const float *>(sq) + row * stride;
-      const int step = kBQ * stride;
-      float m = -INFINITY, l = 0.f, w[4];
-      for (int p = 0; p < a.splits; ++p) m = fmaxf(m, mine[p * step + cols]);
-      for (int p = 0; p < a.splits; ++p) {
-        w[p & 3] = fast_exp2(mine[p * step + cols] - m);
-        l = fmaf(w[p & 3], mine[p * step + cols + 1], l);
-      }
-      const float inv = 1.f / l;
-      __nv_bfloat16 *op = a.O + (tok * a.H + head) * D + part * cols;
-      for (int c = 0; c < cols; c += 2) {
-        float x = 0.f, y = 0.f;
+    if (warp != 0 && sm.ok) {
+      const float *parts = reinterpret_cast<const float *>(sq);
+      const int step = share * kStride, q_tok = q_token(qt);
+      for (int item = threadIdx.x - 32; item < share * (D / 8); item += 128) {
+        const int r = item / (D / 8), ch = item % (D / 8) * 8, qr = part * share + r;
+        if (q_tok + qr >= a.L) continue;
+        const float *mine = parts + r * kStride;
+        float m = -INFINITY, l = 0.f, x[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        for (int p = 0; p < a.splits; ++p) m = fmaxf(m, mine[p * step + D]);
         for (int p = 0; p < a.splits; ++p) {
-          const float2 v = *reinterpret_cast<const float2 *>(mine + p * step + c);
-          x = fmaf(w[p & 3], v.x, x);
-          y = fmaf(w[p & 3], v.y, y);
+          const float *o = mine + p * step;
+          const float w = fast_exp2(o[D] - m);
+          const float4 u = *reinterpret_cast<const float4 *>(o + ch), v = *reinterpret_cast<const float4 *>(o + ch + 4);
+          l = fmaf(w, o[D + 1], l);
+          x[0] = fmaf(w, u.x, x[0]); x[1] = fmaf(w, u.y, x[1]); x[2] = fmaf(w, u.z, x[2]); x[3] = fmaf(w, u.w, x[3]);
+          x[4] = fmaf(w, v.x, x[4]); x[5] = fmaf(w, v.y, x[5]); x[6] = fmaf(w, v.z, x[6]); x[7] = fmaf(w, v.w, x[7]);
         }
-        *reinterpret_cast<uint32_t *>(op + c) = pack_p2<F16>(x * inv, y * inv);
+        const float inv = 1.f / l;
+        const size_t tok = (size_t)row0 + q_tok + qr;
+        *reinterpret_cast<uint4 *>(a.O + (tok * a.H + head) * D + ch) =
+            make_uint4(pack_p2<F16>(x[0] * inv, x[1] * inv), pack_p2<F16>(x[2] * inv, x[3] * inv), pack_p2<F16>(x[4] * inv, x[5] * inv),
+                       pack_p2<F16>(x[6] * inv, x[7] * inv));
+        if (ch == 0) a.lse[tok * a.H + head] = (m + log2f(l)) * 0.6931471805599453f;
       }
-      if (part == 0) a.lse[tok * a.H + head] = (m + log2f(l)) * 0.6931471805599453f;
     }
   }
 
@@ -491,39 +526,55 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 template <int D, bool F16>
 static int launch_attn_fwd(const void *Q, const void *K, const void *V, AttnFwdArgs a, int device, cudaStream_t st) {
   using C = AttnCfg<D>;
-  auto kern = attn_fwd_kernel<D, F16>;
   const int dt = F16 ? 1 : 0;
-  F3D_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(kern), device, C::kSmem));
   CUtensorMap mq, mk, mv;
   const uint64_t rows = (uint64_t)a.B * a.L;
   const uint64_t s1 = (uint64_t)D * 2, s2 = (uint64_t)a.H * D * 2;
   F3D_TRY(encode_tmap_3d(&mq, dt, Q, D, a.H, rows, s1, s2, C::DCH, 1, kBQ, C::RB));
   F3D_TRY(encode_tmap_3d(&mk, dt, K, D, a.H, rows, s1, s2, C::DCH, 1, C::BKV, C::RB));
   F3D_TRY(encode_tmap_3d(&mv, dt, V, D, a.H, rows, s1, s2, C::DCH, 1, C::BKV, C::RB));
-  // A query tile is a chain of key tiles, 0.4 us each on an SM that has little else to do.  Where the tiles are so few that
-  // the SMs would hold less than half of the CTAs they have room for, the keys of a tile are shared out to two or four CTAs
-  // of a cluster; a part keeps at least 512 keys, below which joining the parts costs what the split saves.
-  const long long tiles = (long long)a.num_scopes * a.k * a.q_blocks_per_bucket;
+  const int tiles_per_scope = a.k * a.q_blocks_per_bucket;
+  const long long tiles = (long long)a.num_scopes * tiles_per_scope, heads = (long long)a.H * a.B;
   const long long room = (long long)sm_count(device) * C::kMinCtas;
+  // A query tile is a chain of key tiles, 0.4 us each on an SM that has little else to do.  Where the tiles are so few that
+  // the SMs would hold less than half of the CTAs they have room for, the keys of a tile are shared out to a cluster of two
+  // or four CTAs (three, and five to eight, measure slower: their clusters pack the SMs badly); a part keeps at least 512
+  // keys, below which joining the parts costs what the split saves.  One head, D = 32, W = 4096: 12,288 tokens 49 -> 29 us
+  // (four), 24,576 tokens 59 -> 45 us (two; four, which no longer fit at once: 48).
   a.splits = 1;
-  while (a.splits < 4 && tiles * a.H * a.B * a.splits * 2 <= room && a.k * a.q_blocks_per_bucket / (2 * a.splits) >= 4) a.splits *= 2;
-  dim3 grid((unsigned)(tiles * a.splits), a.H, a.B);
-  if (a.splits == 1) {
-    kern<<<grid, C::kThreads, C::kSmem, st>>>(mq, mk, mv, a);
+  while (a.splits < 4 && tiles * heads * a.splits * 2 <= room && tiles_per_scope / (2 * a.splits) >= 4) a.splits *= 2;
+  if (a.splits > 1) {
+    auto kern = attn_fwd_kernel<D, F16, kSplit>;
+    F3D_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(kern), device, C::template smem<kSplit>()));
+    cudaLaunchAttribute cluster[1];
+    cluster[0].id = cudaLaunchAttributeClusterDimension;
+    cluster[0].val.clusterDim.x = (unsigned)a.splits;
+    cluster[0].val.clusterDim.y = cluster[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(tiles * a.splits), a.H, a.B);
+    cfg.blockDim = dim3(C::kThreads);
+    cfg.dynamicSmemBytes = C::template smem<kSplit>();
+    cfg.stream = st;
+    cfg.attrs = cluster;
+    cfg.numAttrs = 1;
+    F3D_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, mq, mk, mv, a));
     return check_launch("buck_swin_fwd");
   }
-  cudaLaunchAttribute cluster[1];
-  cluster[0].id = cudaLaunchAttributeClusterDimension;
-  cluster[0].val.clusterDim.x = (unsigned)a.splits;
-  cluster[0].val.clusterDim.y = cluster[0].val.clusterDim.z = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(C::kThreads);
-  cfg.dynamicSmemBytes = C::kSmem;
-  cfg.stream = st;
-  cfg.attrs = cluster;
-  cfg.numAttrs = 1;
-  F3D_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, mq, mk, mv, a));
+  // A CTA spends 4,000 cycles before its first scores (tensor memory, scope table, Q and K from memory) and 1,300 after its
+  // last: a fifth of its life at W = 512.  There it takes two query tiles of its scope, the second one's Q and keys arriving
+  // under the first (8 heads: W = 512 1497 -> 1391 us, W = 1024 1253 -> 1202 us, W = 256 528 -> 495 us; four tiles: 1685, the
+  // CTAs of an SM then run in step; nothing at W = 4096).
+  if constexpr (D <= 32) {
+    if (tiles_per_scope % 2 == 0 && tiles_per_scope <= kShortWindow && tiles * heads >= 8 * room) {
+      auto kern = attn_fwd_kernel<D, F16, kTwoTiles>;
+      F3D_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(kern), device, C::template smem<kTwoTiles>()));
+      kern<<<dim3((unsigned)(tiles / 2), a.H, a.B), C::kThreads, C::template smem<kTwoTiles>(), st>>>(mq, mk, mv, a);
+      return check_launch("buck_swin_fwd");
+    }
+  }
+  auto kern = attn_fwd_kernel<D, F16, kPlain>;
+  F3D_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(kern), device, C::template smem<kPlain>()));
+  kern<<<dim3((unsigned)tiles, a.H, a.B), C::kThreads, C::template smem<kPlain>(), st>>>(mq, mk, mv, a);
   return check_launch("buck_swin_fwd");
 }
 

@@ -107,6 +107,34 @@ def test_growing_scores(cuda_device, d, dtype, steps, bucket):
     assert ((lse.cpu() - ref_lse).abs() / ref_lse.abs().clamp(min=1)).max().item() <= 1e-4
 
 
+@pytest.mark.parametrize("d,dtype", [(16, torch.bfloat16), (32, torch.bfloat16), (32, torch.float16)])
+@pytest.mark.parametrize("bucket,k,jump", [(256, 1, False), (128, 2, False), (512, 2, False), (256, 1, True)])
+def test_many_short_scopes(cuda_device, d, dtype, bucket, k, jump):
+    """So many tiles of a short window that a CTA takes two query tiles of its scope: the buckets of a scope in any order, and
+    rows of the second tile that send the CTA into the careful pass.  Checked on the first, a middle and the last scope."""
+    from flash3dtransformer_b200.lib import pshattn
+    dev = cuda_device
+    w, h = bucket * k, 16
+    n = 5120 * 128 // (h * w) + 1                                 # scopes: past eight CTAs for every slot of 148 SMs
+    l = n * w
+    g = torch.Generator(dev).manual_seed(3)
+    q, kk, v = (torch.randn(1, l, h, d, generator=g, device=dev).to(dtype) for _ in range(3))
+    if jump:
+        kk[:, 60::w] *= 12.0
+        q[:, 128::w] *= 4.0
+    sc = torch.randperm(l // bucket, generator=torch.Generator().manual_seed(4)).reshape(n, k)
+    o = torch.zeros(1, l, h, d, dtype=dtype, device=dev)
+    lse = torch.zeros(1, l, h, dtype=torch.float32, device=dev)
+    pshattn.buck_swin_fwd(q, kk, v, o, lse, sc.to(torch.uint32).to(dev), bucket)
+    pshattn.device_status()
+    for s in (0, n // 2, n - 1):
+        rows = torch.cat([torch.arange(b * bucket, (b + 1) * bucket) for b in sc[s].tolist()])
+        sub = [t[:, rows.to(dev)].cpu() for t in (q, kk, v, o, lse)]
+        ref_o, ref_lse = ao.buck_swin_fwd(sub[0], sub[1], sub[2], torch.arange(k).reshape(1, k), bucket)
+        assert (sub[3].float() - ref_o).abs().max().item() <= 3e-2
+        assert (sub[4] - ref_lse).abs().max().item() <= 2e-2
+
+
 def test_errors(cuda_device):
     from flash3dtransformer_b200.lib import pshattn
     dev = cuda_device
