@@ -537,6 +537,32 @@ __global__ void attn_bwd_dq_convert_kernel(const float *__restrict__ acc, __nv_b
   reinterpret_cast<uint4 *>(dQ)[i] = w;
 }
 
+// Clears the rows of the buckets that no scope lists in `mats` matrices of [batch][L rows of row16 16-byte words].  A block
+// takes 32 buckets: it reads the whole table once (a few KB) and clears what is left over, which is nothing when the scopes
+// cover every bucket.  (A zero fill of the gradients of an attention layer, 960,000 rows of 3 x 256, took 372 us.)
+__global__ void __launch_bounds__(256) clear_unlisted_kernel(uint4 *__restrict__ t, const uint32_t *__restrict__ scopes, uint32_t entries,
+                                                             uint32_t buckets, uint32_t bucket, uint32_t L, uint32_t row16, uint32_t mats) {
+  __shared__ uint32_t listed;
+  if (threadIdx.x == 0) listed = 0u;
+  __syncthreads();
+  const uint32_t b0 = blockIdx.x * 32;
+  uint32_t mine = 0u;
+  for (uint32_t e = threadIdx.x; e < entries; e += 256) {
+    const uint32_t d = __ldg(scopes + e) - b0;
+    if (d < 32u) mine |= 1u << d;
+  }
+  if (mine) atomicOr(&listed, mine);
+  __syncthreads();
+  const uint64_t words = (uint64_t)bucket * row16;                // of one bucket in one matrix
+  for (uint32_t i = 0; i < 32 && b0 + i < buckets; ++i) {
+    if ((listed >> i) & 1u) continue;
+    for (uint32_t m = 0; m < mats; ++m) {
+      uint4 *p = t + ((uint64_t)m * L + (uint64_t)(b0 + i) * bucket) * row16;
+      for (uint64_t w = threadIdx.x; w < words; w += 256) p[w] = make_uint4(0u, 0u, 0u, 0u);
+    }
+  }
+}
+
 template <int D>
 static int launch_attn_bwd(const void *Q, const void *K, const void *V, const void *dO, AttnBwdArgs a, int device, cudaStream_t st) {
   using C = BwdCfg<D>;
@@ -604,4 +630,20 @@ extern "C" int f3d_buck_swin_bwd(const void *Q, const void *K, const void *V, co
   attn_bwd_dq_convert_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, st>>>(static_cast<const float *>(acc), static_cast<__nv_bfloat16 *>(dQ), n8, scale);
   F3D_TRY(check_launch("buck_swin_bwd (dq convert)"));
   return maybe_sync(st, "buck_swin_bwd");
+}
+
+extern "C" int f3d_clear_unlisted(void *rows, const void *scope_buckets, int mats, int L, uint64_t row_bytes, int num_scopes,
+                                  int scope_size, uint32_t bucket_size, int device, void *stream) {
+  if (mats < 0 || L < 0 || num_scopes < 0 || scope_size < 0 || bucket_size == 0 || L % (int)bucket_size || row_bytes % 16 ||
+      reinterpret_cast<uintptr_t>(rows) % 16)
+    return set_error(F3D_ERR_ARG, "clear_unlisted: %d x %d rows of %llu bytes in buckets of %u", mats, L, (unsigned long long)row_bytes, bucket_size);
+  const uint32_t buckets = (uint32_t)L / bucket_size;
+  if (mats == 0 || buckets == 0 || row_bytes == 0) return F3D_OK;
+  DeviceGuard guard(device);
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  clear_unlisted_kernel<<<(buckets + 31) / 32, 256, 0, st>>>(static_cast<uint4 *>(rows), static_cast<const uint32_t *>(scope_buckets),
+                                                             (uint32_t)num_scopes * (uint32_t)scope_size, buckets, bucket_size, (uint32_t)L,
+                                                             (uint32_t)(row_bytes / 16), (uint32_t)mats);
+  F3D_TRY(check_launch("clear_unlisted"));
+  return maybe_sync(st, "clear_unlisted");
 }

@@ -35,7 +35,11 @@ class BuckSwinFwdFunction(Function):
     @staticmethod
     def backward(ctx, grad_output) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor, None, None]:
         Q, K, V, O, lse = ctx.saved_tensors
-        bwd = sa.BuckSwinBwdBuffers.create_buckswin_buffers(O, ctx.scope_buckets, ctx.buck_size)
+        bwd = sa.BuckSwinBwdBuffers.create_buckswin_buffers(O, ctx.scope_buckets, ctx.buck_size, fill=False)
+        b, l, h, d = O.shape
+        if getattr(ctx.scope_buckets, "_f3d_partition_of", -1) != l:
+            for t in (bwd.dK, bwd.dV):
+                pshattn.clear_unlisted(t.view(b, l, h * d), ctx.scope_buckets, ctx.buck_size)
         pshattn.buck_swin_bwd(Q, K, V, O, grad_output.contiguous(), lse, bwd.Delta, bwd.dQ, bwd.dK, bwd.dV,
                               ctx.scope_buckets, ctx.buck_size)
         return bwd.dQ, bwd.dK, bwd.dV, None, None
@@ -63,9 +67,10 @@ class BuckSwinPackedFunction(Function):
         shape, scope_buckets, buck_size = ctx.cfg
         b, l, h, d = shape
         # scope tables made by SwinPlan are marked when they put every bucket in exactly one scope; then every row of
-        # the gradient is written by the kernel and the buffer needs no zero fill
-        covered = getattr(scope_buckets, "_f3d_partition_of", -1) == l
-        grad = torch.empty_like(qkv) if covered else torch.zeros_like(qkv)
+        # the gradient is written by the kernel.  Otherwise the rows of unlisted buckets are cleared.
+        grad = torch.empty_like(qkv)
+        if getattr(scope_buckets, "_f3d_partition_of", -1) != l:
+            pshattn.clear_unlisted(grad.view(3 * b, l, h * d), scope_buckets, buck_size)
         Q, K, V = (qkv[i].view(b, l, h, d) for i in range(3))
         dQ, dK, dV = (grad[i].view(b, l, h, d) for i in range(3))
         delta = torch.empty(b, l, h, dtype=torch.float32, device=O.device)      # every row is written by the delta kernel

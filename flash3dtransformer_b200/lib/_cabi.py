@@ -51,6 +51,7 @@ PROTOTYPES = {
     "f3d_buck_swin_fwd_dtype": (_int, [_vp, _vp, _vp, _vp, _vp, _vp, _int, _int, _int, _int, _int, _int, _u32, _int, _int, _vp]),
     "f3d_linear_fused": (_int, [_vp, _vp, _vp, _vp, _vp, _int, _int, _int, _int, _int, _int, _vp, _vp, _f32, _vp, _int, _vp]),
     "f3d_bbox_f16": (_int, [_vp, _vp, _vp, _u32, _int, _vp]),
+    "f3d_clear_unlisted": (_int, [_vp, _vp, _int, _int, c_uint64, _int, _int, _u32, _int, _vp]),
     "f3d_row_stats_bf16": (_int, [_vp, _vp, _u32, _u32, _int, _vp]),
     "f3d_xfmr_stack_bf16": (_int, [ctypes.POINTER(XfmrBlock), _int, _vp, _vp, _vp, _vp, c_uint64, _u32, _u32, _int, _vp]),
     "f3d_xfmr_stack_scratch": (c_uint64, [_u32, _u32, _u32]),

@@ -775,3 +775,18 @@ def buck_swin_bwd(Q, K, V, O, dO, LSE, Delta, dQ, dK, dV, Scope_buckets, bucket_
                                         _ptr(dK), _ptr(dV), _ptr(Scope_buckets), b, l, h, d, Scope_buckets.shape[0],
                                         Scope_buckets.shape[1], int(bucket_size), dev, _stream(dev))
     _cabi.check(st, "buck_swin_bwd")
+
+
+def clear_unlisted(rows, Scope_buckets, bucket_size) -> None:
+    """rows [mats, L, ...] = 0 for the tokens of every bucket that no scope lists (buck_swin_bwd leaves their dK and dV as
+    they are).  No counterpart in the reference, which fills the whole gradient with zeros first."""
+    dev = _check_tensors([rows, Scope_buckets], ["rows", "Scope_buckets"])
+    _check_dtype([Scope_buckets], ["Scope_buckets"], torch.uint32)
+    if rows.dim() < 2 or Scope_buckets.dim() != 2:
+        raise RuntimeError("rows must be [mats, L, ...] and Scope_buckets [num_scopes, scope_size]")
+    mats, l = rows.shape[0], rows.shape[1]
+    if mats * l == 0:
+        return
+    st = _cabi.load().f3d_clear_unlisted(_ptr(rows), _ptr(Scope_buckets), mats, l, rows.numel() // (mats * l) * rows.element_size(),
+                                         Scope_buckets.shape[0], Scope_buckets.shape[1], int(bucket_size), dev, _stream(dev))
+    _cabi.check(st, "clear_unlisted")

@@ -37,7 +37,12 @@ class BuckSwinBwdBuffers:
     buck_size: int
 
     @staticmethod
-    def create_buckswin_buffers(O: torch.Tensor, Scope_buckets: torch.Tensor, buck_size: int):
+    def create_buckswin_buffers(O: torch.Tensor, Scope_buckets: torch.Tensor, buck_size: int, fill: bool = True):
+        """`fill` False leaves the buffers as allocated: the backward writes Delta and dQ whole, dK and dV for the tokens of
+        listed buckets."""
         b, l, h, _ = O.shape
+        if not fill:
+            return BuckSwinBwdBuffers(O, torch.empty_like(O), torch.empty_like(O), torch.empty_like(O), Scope_buckets,
+                                      torch.empty(b, l, h, dtype=torch.float32, device=O.device), buck_size)
         return BuckSwinBwdBuffers(O, torch.zeros_like(O), torch.zeros_like(O), torch.zeros_like(O), Scope_buckets,
                                   torch.zeros(b, l, h, dtype=torch.float32, device=O.device), buck_size)

@@ -261,6 +261,11 @@ uint64_t f3d_xfmr_stack_scratch(uint32_t rows, uint32_t channels, uint32_t hidde
  * bf16 in/out, fp32 accumulation; synchronises the stream like the reference (:77).  Any M; N, K multiples of 8. */
 int f3d_gemm_sm_bf16(const void *A, const void *B, void *O, int M, int N, int K, int device, void *stream);
 
+/* zeroes the rows of every bucket that no scope lists in `mats` consecutive matrices of L rows of row_bytes bytes (a multiple
+ * of 16): the gradients of tokens that f3d_buck_swin_bwd does not write */
+int f3d_clear_unlisted(void *rows, const void *scope_buckets, int mats, int L, uint64_t row_bytes, int num_scopes,
+                       int scope_size, uint32_t bucket_size, int device, void *stream);
+
 /* bounding box of fp16 coords [rows, 3]: bbox_min / bbox_max fp16 [3], NaN where a column holds one (coords.min(0) and
  * coords.max(0) of flash3dxfmr/psh/psh_main.py:117-118); rows > 0 */
 int f3d_bbox_f16(const void *coords, void *bbox_min, void *bbox_max, uint32_t rows, int device, void *stream);

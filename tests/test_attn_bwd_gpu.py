@@ -196,3 +196,30 @@ def test_full_size_layer_sampled_scopes_and_properties(cuda_device, k):
     scale = do.float().abs().mean().item()
     assert dq1[:, :n_listed].float().abs().max().item() <= 0.05 * scale * 8
     assert dk1[:, :n_listed].float().abs().max().item() <= 0.05 * scale * 8
+
+
+@pytest.mark.parametrize("b,d,listed", [(1, 32, [[0, 2], [5, 39]]), (2, 16, [[1], [33]]), (1, 64, [])])
+def test_layer_gradient_of_unlisted_buckets_is_zero(cuda_device, b, d, listed):
+    """The layer's gradients start uninitialised: the rows of buckets that no scope lists are cleared, the listed ones are what
+    a zero-filled buffer gives."""
+    from flash3dtransformer_b200.layers.buck_swin import BuckSwinFwdFunction, BuckSwinPackedFunction
+    dev = cuda_device
+    h, bucket, n = 2, 128, 40
+    l = n * bucket
+    g = torch.Generator(dev).manual_seed(0)
+    qkv = torch.randn(3, b * l, h * d, generator=g, device=dev).bfloat16()
+    do = torch.randn(b, l, h, d, generator=g, device=dev).bfloat16()
+    sc = torch.tensor(listed if listed else [[0]], dtype=torch.int64).to(torch.uint32).to(dev)
+    sc = sc if listed else sc[:0]
+    rows = torch.zeros(l, dtype=torch.bool)
+    for bk in [x for s in listed for x in s]:
+        rows[bk * bucket:(bk + 1) * bucket] = True
+    torch.empty(64 << 20, device=dev).fill_(float("nan"))             # what the allocator hands out next is not zero
+    x = qkv.clone().requires_grad_(True)
+    BuckSwinPackedFunction.apply(x, (b, l, h, d), sc, bucket).backward(do)
+    parts = [qkv[i].view(b, l, h, d).clone().requires_grad_(True) for i in range(3)]
+    BuckSwinFwdFunction.apply(*parts, sc, bucket).backward(do)
+    for i in range(3):
+        got = x.grad[i].view(b, l, h, d)
+        assert torch.isfinite(got.float()).all() and torch.equal(got, parts[i].grad)
+        assert torch.all(got[:, ~rows.to(dev)] == 0) and (not listed or got[:, rows.to(dev)].abs().max() > 0)
