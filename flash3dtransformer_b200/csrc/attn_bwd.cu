@@ -180,6 +180,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   __syncthreads();
   tc::tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  grid_enter();
   tc::WaitCtx wc{abort_flag, a.status};
 
   if (warp == 0) {
@@ -513,6 +514,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 // Delta[b,t,h] = sum_d dO * O  (tests/test_attn_bwd.py:24-27)
 __global__ void attn_bwd_delta_kernel(const __nv_bfloat16 *__restrict__ O, const __nv_bfloat16 *__restrict__ dO,
                                       float *__restrict__ delta, size_t rows, int D) {
+  const uint32_t after = grid_enter();
+  O += after; dO += after;
   size_t r = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= rows) return;
   const uint4 *po = reinterpret_cast<const uint4 *>(O + r * D), *pd = reinterpret_cast<const uint4 *>(dO + r * D);
@@ -527,6 +530,8 @@ __global__ void attn_bwd_delta_kernel(const __nv_bfloat16 *__restrict__ O, const
 }
 
 __global__ void attn_bwd_dq_convert_kernel(const float *__restrict__ acc, __nv_bfloat16 *__restrict__ dQ, size_t n8, float scale) {
+  const uint32_t after = grid_enter();
+  acc += after;
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n8) return;
   float4 a4 = reinterpret_cast<const float4 *>(acc)[2 * i], b4 = reinterpret_cast<const float4 *>(acc)[2 * i + 1];
@@ -542,6 +547,8 @@ __global__ void attn_bwd_dq_convert_kernel(const float *__restrict__ acc, __nv_b
 // cover every bucket.  (A zero fill of the gradients of an attention layer, 960,000 rows of 3 x 256, took 372 us.)
 __global__ void __launch_bounds__(256) clear_unlisted_kernel(uint4 *__restrict__ t, const uint32_t *__restrict__ scopes, uint32_t entries,
                                                              uint32_t buckets, uint32_t bucket, uint32_t L, uint32_t row16, uint32_t mats) {
+  const uint32_t after = grid_enter();
+  scopes += after;
   __shared__ uint32_t listed;
   if (threadIdx.x == 0) listed = 0u;
   __syncthreads();
@@ -581,7 +588,7 @@ static int launch_attn_bwd(const void *Q, const void *K, const void *V, const vo
   if (C::kTmaDq)
     F3D_TRY(encode_tmap_2d(&mdq, 2, a.dq_acc, (uint64_t)a.H * D, rows, (uint64_t)a.H * D * 4, D, C::BQ, 128));
   dim3 grid(a.num_scopes * a.k * a.kblocks_per_bucket, a.H, a.B);
-  kern<<<grid, C::kThreads, C::kSmem, st>>>(mq, mk, mv, mdo, mdq, a);
+  launch(kern, grid, C::kThreads, C::kSmem, st, mq, mk, mv, mdo, mdq, a);
   return check_launch("buck_swin_bwd");
 }
 
@@ -602,7 +609,7 @@ extern "C" int f3d_buck_swin_bwd(const void *Q, const void *K, const void *V, co
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   F3D_TRY(maybe_sync(st, "buck_swin_bwd"));
   const size_t rows = (size_t)B * L * H;
-  attn_bwd_delta_kernel<<<(unsigned)((rows + 255) / 256), 256, 0, st>>>(static_cast<const __nv_bfloat16 *>(O), static_cast<const __nv_bfloat16 *>(dO),
+  launch(attn_bwd_delta_kernel, (unsigned)((rows + 255) / 256), 256, 0, st, static_cast<const __nv_bfloat16 *>(O), static_cast<const __nv_bfloat16 *>(dO),
                                                                        static_cast<float *>(Delta), rows, D);
   F3D_TRY(check_launch("buck_swin_bwd (delta)"));
   if (num_scopes == 0) {          // no bucket is listed: dQ is all zero, dK and dV have no listed rows
@@ -627,7 +634,7 @@ extern "C" int f3d_buck_swin_bwd(const void *Q, const void *K, const void *V, co
   }
   F3D_TRY(rc);
   const size_t n8 = rows * D / 8;
-  attn_bwd_dq_convert_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, st>>>(static_cast<const float *>(acc), static_cast<__nv_bfloat16 *>(dQ), n8, scale);
+  launch(attn_bwd_dq_convert_kernel, (unsigned)((n8 + 255) / 256), 256, 0, st, static_cast<const float *>(acc), static_cast<__nv_bfloat16 *>(dQ), n8, scale);
   F3D_TRY(check_launch("buck_swin_bwd (dq convert)"));
   return maybe_sync(st, "buck_swin_bwd");
 }
@@ -641,7 +648,7 @@ extern "C" int f3d_clear_unlisted(void *rows, const void *scope_buckets, int mat
   if (mats == 0 || buckets == 0 || row_bytes == 0) return F3D_OK;
   DeviceGuard guard(device);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  clear_unlisted_kernel<<<(buckets + 31) / 32, 256, 0, st>>>(static_cast<uint4 *>(rows), static_cast<const uint32_t *>(scope_buckets),
+  launch(clear_unlisted_kernel, (buckets + 31) / 32, 256, 0, st, static_cast<uint4 *>(rows), static_cast<const uint32_t *>(scope_buckets),
                                                              (uint32_t)num_scopes * (uint32_t)scope_size, buckets, bucket_size, (uint32_t)L,
                                                              (uint32_t)(row_bytes / 16), (uint32_t)mats);
   F3D_TRY(check_launch("clear_unlisted"));

@@ -326,11 +326,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     // four key tiles always lie in one bucket.
     if (warp == 0 && tc::elect_one()) {
       if (pass) for (uint64_t *bar = bars; bar <= q_full + 1; ++bar) tc::mbar_inval(bar);
+      if (pass == 0) { tc::tma_prefetch_desc(&map_q); tc::tma_prefetch_desc(&map_k); tc::tma_prefetch_desc(&map_v); }
       *abort_flag = 0;
       for (int s = 0; s < R; ++s) tc::mbar_init(&kv_full[s], 1);
       for (int b = 0; b < 2; ++b) { tc::mbar_init(&s_full[b], 1); tc::mbar_init(&p_full[b], 128); }
       tc::mbar_init(&q_full[0], 1); tc::mbar_init(&q_full[1], 1);
       tc::mbar_fence_init();
+      grid_wait();                                                // in the first pass; the kernel in front has long ended in the second
       const int q_tok = q_token(qt);
       const int tok0 = row0 + (int)my_scope[slot0] * a.bucket + at0;
       tc::mbar_expect_tx(q_full, C::kQBytes + 2 * C::kTileBytes);
@@ -348,6 +350,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     __syncthreads();
     tc::tc_fence_after_sync();
     tmem_base = *tmem_slot;
+    if (pass == 0) grid_enter();                                  // the other warps store O, which the kernel in front may still read
     if (warp == 0) {
       if (tc::elect_one()) {
         // position of a stream of key tiles: row inside its bucket, first token of the bucket and of the next one (the scope
@@ -546,17 +549,19 @@ static int launch_attn_fwd(const void *Q, const void *K, const void *V, AttnFwdA
   if (a.splits > 1) {
     auto kern = attn_fwd_kernel<D, F16, kSplit>;
     F3D_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(kern), device, C::template smem<kSplit>()));
-    cudaLaunchAttribute cluster[1];
+    cudaLaunchAttribute cluster[2];
     cluster[0].id = cudaLaunchAttributeClusterDimension;
     cluster[0].val.clusterDim.x = (unsigned)a.splits;
     cluster[0].val.clusterDim.y = cluster[0].val.clusterDim.z = 1;
+    cluster[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    cluster[1].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)(tiles * a.splits), a.H, a.B);
     cfg.blockDim = dim3(C::kThreads);
     cfg.dynamicSmemBytes = C::template smem<kSplit>();
     cfg.stream = st;
     cfg.attrs = cluster;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     F3D_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, mq, mk, mv, a));
     return check_launch("buck_swin_fwd");
   }
@@ -568,13 +573,13 @@ static int launch_attn_fwd(const void *Q, const void *K, const void *V, AttnFwdA
     if (tiles_per_scope % 2 == 0 && tiles_per_scope <= kShortWindow && tiles * heads >= 8 * room) {
       auto kern = attn_fwd_kernel<D, F16, kTwoTiles>;
       F3D_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(kern), device, C::template smem<kTwoTiles>()));
-      kern<<<dim3((unsigned)(tiles / 2), a.H, a.B), C::kThreads, C::template smem<kTwoTiles>(), st>>>(mq, mk, mv, a);
+      launch(kern, dim3((unsigned)(tiles / 2), a.H, a.B), C::kThreads, C::template smem<kTwoTiles>(), st, mq, mk, mv, a);
       return check_launch("buck_swin_fwd");
     }
   }
   auto kern = attn_fwd_kernel<D, F16, kPlain>;
   F3D_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(kern), device, C::template smem<kPlain>()));
-  kern<<<dim3((unsigned)tiles, a.H, a.B), C::kThreads, C::template smem<kPlain>(), st>>>(mq, mk, mv, a);
+  launch(kern, dim3((unsigned)tiles, a.H, a.B), C::kThreads, C::template smem<kPlain>(), st, mq, mk, mv, a);
   return check_launch("buck_swin_fwd");
 }
 

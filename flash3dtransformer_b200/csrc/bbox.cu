@@ -60,6 +60,8 @@ __device__ __forceinline__ void box_store(Box3 b, __half *lo, __half *hi) {
 // VEC: the coordinates start on a 16-byte boundary.  Block b of `gridDim.x` leaves its box at lo + 6 b, hi + 6 b.
 template <bool VEC>
 __global__ void __launch_bounds__(kBoxThreads) bbox_kernel(const __half *__restrict__ c, uint32_t n, __half *lo, __half *hi) {
+  const uint32_t after = grid_enter();
+  c += after;
   Box3 b;
   box_init(b);
   const uint32_t stride = gridDim.x * kBoxThreads, first = blockIdx.x * kBoxThreads + threadIdx.x;
@@ -86,6 +88,8 @@ __global__ void __launch_bounds__(kBoxThreads) bbox_kernel(const __half *__restr
 }
 
 __global__ void __launch_bounds__(kBoxThreads) bbox_final_kernel(const __half *__restrict__ part, uint32_t blocks, __half *lo, __half *hi) {
+  const uint32_t after = grid_enter();
+  part += after;
   Box3 b;
   box_init(b);
   for (uint32_t r = threadIdx.x; r < blocks; r += kBoxThreads) {
@@ -122,9 +126,9 @@ extern "C" int f3d_bbox_f16(const void *coords, void *bbox_min, void *bbox_max, 
     out_lo = static_cast<__half *>(part);
     out_hi = out_lo + 3;
   }
-  if (vec) bbox_kernel<true><<<blocks, kBoxThreads, 0, st>>>(c, rows, out_lo, out_hi);
-  else bbox_kernel<false><<<blocks, kBoxThreads, 0, st>>>(c, rows, out_lo, out_hi);
-  if (!one) bbox_final_kernel<<<1, kBoxThreads, 0, st>>>(out_lo, blocks, lo, hi);
+  if (vec) launch(bbox_kernel<true>, blocks, kBoxThreads, 0, st, c, rows, out_lo, out_hi);
+  else launch(bbox_kernel<false>, blocks, kBoxThreads, 0, st, c, rows, out_lo, out_hi);
+  if (!one) launch(bbox_final_kernel, 1, kBoxThreads, 0, st, out_lo, blocks, lo, hi);
   F3D_TRY(check_launch("bbox", one ? 1 : 2));
   return maybe_sync(st, "bbox");
 }

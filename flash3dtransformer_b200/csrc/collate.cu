@@ -19,6 +19,8 @@ constexpr int kCollatePerThread = 4;     // points per thread: independent loads
 template <int DIM>
 __global__ void __launch_bounds__(kCollateThreads) collate_points_kernel(const float *__restrict__ rec, __half *__restrict__ coords,
                                                                          float *__restrict__ extra, uint64_t rows) {
+  const uint32_t after = grid_enter();
+  rec += after;
   const uint64_t base = (uint64_t)blockIdx.x * (kCollateThreads * kCollatePerThread) + threadIdx.x;
   float v[kCollatePerThread][DIM];
 #pragma unroll
@@ -63,7 +65,7 @@ __global__ void __launch_bounds__(kCollateThreads) collate_points_kernel(const f
 template <int DIM>
 static int launch_collate(const void *rec, void *coords, void *extra, uint64_t rows, cudaStream_t st) {
   const uint64_t per_cta = (uint64_t)kCollateThreads * kCollatePerThread;
-  collate_points_kernel<DIM><<<(unsigned)((rows + per_cta - 1) / per_cta), kCollateThreads, 0, st>>>(
+  launch(collate_points_kernel<DIM>, (unsigned)((rows + per_cta - 1) / per_cta), kCollateThreads, 0, st,
       static_cast<const float *>(rec), static_cast<__half *>(coords), static_cast<float *>(extra), rows);
   return check_launch("collate_points");
 }

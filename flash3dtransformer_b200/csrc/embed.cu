@@ -16,6 +16,8 @@ constexpr int kEmbedThreads = 256;
 __global__ void __launch_bounds__(kEmbedThreads) coord_embed_kernel(const __half *__restrict__ x, const float *__restrict__ w,
                                                                     const float *__restrict__ b, __nv_bfloat16 *__restrict__ y,
                                                                     uint32_t rows, uint32_t C, uint32_t rows_per_block) {
+  const uint32_t after = grid_enter();
+  x += after; w += after; b += after;
   const uint32_t chunks = C / 8;                         // 16-byte output chunks per row
   const uint32_t ch = threadIdx.x % chunks, rsub = threadIdx.x / chunks, rstep = kEmbedThreads / chunks;
   if (rsub >= rstep) return;                             // threads beyond a whole number of rows idle
@@ -49,6 +51,8 @@ __global__ void __launch_bounds__(kEmbedThreads) coord_embed_kernel(const __half
 __global__ void __launch_bounds__(kEmbedThreads) coord_embed_bwd_partial_kernel(const __half *__restrict__ x, const __nv_bfloat16 *__restrict__ g,
                                                                                 float *__restrict__ partial, uint32_t rows, uint32_t C,
                                                                                 uint32_t rows_per_block) {
+  const uint32_t after = grid_enter();
+  x += after; g += after;
   extern __shared__ float red[];                         // [slots][4][C]
   const uint32_t chunks = C / 8;
   const uint32_t ch = threadIdx.x % chunks, rsub = threadIdx.x / chunks, rstep = kEmbedThreads / chunks;
@@ -88,6 +92,8 @@ __global__ void __launch_bounds__(kEmbedThreads) coord_embed_bwd_partial_kernel(
 
 __global__ void __launch_bounds__(256) coord_embed_bwd_reduce_kernel(const float *__restrict__ partial, float *__restrict__ gw,
                                                                      float *__restrict__ gb, uint32_t blocks, uint32_t C) {
+  const uint32_t after = grid_enter();
+  partial += after;
   const uint32_t q = blockIdx.x * 256 + threadIdx.x;      // q = j * C + c
   if (q >= 4 * C) return;
   float s = 0.f;
@@ -120,10 +126,10 @@ extern "C" int f3d_coord_embed_bwd(const void *coords, const void *grad_out, voi
   blocks = (rows + rows_per_block - 1) / rows_per_block;
   void *partial = nullptr;
   F3D_TRY(workspace(device, 4, (size_t)blocks * 4 * C * sizeof(float), st, &partial));
-  coord_embed_bwd_partial_kernel<<<blocks, kEmbedThreads, smem, st>>>(static_cast<const __half *>(coords), static_cast<const __nv_bfloat16 *>(grad_out),
+  launch(coord_embed_bwd_partial_kernel, blocks, kEmbedThreads, smem, st, static_cast<const __half *>(coords), static_cast<const __nv_bfloat16 *>(grad_out),
                                                                      static_cast<float *>(partial), rows, C, rows_per_block);
   F3D_TRY(check_launch("coord_embed_bwd"));
-  coord_embed_bwd_reduce_kernel<<<(4 * C + 255) / 256, 256, 0, st>>>(static_cast<const float *>(partial), static_cast<float *>(grad_weight),
+  launch(coord_embed_bwd_reduce_kernel, (4 * C + 255) / 256, 256, 0, st, static_cast<const float *>(partial), static_cast<float *>(grad_weight),
                                                                     static_cast<float *>(grad_bias), blocks, C);
   return check_launch("coord_embed_bwd (reduce)");
 }
@@ -137,7 +143,7 @@ extern "C" int f3d_coord_embed_bf16(const void *coords, const void *weight, cons
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const uint32_t rows_per_block = 512;
   const uint32_t grid = (rows + rows_per_block - 1) / rows_per_block;
-  coord_embed_kernel<<<grid, kEmbedThreads, 0, st>>>(static_cast<const __half *>(coords), static_cast<const float *>(weight),
+  launch(coord_embed_kernel, grid, kEmbedThreads, 0, st, static_cast<const __half *>(coords), static_cast<const float *>(weight),
                                                     static_cast<const float *>(bias), static_cast<__nv_bfloat16 *>(out), rows, C,
                                                     rows_per_block);
   return check_launch("coord_embed_bf16");

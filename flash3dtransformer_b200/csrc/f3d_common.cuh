@@ -46,6 +46,43 @@ static inline int check_launch(const char *what, int kernels = 1) {
   return F3D_OK;
 }
 
+// Every kernel of the library is launched so that its blocks may start while the kernel before it in the stream is still
+// running its last ones (programmatic stream serialisation); each block waits for that kernel, and with it for everything in
+// front of it, before it touches memory.  What overlaps is the launch itself and, in the tensor-core kernels, the setup of
+// barriers, tensor memory and descriptors: 2-4 us of every launch, which is half of a small batch's forward.
+// A kernel that does not wait, a copy or a memset behind such a launch keeps the full order of the stream.
+template <class... P, class... A>
+static inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<A &&>(args)...);      // the caller's check_launch reads the error
+}
+
+// Waits for the kernel in front.  The zero it returns goes into the addresses of what that kernel may have written: loads the
+// compiler takes for invariant (__ldg, __restrict__) can then not move in front of the wait.
+__device__ __forceinline__ uint32_t grid_wait() {
+  uint32_t zero;
+  asm volatile("griddepcontrol.wait;\n\tmov.u32 %0, 0;" : "=r"(zero)::"memory");
+  return zero;
+}
+// Lets the next kernel's blocks start.  Only behind everything this block allocates (tensor memory): a block of the next
+// kernel may hold what is left of it until this kernel has ended.
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// both, for kernels that allocate nothing: the first statement of the kernel
+__device__ __forceinline__ uint32_t grid_enter() {
+  const uint32_t zero = grid_wait();
+  grid_release();
+  return zero;
+}
+
 static inline int maybe_sync(cudaStream_t s, const char *what) {
   if (!sync_flag()) return F3D_OK;
   cudaError_t e = cudaStreamSynchronize(s);

@@ -170,6 +170,16 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   // neither loads nor adds it.  Every 16-byte half of the ones rows is (1, 1, 1, 0, ...), the bias rows carry their terms
   // in the first half and zeros in the second, so the sum does not depend on where the 32-byte swizzle puts the halves.
   const bool fold_bias = g.bias != nullptr && g.ln_stats == nullptr && n_tiles == 1 && g.ksplit == 1;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kStages; ++s) { tc::mbar_init(&full[s], 1); tc::mbar_init(&empty[s], 1); }
+    for (int a = 0; a < kAcc; ++a) { tc::mbar_init(&acc_full[a], 1); tc::mbar_init(&acc_empty[a], kEpiWarps); }
+    if (!LEAN) for (int a = 0; a < kAcc * 4; ++a) stat_cnt[a] = 0;
+    *abort_flag = 0;
+    tc::mbar_fence_init();
+    tc::tma_prefetch_desc(&map_a); tc::tma_prefetch_desc(&map_b); tc::tma_prefetch_desc(&map_c);
+  }
+  if (warp == 1) { tc::tmem_alloc(tmem_slot, kTmemCols); tc::tmem_relinquish(); }
+  const uint32_t after = grid_wait();
   if (fold_bias) {
     const uint32_t one2 = F16 ? 0x3C003C00u : 0x3F803F80u, one1 = F16 ? 0x00003C00u : 0x00003F80u;
     for (int c = threadIdx.x; c < BM * 2; c += kGemmThreads) tc::sts128(tc::smem_u32(fold_base) + c * 16, make_uint4(one2, one1, 0u, 0u));
@@ -178,7 +188,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       int col = r;
       if (g.epilogue == EPI_SWIGLU) col = r < BN / 2 ? r : g.N / 2 + (r - BN / 2);
       const bool live = g.epilogue == EPI_SWIGLU ? (r < BN / 2 ? r < g.N / 2 : r - BN / 2 < g.N / 2) : r < g.N;
-      const float b = live ? __ldg(g.bias + col) : 0.f;
+      const float b = live ? __ldg(g.bias + col + after) : 0.f;
       uint32_t w0, w1;
       if (F16) {
         const __half h0 = __float2half_rn(b);
@@ -202,23 +212,15 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     tc::fence_proxy_async();
   }
 
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) { tc::mbar_init(&full[s], 1); tc::mbar_init(&empty[s], 1); }
-    for (int a = 0; a < kAcc; ++a) { tc::mbar_init(&acc_full[a], 1); tc::mbar_init(&acc_empty[a], kEpiWarps); }
-    if (!LEAN) for (int a = 0; a < kAcc * 4; ++a) stat_cnt[a] = 0;
-    *abort_flag = 0;
-    tc::mbar_fence_init();
-  }
-  if (warp == 1) { tc::tmem_alloc(tmem_slot, kTmemCols); tc::tmem_relinquish(); }
   tc::tc_fence_before_sync();
   __syncthreads();
   tc::tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  grid_release();
   tc::WaitCtx wc{abort_flag, g.status};
 
   if (warp == 0) {
     if (tc::elect_one()) {
-      tc::tma_prefetch_desc(&map_a); tc::tma_prefetch_desc(&map_b); tc::tma_prefetch_desc(&map_c);
       uint32_t it = 0;
       bool ok = true;
       // With a single column tile and a k-block count that divides the ring, stage s always carries k-block
@@ -553,7 +555,7 @@ static int launch_gemm_build(const CUtensorMap &ma, const CUtensorMap &mb, const
   F3D_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(kern), device, GemmSmem<BN, LEAN>::kTotal));
   int tiles = ((g.M + BM - 1) / BM) * ((g.N + BN - 1) / BN);
   int grid = tiles < sm_count(device) ? tiles : sm_count(device);
-  kern<<<grid, gemm_threads(LEAN), GemmSmem<BN, LEAN>::kTotal, st>>>(ma, mb, mc, g);
+  launch(kern, grid, gemm_threads(LEAN), GemmSmem<BN, LEAN>::kTotal, st, ma, mb, mc, g);
   return check_launch("gemm_bf16_tcgen05");
 }
 
@@ -685,6 +687,8 @@ extern "C" int f3d_linear_ksplit_bf16(const void *A, const void *W, const void *
 // transposed into a scratch [N,K] matrix first so that both operands are K-major for the tensor cores.
 namespace f3d {
 __global__ void transpose_bf16_kernel(const __nv_bfloat16 *in, __nv_bfloat16 *out, int rows, int cols) {
+  const uint32_t after = grid_enter();
+  in += after;
   __shared__ __nv_bfloat16 t[32][33];
   int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 32 + threadIdx.y;
   for (int j = 0; j < 32; j += 8) if (x < cols && y + j < rows) t[threadIdx.y + j][threadIdx.x] = in[(size_t)(y + j) * cols + x];
@@ -701,7 +705,7 @@ extern "C" int f3d_gemm_sm_bf16(const void *A, const void *B, void *O, int M, in
   void *bt = nullptr;
   F3D_TRY(workspace(device, 1, (size_t)N * K * 2, st, &bt));
   dim3 grid((N + 31) / 32, (K + 31) / 32), block(32, 8);
-  transpose_bf16_kernel<<<grid, block, 0, st>>>(static_cast<const __nv_bfloat16 *>(B), static_cast<__nv_bfloat16 *>(bt), K, N);
+  launch(transpose_bf16_kernel, grid, block, 0, st, static_cast<const __nv_bfloat16 *>(B), static_cast<__nv_bfloat16 *>(bt), K, N);
   F3D_TRY(check_launch("transpose"));
   F3D_TRY(linear_bf16(A, K, bt, K, nullptr, nullptr, 0, O, (long long)M * N, M, N, K, 1, EPI_NONE, device, st));
   // the reference synchronises here (src/psh/gemm_dispatcher.cu:77)

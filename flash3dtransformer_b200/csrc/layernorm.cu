@@ -39,6 +39,8 @@ template <int LPR, int CHUNKS, int ROWS, int MODE>
 __global__ void __launch_bounds__(kLnThreads) layernorm_bf16_kernel(const __nv_bfloat16 *__restrict__ x, const float *__restrict__ w,
                                                                     const float *__restrict__ b, __nv_bfloat16 *__restrict__ y,
                                                                     uint32_t rows, uint32_t C, float eps, float2 *__restrict__ stats) {
+  const uint32_t after = grid_enter();
+  x += after; w += after; b += after;
   constexpr bool GELU = MODE == 1;
   constexpr uint32_t kRowsPerWarp = 32 / LPR;
   const uint32_t lane = threadIdx.x & 31;
@@ -124,9 +126,9 @@ static void launch_ln(const __nv_bfloat16 *x, const float *w, const float *b, __
                       int gelu, cudaStream_t st) {
   const uint32_t rows_per_block = (kLnThreads / 32) * (32 / LPR) * ROWS;
   const uint32_t grid = (rows + rows_per_block - 1) / rows_per_block;
-  if (gelu == 2) layernorm_bf16_kernel<LPR, CHUNKS, ROWS, 2><<<grid, kLnThreads, 0, st>>>(x, w, b, y, rows, C, eps, reinterpret_cast<float2 *>(y));
-  else if (gelu) layernorm_bf16_kernel<LPR, CHUNKS, ROWS, 1><<<grid, kLnThreads, 0, st>>>(x, w, b, y, rows, C, eps, nullptr);
-  else layernorm_bf16_kernel<LPR, CHUNKS, ROWS, 0><<<grid, kLnThreads, 0, st>>>(x, w, b, y, rows, C, eps, nullptr);
+  if (gelu == 2) launch(layernorm_bf16_kernel<LPR, CHUNKS, ROWS, 2>, grid, kLnThreads, 0, st, x, w, b, y, rows, C, eps, reinterpret_cast<float2 *>(y));
+  else if (gelu) launch(layernorm_bf16_kernel<LPR, CHUNKS, ROWS, 1>, grid, kLnThreads, 0, st, x, w, b, y, rows, C, eps, nullptr);
+  else launch(layernorm_bf16_kernel<LPR, CHUNKS, ROWS, 0>, grid, kLnThreads, 0, st, x, w, b, y, rows, C, eps, nullptr);
 }
 
 }  // namespace f3d

@@ -18,6 +18,8 @@ template <int LPR, int CHUNKS>
 __global__ void __launch_bounds__(kLnbThreads) layernorm_bwd_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ g,
                                                                     const float *__restrict__ w, __nv_bfloat16 *__restrict__ dx,
                                                                     float *__restrict__ partial, uint32_t rows, uint32_t C, float eps) {
+  const uint32_t after = grid_enter();
+  x += after; g += after; w += after;
   constexpr uint32_t kRowsPerWarp = 32 / LPR;
   constexpr uint32_t kRowsPerBlock = (kLnbThreads / 32) * kRowsPerWarp;
   __shared__ float red[kLnbThreads / 32][LPR * CHUNKS * 8];      // one warp row per warp, used for dweight then dbias
@@ -136,6 +138,8 @@ __global__ void __launch_bounds__(kLnbThreads) layernorm_bwd_kernel(const __nv_b
 constexpr int kLnbStrands = 32;
 __global__ void __launch_bounds__(32 * kLnbStrands) layernorm_bwd_reduce_kernel(const float *__restrict__ partial, float *__restrict__ dweight,
                                                                                 float *__restrict__ dbias, uint32_t blocks, uint32_t C) {
+  const uint32_t after = grid_enter();
+  partial += after;
   __shared__ float red[2][kLnbStrands][32];
   const uint32_t tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const uint32_t c = blockIdx.x * 32 + tx;
@@ -156,7 +160,7 @@ __global__ void __launch_bounds__(32 * kLnbStrands) layernorm_bwd_reduce_kernel(
 template <int LPR, int CHUNKS>
 static void launch_lnb(const __nv_bfloat16 *x, const __nv_bfloat16 *g, const float *w, __nv_bfloat16 *dx, float *partial, uint32_t rows,
                        uint32_t C, float eps, uint32_t grid, cudaStream_t st) {
-  layernorm_bwd_kernel<LPR, CHUNKS><<<grid, kLnbThreads, 0, st>>>(x, g, w, dx, partial, rows, C, eps);
+  launch(layernorm_bwd_kernel<LPR, CHUNKS>, grid, kLnbThreads, 0, st, x, g, w, dx, partial, rows, C, eps);
 }
 
 }  // namespace f3d
@@ -204,6 +208,6 @@ extern "C" int f3d_layernorm_bwd_bf16(const void *x, const void *grad_out, const
     }
   }
   F3D_TRY(check_launch("layernorm_bwd_bf16"));
-  layernorm_bwd_reduce_kernel<<<(C + 31) / 32, 32 * kLnbStrands, 0, st>>>(pp, static_cast<float *>(grad_weight), static_cast<float *>(grad_bias), grid, C);
+  launch(layernorm_bwd_reduce_kernel, (C + 31) / 32, 32 * kLnbStrands, 0, st, pp, static_cast<float *>(grad_weight), static_cast<float *>(grad_bias), grid, C);
   return check_launch("layernorm_bwd_bf16 (reduce)");
 }

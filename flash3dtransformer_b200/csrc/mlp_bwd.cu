@@ -15,6 +15,8 @@ namespace f3d {
 
 __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const __nv_bfloat16 *__restrict__ y, const __nv_bfloat16 *__restrict__ g,
                                                          __nv_bfloat16 *__restrict__ dy, size_t rows, uint32_t F) {
+  const uint32_t after = grid_enter();
+  y += after; g += after;
   const uint32_t chunks = F / 8;
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= rows * chunks) return;
@@ -52,6 +54,8 @@ template <bool TANH> __device__ __forceinline__ float gelu_grad(float x) {
 template <bool TANH>
 __global__ void __launch_bounds__(256) gelu_bwd_kernel(const __nv_bfloat16 *__restrict__ y, const __nv_bfloat16 *__restrict__ g,
                                                        __nv_bfloat16 *__restrict__ dy, size_t chunks) {
+  const uint32_t after = grid_enter();
+  y += after; g += after;
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= chunks) return;
   const uint4 qy = __ldg(reinterpret_cast<const uint4 *>(y) + idx), qg = __ldg(reinterpret_cast<const uint4 *>(g) + idx);
@@ -69,6 +73,8 @@ __global__ void __launch_bounds__(256) gelu_bwd_kernel(const __nv_bfloat16 *__re
 // partial[b][c] = sum over the rows of block b; blocks stride over the rows
 __global__ void __launch_bounds__(256) colsum_partial_kernel(const __nv_bfloat16 *__restrict__ x, float *__restrict__ partial, size_t rows,
                                                              uint32_t C, uint32_t ld, uint32_t rows_per_block) {
+  const uint32_t after = grid_enter();
+  x += after;
   const uint32_t chunks = C / 8;                      // threads of a block: [row slots][chunks]
   const uint32_t ch = threadIdx.x % chunks, slot = threadIdx.x / chunks, slots = blockDim.x / chunks;
   __shared__ float red[256 * 8];
@@ -110,6 +116,8 @@ __global__ void __launch_bounds__(256) colsum_partial_kernel(const __nv_bfloat16
 // slices in order (fixed summation order)
 __global__ void __launch_bounds__(256) colsum_reduce_kernel(const float *__restrict__ partial, float *__restrict__ out, uint32_t blocks,
                                                             uint32_t C) {
+  const uint32_t after = grid_enter();
+  partial += after;
   __shared__ float red[8][32];
   const uint32_t tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const uint32_t c = blockIdx.x * 32 + tx;
@@ -140,7 +148,7 @@ extern "C" int f3d_swiglu_bwd_bf16(const void *pre_act, const void *grad_out, vo
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const size_t n = (size_t)rows * (F / 8);
   if ((n + 255) / 256 > 0x7FFFFFFFull) return set_error(F3D_ERR_UNSUPPORTED, "swiglu_bwd: tensor too large");
-  swiglu_bwd_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(static_cast<const __nv_bfloat16 *>(pre_act), static_cast<const __nv_bfloat16 *>(grad_out),
+  launch(swiglu_bwd_kernel, (unsigned)((n + 255) / 256), 256, 0, st, static_cast<const __nv_bfloat16 *>(pre_act), static_cast<const __nv_bfloat16 *>(grad_out),
                                                                 static_cast<__nv_bfloat16 *>(grad_pre_act), (size_t)rows, F);
   return check_launch("swiglu_bwd_bf16");
 }
@@ -157,8 +165,8 @@ extern "C" int f3d_gelu_bwd_bf16(const void *pre_act, const void *grad_out, void
   if ((n + 255) / 256 > 0x7FFFFFFFull) return set_error(F3D_ERR_UNSUPPORTED, "gelu_bwd: tensor too large");
   const unsigned grid = (unsigned)((n + 255) / 256);
   const __nv_bfloat16 *y = static_cast<const __nv_bfloat16 *>(pre_act), *g = static_cast<const __nv_bfloat16 *>(grad_out);
-  if (tanh_form) gelu_bwd_kernel<true><<<grid, 256, 0, st>>>(y, g, static_cast<__nv_bfloat16 *>(grad_pre_act), n);
-  else gelu_bwd_kernel<false><<<grid, 256, 0, st>>>(y, g, static_cast<__nv_bfloat16 *>(grad_pre_act), n);
+  if (tanh_form) launch(gelu_bwd_kernel<true>, grid, 256, 0, st, y, g, static_cast<__nv_bfloat16 *>(grad_pre_act), n);
+  else launch(gelu_bwd_kernel<false>, grid, 256, 0, st, y, g, static_cast<__nv_bfloat16 *>(grad_pre_act), n);
   return check_launch("gelu_bwd_bf16");
 }
 
@@ -180,10 +188,10 @@ extern "C" int f3d_colsum_bf16(const void *x, void *out, uint64_t rows, uint32_t
     // a block is [row slots][chunks of 8 channels]
     const uint32_t chunks = cb / 8;
     const uint32_t threads = 256 / chunks * chunks;
-    colsum_partial_kernel<<<blocks, threads, 0, st>>>(static_cast<const __nv_bfloat16 *>(x) + c0, static_cast<float *>(partial), (size_t)rows, cb, C,
+    launch(colsum_partial_kernel, blocks, threads, 0, st, static_cast<const __nv_bfloat16 *>(x) + c0, static_cast<float *>(partial), (size_t)rows, cb, C,
                                                       rows_per_block);
     F3D_TRY(check_launch("colsum_bf16"));
-    colsum_reduce_kernel<<<(cb + 31) / 32, 256, 0, st>>>(static_cast<const float *>(partial), static_cast<float *>(out) + c0, blocks, cb);
+    launch(colsum_reduce_kernel, (cb + 31) / 32, 256, 0, st, static_cast<const float *>(partial), static_cast<float *>(out) + c0, blocks, cb);
     F3D_TRY(check_launch("colsum_bf16 (reduce)"));
   }
   return F3D_OK;

@@ -93,6 +93,8 @@ struct GatherArgs {
 // ------------------------------------------------------------------------------------------- pooling forward
 template <typename T>
 __global__ void __launch_bounds__(kPoolThreads) pool_reduce_kernel(const T *__restrict__ in, T *__restrict__ out, GatherArgs a) {
+  const uint32_t after = grid_enter();
+  in += after; a.unpool_ind += after;
   constexpr int N = Chunk<T>::N;
   // A thread reduces two 16-byte chunks of the output (slots 2 * gid and 2 * gid + 1).  Members are taken two at a
   // time: the indices and then the 16-byte loads of both chunks are issued before the first value is used, so a thread
@@ -165,6 +167,8 @@ __global__ void __launch_bounds__(kPoolThreads) pool_reduce_kernel(const T *__re
 template <typename T>
 __global__ void __launch_bounds__(kPoolThreads) pool_reduce_bwd_kernel(const T *__restrict__ grad_red, const T *__restrict__ in,
                                                                        T *__restrict__ grad_in, GatherArgs a) {
+  const uint32_t after = grid_enter();
+  grad_red += after; in += after; a.unpool_ind += after;
   constexpr int N = Chunk<T>::N;
   uint64_t gid = (uint64_t)blockIdx.x * kPoolThreads + threadIdx.x;
   uint32_t row = (uint32_t)(gid / a.chunks_per_row), ch = (uint32_t)(gid % a.chunks_per_row);
@@ -217,6 +221,8 @@ template <typename T>
 __global__ void __launch_bounds__(kPoolThreads) unpool_add_kernel(const T *__restrict__ res, const T *__restrict__ down,
                                                                   T *__restrict__ up, GatherArgs a, uint32_t covered_rows,
                                                                   uint32_t up_rows, uint32_t zero_blocks) {
+  const uint32_t after = grid_enter();
+  res += after; down += after; a.unpool_ind += after;
   constexpr int N = Chunk<T>::N;
   // The blocks that clear the tail come first in the grid.  The mark of an unfilled slot (rows of the pooled input + 3) is
   // out of range for the pooling, but not for a residual padded by more than three rows: what the gather blocks store
@@ -254,6 +260,8 @@ __global__ void __launch_bounds__(kPoolThreads) unpool_add_kernel(const T *__res
 template <typename T>
 __global__ void __launch_bounds__(kPoolThreads) unpool_add_bwd_kernel(T *__restrict__ grad_res, T *__restrict__ grad_down,
                                                                       const T *__restrict__ grad_up, GatherArgs a) {
+  const uint32_t after = grid_enter();
+  grad_up += after; a.unpool_ind += after;
   constexpr int N = Chunk<T>::N;
   uint64_t gid = (uint64_t)blockIdx.x * kPoolThreads + threadIdx.x;
   uint32_t row = (uint32_t)(gid / a.chunks_per_row), ch = (uint32_t)(gid % a.chunks_per_row);
@@ -323,7 +331,7 @@ extern "C" int f3d_batch_subbuck_reduce(
   GatherArgs a{static_cast<const uint32_t *>(unpool_ind), unpool_rows, reduced_rows, total_N, feat_dim, subbuck_size, red_op,
                feat_dim * (uint32_t)esize(feat_dtype) / 16};
   if (reduced_rows > 0) {
-    F3D_DISPATCH_DT(feat_dtype, pool_reduce_kernel<T><<<(blocks_for(reduced_rows, a.chunks_per_row) + 1) / 2, kPoolThreads, 0, st>>>(
+    F3D_DISPATCH_DT(feat_dtype, launch(pool_reduce_kernel<T>, (blocks_for(reduced_rows, a.chunks_per_row) + 1) / 2, kPoolThreads, 0, st,
         static_cast<const T *>(scattered_feat), static_cast<T *>(reduced_feat), a));
   }
   F3D_TRY(check_launch("batch_subbuck_reduce"));
@@ -343,7 +351,7 @@ extern "C" int f3d_batch_subbuck_reduce_backward(
   GatherArgs a{static_cast<const uint32_t *>(unpool_ind), unpool_rows, unpool_rows, total_N, feat_dim, subbuck_size, red_op,
                feat_dim * (uint32_t)esize(feat_dtype) / 16};
   if (unpool_rows > 0) {
-    F3D_DISPATCH_DT(feat_dtype, pool_reduce_bwd_kernel<T><<<blocks_for(unpool_rows, a.chunks_per_row), kPoolThreads, 0, st>>>(
+    F3D_DISPATCH_DT(feat_dtype, launch(pool_reduce_bwd_kernel<T>, blocks_for(unpool_rows, a.chunks_per_row), kPoolThreads, 0, st,
         static_cast<const T *>(grad_red_feat), static_cast<const T *>(input_feat), static_cast<T *>(grad_input_feat), a));
   }
   F3D_TRY(check_launch("batch_subbuck_reduce_backward"));
@@ -365,7 +373,7 @@ extern "C" int f3d_additive_unpool_fwd(
   uint32_t gb = blocks_for(unpool_rows, a.chunks_per_row);
   uint32_t zb = blocks_for(up_rows - covered_rows, a.chunks_per_row);
   if (gb + zb > 0) {
-    F3D_DISPATCH_DT(feat_dtype, unpool_add_kernel<T><<<gb + zb, kPoolThreads, 0, st>>>(
+    F3D_DISPATCH_DT(feat_dtype, launch(unpool_add_kernel<T>, gb + zb, kPoolThreads, 0, st,
         static_cast<const T *>(res_feat), static_cast<const T *>(down_feat), static_cast<T *>(up_add_feat), a, covered_rows,
         up_rows, zb));
   }
@@ -384,7 +392,7 @@ extern "C" int f3d_additive_unpool_bwd(
   GatherArgs a{static_cast<const uint32_t *>(unpool_ind), unpool_rows, unpool_rows, up_rows, feat_dim, subbuck_size, 0,
                feat_dim * (uint32_t)esize(feat_dtype) / 16};
   if (unpool_rows > 0) {
-    F3D_DISPATCH_DT(feat_dtype, unpool_add_bwd_kernel<T><<<blocks_for(unpool_rows, a.chunks_per_row), kPoolThreads, 0, st>>>(
+    F3D_DISPATCH_DT(feat_dtype, launch(unpool_add_bwd_kernel<T>, blocks_for(unpool_rows, a.chunks_per_row), kPoolThreads, 0, st,
         static_cast<T *>(grad_res), static_cast<T *>(grad_down), static_cast<const T *>(grad_up_added), a));
   }
   F3D_TRY(check_launch("additive_unpool_bwd"));

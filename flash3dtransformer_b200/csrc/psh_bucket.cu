@@ -228,6 +228,7 @@ __device__ __forceinline__ void warp_prefix(const TileSmem &s, uint32_t nbp) {
 // ---------------------------------------------------------------------------------------------------------
 // K1: first-hash key of every point (kept in scratch) and the key histogram of every tile
 __global__ void __launch_bounds__(kPshThreads) psh_hist_kernel(PshArgs a) {
+  grid_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   TileSmem s = carve(smem_raw, a.nbp, 0);
   TileInfo t = tile_info(a);
@@ -299,6 +300,7 @@ __device__ __forceinline__ uint32_t scene_tiles(const PshArgs &a, uint32_t scene
 // prefixes over the scene's tiles in place (32 tiles per step, warp shuffle scan) and writes the column total.
 // which = 0: round A (totals -> count0, kept), 1: round B attempts (-> attB), 2: round C movers (-> movC).
 __global__ void __launch_bounds__(kPshThreads) psh_scan_kernel(PshArgs a, int which) {
+  grid_enter();
   const int lane = threadIdx.x & 31;
   const uint32_t col_lin = blockIdx.x * kPshWarps + (threadIdx.x >> 5);
   if (col_lin >= a.batch * a.nbp) return;
@@ -333,6 +335,7 @@ __global__ void __launch_bounds__(kPshThreads) psh_scan_kernel(PshArgs a, int wh
 // ---------------------------------------------------------------------------------------------------------
 // K3: round A ranks, overflow detection, probe walk, round B histogram
 __global__ void __launch_bounds__(kPshThreads) psh_rankA_kernel(PshArgs a) {
+  grid_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ uint32_t pending_cnt;
   TileSmem s = carve(smem_raw, a.nbp, a.tile);
@@ -500,6 +503,7 @@ __global__ void __launch_bounds__(kPshThreads) psh_rankA_kernel(PshArgs a) {
 // ---------------------------------------------------------------------------------------------------------
 // K5: resolve round B, choose round C targets, round C histogram
 __global__ void __launch_bounds__(kPshThreads) psh_resolveB_kernel(PshArgs a) {
+  grid_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ uint32_t mover_cnt;
   __shared__ uint32_t wsum[kPshWarps + 1];
@@ -642,6 +646,7 @@ __global__ void __launch_bounds__(kPshThreads) psh_resolveB_kernel(PshArgs a) {
 // ---------------------------------------------------------------------------------------------------------
 // K7: round C ranks, final (id, offset), scatter of the coordinates, tail padding (grid row y == batch)
 __global__ void __launch_bounds__(kPshThreads) psh_scatter_kernel(PshArgs a) {
+  grid_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   if (blockIdx.y == a.batch) {
     // tail rows [total_N, pad_to) take the pad value (src/psh/batch_psh_bucket.cuh:538-547)
@@ -844,12 +849,12 @@ static int psh_run(PshArgs a, const PshPlan &p, uint32_t *scratch, uint32_t max_
   // accumulated with atomics and must start at zero (they are adjacent: one memset)
   if (max_n > 0) {
     F3D_CUDA_TRY(cudaMemsetAsync(a.tabB, 0, 2 * rows * p.nbp * sizeof(uint32_t), st));
-    psh_hist_kernel<<<grid, kPshThreads, p.smem_hist, st>>>(a);
-    psh_scan_kernel<<<scan_blocks, kPshThreads, 0, st>>>(a, 0);
-    psh_rankA_kernel<<<grid, kPshThreads, p.smem_rank, st>>>(a);
-    psh_scan_kernel<<<scan_blocks, kPshThreads, 0, st>>>(a, 1);
-    psh_resolveB_kernel<<<grid, kPshThreads, p.smem_rank, st>>>(a);
-    psh_scan_kernel<<<scan_blocks, kPshThreads, 0, st>>>(a, 2);
+    launch(psh_hist_kernel, grid, kPshThreads, p.smem_hist, st, a);
+    launch(psh_scan_kernel, scan_blocks, kPshThreads, 0, st, a, 0);
+    launch(psh_rankA_kernel, grid, kPshThreads, p.smem_rank, st, a);
+    launch(psh_scan_kernel, scan_blocks, kPshThreads, 0, st, a, 1);
+    launch(psh_resolveB_kernel, grid, kPshThreads, p.smem_rank, st, a);
+    launch(psh_scan_kernel, scan_blocks, kPshThreads, 0, st, a, 2);
   } else {
     F3D_CUDA_TRY(cudaMemsetAsync(a.bucket_counter, 0, (size_t)a.batch * a.nb * 4, st));
     F3D_CUDA_TRY(cudaMemsetAsync(a.cumsum_counter, 0, (size_t)a.batch * a.nb * 4, st));
@@ -861,7 +866,7 @@ static int psh_run(PshArgs a, const PshPlan &p, uint32_t *scratch, uint32_t max_
   if (gx > 0) {
     dim3 grid2(gx, a.batch + 1);
     a.tiles_max = p.tiles_max;
-    psh_scatter_kernel<<<grid2, kPshThreads, p.smem_rank, st>>>(a);
+    launch(psh_scatter_kernel, grid2, kPshThreads, p.smem_rank, st, a);
   }
   return check_launch("psh kernels", (max_n > 0 ? 6 : 0) + (gx > 0 ? 1 : 0));
 }

@@ -21,6 +21,8 @@ __global__ void __launch_bounds__(256) scatter_index_kernel(const uint16_t *__re
                                                             const uint32_t *__restrict__ cumsum, const uint32_t *__restrict__ batch_sep,
                                                             uint32_t *__restrict__ out2in, uint32_t *__restrict__ in2out, uint32_t total_N,
                                                             uint32_t batch, uint32_t nb, uint32_t pad_to) {
+  const uint32_t after = grid_enter();
+  bucket_id += after; bucket_offset += after; cumsum += after; batch_sep += after;
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= pad_to) return;
   if (i >= total_N) { out2in[i] = total_N + 3u; return; }
@@ -43,6 +45,8 @@ constexpr int kGatherUnroll = 4;   // 16-byte chunks in flight per thread
 template <typename V>
 __global__ void __launch_bounds__(256) gather_rows_kernel(const V *__restrict__ src, const uint32_t *__restrict__ index, V *__restrict__ out,
                                                           uint64_t total, uint32_t rows_src, uint32_t vecs_per_row, int shift) {
+  const uint32_t after = grid_enter();
+  src += after; index += after;
   const uint64_t t0 = (uint64_t)blockIdx.x * (256 * kGatherUnroll) + threadIdx.x;
   V v[kGatherUnroll];
   uint32_t s[kGatherUnroll], c[kGatherUnroll];
@@ -81,7 +85,7 @@ extern "C" int f3d_scatter_index(const void *bucket_id, const void *bucket_offse
   if (pad_to_N == 0) return F3D_OK;
   DeviceGuard guard(device);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  scatter_index_kernel<<<(pad_to_N + 255) / 256, 256, 0, st>>>(static_cast<const uint16_t *>(bucket_id), static_cast<const uint32_t *>(bucket_offset),
+  launch(scatter_index_kernel, (pad_to_N + 255) / 256, 256, 0, st, static_cast<const uint16_t *>(bucket_id), static_cast<const uint32_t *>(bucket_offset),
                                                               static_cast<const uint32_t *>(cumsum_counter), static_cast<const uint32_t *>(batch_sep),
                                                               static_cast<uint32_t *>(out2in), static_cast<uint32_t *>(in2out), total_N, batch_size,
                                                               num_bucket, pad_to_N);
@@ -105,8 +109,8 @@ extern "C" int f3d_gather_rows(const void *src, const void *index, void *out, ui
   int shift = -1;
   if ((vpr & (vpr - 1)) == 0) for (shift = 0; (1u << shift) < vpr; ++shift) {}
   auto idx = static_cast<const uint32_t *>(index);
-  if (vec == 16) gather_rows_kernel<uint4><<<grid, 256, 0, st>>>(static_cast<const uint4 *>(src), idx, static_cast<uint4 *>(out), n, rows_src, vpr, shift);
-  else if (vec == 8) gather_rows_kernel<uint2><<<grid, 256, 0, st>>>(static_cast<const uint2 *>(src), idx, static_cast<uint2 *>(out), n, rows_src, vpr, shift);
-  else gather_rows_kernel<uint32_t><<<grid, 256, 0, st>>>(static_cast<const uint32_t *>(src), idx, static_cast<uint32_t *>(out), n, rows_src, vpr, shift);
+  if (vec == 16) launch(gather_rows_kernel<uint4>, grid, 256, 0, st, static_cast<const uint4 *>(src), idx, static_cast<uint4 *>(out), n, rows_src, vpr, shift);
+  else if (vec == 8) launch(gather_rows_kernel<uint2>, grid, 256, 0, st, static_cast<const uint2 *>(src), idx, static_cast<uint2 *>(out), n, rows_src, vpr, shift);
+  else launch(gather_rows_kernel<uint32_t>, grid, 256, 0, st, static_cast<const uint32_t *>(src), idx, static_cast<uint32_t *>(out), n, rows_src, vpr, shift);
   return check_launch("gather_rows");
 }

@@ -43,6 +43,7 @@ __device__ __forceinline__ float warp_max(float v) {
 }
 
 __global__ void __launch_bounds__(kSbThreads) subbuck_build_kernel(SubbuckArgs a) {
+  grid_enter();
   __shared__ uint32_t hist[kSbBins];
   __shared__ uint16_t sorted_tid[kSbThreads];
   __shared__ float sc[3][kSbThreads];
@@ -168,6 +169,7 @@ __global__ void __launch_bounds__(kSbThreads) subbuck_build_kernel(SubbuckArgs a
 
 // rows [from, to) of a [rows,3] fp16 array := 0 (alignment padding of reduced_coord)
 __global__ void zero_rows3_kernel(__half *p, uint32_t from, uint32_t to) {
+  grid_enter();
   uint64_t i = (uint64_t)from * 3 + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   if (i < (uint64_t)to * 3) p[i] = __float2half_rn(0.f);
 }
@@ -187,11 +189,11 @@ int subbuck_build(const void *coord, const void *batch_sep, const void *red_sep,
   a.red_rows = red_rows; a.red_coord_rows = red_coord_rows;
   if (max_n > 0 && batch > 0) {
     dim3 grid(cdiv_u32(max_n, kSbThreads), batch);
-    subbuck_build_kernel<<<grid, kSbThreads, 0, st>>>(a);
+    launch(subbuck_build_kernel, grid, kSbThreads, 0, st, a);
   }
   if (red_coord_rows > red_rows) {
     uint32_t cnt = (red_coord_rows - red_rows) * 3;
-    zero_rows3_kernel<<<cdiv_u32(cnt, 256), 256, 0, st>>>(a.reduced_coord, red_rows, red_coord_rows);
+    launch(zero_rows3_kernel, cdiv_u32(cnt, 256), 256, 0, st, a.reduced_coord, red_rows, red_coord_rows);
   }
   return check_launch("subbuck_build", ((max_n > 0 && batch > 0) ? 1 : 0) + (red_coord_rows > red_rows ? 1 : 0));
 }

@@ -67,6 +67,7 @@ wgrad_tcgen05_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
   __syncthreads();
   tc::tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  grid_enter();
   tc::WaitCtx wc{abort_flag, a.status};
 
   if (warp == 0) {
@@ -177,6 +178,8 @@ wgrad_tcgen05_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
 // bias sums
 __global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float *__restrict__ partial, float *__restrict__ out_w, float *__restrict__ out_b,
                                                            uint32_t slabs, size_t nw, size_t nb) {
+  const uint32_t after = grid_enter();
+  partial += after;
   // 32 x 8 threads: thread (tx, ty) adds slabs ty, ty + 8, ... of four consecutive elements, then the eight strands
   // are added in order (a fixed order, with eight loads in flight per element instead of one)
   __shared__ float4 red[8][32];
@@ -242,9 +245,9 @@ extern "C" int f3d_linear_wgrad_bf16(const void *grad_out, const void *x, void *
   const int smem = kWgStages * (2 + a.x_panels) * kWgPanelBytes + 256 + 1024;
   F3D_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(wgrad_tcgen05_kernel), device, kWgStages * 6 * kWgPanelBytes + 256 + 1024));
   dim3 grid(tiles, a.slabs);
-  wgrad_tcgen05_kernel<<<grid, kWgThreads, smem, st>>>(mg, mx, a);
+  launch(wgrad_tcgen05_kernel, grid, kWgThreads, smem, st, mg, mx, a);
   F3D_TRY(check_launch("linear_wgrad"));
-  wgrad_reduce_kernel<<<(unsigned)(((nw + nb) / 4 + 31) / 32), 256, 0, st>>>(a.partial_w, static_cast<float *>(grad_weight),
+  launch(wgrad_reduce_kernel, (unsigned)(((nw + nb) / 4 + 31) / 32), 256, 0, st, a.partial_w, static_cast<float *>(grad_weight),
                                                                                static_cast<float *>(grad_bias), (uint32_t)a.slabs, nw, nb);
   F3D_TRY(check_launch("linear_wgrad (reduce)"));
   return F3D_OK;
