@@ -41,6 +41,10 @@ namespace f3d {
 // and SwiGLU without a folded LayerNorm:
 // without the other epilogues' code a thread needs fewer registers, so 16 epilogue warps fit, and the epilogue, a chain
 // of latencies per 32-column task, is what bounds those projections.
+// A third build takes the gradient through SwiGLU: the product recomputes the pre-activation [gate | up] of a projection and
+// the epilogue turns it, with the gradient of the activation, into the gradient of [gate | up], so the pre-activation never
+// leaves the chip.
+enum GemmBuild : int { kGeneral = 0, kLean = 1, kSwigluBwd = 2 };
 constexpr int epi_warps(bool lean) { return lean ? 16 : 12; }
 constexpr int gemm_threads(bool lean) { return 64 + 32 * epi_warps(lean); }     // TMA warp, MMA warp, epilogue warps
 constexpr int BM = 128;
@@ -139,10 +143,11 @@ template <bool F16> __device__ __forceinline__ float unpack_in1(const __nv_bfloa
   return __bfloat162float(*p);
 }
 
-template <int BN, bool F16, bool LEAN>
-__global__ void __launch_bounds__(gemm_threads(LEAN), 1)
+template <int BN, bool F16, int BUILD>
+__global__ void __launch_bounds__(gemm_threads(BUILD != kGeneral), 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                          const __grid_constant__ CUtensorMap map_c, GemmArgs g) {
+  constexpr bool LEAN = BUILD != kGeneral;
   using S = GemmSmem<BN, LEAN>;
   constexpr int kEpiWarps = S::kEpiWarps, kGemmThreads = gemm_threads(LEAN);
   constexpr int kStages = S::kStages;
@@ -328,6 +333,55 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       for (int c0 = (int)((sub + kSub - task % kSub) % kSub) * 32; c0 < out_cols; c0 += 32 * (int)kSub) {
         float v[32];
         const int oc0 = (g.epilogue == EPI_SWIGLU ? n0 / 2 : n0) + c0;      // first output column of the task
+        if constexpr (BUILD == kSwigluBwd) {
+          // 16 columns at a time: gate a, up u, gradient o of the activation -> o u s (1 + a (1 - s)) and o a s, s = sigmoid(a)
+          if (tc::elect_one()) tc::tma_wait_read<0>();            // both staging buffers, one for each half of the output
+          __syncwarp();
+#pragma unroll
+          for (int hh = 0; hh < 2; ++hh) {
+            uint32_t r[16], u[16];
+            tc::tmem_ld_32x32b_x16(t_row + c0 + hh * 16, r);
+            tc::tmem_ld_32x32b_x16(t_row + BN / 2 + c0 + hh * 16, u);
+            uint4 o4[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
+            if (row < g.M) {
+              const uint4 *op = reinterpret_cast<const uint4 *>(g.residual + (size_t)row * g.ldr + oc0 + hh * 16);
+              o4[0] = __ldg(op); o4[1] = __ldg(op + 1);
+            }
+            tc::tmem_ld_wait();
+            const uint32_t *ow = reinterpret_cast<const uint32_t *>(o4);
+            const bool add_bias = g.bias && !fold_bias;
+            const float2 *pg = reinterpret_cast<const float2 *>(g.bias + oc0 + hh * 16), *pu = reinterpret_cast<const float2 *>(g.bias + g.N / 2 + oc0 + hh * 16);
+            uint32_t wg[8], wu[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              float2 a = make_float2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1]));
+              float2 b = make_float2(__uint_as_float(u[2 * e]), __uint_as_float(u[2 * e + 1]));
+              if (add_bias) {
+                const float2 ba = __ldg(pg + e), bb = __ldg(pu + e);
+                a.x += ba.x; a.y += ba.y; b.x += bb.x; b.y += bb.y;
+              }
+              const float2 o = unpack_in2<F16>(ow[e]);
+              const float s0 = __fdividef(1.f, 1.f + __expf(-a.x)), s1 = __fdividef(1.f, 1.f + __expf(-a.y));
+              const float t0 = o.x * s0, t1 = o.y * s1;
+              wg[e] = pack_out2<F16>(t0 * b.x * fmaf(a.x, 1.f - s0, 1.f), t1 * b.y * fmaf(a.y, 1.f - s1, 1.f));
+              wu[e] = pack_out2<F16>(t0 * a.x, t1 * a.y);
+            }
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+              const uint32_t at = tc::smem_u32(my_out) + lane * 64 + (((hh * 2 + j) ^ ((lane >> 1) & 3)) * 16);
+              tc::sts128(at, make_uint4(wg[4 * j], wg[4 * j + 1], wg[4 * j + 2], wg[4 * j + 3]));
+              tc::sts128(at + 32 * 64, make_uint4(wu[4 * j], wu[4 * j + 1], wu[4 * j + 2], wu[4 * j + 3]));
+            }
+          }
+          tc::fence_proxy_async();
+          __syncwarp();
+          if (tc::elect_one()) {
+            tc::tma_store_3d(&map_c, my_out, oc0, m0 + q * 32, 0);
+            tc::tma_store_3d(&map_c, my_out + 32 * 64, g.N / 2 + oc0, m0 + q * 32, 0);
+            tc::tma_commit();
+          }
+          continue;
+        }
         // runtime switches (bias, activation) are tested once per task, never per element
         if (LEAN && g.epilogue == EPI_SWIGLU) {
           // lean build: gate and up accumulators of 16 output columns at a time, so that a thread stays within the
@@ -548,10 +602,11 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
 
 int *status_word(int device);   // device word, zero until a kernel reports an abandoned wait
 
-template <int BN, bool F16, bool LEAN>
+template <int BN, bool F16, int BUILD>
 static int launch_gemm_build(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &mc, const GemmArgs &g, int device,
                              cudaStream_t st) {
-  auto kern = gemm_bf16_tcgen05_kernel<BN, F16, LEAN>;
+  constexpr bool LEAN = BUILD != kGeneral;
+  auto kern = gemm_bf16_tcgen05_kernel<BN, F16, BUILD>;
   F3D_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(kern), device, GemmSmem<BN, LEAN>::kTotal));
   int tiles = ((g.M + BM - 1) / BM) * ((g.N + BN - 1) / BN);
   int grid = tiles < sm_count(device) ? tiles : sm_count(device);
@@ -564,8 +619,8 @@ static int launch_gemm(const CUtensorMap &ma, const CUtensorMap &mb, const CUten
                        cudaStream_t st) {
   // the plain projections (bias, residual, column splits, TMA stores) take the lean build
   const bool lean = (g.epilogue == EPI_NONE || g.epilogue == EPI_SWIGLU) && !g.ln_stats && !g.stats_out && !g.direct_store;
-  if (lean) return launch_gemm_build<BN, F16, true>(ma, mb, mc, g, device, st);
-  return launch_gemm_build<BN, F16, false>(ma, mb, mc, g, device, st);
+  if (lean) return launch_gemm_build<BN, F16, kLean>(ma, mb, mc, g, device, st);
+  return launch_gemm_build<BN, F16, kGeneral>(ma, mb, mc, g, device, st);
 }
 
 struct LinearFusion {
@@ -634,9 +689,33 @@ int linear_bf16(const void *A, int lda, const void *W, int ldw, const void *bias
   }
 }
 
+// dY [M, N] = gradient of silu(gate) * up with respect to [gate | up] = A W^T + bias, for the gradient dH [M, N / 2]
+static int linear_swiglu_bwd(const void *A, const void *W, const void *bias, const void *dH, void *dY, int M, int N, int K, int device, cudaStream_t st) {
+  if (M <= 0 || N <= 0 || K <= 0 || K % 8 || N % 128) return set_error(F3D_ERR_ARG, "swiglu gradient: M, N, K = %d, %d, %d (N %% 128, K %% 8 must be 0)", M, N, K);
+  if (reinterpret_cast<uintptr_t>(dY) % 16 || reinterpret_cast<uintptr_t>(dH) % 16) return set_error(F3D_ERR_ARG, "swiglu gradient: pointers must be 16-byte aligned");
+  const int BN = N % 256 == 0 ? 256 : 128;
+  CUtensorMap ma, mb, mc;
+  F3D_TRY(encode_tmap_2d(&ma, 0, A, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, BK, BM, 128));
+  F3D_TRY(encode_tmap_2d(&mb, 0, W, (uint64_t)K, (uint64_t)N, (uint64_t)K * 2, BK, BN / 2, 128));
+  F3D_TRY(encode_tmap_3d(&mc, 0, dY, (uint64_t)N, (uint64_t)M, 1, (uint64_t)N * 2, (uint64_t)M * N * 2, 32, 32, 1, 64));
+  GemmArgs g{M, N, K, 1, N, static_cast<const float *>(bias), static_cast<const __nv_bfloat16 *>(dH), N / 2, EPI_SWIGLU, 0,
+             static_cast<__nv_bfloat16 *>(dY), (long long)M * N, status_word(device), 1, nullptr, nullptr, 0.f, 0.f, nullptr};
+  if (!g.status) return F3D_ERR_CUDA;
+  return BN == 256 ? launch_gemm_build<256, false, kSwigluBwd>(ma, mb, mc, g, device, st) : launch_gemm_build<128, false, kSwigluBwd>(ma, mb, mc, g, device, st);
+}
+
 }  // namespace f3d
 
 using namespace f3d;
+
+extern "C" int f3d_linear_swiglu_bwd_bf16(const void *A, const void *W, const void *bias, const void *grad_out, void *grad_pre_act, int M, int N, int K,
+                                          int device, void *stream) {
+  DeviceGuard guard(device);
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  F3D_TRY(maybe_sync(st, "linear_swiglu_bwd"));
+  F3D_TRY(linear_swiglu_bwd(A, W, bias, grad_out, grad_pre_act, M, N, K, device, st));
+  return maybe_sync(st, "linear_swiglu_bwd");
+}
 
 extern "C" int f3d_linear_bf16(const void *A, const void *W, const void *bias, const void *residual, void *C, int M, int N,
                                int K, int nsplit, int epilogue, int device, void *stream) {

@@ -16,10 +16,12 @@ constexpr int kLnbThreads = 256;
 
 template <int LPR, int CHUNKS>
 __global__ void __launch_bounds__(kLnbThreads) layernorm_bwd_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ g,
-                                                                    const float *__restrict__ w, __nv_bfloat16 *__restrict__ dx,
+                                                                    const float *__restrict__ w, const __nv_bfloat16 *__restrict__ add,
+                                                                    __nv_bfloat16 *__restrict__ dx,
                                                                     float *__restrict__ partial, uint32_t rows, uint32_t C, float eps) {
   const uint32_t after = grid_enter();
   x += after; g += after; w += after;
+  if (add) add += after;                                         // gradient that reaches x past the LayerNorm (the residual)
   constexpr uint32_t kRowsPerWarp = 32 / LPR;
   constexpr uint32_t kRowsPerBlock = (kLnbThreads / 32) * kRowsPerWarp;
   __shared__ float red[kLnbThreads / 32][LPR * CHUNKS * 8];      // one warp row per warp, used for dweight then dbias
@@ -93,12 +95,15 @@ __global__ void __launch_bounds__(kLnbThreads) layernorm_bwd_kernel(const __nv_b
     for (int i = 0; i < CHUNKS; ++i) {
       const uint32_t ch = sl + i * LPR;
       if (live && ch < nchunk) {
-        uint4 q;
+        uint4 q, qa = make_uint4(0u, 0u, 0u, 0u);
+        if (add) qa = __ldg(reinterpret_cast<const uint4 *>(add + (size_t)row * C) + ch);
         __nv_bfloat162 *h = reinterpret_cast<__nv_bfloat162 *>(&q);
+        const __nv_bfloat162 *ha = reinterpret_cast<const __nv_bfloat162 *>(&qa);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const float o0 = rstd * (gv[i][2 * e] * ww[i][2 * e] - m1 - xv[i][2 * e] * m2);
-          const float o1 = rstd * (gv[i][2 * e + 1] * ww[i][2 * e + 1] - m1 - xv[i][2 * e + 1] * m2);
+          float o0 = rstd * (gv[i][2 * e] * ww[i][2 * e] - m1 - xv[i][2 * e] * m2);
+          float o1 = rstd * (gv[i][2 * e + 1] * ww[i][2 * e + 1] - m1 - xv[i][2 * e + 1] * m2);
+          if (add) { const float2 f = __bfloat1622float2(ha[e]); o0 += f.x; o1 += f.y; }
           h[e] = __floats2bfloat162_rn(o0, o1);
         }
         *(reinterpret_cast<uint4 *>(dx + (size_t)row * C) + ch) = q;
@@ -158,9 +163,9 @@ __global__ void __launch_bounds__(32 * kLnbStrands) layernorm_bwd_reduce_kernel(
 }
 
 template <int LPR, int CHUNKS>
-static void launch_lnb(const __nv_bfloat16 *x, const __nv_bfloat16 *g, const float *w, __nv_bfloat16 *dx, float *partial, uint32_t rows,
+static void launch_lnb(const __nv_bfloat16 *x, const __nv_bfloat16 *g, const float *w, const __nv_bfloat16 *add, __nv_bfloat16 *dx, float *partial, uint32_t rows,
                        uint32_t C, float eps, uint32_t grid, cudaStream_t st) {
-  launch(layernorm_bwd_kernel<LPR, CHUNKS>, grid, kLnbThreads, 0, st, x, g, w, dx, partial, rows, C, eps);
+  launch(layernorm_bwd_kernel<LPR, CHUNKS>, grid, kLnbThreads, 0, st, x, g, w, add, dx, partial, rows, C, eps);
 }
 
 }  // namespace f3d
@@ -169,8 +174,14 @@ using namespace f3d;
 
 extern "C" int f3d_layernorm_bwd_bf16(const void *x, const void *grad_out, const void *weight, void *grad_x, void *grad_weight,
                                       void *grad_bias, uint32_t rows, uint32_t C, float eps, int device, void *stream) {
+  return f3d_layernorm_bwd_add_bf16(x, grad_out, weight, nullptr, grad_x, grad_weight, grad_bias, rows, C, eps, device, stream);
+}
+
+extern "C" int f3d_layernorm_bwd_add_bf16(const void *x, const void *grad_out, const void *weight, const void *grad_residual, void *grad_x,
+                                          void *grad_weight, void *grad_bias, uint32_t rows, uint32_t C, float eps, int device, void *stream) {
   if (C == 0 || C % 8 || C > 1024) return set_error(F3D_ERR_ARG, "layernorm_bwd: channel count %u must be a multiple of 8, at most 1024", C);
-  if (reinterpret_cast<uintptr_t>(x) % 16 || reinterpret_cast<uintptr_t>(grad_out) % 16 || reinterpret_cast<uintptr_t>(grad_x) % 16)
+  if (reinterpret_cast<uintptr_t>(x) % 16 || reinterpret_cast<uintptr_t>(grad_out) % 16 || reinterpret_cast<uintptr_t>(grad_x) % 16 ||
+      reinterpret_cast<uintptr_t>(grad_residual) % 16)
     return set_error(F3D_ERR_ARG, "layernorm_bwd: pointers must be 16-byte aligned");
   DeviceGuard guard(device);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
@@ -190,21 +201,22 @@ extern "C" int f3d_layernorm_bwd_bf16(const void *x, const void *grad_out, const
   F3D_TRY(workspace(device, 3, (size_t)grid * 2 * C * sizeof(float), st, &partial));
   auto xp = static_cast<const __nv_bfloat16 *>(x), gp = static_cast<const __nv_bfloat16 *>(grad_out);
   auto dxp = static_cast<__nv_bfloat16 *>(grad_x);
+  auto ap = static_cast<const __nv_bfloat16 *>(grad_residual);
   auto wp = static_cast<const float *>(weight);
   auto pp = static_cast<float *>(partial);
   if (lpr < 32) {
     switch (lpr) {
-      case 1: launch_lnb<1, 1>(xp, gp, wp, dxp, pp, rows, C, eps, grid, st); break;
-      case 2: launch_lnb<2, 1>(xp, gp, wp, dxp, pp, rows, C, eps, grid, st); break;
-      case 4: launch_lnb<4, 1>(xp, gp, wp, dxp, pp, rows, C, eps, grid, st); break;
-      case 8: launch_lnb<8, 1>(xp, gp, wp, dxp, pp, rows, C, eps, grid, st); break;
-      default: launch_lnb<16, 1>(xp, gp, wp, dxp, pp, rows, C, eps, grid, st); break;
+      case 1: launch_lnb<1, 1>(xp, gp, wp, ap, dxp, pp, rows, C, eps, grid, st); break;
+      case 2: launch_lnb<2, 1>(xp, gp, wp, ap, dxp, pp, rows, C, eps, grid, st); break;
+      case 4: launch_lnb<4, 1>(xp, gp, wp, ap, dxp, pp, rows, C, eps, grid, st); break;
+      case 8: launch_lnb<8, 1>(xp, gp, wp, ap, dxp, pp, rows, C, eps, grid, st); break;
+      default: launch_lnb<16, 1>(xp, gp, wp, ap, dxp, pp, rows, C, eps, grid, st); break;
     }
   } else {
     switch (chunks) {
-      case 1: launch_lnb<32, 1>(xp, gp, wp, dxp, pp, rows, C, eps, grid, st); break;
-      case 2: launch_lnb<32, 2>(xp, gp, wp, dxp, pp, rows, C, eps, grid, st); break;
-      default: launch_lnb<32, 4>(xp, gp, wp, dxp, pp, rows, C, eps, grid, st); break;
+      case 1: launch_lnb<32, 1>(xp, gp, wp, ap, dxp, pp, rows, C, eps, grid, st); break;
+      case 2: launch_lnb<32, 2>(xp, gp, wp, ap, dxp, pp, rows, C, eps, grid, st); break;
+      default: launch_lnb<32, 4>(xp, gp, wp, ap, dxp, pp, rows, C, eps, grid, st); break;
     }
   }
   F3D_TRY(check_launch("layernorm_bwd_bf16"));

@@ -37,6 +37,22 @@ def bf16_weight(p: torch.Tensor) -> torch.Tensor:
     return w
 
 
+_BF16T_CACHE = {}
+
+
+def bf16_weight_t(p: torch.Tensor, parts: int = 1) -> torch.Tensor:
+    """bf16 transpose of a parameter [N, K] (of each of `parts` equal slices of its rows: [parts, K, N / parts]), the operand of
+    the input gradient; refreshed like bf16_weight."""
+    key = (id(p), parts)
+    hit = _BF16T_CACHE.get(key)
+    if hit is not None and hit[0] == p._version and hit[1].device == p.device and hit[2]() is p:
+        return hit[1]
+    w = bf16_weight(p)
+    t = w.view(parts, w.shape[0] // parts, w.shape[1]).transpose(1, 2).contiguous() if parts > 1 else w.t().contiguous()
+    _BF16T_CACHE[key] = (p._version, t, _forget(_BF16T_CACHE, key, p))
+    return t
+
+
 def _fp32_param(p: torch.Tensor) -> torch.Tensor:
     """fp32 contiguous view of a parameter (the parameter itself when it already is one)."""
     d = p.detach()
@@ -127,12 +143,25 @@ class CoordEmbedFn(Function):
 _WGRAD_MAX_ELEMS = 512 * 1024
 
 
+def native_wgrad(n: int, k: int) -> bool:
+    """Whether the gradient of a weight [n, k] goes to the native kernel."""
+    return pshattn.wgrad_supported(n, k) and n * k <= _WGRAD_MAX_ELEMS
+
+
+def param_grads_into(g, xb, gw, gb):
+    """The library's product and the native column sums, for weights that native_wgrad turns away: gw fp32 [N, K] = g^T xb and
+    gb fp32 [N] (or None) = column sums of g."""
+    gw.copy_(g.t() @ xb)
+    if gb is not None:
+        pshattn.colsum_bf16(g, gb)
+
+
 def _param_grads(g, xb, weight, bias):
     """(grad_weight, grad_bias) of y = x W^T + b for the bf16 gradient g [M, N] and input xb [M, K]: one native pass
     over both (fp32 results, fixed summation order) for the shapes it takes, else a library GEMM plus the native
     column sums."""
     n, k = g.shape[1], xb.shape[1]
-    if g.dtype == torch.bfloat16 and pshattn.wgrad_supported(n, k) and n * k <= _WGRAD_MAX_ELEMS:
+    if g.dtype == torch.bfloat16 and native_wgrad(n, k):
         gw = torch.empty(n, k, dtype=torch.float32, device=g.device)
         gb = torch.empty(n, dtype=torch.float32, device=g.device) if bias is not None else None
         pshattn.linear_wgrad_bf16(g, xb, gw, gb)
@@ -196,11 +225,9 @@ class LinearFn(Function):
         g = g.contiguous()
         g_res = g if has_res else None
         if epilogue == pshattn.EPI_SWIGLU:
-            # the pre-activation [gate | up] is recomputed on the native GEMM, its gradient by one fused kernel
-            y = torch.empty(xb.shape[0], wb.shape[0], dtype=torch.bfloat16, device=xb.device)
-            pshattn.linear_bf16(xb, wb, _fp32_bias(bias), y)
-            gy = torch.empty_like(y)
-            pshattn.swiglu_bwd_bf16(y, g if g.dtype == torch.bfloat16 else g.to(torch.bfloat16), gy)
+            # the pre-activation [gate | up] is recomputed, and its gradient taken, inside one product
+            gy = torch.empty(xb.shape[0], wb.shape[0], dtype=torch.bfloat16, device=xb.device)
+            pshattn.linear_swiglu_bwd_bf16(xb, wb, _fp32_bias(bias), g if g.dtype == torch.bfloat16 else g.to(torch.bfloat16), gy)
             g = gy
         elif epilogue == pshattn.EPI_GELU:
             # the same for the tanh-form GELU epilogue
@@ -209,9 +236,9 @@ class LinearFn(Function):
             gy = torch.empty_like(y)
             pshattn.gelu_bwd_bf16(y, g if g.dtype == torch.bfloat16 else g.to(torch.bfloat16), gy, tanh_form=True)
             g = gy
-        # gx = g W: the native GEMM computes A B^T, so W^T ([in, out], a small matrix) is materialised
+        # gx = g W: the native GEMM computes A B^T, so it takes W^T ([in, out], a small matrix)
         gx = torch.empty(g.shape[0], wb.shape[1], dtype=torch.bfloat16, device=g.device)
-        pshattn.linear_bf16(g, wb.t().contiguous(), None, gx)
+        pshattn.linear_bf16(g, bf16_weight_t(weight), None, gx)
         gw, gb = _param_grads(g, xb, weight, bias)
         return gx, gw, gb, g_res, None, None
 
@@ -220,7 +247,7 @@ def _split_backward(xb, weight, bias, wb, g):
     """Backward of a projection whose output is nsplit separate matrices: g is the packed gradient [S, M, C]."""
     s, m, c = g.shape
     # grad_x = sum_s g[s] W_s as one GEMM over the slices; W_s^T ([in, C] per slice) is a small matrix
-    wt = wb.view(s, c, wb.shape[1]).transpose(1, 2).contiguous()
+    wt = bf16_weight_t(weight, s)
     gx = torch.empty(m, wb.shape[1], dtype=torch.bfloat16, device=g.device)
     pshattn.linear_ksplit_bf16(g, wt, gx)
     parts = [_param_grads(g[i], xb, weight, bias[i * c:(i + 1) * c] if bias is not None else None) for i in range(s)]

@@ -12,6 +12,7 @@ from typing import List
 import torch
 import torch.cuda.nvtx as nvtx
 from torch import nn
+from torch.autograd import Function
 from torch.nn.modules import module as nn_module
 
 from . import buck_swin, elem_wise
@@ -53,7 +54,10 @@ class XFMR(nn.Module):
         if f3ddev.get_nvtx():
             nvtx.range_push(self.NVTX_SCOPE)
         feat = reduced_feat if reduced_feat.dtype == torch.bfloat16 else reduced_feat.to(torch.bfloat16)
-        if self._can_fold(feat):
+        params = self._trainable(feat)
+        if params is not None:
+            out = XfmrBlockFunction.apply(feat, self, scope_bucks, *params)
+        elif self._can_fold(feat):
             out = self._forward_folded(feat, reduced_feat, scope_bucks, n, c)
         else:
             x = F3.apply_norm(self.norm, feat)
@@ -62,6 +66,20 @@ class XFMR(nn.Module):
         if f3ddev.get_nvtx():
             nvtx.range_pop()
         return out
+
+    def _trainable(self, feat):
+        """The block's parameters when autograd can take the block as one node (XfmrBlockFunction), else None."""
+        if not BlockStack.ENABLED or not torch.is_grad_enabled() or not feat.is_cuda or f3ddev.get_nvtx() or nn_module._has_any_global_hook():
+            return None
+        n, c = feat.shape
+        ps = _plain_block(self)
+        if ps is None or n == 0 or any(ps[i] is None for i in (0, 1, 2, 4, 6, 7, 8, 10)):
+            return None
+        f = ps[10].shape[1]
+        if ((c != 32 and c % 64) or c > 1024 or f % 64 or tuple(self.norm.normalized_shape) != (c,) or self.bwa.head_dim not in (16, 32, 64, 128)
+                or ps[8].shape[0] != 2 * f or any(p is not None and (p.device != feat.device or p.dtype != torch.float32) for p in ps)):
+            return None
+        return ps
 
     # Narrowest block that takes the folded path.  Measured per block on 16 x 120k points (LayerNorm kernels + four
     # GEMMs against four fused GEMMs): C = 32 / 64 / 128 lose 57 / 32 / 9 us (their epilogues are bound by instruction
@@ -120,27 +138,17 @@ class BlockStack:
         the plain one."""
         key, params = [], []
         for b in blocks:
-            if type(b) is not XFMR:
+            if type(b) is not XFMR or b._forward_hooks or b._forward_pre_hooks:
                 return None, None
-            m = b._modules
-            norm, bwa, mlp = m["norm"], m["bwa"], m["mlp"]
-            if type(norm) is not nn.LayerNorm or type(bwa) is not buck_swin.BucketSwinAttentionModule or type(mlp) is not elem_wise.MLP:
+            ps = _plain_block(b)
+            if ps is None:
                 return None, None
-            qkv, proj, inner = bwa._modules["qkv"], bwa._modules["proj"], mlp._modules["mlp"]
-            if type(inner) is not elem_wise.LayerNormMLP or inner.activation != "swiglu" or type(qkv) is not nn.Linear or type(proj) is not nn.Linear:
-                return None, None
-            for mod in (b, bwa, mlp, inner):
-                if mod._forward_hooks or mod._forward_pre_hooks:
-                    return None, None
-            n, q, o, i = norm._parameters, qkv._parameters, proj._parameters, inner._parameters
-            ps = (n["weight"], n["bias"], q["weight"], q["bias"], o["weight"], o["bias"], i["layer_norm_weight"], i["layer_norm_bias"],
-                  i["fc1_weight"], i["fc1_bias"], i["fc2_weight"], i["fc2_bias"])
             for p in ps:
                 if p is None:
                     key.append(None)
                 else:
                     key += (id(p), p._version, p.data_ptr())
-            key += (id(b.swin_plan), norm.eps, inner.eps, bwa.num_heads, bwa.attn.buck_size)
+            key += (id(b.swin_plan), b.norm.eps, b.mlp.mlp.eps, b.bwa.num_heads, b.bwa.attn.buck_size)
             params.append(ps)
         return key, params
 
@@ -205,6 +213,112 @@ class BlockStack:
                                               plan[1], n, c, x.get_device(), pshattn._stream(x.get_device()))
         _cabi.check(st, "xfmr_stack")
         return out
+
+
+def _plain_block(b):
+    """The parameters of a block whose forward is all there is to it (the layer types of this package, no hooks inside), else
+    None."""
+    m = b._modules
+    norm, bwa, mlp = m["norm"], m["bwa"], m["mlp"]
+    if type(norm) is not nn.LayerNorm or type(bwa) is not buck_swin.BucketSwinAttentionModule or type(mlp) is not elem_wise.MLP:
+        return None
+    qkv, proj, inner = bwa._modules["qkv"], bwa._modules["proj"], mlp._modules["mlp"]
+    if type(inner) is not elem_wise.LayerNormMLP or inner.activation != "swiglu" or type(qkv) is not nn.Linear or type(proj) is not nn.Linear:
+        return None
+    for mod in (norm, bwa, bwa._modules["attn"], qkv, proj, mlp, inner):
+        if mod._forward_hooks or mod._forward_pre_hooks or mod._backward_hooks or mod._backward_pre_hooks:
+            return None
+    n, q, o, i = norm._parameters, qkv._parameters, proj._parameters, inner._parameters
+    return (n["weight"], n["bias"], q["weight"], q["bias"], o["weight"], o["bias"], i["layer_norm_weight"], i["layer_norm_bias"],
+            i["fc1_weight"], i["fc1_bias"], i["fc2_weight"], i["fc2_bias"])
+
+
+class XfmrBlockFunction(Function):
+    """A whole block as one autograd node: forward and backward are one native call each (f3d_xfmr_block_fwd_bf16,
+    f3d_xfmr_block_bwd_bf16).  The same kernels as layer by layer, except that the residual gradients are added in fp32 inside
+    the LayerNorm gradients and the pre-activation of the MLP is never stored."""
+
+    @staticmethod
+    def forward(ctx, x, block, scopes, *params):
+        nw, nb, qw, qb, ow, ob, lw, lb, w1, b1, w2, b2 = params
+        xb = (x if x.dtype == torch.bfloat16 else x.to(torch.bfloat16)).contiguous()
+        n, c = xb.shape
+        h, f, dev = block.bwa.num_heads, w2.shape[1], xb.device
+        # n1, attn, mid, n2 | qkv | hid of one allocation: they live and die together
+        buf = torch.empty(n * (7 * c + f), dtype=torch.bfloat16, device=dev)
+        row = n * c
+        n1, attn, mid, n2 = (buf[i * row:(i + 1) * row].view(n, c) for i in range(4))
+        qkv, hid = buf[4 * row:7 * row].view(3, n, c), buf[7 * row:].view(n, f)
+        lse = torch.empty(n, h, dtype=torch.float32, device=dev)
+        out = torch.empty_like(xb)
+        a, keep = XfmrBlockFunction._block(block, scopes, params)
+        t = _cabi.XfmrSaved(xb.data_ptr(), n1.data_ptr(), qkv.data_ptr(), attn.data_ptr(), lse.data_ptr(), mid.data_ptr(), n2.data_ptr(),
+                            hid.data_ptr(), out.data_ptr())
+        st = _cabi.load().f3d_xfmr_block_fwd_bf16(a, t, n, c, x.get_device(), pshattn._stream(x.get_device()))
+        _cabi.check(st, "xfmr_block_fwd")
+        ctx.save_for_backward(xb, buf, lse, *params)
+        ctx.cfg = (block, scopes)
+        return out
+
+    @staticmethod
+    def _block(block, scopes, params):
+        """The native description of the block, and the tensors its pointers need kept alive."""
+        nw, nb, qw, qb, ow, ob, lw, lb, w1, b1, w2, b2 = params
+        keep = [F3._fp32_param(nw), F3._fp32_param(nb), F3.bf16_weight(qw), F3._fp32_bias(qb), F3.bf16_weight(ow), F3._fp32_bias(ob),
+                F3._fp32_param(lw), F3._fp32_param(lb), F3.bf16_weight(w1), F3._fp32_bias(b1), F3.bf16_weight(w2), F3._fp32_bias(b2)]
+        a = _cabi.XfmrBlock(*[None if t is None else t.data_ptr() for t in keep], None, None, scopes.data_ptr(), block.norm.eps,
+                            block.mlp.mlp.eps, block.bwa.num_heads, w2.shape[1], scopes.shape[0], scopes.shape[1], block.bwa.attn.buck_size)
+        return a, keep
+
+    @staticmethod
+    def backward(ctx, g):
+        xb, buf, lse, *params = ctx.saved_tensors
+        block, scopes = ctx.cfg
+        nw, nb, qw, qb, ow, ob, lw, lb, w1, b1, w2, b2 = params
+        n, c = xb.shape
+        h, f, dev = block.bwa.num_heads, w2.shape[1], xb.device
+        g = (g if g.dtype == torch.bfloat16 else g.to(torch.bfloat16)).contiguous()
+        row = n * c
+        p0 = buf.data_ptr()
+        t = _cabi.XfmrSaved(xb.data_ptr(), p0, p0 + 8 * row, p0 + 2 * row, lse.data_ptr(), p0 + 4 * row, p0 + 6 * row, p0 + 14 * row, None)
+        a, keep = XfmrBlockFunction._block(block, scopes, params)
+        wt = (F3.bf16_weight_t(qw, 3), F3.bf16_weight_t(ow), F3.bf16_weight_t(w1), F3.bf16_weight_t(w2))
+        # g_mid | g_qkv | g_pre, then the fp32 parameter gradients in one buffer each
+        gbuf = torch.empty(n * (4 * c + 2 * f), dtype=torch.bfloat16, device=dev)
+        gx = torch.empty_like(xb)
+        flat = torch.empty(sum(p.numel() for p in params if p is not None), dtype=torch.float32, device=dev)
+        grads, at = [], 0
+        for p in params:
+            if p is None:
+                grads.append(None)
+            else:
+                grads.append(flat[at:at + p.numel()].view(p.shape))
+                at += p.numel()
+        q0, f0 = gbuf.data_ptr(), flat.data_ptr()
+        # weights past the native kernel's limit take a library product from the same gradients
+        native = [F3.native_wgrad(w.shape[0] // s, w.shape[1]) for w, s in ((qw, 3), (ow, 1), (w1, 1), (w2, 1))]
+        ptr = [None if t is None else t.data_ptr() for t in grads]
+        for i, ok in zip((2, 4, 8, 10), native):
+            if not ok:
+                ptr[i] = ptr[i + 1] = None
+        gr = _cabi.XfmrGrads(*[w.data_ptr() for w in wt], *ptr, gx.data_ptr(), q0 + 8 * row, q0, q0 + 2 * row,
+                             int(getattr(scopes, "_f3d_partition_of", -1) == n))
+        lib = _cabi.load()
+        size = int(lib.f3d_xfmr_block_bwd_scratch(n, c, f, h))
+        scratch = torch.empty(size, dtype=torch.uint8, device=dev)
+        st = lib.f3d_xfmr_block_bwd_bf16(a, t, gr, g.data_ptr(), scratch.data_ptr(), size, n, c, g.get_device(), pshattn._stream(g.get_device()))
+        _cabi.check(st, "xfmr_block_bwd")
+        if not all(native):
+            n1, attn, n2, hid = buf[:row].view(n, c), buf[row:2 * row].view(n, c), buf[3 * row:4 * row].view(n, c), buf[7 * row:].view(n, f)
+            g_mid, g_qkv, g_pre = gbuf[:row].view(n, c), gbuf[row:4 * row].view(3, n, c), gbuf[4 * row:].view(n, 2 * f)
+            if not native[0]:
+                for i in range(3):
+                    F3.param_grads_into(g_qkv[i], n1, grads[2][i * c:(i + 1) * c], None if qb is None else grads[3][i * c:(i + 1) * c])
+            for ok, gg, xx, i in ((native[1], g_mid, attn, 4), (native[2], g_pre, n2, 8), (native[3], g, hid, 10)):
+                if not ok:
+                    F3.param_grads_into(gg, xx, grads[i], grads[i + 1])
+        grads = [None if t is None else t.to(p.dtype) for t, p in zip(grads, params)]
+        return (gx, None, None, *grads)
 
 
 class Stage(nn.Module):

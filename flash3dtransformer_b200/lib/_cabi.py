@@ -22,6 +22,18 @@ class XfmrBlock(ctypes.Structure):
                 (n, c_int) for n in ("heads", "hidden", "num_scopes", "scope_size", "bucket")]
 
 
+class XfmrSaved(ctypes.Structure):
+    """f3d_xfmr_saved of include/f3d_b200.h."""
+    _fields_ = [(n, c_void_p) for n in ("x", "n1", "qkv", "attn", "lse", "mid", "n2", "hid", "out")]
+
+
+class XfmrGrads(ctypes.Structure):
+    """f3d_xfmr_grads of include/f3d_b200.h."""
+    _fields_ = [(n, c_void_p) for n in ("qkv_wt", "proj_wt", "fc1_wt", "fc2_wt", "norm_w", "norm_b", "qkv_w", "qkv_b", "proj_w", "proj_b",
+                                        "ln2_w", "ln2_b", "fc1_w", "fc1_b", "fc2_w", "fc2_b", "grad_x", "g_pre", "g_mid", "g_qkv")] + [
+                ("covered", c_int)]
+
+
 # name -> (restype, argtypes); mirrors include/f3d_b200.h declaration by declaration
 PROTOTYPES = {
     "f3d_last_error": (c_char_p, []),
@@ -55,6 +67,12 @@ PROTOTYPES = {
     "f3d_row_stats_bf16": (_int, [_vp, _vp, _u32, _u32, _int, _vp]),
     "f3d_xfmr_stack_bf16": (_int, [ctypes.POINTER(XfmrBlock), _int, _vp, _vp, _vp, _vp, c_uint64, _u32, _u32, _int, _vp]),
     "f3d_xfmr_stack_scratch": (c_uint64, [_u32, _u32, _u32]),
+    "f3d_xfmr_block_fwd_bf16": (_int, [ctypes.POINTER(XfmrBlock), ctypes.POINTER(XfmrSaved), _u32, _u32, _int, _vp]),
+    "f3d_xfmr_block_bwd_bf16": (_int, [ctypes.POINTER(XfmrBlock), ctypes.POINTER(XfmrSaved), ctypes.POINTER(XfmrGrads), _vp, _vp, c_uint64, _u32,
+                                       _u32, _int, _vp]),
+    "f3d_xfmr_block_bwd_scratch": (c_uint64, [_u32, _u32, _u32, _u32]),
+    "f3d_linear_swiglu_bwd_bf16": (_int, [_vp, _vp, _vp, _vp, _vp, _int, _int, _int, _int, _vp]),
+    "f3d_layernorm_bwd_add_bf16": (_int, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _u32, _u32, _f32, _int, _vp]),
     "f3d_gemm_sm_bf16": (_int, [_vp, _vp, _vp, _int, _int, _int, _int, _vp]),
     "f3d_buck_swin_fwd": (_int, [_vp, _vp, _vp, _vp, _vp, _vp, _int, _int, _int, _int, _int, _int, _u32, _int, _vp]),
     "f3d_layernorm_bf16": (_int, [_vp, _vp, _vp, _vp, _u32, _u32, _f32, _int, _int, _vp]),

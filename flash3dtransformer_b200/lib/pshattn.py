@@ -566,9 +566,9 @@ def layernorm_bf16(x, weight, bias, out, eps=1e-5, gelu=False) -> None:
     _cabi.check(st, "layernorm_bf16")
 
 
-def layernorm_bwd_bf16(x, grad_out, weight, grad_x, grad_weight, grad_bias, eps=1e-5) -> None:
+def layernorm_bwd_bf16(x, grad_out, weight, grad_x, grad_weight, grad_bias, eps=1e-5, grad_residual=None) -> None:
     """Backward of layernorm_bf16 (without GELU): x, grad_out, grad_x bf16 [rows, C]; weight, grad_weight, grad_bias
-    fp32 [C].  Not part of the reference's operator module (its LayerNorm backward comes from TransformerEngine)."""
+    fp32 [C]; grad_residual bf16 [rows, C], the gradient that reaches x past the LayerNorm, is added to grad_x.  Not part of the reference's operator module (its LayerNorm backward comes from TransformerEngine)."""
     dev = _check_tensors([x, grad_out, weight, grad_x, grad_weight, grad_bias], ["x", "grad_out", "weight", "grad_x", "grad_weight", "grad_bias"])
     _check_dtype([x, grad_out, grad_x], ["x", "grad_out", "grad_x"], torch.bfloat16)
     _check_dtype([weight, grad_weight, grad_bias], ["weight", "grad_weight", "grad_bias"], torch.float32)
@@ -576,8 +576,13 @@ def layernorm_bwd_bf16(x, grad_out, weight, grad_x, grad_weight, grad_bias, eps=
         raise RuntimeError("x, grad_out and grad_x must be [rows, C] of equal shape")
     if not (weight.numel() == x.shape[1] == grad_weight.numel() == grad_bias.numel()):
         raise RuntimeError("weight, grad_weight, grad_bias must be [C]")
-    st = _cabi.load().f3d_layernorm_bwd_bf16(_ptr(x), _ptr(grad_out), _ptr(weight), _ptr(grad_x), _ptr(grad_weight), _ptr(grad_bias),
-                                             x.shape[0], x.shape[1], float(eps), dev, _stream(dev))
+    if grad_residual is not None:
+        _check_tensors([x, grad_residual], ["x", "grad_residual"])
+        _check_dtype([grad_residual], ["grad_residual"], torch.bfloat16)
+        if grad_residual.shape != x.shape:
+            raise RuntimeError("grad_residual must have the shape of x")
+    st = _cabi.load().f3d_layernorm_bwd_add_bf16(_ptr(x), _ptr(grad_out), _ptr(weight), _ptr(grad_residual) if grad_residual is not None else None,
+                                             _ptr(grad_x), _ptr(grad_weight), _ptr(grad_bias), x.shape[0], x.shape[1], float(eps), dev, _stream(dev))
     _cabi.check(st, "layernorm_bwd_bf16")
 
 
@@ -593,6 +598,26 @@ def swiglu_bwd_bf16(pre_act, grad_out, grad_pre_act) -> None:
     st = _cabi.load().f3d_swiglu_bwd_bf16(_ptr(pre_act), _ptr(grad_out), _ptr(grad_pre_act), pre_act.shape[0], grad_out.shape[1],
                                           dev, _stream(dev))
     _cabi.check(st, "swiglu_bwd_bf16")
+
+
+def linear_swiglu_bwd_bf16(x, weight, bias, grad_out, grad_pre_act) -> None:
+    """grad_pre_act bf16 [M, 2F] = gradient of silu(gate) * up with respect to [gate | up] = x weight^T + bias for grad_out
+    bf16 [M, F]: linear_bf16 followed by swiglu_bwd_bf16 without the pre-activation in between.  x bf16 [M, K], weight bf16
+    [2F, K], bias fp32 [2F] or None."""
+    dev = _check_tensors([x, weight, grad_out, grad_pre_act], ["x", "weight", "grad_out", "grad_pre_act"])
+    _check_dtype([x, weight, grad_out, grad_pre_act], ["x", "weight", "grad_out", "grad_pre_act"], torch.bfloat16)
+    m, k = x.shape
+    n = weight.shape[0]
+    if weight.shape[1] != k or tuple(grad_out.shape) != (m, n // 2) or tuple(grad_pre_act.shape) != (m, n):
+        raise RuntimeError(f"weight must be [2F,{k}], grad_out [{m}, F] and grad_pre_act [{m}, 2F]")
+    if bias is not None:
+        _check_tensors([x, bias], ["x", "bias"])
+        _check_dtype([bias], ["bias"], torch.float32)
+        if bias.numel() != n:
+            raise RuntimeError(f"bias must have {n} elements")
+    st = _cabi.load().f3d_linear_swiglu_bwd_bf16(_ptr(x), _ptr(weight), _ptr(bias) if bias is not None else None, _ptr(grad_out),
+                                                 _ptr(grad_pre_act), m, n, k, dev, _stream(dev))
+    _cabi.check(st, "linear_swiglu_bwd_bf16")
 
 
 def gelu_bwd_bf16(pre_act, grad_out, grad_pre_act, tanh_form: bool = False) -> None:

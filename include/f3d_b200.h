@@ -239,6 +239,35 @@ int f3d_linear_fused(const void *A, const void *W, const void *bias, const void 
  * of f3d_linear_fused for rows that no GEMM of this library produced.  C a multiple of 8, <= 2048. */
 int f3d_row_stats_bf16(const void *x, void *stats, uint32_t rows, uint32_t C, int device, void *stream);
 
+/* grad_pre_act [M, N] = gradient of silu(gate) * up with respect to [gate | up] = A W^T + bias (fp32 [N] or NULL) for
+ * grad_out [M, N / 2]; bf16, the pre-activation is recomputed inside the product.  N a multiple of 128, K of 8. */
+int f3d_linear_swiglu_bwd_bf16(const void *A, const void *W, const void *bias, const void *grad_out, void *grad_pre_act, int M, int N,
+                               int K, int device, void *stream);
+
+/* f3d_layernorm_bwd_bf16 with grad_residual bf16 [rows, C] (or NULL) added to grad_x: the gradient that reaches x past the
+ * LayerNorm */
+int f3d_layernorm_bwd_add_bf16(const void *x, const void *grad_out, const void *weight, const void *grad_residual, void *grad_x,
+                               void *grad_weight, void *grad_bias, uint32_t rows, uint32_t C, float eps, int device, void *stream);
+
+/* What a block (see f3d_xfmr_block below) keeps between its forward and its backward pass, all of [rows, ...]: bf16 x, n1, mid,
+ * n2, out [C], qkv [3][rows][C], attn [C], hid [hidden]; fp32 lse [heads]. */
+typedef struct f3d_xfmr_saved {
+  const void *x;
+  void *n1, *qkv, *attn, *lse, *mid, *n2, *hid, *out;
+} f3d_xfmr_saved;
+
+/* Inputs and outputs of a block's backward pass beside its grad_out: bf16 transposed weights (qkv_wt [3][C][C]: the transpose of
+ * each third; proj_wt [C][C]; fc1_wt [C][2 hidden]; fc2_wt [hidden][C]), fp32 parameter gradients (a NULL weight gradient is
+ * left out; the biases' are then left out with it), bf16 grad_x [rows, C], and the gradients that a caller needs to compute a
+ * left-out weight gradient itself: g_pre [rows, 2 hidden] (fc1), g_mid [rows, C] (proj), g_qkv [3][rows][C].  covered: every
+ * bucket is listed by a scope. */
+typedef struct f3d_xfmr_grads {
+  const void *qkv_wt, *proj_wt, *fc1_wt, *fc2_wt;
+  void *norm_w, *norm_b, *qkv_w, *qkv_b, *proj_w, *proj_b, *ln2_w, *ln2_b, *fc1_w, *fc1_b, *fc2_w, *fc2_b;
+  void *grad_x, *g_pre, *g_mid, *g_qkv;
+  int covered;
+} f3d_xfmr_grads;
+
 /* One transformer block of f3d_xfmr_stack_bf16 (the reference's XFMR, flash3dxfmr/layers/stage.py:90-101): weights bf16
  * [out, in], biases, LayerNorm parameters and column sums fp32.  With qkv_colsum and fc1_colsum (both or neither) the two
  * LayerNorms are folded into the projections behind them as in f3d_linear_fused (qkv_w / fc1_w then hold the scaled weights,
@@ -254,6 +283,12 @@ typedef struct f3d_xfmr_block {
  * issued by one call.  lse: fp32 [rows, most heads of a block], overwritten; scratch: at least f3d_xfmr_stack_scratch bytes of device memory, 256-byte aligned. */
 int f3d_xfmr_stack_bf16(const f3d_xfmr_block *blocks, int count, const void *x, void *out, void *lse,
                         void *scratch, uint64_t scratch_bytes, uint32_t rows, uint32_t channels, int device, void *stream);
+/* forward pass of one block (without folded LayerNorms) that keeps what its backward pass reads */
+int f3d_xfmr_block_fwd_bf16(const f3d_xfmr_block *block, const f3d_xfmr_saved *t, uint32_t rows, uint32_t channels, int device, void *stream);
+/* its backward pass; scratch as f3d_xfmr_block_bwd_scratch says */
+int f3d_xfmr_block_bwd_bf16(const f3d_xfmr_block *block, const f3d_xfmr_saved *t, const f3d_xfmr_grads *g, const void *grad_out, void *scratch,
+                            uint64_t scratch_bytes, uint32_t rows, uint32_t channels, int device, void *stream);
+uint64_t f3d_xfmr_block_bwd_scratch(uint32_t rows, uint32_t channels, uint32_t hidden, uint32_t heads);
 /* scratch bytes for the widest hidden layer among the blocks */
 uint64_t f3d_xfmr_stack_scratch(uint32_t rows, uint32_t channels, uint32_t hidden);
 

@@ -63,3 +63,29 @@ def test_follows_parameters_modules_and_hooks(cuda_device):
     y = stage(None, x.float().requires_grad_(True), None)             # autograd: block by block
     y.float().sum().backward()
     assert stage.encoder_blocks[0].norm.weight.grad is not None
+
+
+@pytest.mark.parametrize("c,rows,hd", [(32, 512, 16), (32, 4096, 32), (64, 4608, 32), (256, 1024, 32), (512, 1024, 64)])
+def test_block_as_one_autograd_node(cuda_device, c, rows, hd):
+    """Output and every gradient of the native block against the layers taken one by one (c = 512: weights past the native
+    weight gradient's limit)."""
+    from flash3dtransformer_b200.layers import stage as st
+    stage = _stage(cuda_device, c, 1, hd)
+    block = stage.encoder_blocks[0]
+    x = torch.randn(rows, c, device=cuda_device).bfloat16()
+    g = torch.randn(rows, c, device=cuda_device).bfloat16()
+    got = []
+    for native in (True, False):
+        st.BlockStack.ENABLED = native
+        try:
+            block.zero_grad()
+            xx = x.clone().requires_grad_(True)
+            out = block(None, xx, None)
+            assert (type(out.grad_fn).__name__ == "XfmrBlockFunctionBackward") == native
+            out.backward(g)
+        finally:
+            st.BlockStack.ENABLED = True
+        got.append([out.detach(), xx.grad] + [p.grad for p in block.parameters()])
+    assert torch.equal(got[0][0], got[1][0])
+    for a, b in zip(*got):
+        assert a.dtype == b.dtype and (a.float() - b.float()).norm() <= 1e-2 * b.float().norm() + 1e-6

@@ -324,3 +324,22 @@ def test_linear_wgrad_errors(cuda_device):
     with pytest.raises(RuntimeError):
         pshattn.linear_wgrad_bf16(g, torch.zeros(15, 64, device=cuda_device, dtype=torch.bfloat16), torch.zeros(32, 64, device=cuda_device))
     assert pshattn.wgrad_supported(96, 32) and not pshattn.wgrad_supported(96, 48) and not pshattn.wgrad_supported(20, 64)
+
+
+@pytest.mark.parametrize("m,n,k,bias", [(1, 128, 32, True), (127, 256, 64, False), (129, 384, 96, True), (300, 512, 128, True), (20000, 128, 32, False),
+                                        (5000, 2048, 256, True)])
+def test_linear_swiglu_gradient(cuda_device, m, n, k, bias):
+    """The gradient of [gate | up] through silu(gate) * up, taken inside the product that recomputes them."""
+    from flash3dtransformer_b200.lib import pshattn
+    gen = torch.Generator(cuda_device).manual_seed(m + n)
+    x = torch.randn(m, k, device=cuda_device, generator=gen).bfloat16()
+    w = (torch.randn(n, k, device=cuda_device, generator=gen) / k ** 0.5).bfloat16()
+    b = torch.randn(n, device=cuda_device, generator=gen) if bias else None
+    go = torch.randn(m, n // 2, device=cuda_device, generator=gen).bfloat16()
+    out = torch.full((m, n), float("nan"), device=cuda_device, dtype=torch.bfloat16)
+    pshattn.linear_swiglu_bwd_bf16(x, w, b, go, out)
+    pshattn.device_status()
+    y = (x.float() @ w.float().t() + (b if bias else 0.0)).requires_grad_(True)
+    gate, up = y.chunk(2, dim=1)
+    ref, = torch.autograd.grad(torch.nn.functional.silu(gate) * up, y, go.float())
+    _check(out, ref)

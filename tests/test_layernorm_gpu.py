@@ -88,3 +88,19 @@ def test_layernorm_gelu_autograd_path(cuda_device):
     assert err.mean().item() <= 2e-3 * rx.abs().mean().item() + 1e-4
     assert (wr.grad - rw).abs().max().item() <= 5e-3 * rw.abs().max().item() + 5e-2
     assert (br.grad - rb).abs().max().item() <= 5e-3 * rb.abs().max().item() + 5e-2
+
+
+@pytest.mark.parametrize("rows,c", [(1, 8), (33, 32), (4097, 64), (300, 512), (77, 1024)])
+def test_layernorm_backward_adds_the_residual_gradient(cuda_device, rows, c):
+    from flash3dtransformer_b200.lib import pshattn
+    x, w, b, go = _inputs(cuda_device, rows, c, 5)
+    res = torch.randn(rows, c, device=cuda_device).bfloat16()
+    dx, dw, db = torch.empty_like(x), torch.empty(c, device=cuda_device), torch.empty(c, device=cuda_device)
+    pshattn.layernorm_bwd_bf16(x, go, w, dx, dw, db, 1e-5, grad_residual=res)
+    xf = x.float().requires_grad_(True)
+    rx, = torch.autograd.grad(torch.nn.functional.layer_norm(xf, (c,), w, b, 1e-5), xf, go.float())
+    ref = rx + res.float()
+    assert ((dx.float() - ref).abs() <= ref.abs() * 2.0 ** -7 + 3e-3).all()
+    dw2, db2 = torch.empty_like(dw), torch.empty_like(db)
+    pshattn.layernorm_bwd_bf16(x, go, w, dx, dw2, db2, 1e-5)
+    assert torch.equal(dw, dw2) and torch.equal(db, db2)
