@@ -22,7 +22,7 @@ namespace f3d {
 
 int subbuck_build(const void *coord, const void *batch_sep, const void *red_sep, void *subbuck_id, void *subbuck_off,
                   void *unpool_ind, void *reduced_coord, uint32_t total_N, uint32_t batch, uint32_t max_n, uint32_t S,
-                  uint32_t num_vox, uint32_t hash_type, uint32_t red_rows, uint32_t red_coord_rows, cudaStream_t st);
+                  uint32_t num_vox, uint32_t hash_type, uint32_t red_rows, uint32_t red_coord_rows, int device, cudaStream_t st);
 
 enum RedOp : uint32_t { O_MEAN = 0, O_SUM = 1, O_MIN = 2, O_MAX = 3 };
 constexpr int kMaxS = 8;
@@ -327,7 +327,7 @@ extern "C" int f3d_batch_subbuck_reduce(
   F3D_TRY(maybe_sync(st, "batch_subbuck_reduce"));
   if (instance_max_N > total_N) instance_max_N = total_N;
   F3D_TRY(subbuck_build(scattered_coord, batch_sep, reduced_batch_sep, subbuck_id, subbuck_off, unpool_ind, reduced_coord,
-                        total_N, batch_size, instance_max_N, subbuck_size, num_vox, hash_type, unpool_rows, reduced_rows, st));
+                        total_N, batch_size, instance_max_N, subbuck_size, num_vox, hash_type, unpool_rows, reduced_rows, device, st));
   GatherArgs a{static_cast<const uint32_t *>(unpool_ind), unpool_rows, reduced_rows, total_N, feat_dim, subbuck_size, red_op,
                feat_dim * (uint32_t)esize(feat_dtype) / 16};
   if (reduced_rows > 0) {

@@ -32,6 +32,34 @@ def _build(dev, c16, seps, S, feat32, dtype, op, align=1, hash_type=1):
     return coords, feat, sb
 
 
+@pytest.mark.parametrize("scenes,S,kind", [(3, 2, "crowded"), (160, 2, "crowded"), (160, 3, "one voxel"), (160, 7, "spread"), (150, 5, "flat"),
+                                           (75, 4, "ramp")])
+def test_subbuck_order_of_crowded_bins(cuda_device, scenes, S, kind):
+    """Both thread shapes (scenes of up to 1100 points: more than an SM's worth of blocks or fewer), bins below, at and past
+    the size from which a mask orders them, one bin of a whole block, a flat axis."""
+    rng = np.random.default_rng(scenes + S)
+    sizes = rng.integers(1, 1101, scenes)
+    sizes[:3] = (1024, 1025, 33)
+    n = int(sizes.sum())
+    c = rng.uniform(-1.0, 1.0, (n, 3))
+    if kind == "crowded":
+        c[:] = rng.uniform(-1.0, 1.0, (40, 3))[np.minimum(rng.zipf(1.3, n), 40) - 1]
+    elif kind == "one voxel":
+        c[:] = 0.25
+    elif kind == "flat":
+        c[:, 1] = 0.5
+    elif kind == "ramp":                                   # bins of 31, 32, 33, 34 points in turn
+        c[:] = rng.uniform(-1.0, 1.0, (64, 3))[np.repeat(np.arange(64), 31 + np.arange(64) % 4)[np.arange(n) % 2080]]
+    c16 = c.astype(np.float16)
+    seps = np.cumsum(sizes)
+    feat32 = pl._round(rng.normal(size=(n, 8)).astype(np.float32), "bf16")
+    _, _, sb = _build(cuda_device, c16, seps, S, feat32, "bf16", 0, align=64)
+    sid, soff, unpool, rcoord, red_sep = pl.subbuck_build(c16, seps, S, red_rows_aligned=sb.reduced_coord.shape[0])
+    assert np.array_equal(sb.subbuck_id.cpu().numpy(), sid) and np.array_equal(sb.subbuck_off.cpu().numpy(), soff)
+    assert np.array_equal(sb.unpool_ind.cpu().numpy(), unpool)
+    assert np.array_equal(sb.reduced_coord.cpu().numpy().view(np.uint16), np.asarray(rcoord, np.float16).view(np.uint16))
+
+
 @pytest.mark.parametrize("S,dtype,op", [(2, "bf16", 0), (2, "fp32", 1), (3, "bf16", 2), (4, "fp16", 3), (2, "bf16", 3)])
 def test_subbuck_and_reduce_bit_exact(cuda_device, S, dtype, op):
     c32, seps = synthetic.batch(synthetic.lidar_scan, [5000, 1, 1025, 2048, 777, 3333], seed=1)
