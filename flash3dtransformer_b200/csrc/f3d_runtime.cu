@@ -103,6 +103,7 @@ int workspace(int device, int slot, size_t bytes, cudaStream_t stream, void **ou
     }
     F3D_CUDA_TRY(cudaMalloc(&s.ptr, want));
     s.bytes = want;
+    F3D_CUDA_TRY(cudaMemsetAsync(s.ptr, 0, want, stream));       // counters that their kernels leave at zero start there
   }
   *out = s.ptr;
   return F3D_OK;

@@ -22,8 +22,9 @@
 // with `stats_out` the epilogue adds up each output row and its squares, so a chain projection -> LayerNorm ->
 // projection needs neither a LayerNorm kernel nor a pass over x for statistics.  The sums are the same bits on every
 // run: a warp adds its tasks of a tile in column order, the three warps of a lane quadrant leave their partial sums in
-// shared memory and the last one to finish adds them in a fixed order and stores the row's pair (with more than one
-// column tile per row, N > 256, the tiles' pairs meet in an atomic add: two addends commute, so N <= 512 stays exact).
+// shared memory and the last one to finish adds them in a fixed order and stores the row's pair.  With more than one
+// column tile per row the tiles leave their pairs side by side: either the projection behind adds them in column order as it
+// reads them, or (when one pair a row is asked for) the last tile to finish does.
 // Outputs may be split column-wise into `nsplit` separate [M, N/nsplit] matrices (Q, K, V written directly in
 // the [L, H*D] layout the attention kernel reads, instead of three .contiguous() copies,
 // flash3dxfmr/layers/buck_swin.py:188-190).
@@ -44,7 +45,11 @@ namespace f3d {
 // A third build takes the gradient through SwiGLU: the product recomputes the pre-activation [gate | up] of a projection and
 // the epilogue turns it, with the gradient of the activation, into the gradient of [gate | up], so the pre-activation never
 // leaves the chip.
-enum GemmBuild : int { kGeneral = 0, kLean = 1, kSwigluBwd = 2 };
+// Two more carry one of the general build's additions each, the folded LayerNorm or the row sums: what a backbone's inference
+// runs at its wide levels, without the code of the others (8192 rows, N = 4096, K = 512 folded: 30.5 -> 28.4 us; N = 1536
+// 17.0 -> 15.6).  SwiGLU has builds of its own as well: the choice of the activation costs nothing at run time.
+enum GemmBuild : int { kGeneral = 0, kLean = 1, kSwigluBwd = 2, kFold = 3, kSums = 4, kLeanSwiglu = 5, kFoldSwiglu = 6 };
+constexpr bool is_lean(int build) { return build == kLean || build == kLeanSwiglu || build == kSwigluBwd; }
 constexpr int epi_warps(bool lean) { return lean ? 16 : 12; }
 constexpr int gemm_threads(bool lean) { return 64 + 32 * epi_warps(lean); }     // TMA warp, MMA warp, epilogue warps
 constexpr int BM = 128;
@@ -68,7 +73,10 @@ struct GemmArgs {
   const float2 *ln_stats;   // [M] (sum, sum of squares) of every row of A over its K channels, or null: folded LayerNorm
   const float *ln_colsum;   // [N] column sums s of the scaled weight (with ln_stats)
   float ln_eps, ln_inv_k;
-  float2 *stats_out;        // [M] or null: (sum, sum of squares) of every output row, accumulated with atomic adds
+  float2 *stats_out;        // [M] or null: (sum, sum of squares) of every output row
+  float2 *stats_part;       // [column tiles][M] each tile's pairs, and
+  int *stats_cnt;           // [row tiles][4] tiles that have left theirs, per lane quadrant; zero before and after the launch
+  int ln_parts;             // ln_stats is [ln_parts][M], pairs to be added in order
 };
 
 template <int BN, bool LEAN> struct GemmSmem {
@@ -144,10 +152,11 @@ template <bool F16> __device__ __forceinline__ float unpack_in1(const __nv_bfloa
 }
 
 template <int BN, bool F16, int BUILD>
-__global__ void __launch_bounds__(gemm_threads(BUILD != kGeneral), 1)
+__global__ void __launch_bounds__(gemm_threads(is_lean(BUILD)), 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                          const __grid_constant__ CUtensorMap map_c, GemmArgs g) {
-  constexpr bool LEAN = BUILD != kGeneral;
+  constexpr bool LEAN = is_lean(BUILD), kFolded = BUILD == kFold || BUILD == kFoldSwiglu;
+  constexpr bool kLn = BUILD == kGeneral || kFolded, kRowSums = BUILD == kGeneral || BUILD == kSums, kRest = BUILD == kGeneral;
   using S = GemmSmem<BN, LEAN>;
   constexpr int kEpiWarps = S::kEpiWarps, kGemmThreads = gemm_threads(LEAN);
   constexpr int kStages = S::kStages;
@@ -165,6 +174,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   float2 *stat_slots = reinterpret_cast<float2 *>(fold_base + S::kFoldBytes + S::kBarBytes);
   int *stat_cnt = reinterpret_cast<int *>(stat_slots + kAcc * 4 * (kEpiWarps / 4) * 32);
 
+  const bool swiglu = kRest ? g.epilogue == EPI_SWIGLU : BUILD == kSwigluBwd || BUILD == kLeanSwiglu || BUILD == kFoldSwiglu;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m_tiles = (g.M + BM - 1) / BM, n_tiles = (g.N + BN - 1) / BN;
   const int num_tiles = m_tiles * n_tiles;
@@ -178,7 +188,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) { tc::mbar_init(&full[s], 1); tc::mbar_init(&empty[s], 1); }
     for (int a = 0; a < kAcc; ++a) { tc::mbar_init(&acc_full[a], 1); tc::mbar_init(&acc_empty[a], kEpiWarps); }
-    if (!LEAN) for (int a = 0; a < kAcc * 4; ++a) stat_cnt[a] = 0;
+    if (kRowSums) for (int a = 0; a < kAcc * 4; ++a) stat_cnt[a] = 0;
     *abort_flag = 0;
     tc::mbar_fence_init();
     tc::tma_prefetch_desc(&map_a); tc::tma_prefetch_desc(&map_b); tc::tma_prefetch_desc(&map_c);
@@ -191,8 +201,8 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     for (int r = threadIdx.x; r < BN; r += kGemmThreads) {
       // row r of the W tile is output column r, or for SwiGLU gate column r | up column r - BN / 2
       int col = r;
-      if (g.epilogue == EPI_SWIGLU) col = r < BN / 2 ? r : g.N / 2 + (r - BN / 2);
-      const bool live = g.epilogue == EPI_SWIGLU ? (r < BN / 2 ? r < g.N / 2 : r - BN / 2 < g.N / 2) : r < g.N;
+      if (swiglu) col = r < BN / 2 ? r : g.N / 2 + (r - BN / 2);
+      const bool live = swiglu ? (r < BN / 2 ? r < g.N / 2 : r - BN / 2 < g.N / 2) : r < g.N;
       const float b = live ? __ldg(g.bias + col + after) : 0.f;
       uint32_t w0, w1;
       if (F16) {
@@ -257,7 +267,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
           }
           tc::mbar_expect_tx(&full[s], S::kStageBytes);
           tc::tma_load_2d(sa, &map_a, &full[s], kx, ya);
-          if (g.epilogue == EPI_SWIGLU) {
+          if (swiglu) {
             // gate rows [n0/2, n0/2 + BN/2) and up rows [N/2 + n0/2, ...) of W share one tile
             tc::tma_load_2d(sa + S::kABytes, &map_b, &full[s], kb * BK, n0 / 2);
             tc::tma_load_2d(sa + S::kABytes + S::kBBytes / 2, &map_b, &full[s], kb * BK, g.N / 2 + n0 / 2);
@@ -304,20 +314,22 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     unsigned char *my_out = out_base + (warp - 2) * 2 * 32 * 64;
     uint32_t t_local = 0, obuf = 0, task = 0;
     bool ok = true;
-    const int tile_cols = g.epilogue == EPI_SWIGLU ? BN / 2 : BN;    // output columns a tile can produce
-    const int total_cols = g.epilogue == EPI_SWIGLU ? g.N / 2 : g.N; // output columns there are
+    const int tile_cols = swiglu ? BN / 2 : BN;    // output columns a tile can produce
+    const int total_cols = swiglu ? g.N / 2 : g.N; // output columns there are
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++t_local) {
       const uint32_t acc = t_local % kAcc, aph = (t_local / kAcc) & 1u;
       const int mt = n_tiles == 1 ? tile : tile / n_tiles;
       const int m0 = mt * BM, n0 = (tile - mt * n_tiles) * BN;
-      if (!tc::mbar_wait(&acc_full[acc], aph, wc, 104)) { ok = false; break; }
-      tc::tc_fence_after_sync();
-      const uint32_t t_row = tmem_base + acc * BN + ((uint32_t)(q * 32) << 16);
       const int row = m0 + q * 32 + lane;
       // folded LayerNorm: this thread's row contributes rstd and -mean * rstd to every column
       float ln_rstd = 1.f, ln_nmr = 0.f;
-      if (!LEAN && g.ln_stats) {
-        const float2 st = row < g.M ? __ldg(g.ln_stats + row) : make_float2(0.f, 0.f);
+      if (kLn && g.ln_stats) {
+        float2 st = make_float2(0.f, 0.f);
+        if (row < g.M)
+          for (int j = 0; j < g.ln_parts; ++j) {
+            const float2 p = __ldg(g.ln_stats + (size_t)j * g.M + row);
+            st.x += p.x; st.y += p.y;
+          }
         const float mean = st.x * g.ln_inv_k;
         const float var = fmaxf(fmaf(-mean, mean, st.y * g.ln_inv_k), 0.f);
         ln_rstd = rsqrtf(var + g.ln_eps);
@@ -328,11 +340,18 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       // this warp's tasks of the tile: numbers congruent to `sub` modulo kSub, `task` being the tile's first
       // tasks of this tile: only the 32-column groups that hold output columns (N = 96 fills three of a 128-column
       // tile's four groups; the fourth would be computed and then clipped by the store)
-      const int first_col = g.epilogue == EPI_SWIGLU ? n0 / 2 : n0;
+      const int first_col = swiglu ? n0 / 2 : n0;
       const int out_cols = min(tile_cols, (total_cols - first_col + 31) & ~31);
+      // the rows of the residual are requested before the product is awaited: a tile's first use of them is a chain of its own
+      if (!kFolded && BUILD != kLeanSwiglu && g.residual && row < g.M)
+        for (int c0 = (int)((sub + kSub - task % kSub) % kSub) * 32; c0 < out_cols; c0 += 32 * (int)kSub)
+          if (first_col + c0 < total_cols) asm volatile("prefetch.global.L1 [%0];" ::"l"(g.residual + (size_t)row * g.ldr + first_col + c0));
+      if (!tc::mbar_wait(&acc_full[acc], aph, wc, 104)) { ok = false; break; }
+      tc::tc_fence_after_sync();
+      const uint32_t t_row = tmem_base + acc * BN + ((uint32_t)(q * 32) << 16);
       for (int c0 = (int)((sub + kSub - task % kSub) % kSub) * 32; c0 < out_cols; c0 += 32 * (int)kSub) {
         float v[32];
-        const int oc0 = (g.epilogue == EPI_SWIGLU ? n0 / 2 : n0) + c0;      // first output column of the task
+        const int oc0 = (swiglu ? n0 / 2 : n0) + c0;      // first output column of the task
         if constexpr (BUILD == kSwigluBwd) {
           // 16 columns at a time: gate a, up u, gradient o of the activation -> o u s (1 + a (1 - s)) and o a s, s = sigmoid(a)
           if (tc::elect_one()) tc::tma_wait_read<0>();            // both staging buffers, one for each half of the output
@@ -383,7 +402,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
           continue;
         }
         // runtime switches (bias, activation) are tested once per task, never per element
-        if (LEAN && g.epilogue == EPI_SWIGLU) {
+        if (LEAN && swiglu) {
           // lean build: gate and up accumulators of 16 output columns at a time, so that a thread stays within the
           // registers that 16 epilogue warps leave it
 #pragma unroll
@@ -412,12 +431,12 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                             gpack2(__uint_as_float(u[2 * j]), __uint_as_float(u[2 * j + 1])), v[hh * 16 + 2 * j], v[hh * 16 + 2 * j + 1]);
             }
           }
-        } else if (!LEAN && g.epilogue == EPI_SWIGLU) {
+        } else if (kLn && swiglu) {
           uint32_t r[32], u[32];
           tc::tmem_ld_32x32b_x32(t_row + c0, r);
           tc::tmem_ld_32x32b_x32(t_row + BN / 2 + c0, u);
           tc::tmem_ld_wait();
-          if (g.ln_stats) {
+          if (kFolded || g.ln_stats) {
             // gate = rstd * acc_g + nmr * s_g + b'_g (likewise up); the host always supplies b' in this mode
             const float4 *pg = reinterpret_cast<const float4 *>(g.bias + oc0), *pu = reinterpret_cast<const float4 *>(g.bias + g.N / 2 + oc0);
             const float4 *sg = reinterpret_cast<const float4 *>(g.ln_colsum + oc0), *su = reinterpret_cast<const float4 *>(g.ln_colsum + g.N / 2 + oc0);
@@ -454,7 +473,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
           tc::tmem_ld_wait();
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-          if (!LEAN && g.ln_stats) {
+          if (kFolded || (kLn && g.ln_stats)) {
             // v = rstd * acc + (nmr * s + b'); columns past N are never stored, so only the loads are guarded
             const float4 *bp = reinterpret_cast<const float4 *>(g.bias + oc0), *sp4 = reinterpret_cast<const float4 *>(g.ln_colsum + oc0);
 #pragma unroll
@@ -484,12 +503,12 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
               }
             }
           }
-          if (!LEAN && g.epilogue == EPI_GELU) {
+          if (kRest && g.epilogue == EPI_GELU) {
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = gelu_tanh(v[j]);
           }
         }
-        if (g.residual && row < g.M) {
+        if (!kFolded && BUILD != kLeanSwiglu && g.residual && row < g.M) {
           const __nv_bfloat16 *rp = g.residual + (size_t)row * g.ldr + oc0;
           if (oc0 + 32 <= g.N && (reinterpret_cast<uintptr_t>(rp) & 15) == 0) {
 #pragma unroll
@@ -504,7 +523,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             for (int j = 0; j < 32; ++j) if (oc0 + j < g.N) v[j] += unpack_in1<F16>(rp + j);
           }
         }
-        if (!LEAN && g.stats_out) {
+        if (BUILD == kSums || (kRowSums && g.stats_out)) {
           // row sums of this task's columns for the LayerNorm that follows (the next projection folds it in)
 #pragma unroll
           for (int j = 0; j < 32; j += 2) {
@@ -515,7 +534,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             }
           }
         }
-        if (!LEAN && g.direct_store) {
+        if (kRest && g.direct_store) {
           if (row < g.M) {
 #pragma unroll
             for (int j = 0; j < 32; j += 8) {
@@ -553,7 +572,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         obuf ^= 1u;
       }
       task += (uint32_t)(out_cols / 32);
-      if (!LEAN && g.stats_out) {
+      if (BUILD == kSums || (kRowSums && g.stats_out)) {
         // leave this warp's partial sums in its slot; the last warp of the quadrant to get here adds the slots in a
         // fixed order.  The slots of an accumulator are free again before its next tile: every epilogue warp arrives
         // on acc_empty only after this block.
@@ -575,9 +594,28 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
           if (row < g.M) {
             if (n_tiles == 1) {
               g.stats_out[row] = tot;
+            } else if (g.stats_part) {               // the consumer's parts, or scratch for the last tile to add up
+              g.stats_part[(size_t)(tile - mt * n_tiles) * g.M + row] = tot;
             } else {
               atomicAdd(&g.stats_out[row].x, tot.x);
               atomicAdd(&g.stats_out[row].y, tot.y);
+            }
+          }
+          if (n_tiles > 1 && g.stats_cnt) {
+            __threadfence();
+            __syncwarp();
+            if (lane == 0) last = atomicAdd(&g.stats_cnt[mt * 4 + q], 1) == n_tiles - 1;
+            if (__shfl_sync(0xFFFFFFFFu, last, 0)) {
+              __threadfence();
+              float2 sum = make_float2(0.f, 0.f);
+              if (row < g.M) {
+                for (int j = 0; j < n_tiles; ++j) {
+                  const float2 p = __ldcg(g.stats_part + (size_t)j * g.M + row);
+                  sum.x += p.x; sum.y += p.y;
+                }
+                g.stats_out[row] = sum;
+              }
+              if (lane == 0) g.stats_cnt[mt * 4 + q] = 0;
             }
           }
           __syncwarp();
@@ -605,7 +643,7 @@ int *status_word(int device);   // device word, zero until a kernel reports an a
 template <int BN, bool F16, int BUILD>
 static int launch_gemm_build(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &mc, const GemmArgs &g, int device,
                              cudaStream_t st) {
-  constexpr bool LEAN = BUILD != kGeneral;
+  constexpr bool LEAN = is_lean(BUILD);
   auto kern = gemm_bf16_tcgen05_kernel<BN, F16, BUILD>;
   F3D_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(kern), device, GemmSmem<BN, LEAN>::kTotal));
   int tiles = ((g.M + BM - 1) / BM) * ((g.N + BN - 1) / BN);
@@ -617,9 +655,18 @@ static int launch_gemm_build(const CUtensorMap &ma, const CUtensorMap &mb, const
 template <int BN, bool F16>
 static int launch_gemm(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &mc, const GemmArgs &g, int device,
                        cudaStream_t st) {
-  // the plain projections (bias, residual, column splits, TMA stores) take the lean build
-  const bool lean = (g.epilogue == EPI_NONE || g.epilogue == EPI_SWIGLU) && !g.ln_stats && !g.stats_out && !g.direct_store;
-  if (lean) return launch_gemm_build<BN, F16, kLean>(ma, mb, mc, g, device, st);
+  // the plain projections (bias, residual, column splits, TMA stores) and those with one addition have builds of their own
+  const bool swiglu = g.epilogue == EPI_SWIGLU, plain = (g.epilogue == EPI_NONE || swiglu) && !g.direct_store && !(swiglu && g.residual);
+  if constexpr (BN >= 128) {
+    if (plain && swiglu && !g.ln_stats && !g.stats_out) return launch_gemm_build<BN, F16, kLeanSwiglu>(ma, mb, mc, g, device, st);
+    if constexpr (!F16)
+      if (plain && swiglu && g.ln_stats && !g.stats_out) return launch_gemm_build<BN, F16, kFoldSwiglu>(ma, mb, mc, g, device, st);
+  }
+  if (plain && !swiglu && !g.ln_stats && !g.stats_out) return launch_gemm_build<BN, F16, kLean>(ma, mb, mc, g, device, st);
+  if constexpr (!F16) {
+    if (plain && !swiglu && g.ln_stats && !g.stats_out && !g.residual) return launch_gemm_build<BN, F16, kFold>(ma, mb, mc, g, device, st);
+    if (plain && !swiglu && !g.ln_stats && g.stats_out) return launch_gemm_build<BN, F16, kSums>(ma, mb, mc, g, device, st);
+  }
   return launch_gemm_build<BN, F16, kGeneral>(ma, mb, mc, g, device, st);
 }
 
@@ -628,6 +675,8 @@ struct LinearFusion {
   const void *ln_colsum = nullptr;
   float ln_eps = 1e-5f;
   void *stats_out = nullptr;         // row sums of the output
+  int ln_parts = 1;                  // ln_stats is [ln_parts][M]
+  int *stats_parts = nullptr;        // leave stats_out as [parts][M], one part per column tile, and report their number here
 };
 
 // C (nsplit matrices of [M, split_n] with leading dimension split_n, `split_stride` elements apart); dtype 0 = bf16,
@@ -658,9 +707,36 @@ int linear_bf16(const void *A, int lda, const void *W, int ldw, const void *bias
   else if (N <= 32) BN = 32;
   else if (N <= 64) BN = 64;
   else if (N <= 128 || (nsplit > 1 && split_n % 256)) BN = 128;
+  // With few row tiles the widest column tile leaves SMs idle, or nearly idle in a second round.  A tile's time grows with its
+  // columns on top of a part that does not depend on them (rows of A, pipeline fill, epilogue start) and is worth about 64
+  // columns: the width with the least rounds x (width + 64) is taken, the wider one of two equal (with many rounds that is the
+  // widest, which reads A the fewest times).  4096 rows: N = 512, K = 2048 19.7 -> 14.4 us with 128 columns instead of 256,
+  // N = 256, K = 1024 12.3 -> 9.5 us with 64.
+  if (epilogue != EPI_SWIGLU) {
+    const long long m_tiles = (M + BM - 1) / BM, sms = sm_count(device);
+    const auto cost = [&](int w) { return (m_tiles * ((N + w - 1) / w) + sms - 1) / sms * (w + 64); };
+    for (int w = BN / 2; w >= 32; w /= 2)
+      if (cost(w) < cost(BN)) BN = w;
+  }
   const int direct = (nsplit > 1 && split_n % 32) ? 1 : 0;      // a 32-column task must not straddle two outputs
-  // rows that span several column tiles add their tiles' sums into a cleared buffer; one tile stores them
-  if (fu.stats_out && N > BN) F3D_CUDA_TRY(cudaMemsetAsync(fu.stats_out, 0, (size_t)M * sizeof(float2), st));
+  float2 *stats_part = nullptr;
+  int *stats_cnt = nullptr;
+  if (fu.stats_parts) {
+    *fu.stats_parts = (N + BN - 1) / BN;
+    stats_part = static_cast<float2 *>(fu.stats_out);
+  } else if (fu.stats_out && N > BN) {
+    void *part = nullptr, *cnt = nullptr;
+    const size_t tiles = (size_t)((N + BN - 1) / BN);
+    const bool have = workspace(device, 9, tiles * M * sizeof(float2), st, &part) == F3D_OK &&
+                      workspace(device, 10, (size_t)((M + BM - 1) / BM) * 4 * sizeof(int), st, &cnt) == F3D_OK;
+    if (have) {
+      stats_part = static_cast<float2 *>(part);
+      stats_cnt = static_cast<int *>(cnt);
+    } else {
+      // no scratch on a stream that captures before it ever ran this: the tiles add into a cleared buffer
+      F3D_CUDA_TRY(cudaMemsetAsync(fu.stats_out, 0, (size_t)M * sizeof(float2), st));
+    }
+  }
   if (reinterpret_cast<uintptr_t>(C) % 16) return set_error(F3D_ERR_ARG, "gemm: output pointer is not 16-byte aligned");
   CUtensorMap ma, mb, mc;
   F3D_TRY(encode_tmap_2d(&ma, dtype, A, (uint64_t)K, (uint64_t)M * ksplit, (uint64_t)lda * 2, BK, BM, 128));
@@ -671,7 +747,7 @@ int linear_bf16(const void *A, int lda, const void *W, int ldw, const void *bias
   GemmArgs g{M, N, K, nsplit, split_n, static_cast<const float *>(bias), static_cast<const __nv_bfloat16 *>(residual), ldr,
              epilogue, direct, static_cast<__nv_bfloat16 *>(C), split_stride, status_word(device), ksplit,
              static_cast<const float2 *>(fu.ln_stats), static_cast<const float *>(fu.ln_colsum), fu.ln_eps, 1.f / (float)K,
-             static_cast<float2 *>(fu.stats_out)};
+             static_cast<float2 *>(fu.stats_out), stats_part, stats_cnt, fu.ln_parts};
   if (!g.status) return F3D_ERR_CUDA;
   if (dtype == 1) {
     switch (BN) {
@@ -752,6 +828,22 @@ extern "C" int f3d_linear_fused(const void *A, const void *W, const void *bias, 
                       epilogue, device, st, 1, dtype, fu));
   return maybe_sync(st, "linear_fused");
 }
+
+namespace f3d {
+// linear_fused for callers that hand row sums from one projection to the next: they stay in parts, one per column tile
+int linear_folded(const void *A, const void *W, const void *bias, const void *residual, void *C, int M, int N, int K, int nsplit, int epilogue,
+                  const void *ln_stats, int ln_parts, const void *ln_colsum, float ln_eps, void *stats_out, int *stats_parts, int device,
+                  cudaStream_t st) {
+  DeviceGuard guard(device);
+  F3D_TRY(maybe_sync(st, "linear_folded"));
+  const int out_n = epilogue == EPI_SWIGLU ? N / 2 : N;
+  LinearFusion fu;
+  fu.ln_stats = ln_stats; fu.ln_parts = ln_parts; fu.ln_colsum = ln_colsum; fu.ln_eps = ln_eps;
+  fu.stats_out = stats_out; fu.stats_parts = stats_out ? stats_parts : nullptr;
+  F3D_TRY(linear_bf16(A, K, W, K, bias, residual, out_n, C, (long long)M * (out_n / nsplit), M, N, K, nsplit, epilogue, device, st, 1, 0, fu));
+  return maybe_sync(st, "linear_folded");
+}
+}  // namespace f3d
 
 extern "C" int f3d_linear_ksplit_bf16(const void *A, const void *W, const void *bias, const void *residual, void *C, int M, int N,
                                       int K, int ksplit, int device, void *stream) {

@@ -10,6 +10,10 @@
 
 namespace f3d {
 
+int linear_folded(const void *A, const void *W, const void *bias, const void *residual, void *C, int M, int N, int K, int nsplit, int epilogue,
+                  const void *ln_stats, int ln_parts, const void *ln_colsum, float ln_eps, void *stats_out, int *stats_parts, int device,
+                  cudaStream_t st);
+
 struct StackScratch {
   // Q, K, V and the attention output of a block; the MLP's hidden rows take their place once the output projection is done
   size_t qkv, attn, hidden, norm, mid, ping, stats[3], total;
@@ -23,7 +27,8 @@ struct StackScratch {
     norm = at; at += row;
     mid = at; at += row;
     ping = at; at += row;
-    for (int i = 0; i < 3; ++i) { stats[i] = at; at += up(rows * 8); }
+    // row sums of a projection come in one part per column tile (32 columns at the least): the projection behind it adds them
+    for (int i = 0; i < 3; ++i) { stats[i] = at; at += up(rows * 8 * ((c + 31) / 32)); }
     total = at;
   }
 };
@@ -54,6 +59,8 @@ extern "C" int f3d_xfmr_stack_bf16(const f3d_xfmr_block *blocks, int count, cons
   const size_t mat = (size_t)rows * channels * 2;
   const void *cur = x;
   void *stats = nullptr;                                          // row sums of cur, once a block has left them
+  int parts = 1, mid_parts = 1;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   for (int i = 0; i < count; ++i) {
     const f3d_xfmr_block &b = blocks[i];
     void *dst = (count - 1 - i) % 2 == 0 ? out : static_cast<void *>(base + s.ping);
@@ -62,9 +69,10 @@ extern "C" int f3d_xfmr_stack_bf16(const f3d_xfmr_block *blocks, int count, cons
       // both LayerNorms ride in the projections behind them, on the row sums of the projections in front of them
       if (!stats) {
         stats = base + s.stats[0];
+        parts = 1;
         F3D_TRY(f3d_row_stats_bf16(cur, stats, rows, channels, device, stream));
       }
-      F3D_TRY(f3d_linear_fused(cur, b.qkv_w, b.qkv_b, nullptr, qkv, m, 3 * c, c, 3, 0, 0, stats, b.qkv_colsum, b.norm_eps, nullptr, device, stream));
+      F3D_TRY(linear_folded(cur, b.qkv_w, b.qkv_b, nullptr, qkv, m, 3 * c, c, 3, 0, stats, parts, b.qkv_colsum, b.norm_eps, nullptr, nullptr, device, st));
     } else {
       F3D_TRY(f3d_layernorm_bf16(cur, b.norm_w, b.norm_b, norm, rows, channels, b.norm_eps, 0, device, stream));
       F3D_TRY(f3d_linear_fused(norm, b.qkv_w, b.qkv_b, nullptr, qkv, m, 3 * c, c, 3, 0, 0, nullptr, nullptr, 0.f, nullptr, device, stream));
@@ -72,9 +80,9 @@ extern "C" int f3d_xfmr_stack_bf16(const f3d_xfmr_block *blocks, int count, cons
     F3D_TRY(f3d_buck_swin_fwd(q, q + mat, q + 2 * mat, attn, lse, b.scopes, 1, m, b.heads, c / b.heads, b.num_scopes, b.scope_size,
                               (uint32_t)b.bucket, device, stream));
     void *mid_stats = fold ? base + s.stats[2] : nullptr;
-    F3D_TRY(f3d_linear_fused(attn, b.proj_w, b.proj_b, cur, mid, m, c, c, 1, 0, 0, nullptr, nullptr, 0.f, mid_stats, device, stream));
+    F3D_TRY(linear_folded(attn, b.proj_w, b.proj_b, cur, mid, m, c, c, 1, 0, nullptr, 1, nullptr, 0.f, mid_stats, &mid_parts, device, st));
     if (fold) {
-      F3D_TRY(f3d_linear_fused(mid, b.fc1_w, b.fc1_b, nullptr, hid, m, 2 * b.hidden, c, 1, 2, 0, mid_stats, b.fc1_colsum, b.ln2_eps, nullptr, device, stream));
+      F3D_TRY(linear_folded(mid, b.fc1_w, b.fc1_b, nullptr, hid, m, 2 * b.hidden, c, 1, 2, mid_stats, mid_parts, b.fc1_colsum, b.ln2_eps, nullptr, nullptr, device, st));
     } else {
       F3D_TRY(f3d_layernorm_bf16(mid, b.ln2_w, b.ln2_b, norm, rows, channels, b.ln2_eps, 0, device, stream));
       F3D_TRY(f3d_linear_fused(norm, b.fc1_w, b.fc1_b, nullptr, hid, m, 2 * b.hidden, c, 1, 2, 0, nullptr, nullptr, 0.f, nullptr, device, stream));
@@ -82,7 +90,7 @@ extern "C" int f3d_xfmr_stack_bf16(const f3d_xfmr_block *blocks, int count, cons
     // row sums of the block's output only where the next block folds its LayerNorm in
     const bool next_folds = i + 1 < count && blocks[i + 1].qkv_colsum != nullptr;
     void *next_stats = next_folds ? base + s.stats[(i + 1) % 2] : nullptr;
-    F3D_TRY(f3d_linear_fused(hid, b.fc2_w, b.fc2_b, mid, dst, m, c, b.hidden, 1, 0, 0, nullptr, nullptr, 0.f, next_stats, device, stream));
+    F3D_TRY(linear_folded(hid, b.fc2_w, b.fc2_b, mid, dst, m, c, b.hidden, 1, 0, nullptr, 1, nullptr, 0.f, next_stats, &parts, device, st));
     stats = next_stats;
     cur = dst;
   }

@@ -127,3 +127,26 @@ def test_block_and_backbone_folded_against_unfused(cuda_device):
     rows = int(seps[-1])
     _check(a[:rows], b[:rows].float(), "backbone_folded_vs_unfused", max_abs=0.1, mean_rel=1e-2)
     assert folded_launches < unfused_launches            # 8 LayerNorm launches gone, 2 statistics passes added
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 512, 64), (129, 256, 256), (4096, 256, 128), (4096, 512, 512), (1000, 1024, 64), (300, 96, 32), (20000, 512, 64)])
+def test_row_sums_over_column_tiles(cuda_device, m, n, k):
+    """Row sums where the width of the column tiles follows from the number of row tiles: one, few and many tiles a row; the
+    same bits on every run."""
+    from flash3dtransformer_b200.lib import pshattn
+    gen = torch.Generator(cuda_device).manual_seed(m + n)
+    x = torch.randn(m, k, device=cuda_device, generator=gen).bfloat16()
+    w = (torch.randn(n, k, device=cuda_device, generator=gen) / k ** 0.5).bfloat16()
+    b = torch.randn(n, device=cuda_device, generator=gen)
+    res = torch.randn(m, n, device=cuda_device, generator=gen).bfloat16()
+    runs = []
+    for _ in range(2):
+        out = torch.empty(m, n, device=cuda_device, dtype=torch.bfloat16)
+        sums = torch.full((m, 2), float("nan"), device=cuda_device)
+        pshattn.linear_fused(x, w, b, out, residual=res, stats_out=sums)
+        runs.append((out, sums))
+    pshattn.device_status()
+    ref = x.float() @ w.float().t() + b + res.float()
+    assert (runs[0][0].float() - ref).abs().max().item() <= 2e-2 * ref.abs().max().item()
+    assert torch.allclose(runs[0][1], torch.stack([ref.sum(1), ref.square().sum(1)], dim=1), rtol=2e-3, atol=2e-2 * n ** 0.5)
+    assert torch.equal(runs[0][0], runs[1][0]) and torch.equal(runs[0][1], runs[1][1])
