@@ -8,6 +8,14 @@
 // shared memory - the bias gradient costs no second pass over g.  Partial tiles go to a scratch and a second kernel adds
 // the slabs in a fixed order: no atomics, the same bits on every run.
 //
+// g may be several matrices [splits][M][C] (the gradients of Q, K and V) whose weight gradients lie one below the other: one
+// launch then reads x once per 128 output rows, and the three reductions are one.
+//
+// What bounds wide outputs is shared memory: a product takes A again for every instruction, so one instruction covers all
+// panels of x (N = 256: 12 KB read per 128 cycles of the tensor core; with one instruction a panel it was 24 KB per 128), and
+// the column sums read two columns a thread, one 128-byte row a warp.  200,704 rows, N = 2048, K = 256: 308 -> @@ us (141 at the
+// copy rate); 100,352 rows, N = K = 512: 103 -> @@.
+//
 // Stands in for the library GEMM g^T x and the separate column-sum pass of the backward of nn.Linear / te.Linear in
 // flash3dxfmr/layers/buck_swin.py:159,163 and the MLP of flash3dxfmr/layers/elem_wise.py.
 #include "f3d_common.cuh"
@@ -24,7 +32,8 @@ constexpr int kWgStages = 4;
 constexpr int kWgPanelBytes = kWgRows * 128;      // 64 rows of 128 bytes
 
 struct WgradArgs {
-  int M, N, K;
+  int M, N, K;            // N = splits * C
+  int splits, C, pps;     // g is [splits][M][C], pps = 64-column panels of a split
   int rb;                 // bytes of one x row inside a panel: 128, or 64 when K == 32
   int x_panels;           // 64-column panels of x per k-tile (1..4)
   int k_tiles, n_tiles, slabs, blocks_per_slab;
@@ -42,12 +51,13 @@ wgrad_tcgen05_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + kWgStages * stage_bytes);
   uint64_t *full = bars, *empty = bars + kWgStages, *acc_full = bars + 2 * kWgStages;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_full + 1);
+  float2 *half_sums = reinterpret_cast<float2 *>(smem + kWgStages * stage_bytes + 256);     // [2][64] column sums of half the rows
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tile = blockIdx.x, slab = blockIdx.y;
   const int nt = tile / a.k_tiles, kt = tile - nt * a.k_tiles;
-  const int n0 = nt * 128, k0 = kt * a.x_panels * 64;
+  const int p0 = nt * 2, k0 = kt * a.x_panels * 64;                  // first g panel of the tile, first column of x
   const int total_blocks = (a.M + kWgRows - 1) / kWgRows;
   const int b0 = slab * a.blocks_per_slab;
   const int b1 = b0 + a.blocks_per_slab < total_blocks ? b0 + a.blocks_per_slab : total_blocks;
@@ -81,18 +91,17 @@ wgrad_tcgen05_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
         // rows past M and columns past N or K are zero-filled by the copies and add nothing
         // (a tile load costs the copy engine about 7 cycles per box row: the second g panel is skipped when it lies
         // past N; tensor-memory lanes 64..127 then hold products of stale shared memory and are never stored)
-        const bool two = n0 + 64 < a.N;
+        const bool two = p0 + 1 < a.splits * a.pps;
         tc::mbar_expect_tx(&full[s], (uint32_t)((two ? 2 : 1) * kWgPanelBytes + a.x_panels * kWgRows * a.rb));
-        tc::tma_load_2d(st, &map_g, &full[s], n0, r0);
-        if (two) tc::tma_load_2d(st + kWgPanelBytes, &map_g, &full[s], n0 + 64, r0);
+        tc::tma_load_3d(st, &map_g, &full[s], p0 % a.pps * 64, r0, p0 / a.pps);
+        if (two) tc::tma_load_3d(st + kWgPanelBytes, &map_g, &full[s], (p0 + 1) % a.pps * 64, r0, (p0 + 1) / a.pps);
         for (int p = 0; p < a.x_panels; ++p)
           tc::tma_load_2d(st + (2 + p) * kWgPanelBytes, &map_x, &full[s], k0 + p * 64, r0);
       }
     }
   } else if (warp == 1) {
     if (tc::elect_one()) {
-      const uint32_t npanel = a.rb == 64 ? 32u : 64u;                // N of one MMA: the columns of one x panel
-      const uint32_t idesc = tc::make_idesc_f16(128, npanel, true, true, true);
+      const uint32_t idesc = tc::make_idesc_f16(128, a.rb == 64 ? 32u : ncols, true, true, true);
       const uint64_t swz = a.rb == 64 ? tc::kSwizzle64 : tc::kSwizzle128;
       bool ok = true;
       for (int i = 0; i < nblk && ok; ++i) {
@@ -100,29 +109,27 @@ wgrad_tcgen05_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
         if (!tc::mbar_wait(&full[s], ph, wc, 402)) { ok = false; break; }
         tc::tc_fence_after_sync();
         const uint32_t g_addr = tc::smem_u32(smem + s * stage_bytes), x_addr = g_addr + 2 * kWgPanelBytes;
-        for (int p = 0; p < a.x_panels; ++p) {
 #pragma unroll
-          for (int ks = 0; ks < kWgRows / 16; ++ks) {
-            // A: 16 rows of the g tile, its 128 columns in two panels kWgPanelBytes apart (leading offset); B: the
-            // same 16 rows of one x panel
-            const uint64_t ad = tc::make_smem_desc(g_addr + ks * 16 * 128, kWgPanelBytes, 1024, tc::kSwizzle128);
-            const uint64_t bd = tc::make_smem_desc(x_addr + p * kWgPanelBytes + ks * 16 * a.rb, 16, 8 * a.rb, swz);
-            tc::mma_f16_ss(tmem_base + p * 64, ad, bd, idesc, (i | ks) != 0 ? 1u : 0u);
-          }
+        for (int ks = 0; ks < kWgRows / 16; ++ks) {
+          // A: 16 rows of the g tile, its 128 columns in two panels kWgPanelBytes apart (leading offset); B: the same 16
+          // rows of x, its columns in panels the same distance apart
+          const uint64_t ad = tc::make_smem_desc(g_addr + ks * 16 * 128, kWgPanelBytes, 1024, tc::kSwizzle128);
+          const uint64_t bd = tc::make_smem_desc(x_addr + ks * 16 * a.rb, kWgPanelBytes, 8 * a.rb, swz);
+          tc::mma_f16_ss(tmem_base, ad, bd, idesc, (i | ks) != 0 ? 1u : 0u);
         }
         tc::mma_commit(&empty[s]);
       }
       if (ok) tc::mma_commit(acc_full);
     }
   } else {
-    // column sums of the g tile while the tensor cores run.  A warp may read the tensor-memory lanes of quadrant
-    // warp % 4 only, so thread (q, lane) owns output row n0 + q * 32 + lane in the sums and in the epilogue alike.
+    // column sums of the g tile while the tensor cores run: warps of quadrants 0 and 1 add up the upper half of a stage's rows
+    // (two columns a thread: the 64 of panel q & 1), those of quadrants 2 and 3 the lower half
     const int q = warp & 3;
-    const int t = q * 32 + lane;                            // 0..127, row of the output tile
-    const int n = n0 + t;
-    const uint32_t col_off = (uint32_t)(t >> 6) * kWgPanelBytes + (uint32_t)(t & 7) * 2u;
-    const uint32_t chunk = (uint32_t)(t & 63) >> 3;
-    float bsum = 0.f;
+    const int t = q * 32 + lane;                            // 0..127, row of the output tile in the epilogue
+    const uint32_t first_row = (uint32_t)(q >> 1) * (kWgRows / 2);
+    const uint32_t col_off = (uint32_t)(q & 1) * kWgPanelBytes + (uint32_t)(lane & 3) * 4u;
+    const uint32_t chunk = (uint32_t)lane >> 2;
+    float2 bsum = make_float2(0.f, 0.f);
     bool ok = true;
     for (int i = 0; i < nblk && ok; ++i) {
       const uint32_t s = i % kWgStages, ph = (i / kWgStages) & 1u;
@@ -131,21 +138,28 @@ wgrad_tcgen05_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
       if (want_bias) {
         const uint32_t g_addr = tc::smem_u32(smem + s * stage_bytes) + col_off;
 #pragma unroll 16
-        for (int r = 0; r < kWgRows; ++r) {
-          uint16_t h;
-          asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h) : "r"(g_addr + (uint32_t)r * 128u + ((chunk ^ ((uint32_t)r & 7u)) << 4)));
-          bsum += __uint_as_float((uint32_t)h << 16);
+        for (uint32_t r = first_row; r < first_row + kWgRows / 2; ++r) {
+          uint32_t h;
+          asm volatile("ld.shared.u32 %0, [%1];" : "=r"(h) : "r"(g_addr + r * 128u + ((chunk ^ (r & 7u)) << 4)));
+          bsum.x += __uint_as_float(h << 16);
+          bsum.y += __uint_as_float(h & 0xFFFF0000u);
         }
       }
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&empty[s]);
     }
-    // epilogue: lane of tensor memory = output row; the partial tile goes to the slab's scratch as fp32
+    half_sums[(q >> 1) * 64 + (q & 1) * 32 + lane] = bsum;
+    asm volatile("bar.sync 1, 128;" ::: "memory");          // the four warps
+    // epilogue: a warp may read the tensor-memory lanes of quadrant warp % 4 only; lane of tensor memory = output row; the
+    // partial tile goes to the slab's scratch as fp32
+    const int panel = p0 + (t >> 6), split = panel / a.pps, col = (panel - split * a.pps) * 64 + (t & 63);
+    const int n = split * a.C + col;
     if (ok && tc::mbar_wait(acc_full, 0, wc, 404)) {
       __syncwarp();
       tc::tc_fence_after_sync();
-      const bool live = n < a.N;
-      if (want_bias && live) a.partial_b[(size_t)slab * a.slab_stride + n] = bsum;
+      const bool live = split < a.splits && col < a.C;
+      const float *sums = reinterpret_cast<const float *>(half_sums);
+      if (want_bias && live) a.partial_b[(size_t)slab * a.slab_stride + n] = sums[t] + sums[128 + t];
       float *dst = a.partial_w + (size_t)slab * a.slab_stride + (size_t)(live ? n : 0) * a.K + k0;
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16);
       const uint32_t width = a.rb == 64 ? 32u : 64u;        // K == 32: only the first 32 columns of the panel hold results
@@ -207,6 +221,13 @@ using namespace f3d;
 
 extern "C" int f3d_linear_wgrad_bf16(const void *grad_out, const void *x, void *grad_weight, void *grad_bias, int M, int N, int K,
                                      int device, void *stream) {
+  return f3d_linear_wgrad_split_bf16(grad_out, x, grad_weight, grad_bias, M, N, K, 1, device, stream);
+}
+
+extern "C" int f3d_linear_wgrad_split_bf16(const void *grad_out, const void *x, void *grad_weight, void *grad_bias, int M, int N, int K,
+                                           int splits, int device, void *stream) {
+  if (splits < 1 || N % splits || N / splits % 8)
+    return set_error(F3D_ERR_ARG, "linear_wgrad: N = %d in %d matrices of a multiple of 8 columns", N, splits);
   if (M <= 0 || N <= 0 || K <= 0) return set_error(F3D_ERR_ARG, "linear_wgrad: M, N, K must be positive (got %d, %d, %d)", M, N, K);
   if (N % 8) return set_error(F3D_ERR_ARG, "linear_wgrad: N = %d must be a multiple of 8", N);
   if (K != 32 && K % 64) return set_error(F3D_ERR_UNSUPPORTED, "linear_wgrad: K = %d must be 32 or a multiple of 64", K);
@@ -216,12 +237,13 @@ extern "C" int f3d_linear_wgrad_bf16(const void *grad_out, const void *x, void *
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   WgradArgs a{};
   a.M = M; a.N = N; a.K = K;
+  a.splits = splits; a.C = N / splits; a.pps = (a.C + 63) / 64;
   a.rb = K == 32 ? 64 : 128;
   const int panels_total = K == 32 ? 1 : K / 64;
   a.x_panels = panels_total < 4 ? panels_total : 4;
   if (panels_total % a.x_panels) a.x_panels = panels_total % 2 == 0 ? 2 : 1;
   a.k_tiles = panels_total / a.x_panels;
-  a.n_tiles = (N + 127) / 128;
+  a.n_tiles = (splits * a.pps + 1) / 2;
   const int tiles = a.n_tiles * a.k_tiles;
   const int total_blocks = (M + kWgRows - 1) / kWgRows;
   // one CTA per SM (a CTA's fixed costs - tensor-memory allocation, filling the ring, writing its partial tile - are
@@ -240,10 +262,10 @@ extern "C" int f3d_linear_wgrad_bf16(const void *grad_out, const void *x, void *
   a.status = status_word(device);
   if (!a.status) return F3D_ERR_CUDA;
   CUtensorMap mg, mx;
-  F3D_TRY(encode_tmap_2d(&mg, 0, grad_out, (uint64_t)N, (uint64_t)M, (uint64_t)N * 2, 64, kWgRows, 128));
+  F3D_TRY(encode_tmap_3d(&mg, 0, grad_out, (uint64_t)a.C, (uint64_t)M, (uint64_t)splits, (uint64_t)a.C * 2, (uint64_t)a.C * M * 2, 64, kWgRows, 1, 128));
   F3D_TRY(encode_tmap_2d(&mx, 0, x, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, K == 32 ? 32 : 64, kWgRows, K == 32 ? 64 : 128));
-  const int smem = kWgStages * (2 + a.x_panels) * kWgPanelBytes + 256 + 1024;
-  F3D_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(wgrad_tcgen05_kernel), device, kWgStages * 6 * kWgPanelBytes + 256 + 1024));
+  const int smem = kWgStages * (2 + a.x_panels) * kWgPanelBytes + 256 + 1024 + 1024;
+  F3D_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(wgrad_tcgen05_kernel), device, kWgStages * 6 * kWgPanelBytes + 256 + 1024 + 1024));
   dim3 grid(tiles, a.slabs);
   launch(wgrad_tcgen05_kernel, grid, kWgThreads, smem, st, mg, mx, a);
   F3D_TRY(check_launch("linear_wgrad"));

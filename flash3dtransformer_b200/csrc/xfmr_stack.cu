@@ -168,9 +168,6 @@ extern "C" int f3d_xfmr_block_bwd_bf16(const f3d_xfmr_block *blk, const f3d_xfmr
   F3D_TRY(f3d_buck_swin_bwd(q, q + mat, q + 2 * mat, t->attn, g_attn, t->lse, delta, gq, gq + mat, gq + 2 * mat, b.scopes, 1, m, b.heads, c / b.heads,
                             b.num_scopes, b.scope_size, (uint32_t)b.bucket, device, stream));
   F3D_TRY(f3d_linear_ksplit_bf16(gr->g_qkv, gr->qkv_wt, nullptr, nullptr, g_n1, m, c, c, 3, device, stream));
-  if (gr->qkv_w)
-    for (int i = 0; i < 3; ++i)
-      F3D_TRY(f3d_linear_wgrad_bf16(gq + i * mat, t->n1, static_cast<float *>(gr->qkv_w) + (size_t)i * c * c,
-                                    gr->qkv_b ? static_cast<float *>(gr->qkv_b) + (size_t)i * c : nullptr, m, c, c, device, stream));
+  if (gr->qkv_w) F3D_TRY(f3d_linear_wgrad_split_bf16(gq, t->n1, gr->qkv_w, gr->qkv_b, m, 3 * c, c, 3, device, stream));
   return f3d_layernorm_bwd_add_bf16(t->x, g_n1, b.norm_w, gr->g_mid, gr->grad_x, gr->norm_w, gr->norm_b, rows, channels, b.norm_eps, device, stream);
 }

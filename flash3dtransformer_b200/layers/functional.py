@@ -250,6 +250,11 @@ def _split_backward(xb, weight, bias, wb, g):
     wt = bf16_weight_t(weight, s)
     gx = torch.empty(m, wb.shape[1], dtype=torch.bfloat16, device=g.device)
     pshattn.linear_ksplit_bf16(g, wt, gx)
+    if g.dtype == torch.bfloat16 and native_wgrad(c, xb.shape[1]):
+        gw = torch.empty(s * c, xb.shape[1], dtype=torch.float32, device=g.device)
+        gb = torch.empty(s * c, dtype=torch.float32, device=g.device) if bias is not None else None
+        pshattn.linear_wgrad_bf16(g, xb, gw, gb)
+        return gx, gw.to(weight.dtype), (gb.to(bias.dtype) if bias is not None else None), None, None, None
     parts = [_param_grads(g[i], xb, weight, bias[i * c:(i + 1) * c] if bias is not None else None) for i in range(s)]
     gw = torch.cat([p[0] for p in parts], dim=0)
     gb = torch.cat([p[1] for p in parts], dim=0) if bias is not None else None

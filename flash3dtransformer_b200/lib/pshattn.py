@@ -469,23 +469,25 @@ def wgrad_supported(n: int, k: int) -> bool:
 
 def linear_wgrad_bf16(grad_out, x, grad_weight, grad_bias=None) -> None:
     """grad_weight fp32 [N, K] = grad_out^T @ x and grad_bias fp32 [N] = grad_out.sum(0) for bf16 grad_out [M, N] and
-    x [M, K]: the parameter gradients of a projection in one pass over both operands, added in a fixed order."""
+    x [M, K]: the parameter gradients of a projection in one pass over both operands, added in a fixed order.  grad_out may
+    be [S, M, N / S], the gradients of S outputs whose weights lie one below the other."""
     ts, names = [grad_out, x, grad_weight], ["grad_out", "x", "grad_weight"]
     if grad_bias is not None:
         ts.append(grad_bias); names.append("grad_bias")
     dev = _check_tensors(ts, names)
     _check_dtype([grad_out, x], ["grad_out", "x"], torch.bfloat16)
     _check_dtype(ts[2:], names[2:], torch.float32)
-    if not (grad_out.dim() == 2 and x.dim() == 2 and grad_out.shape[0] == x.shape[0]):
-        raise RuntimeError("grad_out must be [M, N] and x [M, K]")
-    m, n = grad_out.shape
+    if not (grad_out.dim() in (2, 3) and x.dim() == 2 and grad_out.shape[-2] == x.shape[0]):
+        raise RuntimeError("grad_out must be [M, N] (or [S, M, N / S]) and x [M, K]")
+    splits = grad_out.shape[0] if grad_out.dim() == 3 else 1
+    m, n = grad_out.shape[-2], grad_out.shape[-1] * splits
     k = x.shape[1]
     if tuple(grad_weight.shape) != (n, k):
         raise RuntimeError(f"grad_weight must be [{n},{k}]")
     if not (grad_bias is None or grad_bias.numel() == n):
         raise RuntimeError(f"grad_bias must have {n} elements")
-    st = _cabi.load().f3d_linear_wgrad_bf16(_ptr(grad_out), _ptr(x), _ptr(grad_weight), _ptr(grad_bias) if grad_bias is not None else None,
-                                            m, n, k, dev, _stream(dev))
+    st = _cabi.load().f3d_linear_wgrad_split_bf16(_ptr(grad_out), _ptr(x), _ptr(grad_weight), _ptr(grad_bias) if grad_bias is not None else None,
+                                                  m, n, k, splits, dev, _stream(dev))
     _cabi.check(st, "linear_wgrad_bf16")
 
 

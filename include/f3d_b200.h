@@ -370,6 +370,8 @@ int f3d_coord_embed_bwd(const void *coords, const void *grad_out, void *grad_wei
  * not NULL, grad_bias fp32 [N] = column sums of grad_out, for grad_out bf16 [M, N] and x bf16 [M, K] (both dense).  One
  * pass over grad_out and x on the tensor cores (neither is transposed in memory), sums over row slabs added in a fixed
  * order.  N a multiple of 8; K = 32 or a multiple of 64. */
+int f3d_linear_wgrad_split_bf16(const void *grad_out, const void *x, void *grad_weight, void *grad_bias, int M, int N, int K, int splits,
+                                int device, void *stream);      /* grad_out = [splits][M][N / splits] */
 int f3d_linear_wgrad_bf16(const void *grad_out, const void *x, void *grad_weight, void *grad_bias, int M, int N, int K,
                           int device, void *stream);
 

@@ -343,3 +343,20 @@ def test_linear_swiglu_gradient(cuda_device, m, n, k, bias):
     gate, up = y.chunk(2, dim=1)
     ref, = torch.autograd.grad(torch.nn.functional.silu(gate) * up, y, go.float())
     _check(out, ref)
+
+
+@pytest.mark.parametrize("m,s,c,k", [(1000, 3, 32, 32), (777, 3, 64, 64), (1, 3, 64, 128), (2049, 3, 96, 192), (500, 3, 256, 256), (640, 2, 40, 512),
+                                     (129, 5, 128, 320)])
+def test_linear_wgrad_of_split_outputs(cuda_device, m, s, c, k):
+    """The gradients of several outputs in one launch: 128-row tiles that end inside, at the end of and across the outputs."""
+    from flash3dtransformer_b200.lib import pshattn
+    gen = torch.Generator(cuda_device).manual_seed(m + s * c + k)
+    g = torch.randn(s, m, c, device=cuda_device, generator=gen).bfloat16()
+    x = torch.randn(m, k, device=cuda_device, generator=gen).bfloat16()
+    gw, gb = torch.full((s * c, k), float("nan"), device=cuda_device), torch.full((s * c,), float("nan"), device=cuda_device)
+    pshattn.linear_wgrad_bf16(g, x, gw, gb)
+    pshattn.device_status()
+    ref_w = torch.einsum("smc,mk->sck", g.float(), x.float()).reshape(s * c, k)
+    ref_b = g.float().sum(1).reshape(-1)
+    assert torch.isfinite(gw).all() and (gw - ref_w).abs().max().item() <= 1e-4 * ref_w.abs().max().item() + 1e-5 * m ** 0.5
+    assert (gb - ref_b).abs().max().item() <= 1e-4 * ref_b.abs().max().item() + 1e-5 * m ** 0.5
