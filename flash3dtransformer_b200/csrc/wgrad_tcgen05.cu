@@ -13,8 +13,9 @@
 //
 // What bounds wide outputs is shared memory: a product takes A again for every instruction, so one instruction covers all
 // panels of x (N = 256: 12 KB read per 128 cycles of the tensor core; with one instruction a panel it was 24 KB per 128), and
-// the column sums read two columns a thread, one 128-byte row a warp.  200,704 rows, N = 2048, K = 256: 308 -> @@ us (141 at the
-// copy rate); 100,352 rows, N = K = 512: 103 -> @@.
+// the column sums read two columns a thread, one 128-byte row a warp.  200,704 rows, N = 2048, K = 256: 308 -> 208 us (141 at the
+// copy rate); 100,352 rows, N = K = 512: 103 -> 68.  Narrow ones are bound by the bytes in flight: their stages are small, so the
+// ring takes up to eight (1,605,632 rows, N = K = 32: 71 -> 66 us, 31 at the copy rate).
 //
 // Stands in for the library GEMM g^T x and the separate column-sum pass of the backward of nn.Linear / te.Linear in
 // flash3dxfmr/layers/buck_swin.py:159,163 and the MLP of flash3dxfmr/layers/elem_wise.py.
@@ -28,7 +29,7 @@ int *status_word(int device);
 
 constexpr int kWgThreads = 192;          // producer warp, MMA warp, four column-sum / epilogue warps
 constexpr int kWgRows = 64;              // rows (tokens) per stage
-constexpr int kWgStages = 4;
+constexpr int kWgMinStages = 4, kWgMaxStages = 8;
 constexpr int kWgPanelBytes = kWgRows * 128;      // 64 rows of 128 bytes
 
 struct WgradArgs {
@@ -37,6 +38,7 @@ struct WgradArgs {
   int rb;                 // bytes of one x row inside a panel: 128, or 64 when K == 32
   int x_panels;           // 64-column panels of x per k-tile (1..4)
   int k_tiles, n_tiles, slabs, blocks_per_slab;
+  int stages;             // of the ring
   float *partial_w;       // slab s: partial_w + s * slab_stride, [N][K]
   float *partial_b;       // slab s: partial_b + s * slab_stride, [N]; or null
   size_t slab_stride;     // floats per slab record (N * K weight sums, then N bias sums when wanted)
@@ -48,10 +50,10 @@ wgrad_tcgen05_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
   extern __shared__ unsigned char smem_raw[];
   unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int stage_bytes = (2 + a.x_panels) * kWgPanelBytes;
-  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + kWgStages * stage_bytes);
-  uint64_t *full = bars, *empty = bars + kWgStages, *acc_full = bars + 2 * kWgStages;
+  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + a.stages * stage_bytes);
+  uint64_t *full = bars, *empty = bars + kWgMaxStages, *acc_full = bars + 2 * kWgMaxStages;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_full + 1);
-  float2 *half_sums = reinterpret_cast<float2 *>(smem + kWgStages * stage_bytes + 256);     // [2][64] column sums of half the rows
+  float2 *half_sums = reinterpret_cast<float2 *>(smem + a.stages * stage_bytes + 256);     // [2][64] column sums of half the rows
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -67,7 +69,7 @@ wgrad_tcgen05_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
   const uint32_t tmem_cols = ncols <= 64 ? 64 : (ncols <= 128 ? 128 : 256);
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kWgStages; ++s) { tc::mbar_init(&full[s], 1); tc::mbar_init(&empty[s], 1 + 4); }
+    for (int s = 0; s < a.stages; ++s) { tc::mbar_init(&full[s], 1); tc::mbar_init(&empty[s], 1 + 4); }
     tc::mbar_init(acc_full, 1);
     *abort_flag = 0;
     tc::mbar_fence_init();
@@ -83,8 +85,8 @@ wgrad_tcgen05_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
   if (warp == 0) {
     if (tc::elect_one()) {
       tc::tma_prefetch_desc(&map_g); tc::tma_prefetch_desc(&map_x);
-      for (int i = 0; i < nblk; ++i) {
-        const uint32_t s = i % kWgStages, ph = (i / kWgStages) & 1u;
+      uint32_t s = 0, ph = 0;
+      for (int i = 0; i < nblk; ++i, ph ^= s + 1 == (uint32_t)a.stages, s = s + 1 == (uint32_t)a.stages ? 0u : s + 1) {
         if (!tc::mbar_wait(&empty[s], ph ^ 1u, wc, 401, 100)) break;
         unsigned char *st = smem + s * stage_bytes;
         const int r0 = (b0 + i) * kWgRows;
@@ -104,8 +106,8 @@ wgrad_tcgen05_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
       const uint32_t idesc = tc::make_idesc_f16(128, a.rb == 64 ? 32u : ncols, true, true, true);
       const uint64_t swz = a.rb == 64 ? tc::kSwizzle64 : tc::kSwizzle128;
       bool ok = true;
-      for (int i = 0; i < nblk && ok; ++i) {
-        const uint32_t s = i % kWgStages, ph = (i / kWgStages) & 1u;
+      uint32_t s = 0, ph = 0;
+      for (int i = 0; i < nblk && ok; ++i, ph ^= s + 1 == (uint32_t)a.stages, s = s + 1 == (uint32_t)a.stages ? 0u : s + 1) {
         if (!tc::mbar_wait(&full[s], ph, wc, 402)) { ok = false; break; }
         tc::tc_fence_after_sync();
         const uint32_t g_addr = tc::smem_u32(smem + s * stage_bytes), x_addr = g_addr + 2 * kWgPanelBytes;
@@ -131,8 +133,8 @@ wgrad_tcgen05_kernel(const __grid_constant__ CUtensorMap map_g, const __grid_con
     const uint32_t chunk = (uint32_t)lane >> 2;
     float2 bsum = make_float2(0.f, 0.f);
     bool ok = true;
-    for (int i = 0; i < nblk && ok; ++i) {
-      const uint32_t s = i % kWgStages, ph = (i / kWgStages) & 1u;
+    uint32_t s = 0, ph = 0;
+    for (int i = 0; i < nblk && ok; ++i, ph ^= s + 1 == (uint32_t)a.stages, s = s + 1 == (uint32_t)a.stages ? 0u : s + 1) {
       // also without a bias gradient the warps follow the ring stage by stage: the stage's release counts them
       if (!tc::mbar_wait(&full[s], ph, wc, 403)) { ok = false; break; }
       if (want_bias) {
@@ -264,8 +266,11 @@ extern "C" int f3d_linear_wgrad_split_bf16(const void *grad_out, const void *x, 
   CUtensorMap mg, mx;
   F3D_TRY(encode_tmap_3d(&mg, 0, grad_out, (uint64_t)a.C, (uint64_t)M, (uint64_t)splits, (uint64_t)a.C * 2, (uint64_t)a.C * M * 2, 64, kWgRows, 1, 128));
   F3D_TRY(encode_tmap_2d(&mx, 0, x, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, K == 32 ? 32 : 64, kWgRows, K == 32 ? 64 : 128));
-  const int smem = kWgStages * (2 + a.x_panels) * kWgPanelBytes + 256 + 1024 + 1024;
-  F3D_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(wgrad_tcgen05_kernel), device, kWgStages * 6 * kWgPanelBytes + 256 + 1024 + 1024));
+  // four stages of the widest tile fill the shared memory; narrower ones get more, as many bytes in flight as fit
+  const int stage_bytes = (2 + a.x_panels) * kWgPanelBytes, room = kWgMinStages * 6 * kWgPanelBytes;
+  a.stages = room / stage_bytes < kWgMaxStages ? room / stage_bytes : kWgMaxStages;
+  const int smem = a.stages * stage_bytes + 256 + 1024 + 1024;
+  F3D_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(wgrad_tcgen05_kernel), device, room + 256 + 1024 + 1024));
   dim3 grid(tiles, a.slabs);
   launch(wgrad_tcgen05_kernel, grid, kWgThreads, smem, st, mg, mx, a);
   F3D_TRY(check_launch("linear_wgrad"));

@@ -137,10 +137,10 @@ class CoordEmbedFn(Function):
         return None, gw.to(ctx.dtypes[0]), gb.to(ctx.dtypes[1])
 
 
-# Largest weight (elements) whose gradient goes to the native kernel: above it the output tiles outnumber the SMs, the
-# operands are re-read once per tile column, and the library's split-K GEMM measured faster (N x K = 4096 x 512: 198
-# against 98 us; 2048 x 256 and below: 40-100 us against 48-127 us).
-_WGRAD_MAX_ELEMS = 512 * 1024
+# Largest weight (elements) whose gradient goes to the native kernel, the largest one measured against the library's product
+# and the separate column sums: N x K = 4096 x 512 405 against 498 us at 100,352 rows, 67 against 119 at 11,456; 512 x 2048
+# 200 against 197 and 38 against 43.  Past it the output tiles outnumber the SMs and the operands are read once per tile column.
+_WGRAD_MAX_ELEMS = 2 * 1024 * 1024
 
 
 def native_wgrad(n: int, k: int) -> bool:
