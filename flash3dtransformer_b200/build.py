@@ -3,7 +3,8 @@
 Every .cu file under csrc/ is compiled to an object (only when its sources changed) and linked into
 flash3dtransformer_b200/lib/libf3d_b200.so.  No torch, pybind or glog dependency enters the library; it
 links the static CUDA runtime only; driver entry points (cuTensorMapEncodeTiled) are resolved at run time
-through cudaGetDriverEntryPoint, so the library also loads on a machine without a GPU driver.
+through cudaGetDriverEntryPoint, so the library also loads on a machine without a GPU driver.  Beside it csrc/host is
+compiled with the host compiler into lib/_f3d_host.so, a Python module that takes torch tensors and calls the library.
 
 Usage: python -m flash3dtransformer_b200.build [--force] [--verbose]
 """
@@ -14,6 +15,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -22,6 +24,8 @@ CSRC = PKG / "csrc"
 OUT_DIR = PKG / "lib"
 OBJ_DIR = PKG / "csrc" / "build"
 LIB = OUT_DIR / "libf3d_b200.so"
+HOST_SRC = CSRC / "host" / "f3d_host.cpp"
+HOST_LIB = OUT_DIR / "_f3d_host.so"
 INCLUDE = PKG.parent / "include"
 
 NVCC_FLAGS = [
@@ -65,6 +69,26 @@ def _compile_one(src: Path, force: bool, verbose: bool) -> tuple[Path, bool, str
     return obj, True, res.stderr if verbose else ""
 
 
+def _build_host(force: bool) -> None:
+    import torch
+    root = Path(torch.__file__).resolve().parent
+    cuda = Path(_nvcc()).resolve().parent.parent
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-isystem", str(root / "include"), "-isystem", str(root / "include" / "torch" / "csrc" / "api" / "include"),
+           "-isystem", sysconfig.get_paths()["include"], "-isystem", str(cuda / "include"), str(HOST_SRC), "-o", str(HOST_LIB),
+           "-L", str(root / "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
+    h = hashlib.sha256(" ".join(cmd + [torch.__version__, sys.version]).encode())
+    for d in [HOST_SRC] + sorted(INCLUDE.glob("*.h")):
+        h.update(d.read_bytes())
+    stamp = OBJ_DIR / "f3d_host.sha"
+    if not force and HOST_LIB.exists() and stamp.exists() and stamp.read_text() == h.hexdigest():
+        return
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"{HOST_SRC.name} failed:\n{res.stdout}\n{res.stderr}")
+    stamp.write_text(h.hexdigest())
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
     OBJ_DIR.mkdir(parents=True, exist_ok=True)
     OUT_DIR.mkdir(parents=True, exist_ok=True)
@@ -83,6 +107,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         res = subprocess.run(cmd, capture_output=True, text=True)
         if res.returncode != 0:
             raise RuntimeError(f"link failed:\n{res.stdout}\n{res.stderr}")
+    _build_host(force)
     return LIB
 
 

@@ -5,6 +5,8 @@ There is no CPU fallback: if the shared library is missing or a call fails, a Ru
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 from ctypes import c_char_p, c_float, c_int, c_uint32, c_uint64, c_void_p
 from pathlib import Path
@@ -111,6 +113,37 @@ def load() -> ctypes.CDLL:
         fn.argtypes = args
     _lib = lib
     return lib
+
+
+class _NoHost:
+    """Stands in for the host module where it was not built: every call goes through ctypes."""
+
+    @staticmethod
+    def _none(*_):
+        return None
+
+    linear = swin_fwd = scatter = index = bbox = _none
+
+
+_host = None
+
+
+def host():
+    """The module of csrc/host: operator calls with their checks in native code.  A function returns the status of the call, or
+    None for arguments that it leaves to the checks in Python."""
+    global _host
+    if _host is None:
+        lib = load()
+        try:
+            loader = importlib.machinery.ExtensionFileLoader("_f3d_host", os.fspath(LIB_PATH.with_name("_f3d_host.so")))
+            mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_f3d_host", loader))
+            loader.exec_module(mod)
+            mod.bind(*[ctypes.cast(getattr(lib, n), c_void_p).value for n in (
+                "f3d_linear_dtype", "f3d_buck_swin_fwd_dtype", "f3d_batch_psh_scatter_pad_hash", "f3d_scatter_index", "f3d_bbox_f16")])
+            _host = mod
+        except ImportError:                  # not built, or built for another torch
+            _host = _NoHost
+    return _host
 
 
 def is_loaded() -> bool:

@@ -132,6 +132,10 @@ def batch_psh_scatter_pad_hash(coord, bucket_id, bucket_counter, bucket_offset, 
                                num_bucket, bucket_divisor, bucket_size, num_vox, bbox_min, bbox_max,
                                probe_offsets, cumsum_counter, scatter_coord, pad_num, hash_type) -> None:
     """f3d::batch_psh_scatter_pad_hash (src/psh/batch_psh_bucket_dispatcher.cu:221-326)."""
+    st = _cabi.host().scatter(coord, bucket_id, bucket_counter, bucket_offset, batch_sep, instance_max_N, num_bucket, bucket_divisor,
+                               bucket_size, num_vox, bbox_min, bbox_max, probe_offsets, cumsum_counter, scatter_coord, pad_num, hash_type)
+    if st is not None:
+        return _cabi.check(st, "batch_psh_scatter_pad_hash")
     names = ["coord", "bucket_id", "bucket_counter", "bucket_offset", "batch_sep", "probe_offsets",
              "cumsum_counter", "scatter_coord", "bbox_min", "bbox_max"]
     tensors = [coord, bucket_id, bucket_counter, bucket_offset, batch_sep, probe_offsets, cumsum_counter,
@@ -376,6 +380,9 @@ def linear_bf16(x, weight, bias, out, residual=None, nsplit=1, epilogue=EPI_NONE
     float16 (float16 is the element type of the reference's CPU-runnable configuration; forward only).  Not part of
     the reference's operator module: the reference leaves these projections to nn.Linear / cuBLAS
     (flash3dxfmr/layers/buck_swin.py:159,163)."""
+    st = _cabi.host().linear(x, weight, bias, out, residual, nsplit, epilogue)
+    if st is not None:
+        return _cabi.check(st, "linear_bf16")
     tensors, names = [x, weight, out], ["x", "weight", "out"]
     if residual is not None:
         tensors.append(residual); names.append("residual")
@@ -539,6 +546,9 @@ def buck_swin_fwd(Q, K, V, O, L, Scope_buckets, bucket_size) -> None:
     """f3d::buck_swin_fwd (declared src/f3d_frontend.cu:90-92; caller flash3dxfmr/layers/buck_swin.py:57).
     O[B,L,H,D] and the log-sum-exp L[B,L,H] are written in place.  Q, K, V, O are bfloat16 or float16 (all the
     same)."""
+    st = _cabi.host().swin_fwd(Q, K, V, O, L, Scope_buckets, bucket_size)
+    if st is not None:
+        return _cabi.check(st, "buck_swin_fwd")
     dev, (b, l, h, d) = _check_qkv([Q, K, V, O], ["Q", "K", "V", "O"], (torch.bfloat16, torch.float16))
     _check_tensors([L, Scope_buckets], ["L", "Scope_buckets"])
     _check_dtype([L], ["L"], torch.float32)
@@ -702,6 +712,9 @@ def collate_points_f32(records, coords, extra=None) -> None:
 
 def bbox_f16(coords, bbox_min, bbox_max) -> None:
     """bbox_min / bbox_max fp16 [3] = the bounding box of fp16 coords [rows, 3], rows > 0."""
+    st = _cabi.host().bbox(coords, bbox_min, bbox_max)
+    if st is not None:
+        return _cabi.check(st, "bbox_f16")
     dev = _check_tensors([coords, bbox_min, bbox_max], ["coords", "bbox_min", "bbox_max"])
     _check_dtype([coords, bbox_min, bbox_max], ["coords", "bbox_min", "bbox_max"], torch.float16)
     if coords.dim() != 2 or coords.shape[1] != 3 or bbox_min.numel() != 3 or bbox_max.numel() != 3:
@@ -714,6 +727,9 @@ def scatter_index(bucket_id, bucket_offset, cumsum_counter, batch_sep, out2in, i
     batch_psh_cumsum_scatter_feat_index_postpad_ker, src/psh/batch_psh_bucket.cuh:667) and, when given,
     in2out[input row] = row in bucket order, from the outputs of batch_psh_scatter.  The reference declares the
     operator that would fill scatter_idx_out2in but never binds it."""
+    st = _cabi.host().index(bucket_id, bucket_offset, cumsum_counter, batch_sep, out2in, in2out)
+    if st is not None:
+        return _cabi.check(st, "scatter_index")
     ts = [bucket_id, bucket_offset, cumsum_counter, batch_sep, out2in] + ([in2out] if in2out is not None else [])
     dev = _check_tensors(ts, ["bucket_id", "bucket_offset", "cumsum_counter", "batch_sep", "out2in", "in2out"][:len(ts)])
     _check_dtype([bucket_id], ["bucket_id"], torch.uint16)
