@@ -183,6 +183,32 @@ PyObject *bbox(PyObject *, PyObject *const *a, Py_ssize_t n) {
   });
 }
 
+// empties(device, code, rows, cols, code, rows, cols, ...): uninitialised tensors [rows, cols], or [rows] where cols is 0; code 0
+// uint16, 1 uint32, 2 float16.  None where a tensor cannot be made here.
+PyObject *empties(PyObject *, PyObject *const *a, Py_ssize_t n) {
+  if (n < 4 || n % 3 != 1 || n > 31) Py_RETURN_NONE;
+  at::Tensor out[10];
+  const Py_ssize_t count = n / 3;
+  try {
+    const at::Device dev(at::kCUDA, (c10::DeviceIndex)u32(a[0]));
+    for (Py_ssize_t i = 0; i < count; ++i) {
+      const long long code = integer(a[3 * i + 1]), rows = integer(a[3 * i + 2]), cols = integer(a[3 * i + 3]);
+      want(code >= 0 && code < 3 && rows >= 0 && cols >= 0);
+      const at::TensorOptions opt = at::TensorOptions().device(dev).dtype(code == 0 ? at::kUInt16 : code == 1 ? at::kUInt32 : at::kHalf);
+      const int64_t size[2] = {rows, cols};
+      out[i] = at::empty(at::IntArrayRef(size, cols ? 2 : 1), opt);
+    }
+  } catch (const Bad &) {
+    Py_RETURN_NONE;
+  } catch (const std::exception &) {           // the caller's own allocation raises it
+    Py_RETURN_NONE;
+  }
+  PyObject *const t = PyTuple_New(count);
+  if (!t) return nullptr;
+  for (Py_ssize_t i = 0; i < count; ++i) PyTuple_SET_ITEM(t, i, THPVariable_Wrap(std::move(out[i])));
+  return t;
+}
+
 // bind(linear, swin_fwd, scatter, index, bbox): addresses of the C entry points
 PyObject *bind(PyObject *, PyObject *const *a, Py_ssize_t n) {
   void *p[5];
@@ -201,7 +227,7 @@ PyObject *bind(PyObject *, PyObject *const *a, Py_ssize_t n) {
 
 #define F3D_METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(name)), METH_FASTCALL, nullptr}
 PyMethodDef g_methods[] = {F3D_METHOD(linear), F3D_METHOD(swin_fwd), F3D_METHOD(scatter), F3D_METHOD(index),
-                           F3D_METHOD(bbox), F3D_METHOD(bind), {nullptr, nullptr, 0, nullptr}};
+                           F3D_METHOD(bbox), F3D_METHOD(empties), F3D_METHOD(bind), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_f3d_host", nullptr, -1, g_methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

@@ -29,7 +29,8 @@
 // on global memory and no inter-CTA waiting: seven launches (key + histogram, scan, round A ranks + probe walk, scan,
 // round B resolution, scan, round C ranks + scatter) over tiles of 2048 points, so that even one scan of 120,000
 // points spreads over 59 CTAs and a batch fills every SM.  The first-hash key of a point is computed once (kernel 1)
-// and kept as 16 bits in scratch; the rank kernels read keys, not coordinates.  The scan kernel turns a round's table
+// and kept as 16 bits in scratch; the rank kernels read keys, not coordinates.  Batches whose tables are small leave the scans
+// and the clearing of the tables out: every tile adds up the columns itself (see psh_run), which makes four launches.  The scan kernel turns a round's table
 // of per-tile counts into per-tile exclusive prefixes in place, one warp per (scene, bucket) column, and writes the
 // scene totals.  Warps own contiguous index ranges; equal keys inside a warp are merged with match_any
 // (warp-aggregated counting), per-warp counters live in shared memory, and coordinates are staged into shared memory
@@ -75,6 +76,7 @@ struct PshArgs {
   const __half *bbox_min; const __half *bbox_max; const int16_t *probe;
   uint32_t total_N, batch, nb, nbp, divisor, cap, num_vox, hash_type, pad_to;
   uint32_t tile, tiles_max;
+  uint32_t direct;         // 1: no scan launches, every tile sums the (small) tables itself
   uint16_t pad_bits; uint16_t coord_aligned; uint16_t out_aligned;
   RngKey key;
   uint32_t scene_base;     // added to the scene index in the random-number counter (global scene id of a shard)
@@ -190,6 +192,43 @@ __device__ __forceinline__ TileInfo tile_info(const PshArgs &a) {
   return t;
 }
 
+__device__ __forceinline__ uint32_t scene_tiles(const PshArgs &a, uint32_t scene) {
+  uint32_t start = scene ? a.batch_sep[scene - 1] : 0u;
+  uint32_t end = min(a.batch_sep[scene], a.total_N);
+  uint32_t n = end > start ? end - start : 0u;
+  return (n + a.tile - 1) / a.tile;
+}
+
+// Direct mode: sums of every column of a tile table over the scene's tiles in front of this one (pre) and over all of them
+// (tot), into shared memory.  A warp takes four columns at a time, a lane up to three of a column's words, so that twelve
+// loads are in flight.
+constexpr uint32_t kDirectTiles = 96, kDirectWords = 8192;
+__device__ __forceinline__ void column_sums(const PshArgs &a, const TileInfo &t, const uint32_t *tab, uint32_t *pre, uint32_t *tot) {
+  const uint32_t tiles = scene_tiles(a, t.scene), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (uint32_t b0 = warp * 4; b0 < a.nbp; b0 += kPshWarps * 4) {
+    uint32_t v[4][kDirectTiles / 32];
+#pragma unroll
+    for (uint32_t c = 0; c < 4; ++c)
+#pragma unroll
+      for (uint32_t j = 0; j < kDirectTiles / 32; ++j) {
+        const uint32_t i = j * 32 + lane;
+        v[c][j] = b0 + c < a.nbp && i < tiles ? tab[tab_at(a, t.scene, b0 + c, i)] : 0u;
+      }
+#pragma unroll
+    for (uint32_t c = 0; c < 4; ++c) {
+      uint32_t all = 0, front = 0;
+#pragma unroll
+      for (uint32_t j = 0; j < kDirectTiles / 32; ++j) {
+        all += v[c][j];
+        front += j * 32 + lane < t.tile ? v[c][j] : 0u;
+      }
+      all = __reduce_add_sync(0xFFFFFFFFu, all);
+      front = __reduce_add_sync(0xFFFFFFFFu, front);
+      if (lane == 0 && b0 + c < a.nbp) { pre[b0 + c] = front; tot[b0 + c] = all; }
+    }
+  }
+}
+
 // warp-aggregated counting of one key per lane (all 32 lanes call)
 __device__ __forceinline__ void warp_count(uint16_t *wh, uint32_t key, bool valid, int lane) {
   uint32_t peers = __match_any_sync(0xFFFFFFFFu, valid ? key : 0xFFFFFFFFu);
@@ -261,7 +300,11 @@ __global__ void __launch_bounds__(kPshThreads) psh_hist_kernel(PshArgs a) {
     }
   }
   __syncthreads();
-  for (uint32_t b = threadIdx.x; b < a.nbp; b += kPshThreads) a.tabA[tab_at(a, t.scene, b, t.tile)] = s.aux[b];
+  for (uint32_t b = threadIdx.x; b < a.nbp; b += kPshThreads) {
+    const size_t at = tab_at(a, t.scene, b, t.tile);
+    a.tabA[at] = s.aux[b];
+    if (a.direct) { a.tabB[at] = 0; a.tabC[at] = 0; }
+  }
 }
 
 // ---------------------------------------------------------------------------------------------------------
@@ -286,13 +329,6 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t *wsum /
   *tot = wsum[kPshWarps];
   __syncthreads();
   return ex;
-}
-
-__device__ __forceinline__ uint32_t scene_tiles(const PshArgs &a, uint32_t scene) {
-  uint32_t start = scene ? a.batch_sep[scene - 1] : 0u;
-  uint32_t end = min(a.batch_sep[scene], a.total_N);
-  uint32_t n = end > start ? end - start : 0u;
-  return (n + a.tile - 1) / a.tile;
 }
 
 // ---------------------------------------------------------------------------------------------------------
@@ -346,10 +382,21 @@ __global__ void __launch_bounds__(kPshThreads) psh_rankA_kernel(PshArgs a) {
   // rank base of this tile (the scanned round A table) and the scene's kept counts: requested first, so that their
   // latency runs under the counting sweep
   const uint32_t so = t.scene * a.nbp;
-  for (uint32_t b = threadIdx.x; b < a.nbp; b += kPshThreads) {
-    s.aux4[b] = 0;
-    s.tbase[b] = a.tabA[tab_at(a, t.scene, b, t.tile)];
-    s.aux[b] = a.kept[so + b];
+  if (a.direct) {
+    column_sums(a, t, a.tabA, s.tbase, s.aux);
+    __syncthreads();
+    for (uint32_t b = threadIdx.x; b < a.nbp; b += kPshThreads) {
+      const uint32_t all = s.aux[b], kept = b == kRecycleBucket ? all : min(all, a.cap);
+      s.aux4[b] = 0;
+      s.aux[b] = kept;
+      if (t.tile == 0) { a.count0[so + b] = all; a.kept[so + b] = kept; }
+    }
+  } else {
+    for (uint32_t b = threadIdx.x; b < a.nbp; b += kPshThreads) {
+      s.aux4[b] = 0;
+      s.tbase[b] = a.tabA[tab_at(a, t.scene, b, t.tile)];
+      s.aux[b] = a.kept[so + b];
+    }
   }
   if (threadIdx.x == 0) pending_cnt = 0;
   __syncthreads();
@@ -520,13 +567,17 @@ __global__ void __launch_bounds__(kPshThreads) psh_resolveB_kernel(PshArgs a) {
   // Round B totals of the scene from the attempt table: rank base of this tile (tbase), free capacity (aux),
   // kept count (aux2), recycle offset of the first rejected attempt per bucket (aux3).  The tile-0 CTA also
   // publishes the bucket counts after round B.
+  if (a.direct) {
+    column_sums(a, t, a.tabB, s.tbase, s.aux4);
+    __syncthreads();
+  }
   {
     uint32_t carry = 0;
     for (uint32_t b0 = 0; b0 < a.nbp; b0 += kPshThreads) {
       const uint32_t b = b0 + threadIdx.x;
       uint32_t rej = 0;
       if (b < a.nbp) {
-        const uint32_t pre = a.tabB[tab_at(a, t.scene, b, t.tile)], att = a.attB[so + b];
+        const uint32_t pre = a.direct ? s.tbase[b] : a.tabB[tab_at(a, t.scene, b, t.tile)], att = a.direct ? s.aux4[b] : a.attB[so + b];
         const uint32_t kept = a.kept[so + b];
         const uint32_t fr = (b != kRecycleBucket && b < a.nb && kept < a.cap) ? a.cap - kept : 0u;
         const uint32_t acc = min(att, fr);
@@ -677,13 +728,17 @@ __global__ void __launch_bounds__(kPshThreads) psh_scatter_kernel(PshArgs a) {
   const uint32_t gbase = t.start + t.t0;
   // Round C totals of the scene: final bucket sizes, their exclusive cumsum (aux = first row of each bucket inside
   // the scene) and the rank base of this tile's movers (tbase).  The tile-0 CTA writes the two counter outputs.
+  if (a.direct) {
+    column_sums(a, t, a.tabC, s.tbase, s.aux4);
+    __syncthreads();
+  }
   {
     uint32_t carry = 0;
     for (uint32_t b0 = 0; b0 < a.nbp; b0 += kPshThreads) {
       const uint32_t b = b0 + threadIdx.x;
       uint32_t fin = 0;
       if (b < a.nbp) {
-        const uint32_t pre = a.tabC[tab_at(a, t.scene, b, t.tile)], mv = a.movC[so + b];
+        const uint32_t pre = a.direct ? s.tbase[b] : a.tabC[tab_at(a, t.scene, b, t.tile)], mv = a.direct ? s.aux4[b] : a.movC[so + b];
         const uint32_t cb = a.cntB[so + b];
         if (b == kRecycleBucket) fin = (a.nb > 1) ? min(cb, a.cap) : cb;
         else if (b < a.nb) fin = cb + mv;
@@ -847,14 +902,17 @@ static int psh_run(PshArgs a, const PshPlan &p, uint32_t *scratch, uint32_t max_
   const unsigned scan_blocks = (unsigned)(((size_t)a.batch * p.nbp + kPshWarps - 1) / kPshWarps);
   // the round A table is fully rewritten by the histogram kernel for live tiles; the round B and C tables are
   // accumulated with atomics and must start at zero (they are adjacent: one memset)
+  // Small tables (a scan of 20,000 points: 79 tiles x 80 columns) cost a tile less to add up by itself, 32 words a thread at
+  // the limit, than a scan launch costs the stream and the host: four launches instead of seven and a memset.
+  a.direct = p.tiles_max <= kDirectTiles && (size_t)p.tiles_max * p.nbp <= kDirectWords;
   if (max_n > 0) {
-    F3D_CUDA_TRY(cudaMemsetAsync(a.tabB, 0, 2 * rows * p.nbp * sizeof(uint32_t), st));
+    if (!a.direct) F3D_CUDA_TRY(cudaMemsetAsync(a.tabB, 0, 2 * rows * p.nbp * sizeof(uint32_t), st));
     launch(psh_hist_kernel, grid, kPshThreads, p.smem_hist, st, a);
-    launch(psh_scan_kernel, scan_blocks, kPshThreads, 0, st, a, 0);
+    if (!a.direct) launch(psh_scan_kernel, scan_blocks, kPshThreads, 0, st, a, 0);
     launch(psh_rankA_kernel, grid, kPshThreads, p.smem_rank, st, a);
-    launch(psh_scan_kernel, scan_blocks, kPshThreads, 0, st, a, 1);
+    if (!a.direct) launch(psh_scan_kernel, scan_blocks, kPshThreads, 0, st, a, 1);
     launch(psh_resolveB_kernel, grid, kPshThreads, p.smem_rank, st, a);
-    launch(psh_scan_kernel, scan_blocks, kPshThreads, 0, st, a, 2);
+    if (!a.direct) launch(psh_scan_kernel, scan_blocks, kPshThreads, 0, st, a, 2);
   } else {
     F3D_CUDA_TRY(cudaMemsetAsync(a.bucket_counter, 0, (size_t)a.batch * a.nb * 4, st));
     F3D_CUDA_TRY(cudaMemsetAsync(a.cumsum_counter, 0, (size_t)a.batch * a.nb * 4, st));
@@ -868,7 +926,7 @@ static int psh_run(PshArgs a, const PshPlan &p, uint32_t *scratch, uint32_t max_
     a.tiles_max = p.tiles_max;
     launch(psh_scatter_kernel, grid2, kPshThreads, p.smem_rank, st, a);
   }
-  return check_launch("psh kernels", (max_n > 0 ? 6 : 0) + (gx > 0 ? 1 : 0));
+  return check_launch("psh kernels", (max_n > 0 ? (a.direct ? 3 : 6) : 0) + (gx > 0 ? 1 : 0));
 }
 
 // The kernel arguments of one PSH call from the C-ABI arguments (shared by the two entry points below).

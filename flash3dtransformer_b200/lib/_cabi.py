@@ -122,7 +122,7 @@ class _NoHost:
     def _none(*_):
         return None
 
-    linear = swin_fwd = scatter = index = bbox = _none
+    linear = swin_fwd = scatter = index = bbox = empties = _none
 
 
 _host = None

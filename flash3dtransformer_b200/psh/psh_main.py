@@ -20,7 +20,7 @@ from . import batching as f3dbatch
 from . import bucket as f3dbuck
 from . import dev_context as f3ddev
 from . import plan as f3dplan
-from ..lib import pshattn
+from ..lib import _cabi, pshattn
 
 NUM_VOX = 0xFFFF
 
@@ -72,6 +72,9 @@ class BucketScatterBuffers:
                 probe_offs=f3dbuck.generate_probe_offsets(dev, row_major=True),
                 scattered_coord=torch.empty((pad_to, d), dtype=torch.float16, device=dev)))
         if not fill:
+            new = _cabi.host().empties(dev.index, 0, total_n, 0, 1, b, num_buck, 1, total_n, 0, 1, b, num_buck, 2, pad_to, d) if total_n and coords.is_cuda else None
+            if new is not None:
+                return BucketScatterBuffers(new[0], new[1], new[2], new[3], f3dbuck.generate_probe_offsets(dev, row_major=True), new[4])
             return BucketScatterBuffers(
                 bucket_id=torch.empty(total_n, dtype=torch.uint16, device=dev),
                 bucket_cntr=torch.empty(b, num_buck, dtype=torch.uint32, device=dev),
@@ -119,7 +122,8 @@ def bounding_box(coords: torch.Tensor):
     """(min, max) fp16 [3] over all rows."""
     if coords.dtype != torch.float16 or coords.dim() != 2 or coords.shape[1] != 3 or coords.shape[0] == 0 or not coords.is_contiguous():
         return torch.aminmax(coords, dim=0)
-    bbox_min, bbox_max = torch.empty(2, 3, dtype=torch.float16, device=coords.device).unbind(0)
+    box = _cabi.host().empties(coords.get_device(), 2, 3, 0, 2, 3, 0) if coords.is_cuda else None
+    bbox_min, bbox_max = box if box is not None else torch.empty(2, 3, dtype=torch.float16, device=coords.device).unbind(0)
     pshattn.bbox_f16(coords, bbox_min, bbox_max)
     return bbox_min, bbox_max
 
@@ -131,7 +135,9 @@ def scatter_index(buffers: BucketScatterBuffers, seps: torch.Tensor, pad_to: int
     at the index (batch_psh_bucket.cuh:735)."""
     n = buffers.bucket_id.numel()
     dev = buffers.bucket_id.device
-    out2in = torch.empty(pad_to, dtype=torch.uint32, device=dev)
-    in2out = torch.empty(n, dtype=torch.uint32, device=dev) if inverse else None
+    new = _cabi.host().empties(dev.index, 1, pad_to, 0, 1, n, 0) if inverse and n and dev.type == "cuda" else None
+    if new is None:
+        new = (torch.empty(pad_to, dtype=torch.uint32, device=dev), torch.empty(n, dtype=torch.uint32, device=dev) if inverse else None)
+    out2in, in2out = new
     pshattn.scatter_index(buffers.bucket_id, buffers.bucket_offs, buffers.bucket_cumsum, seps, out2in, in2out)
     return out2in, in2out

@@ -322,3 +322,14 @@ def test_flat_axis_bit_exact(cuda_device):
     for hash_type in (1, 2):
         nb, div, out = _gpu_scatter(cuda_device, c16, seps, 256, hash_type, c16.shape[0])
         _compare(out, _oracle(c16, seps, nb, div, 256, hash_type, c16.shape[0]))
+
+
+@pytest.mark.parametrize("sizes,bucket,hash_type", [([24320], 256, 2), ([24576], 256, 1), ([24577], 256, 2), ([20992], 256, 1), ([21248, 1, 0, 257], 256, 2),
+                                                    ([9000, 22000, 300], 128, 2)])
+def test_small_tables_without_scan_launches(cuda_device, sizes, bucket, hash_type):
+    """Both sides of the line from which tiles add the tables up by themselves: the largest tile count, the largest table."""
+    coords32, seps = synthetic.batch(synthetic.lidar_scan, sizes, seed=13)
+    c16 = coords32.astype(np.float16)
+    pad_to = -(-c16.shape[0] // bucket) * bucket + bucket
+    nb, div, out = _gpu_scatter(cuda_device, c16, seps, bucket, hash_type, pad_to)
+    _compare(out, _oracle(c16, seps, nb, div, bucket, hash_type, pad_to))
