@@ -14,8 +14,13 @@ namespace f3d {
 
 constexpr int kLnbThreads = 256;
 
+// Blocks an SM holds, and the grid's blocks per SM: rows are strided over a resident grid, so that a warp requests its next row
+// while the reductions of the current one run (one row in flight a warp, with the residual gradient requested only behind the
+// reductions: 142 us for 100,352 rows of 512, 101 us for 200,704 of 256, 63 us at the copy rate; now 117 and 93).
+constexpr int lnb_blocks(int chunks) { return chunks == 1 ? 3 : chunks == 2 ? 2 : 1; }
+
 template <int LPR, int CHUNKS>
-__global__ void __launch_bounds__(kLnbThreads) layernorm_bwd_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ g,
+__global__ void __launch_bounds__(kLnbThreads, lnb_blocks(CHUNKS)) layernorm_bwd_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ g,
                                                                     const float *__restrict__ w, const __nv_bfloat16 *__restrict__ add,
                                                                     __nv_bfloat16 *__restrict__ dx,
                                                                     float *__restrict__ partial, uint32_t rows, uint32_t C, float eps) {
@@ -36,17 +41,31 @@ __global__ void __launch_bounds__(kLnbThreads) layernorm_bwd_kernel(const __nv_b
 #pragma unroll
     for (int e = 0; e < 8; ++e) { ww[i][e] = ch < nchunk ? __ldg(w + ch * 8 + e) : 0.f; dw[i][e] = 0.f; db[i][e] = 0.f; }
   }
+  uint4 nx[CHUNKS], ng[CHUNKS], na[CHUNKS];                     // the next row as it is in memory
+  const auto request = [&](uint32_t r) {
+#pragma unroll
+    for (int i = 0; i < CHUNKS; ++i) {
+      const uint32_t ch = sl + i * LPR;
+      if (r < rows && ch < nchunk) {
+        nx[i] = __ldg(reinterpret_cast<const uint4 *>(x + (size_t)r * C) + ch);
+        ng[i] = __ldg(reinterpret_cast<const uint4 *>(g + (size_t)r * C) + ch);
+        if (add) na[i] = __ldg(reinterpret_cast<const uint4 *>(add + (size_t)r * C) + ch);
+      }
+    }
+  };
+  request(blockIdx.x * kRowsPerBlock + warp * kRowsPerWarp + sub);
   for (uint32_t r0 = blockIdx.x * kRowsPerBlock; r0 < rows; r0 += gridDim.x * kRowsPerBlock) {
     const uint32_t row = r0 + warp * kRowsPerWarp + sub;
     const bool live = row < rows;
     float xv[CHUNKS][8], gv[CHUNKS][8];
+    uint4 ca[CHUNKS];
     float sum = 0.f;
 #pragma unroll
     for (int i = 0; i < CHUNKS; ++i) {
       const uint32_t ch = sl + i * LPR;
       if (live && ch < nchunk) {
-        const uint4 qx = __ldg(reinterpret_cast<const uint4 *>(x + (size_t)row * C) + ch);
-        const uint4 qg = __ldg(reinterpret_cast<const uint4 *>(g + (size_t)row * C) + ch);
+        const uint4 qx = nx[i], qg = ng[i];
+        ca[i] = na[i];
         const __nv_bfloat162 *hx = reinterpret_cast<const __nv_bfloat162 *>(&qx), *hg = reinterpret_cast<const __nv_bfloat162 *>(&qg);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
@@ -59,6 +78,7 @@ __global__ void __launch_bounds__(kLnbThreads) layernorm_bwd_kernel(const __nv_b
         for (int e = 0; e < 8; ++e) { xv[i][e] = 0.f; gv[i][e] = 0.f; }
       }
     }
+    request(row + gridDim.x * kRowsPerBlock);
 #pragma unroll
     for (uint32_t d = LPR >> 1; d; d >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, d);
     const float mean = sum * inv_c;
@@ -95,8 +115,8 @@ __global__ void __launch_bounds__(kLnbThreads) layernorm_bwd_kernel(const __nv_b
     for (int i = 0; i < CHUNKS; ++i) {
       const uint32_t ch = sl + i * LPR;
       if (live && ch < nchunk) {
-        uint4 q, qa = make_uint4(0u, 0u, 0u, 0u);
-        if (add) qa = __ldg(reinterpret_cast<const uint4 *>(add + (size_t)row * C) + ch);
+        uint4 q;
+        const uint4 qa = ca[i];
         __nv_bfloat162 *h = reinterpret_cast<__nv_bfloat162 *>(&q);
         const __nv_bfloat162 *ha = reinterpret_cast<const __nv_bfloat162 *>(&qa);
 #pragma unroll
@@ -196,7 +216,8 @@ extern "C" int f3d_layernorm_bwd_add_bf16(const void *x, const void *grad_out, c
   const uint32_t chunks = (nchunk + lpr - 1) / lpr;
   const uint32_t rows_per_block = (kLnbThreads / 32) * (32 / lpr);
   uint32_t grid = (rows + rows_per_block - 1) / rows_per_block;
-  if (grid > 148u * 8u) grid = 148u * 8u;
+  const uint32_t resident = (uint32_t)(sm_count(device) * lnb_blocks(chunks > 2 ? 4 : (int)chunks));
+  if (grid > resident) grid = resident;
   void *partial = nullptr;
   F3D_TRY(workspace(device, 3, (size_t)grid * 2 * C * sizeof(float), st, &partial));
   auto xp = static_cast<const __nv_bfloat16 *>(x), gp = static_cast<const __nv_bfloat16 *>(grad_out);
