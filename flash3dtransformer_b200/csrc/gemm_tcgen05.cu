@@ -45,11 +45,15 @@ namespace f3d {
 // A third build takes the gradient through SwiGLU: the product recomputes the pre-activation [gate | up] of a projection and
 // the epilogue turns it, with the gradient of the activation, into the gradient of [gate | up], so the pre-activation never
 // leaves the chip.
+// A fourth (kMlpBwd) forms the gradient of the activation too, as a second product into accumulators of its own: the k-blocks
+// of A W^T are followed by those of A2 W2^T, so neither that gradient nor the pre-activation exists in memory.  A tile is 64
+// hidden columns (gate, up and gradient: 192 accumulator columns, two tiles in tensor memory).  With few k-blocks only: see
+// kMlpBwdMaxChannels for the measurements.
 // Two more carry one of the general build's additions each, the folded LayerNorm or the row sums: what a backbone's inference
 // runs at its wide levels, without the code of the others (8192 rows, N = 4096, K = 512 folded: 30.5 -> 28.4 us; N = 1536
 // 17.0 -> 15.6).  SwiGLU has builds of its own as well: the choice of the activation costs nothing at run time.
-enum GemmBuild : int { kGeneral = 0, kLean = 1, kSwigluBwd = 2, kFold = 3, kSums = 4, kLeanSwiglu = 5, kFoldSwiglu = 6 };
-constexpr bool is_lean(int build) { return build == kLean || build == kLeanSwiglu || build == kSwigluBwd; }
+enum GemmBuild : int { kGeneral = 0, kLean = 1, kSwigluBwd = 2, kFold = 3, kSums = 4, kLeanSwiglu = 5, kFoldSwiglu = 6, kMlpBwd = 7 };
+constexpr bool is_lean(int build) { return build == kLean || build == kLeanSwiglu || build == kSwigluBwd || build == kMlpBwd; }
 constexpr int epi_warps(bool lean) { return lean ? 16 : 12; }
 constexpr int gemm_threads(bool lean) { return 64 + 32 * epi_warps(lean); }     // TMA warp, MMA warp, epilogue warps
 constexpr int BM = 128;
@@ -154,14 +158,15 @@ template <bool F16> __device__ __forceinline__ float unpack_in1(const __nv_bfloa
 template <int BN, bool F16, int BUILD>
 __global__ void __launch_bounds__(gemm_threads(is_lean(BUILD)), 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                         const __grid_constant__ CUtensorMap map_c, GemmArgs g) {
+                         const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_a2,
+                         const __grid_constant__ CUtensorMap map_b2, GemmArgs g) {
   constexpr bool LEAN = is_lean(BUILD), kFolded = BUILD == kFold || BUILD == kFoldSwiglu;
   constexpr bool kLn = BUILD == kGeneral || kFolded, kRowSums = BUILD == kGeneral || BUILD == kSums, kRest = BUILD == kGeneral;
   using S = GemmSmem<BN, LEAN>;
   constexpr int kEpiWarps = S::kEpiWarps, kGemmThreads = gemm_threads(LEAN);
   constexpr int kStages = S::kStages;
-  constexpr int kAcc = S::kAcc;
-  constexpr uint32_t kTmemCols = kAcc * BN < 32 ? 32 : kAcc * BN;
+  constexpr int kAcc = BUILD == kMlpBwd ? 2 : S::kAcc, kAccCols = BUILD == kMlpBwd ? 256 : BN;
+  constexpr uint32_t kTmemCols = kAcc * kAccCols < 32 ? 32 : kAcc * kAccCols;
   extern __shared__ unsigned char smem_raw[];
   unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char *stage_base = smem;
@@ -174,12 +179,12 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   float2 *stat_slots = reinterpret_cast<float2 *>(fold_base + S::kFoldBytes + S::kBarBytes);
   int *stat_cnt = reinterpret_cast<int *>(stat_slots + kAcc * 4 * (kEpiWarps / 4) * 32);
 
-  const bool swiglu = kRest ? g.epilogue == EPI_SWIGLU : BUILD == kSwigluBwd || BUILD == kLeanSwiglu || BUILD == kFoldSwiglu;
+  const bool swiglu = kRest ? g.epilogue == EPI_SWIGLU : BUILD == kSwigluBwd || BUILD == kLeanSwiglu || BUILD == kFoldSwiglu || BUILD == kMlpBwd;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m_tiles = (g.M + BM - 1) / BM, n_tiles = (g.N + BN - 1) / BN;
   const int num_tiles = m_tiles * n_tiles;
   const int kb_per_split = (g.K + BK - 1) / BK;
-  const int kb_count = kb_per_split * g.ksplit;
+  const int kb_count = kb_per_split * (BUILD == kMlpBwd ? 2 : g.ksplit);
   // The bias enters the product itself when the kernel has one column tile: the tile of ones times the columns' bias
   // terms (hi + mid + lo in the element type, exact to 2^-24) adds b[n] to every accumulator in fp32, and the epilogue
   // neither loads nor adds it.  Every 16-byte half of the ones rows is (1, 1, 1, 0, ...), the bias rows carry their terms
@@ -242,7 +247,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       // s % kb_count, so its W tile never changes: it is loaded on the stage's first use and stays resident.
       // (A TMA tile load costs about 7 cycles per box row whatever the row length; reloading a 128- or 256-row W
       // tile for every 128 rows of A took a third of the time of the narrow-K shapes.)
-      const bool w_resident = n_tiles == 1 && kStages % kb_count == 0;
+      const bool w_resident = BUILD != kMlpBwd && n_tiles == 1 && kStages % kb_count == 0;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
         const int mt = n_tiles == 1 ? tile : tile / n_tiles;      // a single column tile is the common case: no division
         const int m0 = mt * BM, n0 = (tile - mt * n_tiles) * BN;
@@ -250,6 +255,13 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
           const uint32_t s = it % kStages, ph = (it / kStages) & 1u;
           if (!tc::mbar_wait(&empty[s], ph ^ 1u, wc, 101)) { ok = false; break; }
           unsigned char *sa = stage_base + s * S::kStageBytes;
+          if (BUILD == kMlpBwd && kb >= kb_per_split) {            // the second product: 128 rows of A2, 64 of W2
+            const int x2 = (kb - kb_per_split) * BK;
+            tc::mbar_expect_tx(&full[s], S::kABytes + S::kBBytes / 2);
+            tc::tma_load_2d(sa, &map_a2, &full[s], x2, m0);
+            tc::tma_load_2d(sa + S::kABytes, &map_b2, &full[s], x2, n0 / 2);
+            continue;
+          }
           // k-block kb of slice sp starts at column kx of rows [sp * M + m0, ...) of A and [sp * N + n0, ...) of W;
           // columns past K are zero-filled by the copy, rows past a slice's end land in rows or columns never stored
           int kx = kb * BK, ya = m0, yb = n0;
@@ -286,13 +298,21 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         const uint32_t acc = t_local % kAcc, aph = (t_local / kAcc) & 1u;
         if (!tc::mbar_wait(&acc_empty[acc], aph ^ 1u, wc, 102)) { ok = false; break; }
         tc::tc_fence_after_sync();
-        const uint32_t d_tmem = tmem_base + acc * BN;
+        const uint32_t d_tmem = tmem_base + acc * kAccCols;
         for (int kb = 0; kb < kb_count; ++kb, ++it) {
           const uint32_t s = it % kStages, ph = (it / kStages) & 1u;
           if (!tc::mbar_wait(&full[s], ph, wc, 103)) { ok = false; break; }
           tc::tc_fence_after_sync();
           const uint32_t sa = tc::smem_u32(stage_base + s * S::kStageBytes);
           const uint64_t adesc = tc::kmajor_sw128_desc(sa), bdesc = tc::kmajor_sw128_desc(sa + S::kABytes);
+          if (BUILD == kMlpBwd && kb >= kb_per_split) {
+#pragma unroll
+            for (int k = 0; k < BK / 16; ++k)
+              tc::mma_f16_ss(d_tmem + BN, adesc + 2u * k, bdesc + 2u * k, tc::make_idesc_f16(BM, BN / 2, !F16, false, false),
+                             kb != kb_per_split || k ? 1u : 0u);
+            tc::mma_commit(&empty[s]);
+            continue;
+          }
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k)
             tc::mma_f16_ss(d_tmem, adesc + 2u * k, bdesc + 2u * k, idesc, (kb | k) != 0 ? 1u : 0u);
@@ -343,16 +363,16 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       const int first_col = swiglu ? n0 / 2 : n0;
       const int out_cols = min(tile_cols, (total_cols - first_col + 31) & ~31);
       // the rows of the residual are requested before the product is awaited: a tile's first use of them is a chain of its own
-      if (!kFolded && BUILD != kLeanSwiglu && g.residual && row < g.M)
+      if (!kFolded && BUILD != kLeanSwiglu && BUILD != kMlpBwd && g.residual && row < g.M)
         for (int c0 = (int)((sub + kSub - task % kSub) % kSub) * 32; c0 < out_cols; c0 += 32 * (int)kSub)
           if (first_col + c0 < total_cols) asm volatile("prefetch.global.L1 [%0];" ::"l"(g.residual + (size_t)row * g.ldr + first_col + c0));
       if (!tc::mbar_wait(&acc_full[acc], aph, wc, 104)) { ok = false; break; }
       tc::tc_fence_after_sync();
-      const uint32_t t_row = tmem_base + acc * BN + ((uint32_t)(q * 32) << 16);
+      const uint32_t t_row = tmem_base + acc * kAccCols + ((uint32_t)(q * 32) << 16);
       for (int c0 = (int)((sub + kSub - task % kSub) % kSub) * 32; c0 < out_cols; c0 += 32 * (int)kSub) {
         float v[32];
         const int oc0 = (swiglu ? n0 / 2 : n0) + c0;      // first output column of the task
-        if constexpr (BUILD == kSwigluBwd) {
+        if constexpr (BUILD == kSwigluBwd || BUILD == kMlpBwd) {
           // 16 columns at a time: gate a, up u, gradient o of the activation -> o u s (1 + a (1 - s)) and o a s, s = sigmoid(a)
           if (tc::elect_one()) tc::tma_wait_read<0>();            // both staging buffers, one for each half of the output
           __syncwarp();
@@ -362,7 +382,10 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             tc::tmem_ld_32x32b_x16(t_row + c0 + hh * 16, r);
             tc::tmem_ld_32x32b_x16(t_row + BN / 2 + c0 + hh * 16, u);
             uint4 o4[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
-            if (row < g.M) {
+            uint32_t of[16];
+            if constexpr (BUILD == kMlpBwd) {
+              tc::tmem_ld_32x32b_x16(t_row + BN + c0 + hh * 16, of);
+            } else if (row < g.M) {
               const uint4 *op = reinterpret_cast<const uint4 *>(g.residual + (size_t)row * g.ldr + oc0 + hh * 16);
               o4[0] = __ldg(op); o4[1] = __ldg(op + 1);
             }
@@ -379,7 +402,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                 const float2 ba = __ldg(pg + e), bb = __ldg(pu + e);
                 a.x += ba.x; a.y += ba.y; b.x += bb.x; b.y += bb.y;
               }
-              const float2 o = unpack_in2<F16>(ow[e]);
+              const float2 o = BUILD == kMlpBwd ? make_float2(__uint_as_float(of[2 * e]), __uint_as_float(of[2 * e + 1])) : unpack_in2<F16>(ow[e]);
               const float s0 = __fdividef(1.f, 1.f + __expf(-a.x)), s1 = __fdividef(1.f, 1.f + __expf(-a.y));
               const float t0 = o.x * s0, t1 = o.y * s1;
               wg[e] = pack_out2<F16>(t0 * b.x * fmaf(a.x, 1.f - s0, 1.f), t1 * b.y * fmaf(a.y, 1.f - s1, 1.f));
@@ -642,13 +665,13 @@ int *status_word(int device);   // device word, zero until a kernel reports an a
 
 template <int BN, bool F16, int BUILD>
 static int launch_gemm_build(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &mc, const GemmArgs &g, int device,
-                             cudaStream_t st) {
+                             cudaStream_t st, const CUtensorMap *ma2 = nullptr, const CUtensorMap *mb2 = nullptr) {
   constexpr bool LEAN = is_lean(BUILD);
   auto kern = gemm_bf16_tcgen05_kernel<BN, F16, BUILD>;
   F3D_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(kern), device, GemmSmem<BN, LEAN>::kTotal));
   int tiles = ((g.M + BM - 1) / BM) * ((g.N + BN - 1) / BN);
   int grid = tiles < sm_count(device) ? tiles : sm_count(device);
-  launch(kern, grid, gemm_threads(LEAN), GemmSmem<BN, LEAN>::kTotal, st, ma, mb, mc, g);
+  launch(kern, grid, gemm_threads(LEAN), GemmSmem<BN, LEAN>::kTotal, st, ma, mb, mc, ma2 ? *ma2 : ma, mb2 ? *mb2 : mb, g);
   return check_launch("gemm_bf16_tcgen05");
 }
 
@@ -780,9 +803,37 @@ static int linear_swiglu_bwd(const void *A, const void *W, const void *bias, con
   return BN == 256 ? launch_gemm_build<256, false, kSwigluBwd>(ma, mb, mc, g, device, st) : launch_gemm_build<128, false, kSwigluBwd>(ma, mb, mc, g, device, st);
 }
 
+// dY [M, 2 hid] = gradient of silu(gate) * up with respect to [gate | up] = A W^T + bias where the gradient of the activation is
+// A2 W2^T: A, A2 [M, K], W [2 hid, K], W2 [hid, K]
+static int mlp_swiglu_bwd(const void *A, const void *W, const void *bias, const void *A2, const void *W2, void *dY, int M, int hid, int K, int device,
+                          cudaStream_t st) {
+  if (M <= 0 || hid <= 0 || K <= 0 || K % 8 || hid % 64) return set_error(F3D_ERR_ARG, "mlp gradient: M, hidden, K = %d, %d, %d (hidden %% 64, K %% 8 must be 0)", M, hid, K);
+  if (reinterpret_cast<uintptr_t>(dY) % 16) return set_error(F3D_ERR_ARG, "mlp gradient: output pointer is not 16-byte aligned");
+  const int N = 2 * hid;
+  CUtensorMap ma, mb, mc, ma2, mb2;
+  F3D_TRY(encode_tmap_2d(&ma, 0, A, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, BK, BM, 128));
+  F3D_TRY(encode_tmap_2d(&mb, 0, W, (uint64_t)K, (uint64_t)N, (uint64_t)K * 2, BK, 64, 128));
+  F3D_TRY(encode_tmap_2d(&ma2, 0, A2, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, BK, BM, 128));
+  F3D_TRY(encode_tmap_2d(&mb2, 0, W2, (uint64_t)K, (uint64_t)hid, (uint64_t)K * 2, BK, 64, 128));
+  F3D_TRY(encode_tmap_3d(&mc, 0, dY, (uint64_t)N, (uint64_t)M, 1, (uint64_t)N * 2, (uint64_t)M * N * 2, 32, 32, 1, 64));
+  GemmArgs g{M, N, K, 1, N, static_cast<const float *>(bias), nullptr, 0, EPI_SWIGLU, 0,
+             static_cast<__nv_bfloat16 *>(dY), (long long)M * N, status_word(device), 1, nullptr, nullptr, 0.f, 0.f, nullptr};
+  if (!g.status) return F3D_ERR_CUDA;
+  return launch_gemm_build<128, false, kMlpBwd>(ma, mb, mc, g, device, st, &ma2, &mb2);
+}
+
 }  // namespace f3d
 
 using namespace f3d;
+
+extern "C" int f3d_mlp_swiglu_bwd_bf16(const void *A, const void *W, const void *bias, const void *A2, const void *W2, void *grad_pre_act, int M,
+                                       int hidden, int K, int device, void *stream) {
+  DeviceGuard guard(device);
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  F3D_TRY(maybe_sync(st, "mlp_swiglu_bwd"));
+  F3D_TRY(mlp_swiglu_bwd(A, W, bias, A2, W2, grad_pre_act, M, hidden, K, device, st));
+  return maybe_sync(st, "mlp_swiglu_bwd");
+}
 
 extern "C" int f3d_linear_swiglu_bwd_bf16(const void *A, const void *W, const void *bias, const void *grad_out, void *grad_pre_act, int M, int N, int K,
                                           int device, void *stream) {

@@ -98,7 +98,7 @@ extern "C" int f3d_xfmr_stack_bf16(const f3d_xfmr_block *blocks, int count, cons
 }
 
 // ------------------------------------------------------------------------------------------------------- training
-// The same block with what its backward pass needs kept, and that backward pass: 7 and 21 launches issued by one call each.
+// The same block with what its backward pass needs kept, and that backward pass: 7 and 20 or 21 launches issued by one call each.
 // Operator by operator autograd needed 33 ms of host time for a micro-batch that the GPU works on for 34 ms; what falls away
 // besides are the additions of the residual gradients (they ride in the LayerNorm gradients) and the pre-activation of the MLP
 // (its gradient is taken inside the product that recomputes it).
@@ -120,16 +120,23 @@ extern "C" int f3d_xfmr_block_fwd_bf16(const f3d_xfmr_block *blk, const f3d_xfmr
 }
 
 namespace f3d {
-// gradient of the hidden rows first; once the pre-activation's gradient exists the [rows, C] intermediates take its place
+// Widest block whose gradient of the hidden rows is formed inside the SwiGLU gradient.  Its tiles are narrow (64 hidden columns),
+// so A is read more often, while 8 hid bytes a row need not move: with one to four k-blocks that is a gain (gradient of the hidden
+// rows and of [gate | up], separately -> together: C = 32 at 1,605,632 rows 381 -> 218 us, C = 128 at 401,408 400 -> 278, C = 256
+// at 200,704 456 -> 450 and at 22,912 62 -> 56), with eight it is a loss (C = 512 at 100,352 rows 661 -> 792 us).
+constexpr int kMlpBwdMaxChannels = 256;
+
+// gradient of the hidden rows first, where it is needed; once the pre-activation's gradient exists the [rows, C] intermediates
+// take its place
 struct BlockBwdScratch {
   size_t g_hid, g_n2, g_attn, g_n1, delta, total;
   BlockBwdScratch(size_t rows, size_t c, size_t hid, size_t heads) {
     const auto up = [](size_t b) { return (b + 255) & ~size_t(255); };
-    const size_t row = up(rows * c * 2);
+    const size_t row = up(rows * c * 2), first = c > (size_t)kMlpBwdMaxChannels ? up(rows * hid * 2) : 0;
     g_hid = g_n2 = 0;
     g_attn = row;
     g_n1 = 2 * row;
-    delta = up(rows * hid * 2) > 3 * row ? up(rows * hid * 2) : 3 * row;
+    delta = first > 3 * row ? first : 3 * row;
     total = delta + up(rows * heads * 4);
   }
 };
@@ -154,10 +161,14 @@ extern "C" int f3d_xfmr_block_bwd_bf16(const f3d_xfmr_block *blk, const f3d_xfmr
   const auto gemm = [&](const void *a, const void *wt, void *out, int n, int k) {
     return f3d_linear_fused(a, wt, nullptr, nullptr, out, m, n, k, 1, 0, 0, nullptr, nullptr, 0.f, nullptr, device, stream);
   };
-  // MLP: fc2, SwiGLU, fc1, LayerNorm (+ the residual gradient)
-  F3D_TRY(gemm(grad_out, gr->fc2_wt, g_hid, hid, c));
+  // MLP: fc2 and SwiGLU, fc1, LayerNorm (+ the residual gradient)
   if (gr->fc2_w) F3D_TRY(f3d_linear_wgrad_bf16(grad_out, t->hid, gr->fc2_w, gr->fc2_b, m, c, hid, device, stream));
-  F3D_TRY(f3d_linear_swiglu_bwd_bf16(t->n2, b.fc1_w, b.fc1_b, g_hid, gr->g_pre, m, 2 * hid, c, device, stream));
+  if (c <= kMlpBwdMaxChannels) {
+    F3D_TRY(f3d_mlp_swiglu_bwd_bf16(t->n2, b.fc1_w, b.fc1_b, grad_out, gr->fc2_wt, gr->g_pre, m, hid, c, device, stream));
+  } else {
+    F3D_TRY(gemm(grad_out, gr->fc2_wt, g_hid, hid, c));
+    F3D_TRY(f3d_linear_swiglu_bwd_bf16(t->n2, b.fc1_w, b.fc1_b, g_hid, gr->g_pre, m, 2 * hid, c, device, stream));
+  }
   F3D_TRY(gemm(gr->g_pre, gr->fc1_wt, g_n2, c, 2 * hid));
   if (gr->fc1_w) F3D_TRY(f3d_linear_wgrad_bf16(gr->g_pre, t->n2, gr->fc1_w, gr->fc1_b, m, 2 * hid, c, device, stream));
   F3D_TRY(f3d_layernorm_bwd_add_bf16(t->mid, g_n2, b.ln2_w, grad_out, gr->g_mid, gr->ln2_w, gr->ln2_b, rows, channels, b.ln2_eps, device, stream));

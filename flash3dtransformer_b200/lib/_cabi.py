@@ -74,6 +74,7 @@ PROTOTYPES = {
                                        _u32, _int, _vp]),
     "f3d_xfmr_block_bwd_scratch": (c_uint64, [_u32, _u32, _u32, _u32]),
     "f3d_linear_swiglu_bwd_bf16": (_int, [_vp, _vp, _vp, _vp, _vp, _int, _int, _int, _int, _vp]),
+    "f3d_mlp_swiglu_bwd_bf16": (_int, [_vp, _vp, _vp, _vp, _vp, _vp, _int, _int, _int, _int, _vp]),
     "f3d_layernorm_bwd_add_bf16": (_int, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _u32, _u32, _f32, _int, _vp]),
     "f3d_gemm_sm_bf16": (_int, [_vp, _vp, _vp, _int, _int, _int, _int, _vp]),
     "f3d_buck_swin_fwd": (_int, [_vp, _vp, _vp, _vp, _vp, _vp, _int, _int, _int, _int, _int, _int, _u32, _int, _vp]),

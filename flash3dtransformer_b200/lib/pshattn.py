@@ -632,6 +632,26 @@ def linear_swiglu_bwd_bf16(x, weight, bias, grad_out, grad_pre_act) -> None:
     _cabi.check(st, "linear_swiglu_bwd_bf16")
 
 
+def mlp_swiglu_bwd_bf16(x, weight, bias, grad_out, weight2_t, grad_pre_act) -> None:
+    """linear_swiglu_bwd_bf16 for grad_out @ weight2_t^T instead of grad_out, the product formed inside: x, grad_out bf16
+    [M, K], weight bf16 [2F, K], weight2_t bf16 [F, K], grad_pre_act bf16 [M, 2F]."""
+    ts, names = [x, weight, grad_out, weight2_t, grad_pre_act], ["x", "weight", "grad_out", "weight2_t", "grad_pre_act"]
+    dev = _check_tensors(ts, names)
+    _check_dtype(ts, names, torch.bfloat16)
+    m, k = x.shape
+    n = weight.shape[0]
+    if weight.shape[1] != k or grad_out.shape != x.shape or tuple(weight2_t.shape) != (n // 2, k) or tuple(grad_pre_act.shape) != (m, n):
+        raise RuntimeError(f"weight must be [2F,{k}], weight2_t [F,{k}], grad_out [{m},{k}] and grad_pre_act [{m}, 2F]")
+    if bias is not None:
+        _check_tensors([x, bias], ["x", "bias"])
+        _check_dtype([bias], ["bias"], torch.float32)
+        if bias.numel() != n:
+            raise RuntimeError(f"bias must have {n} elements")
+    st = _cabi.load().f3d_mlp_swiglu_bwd_bf16(_ptr(x), _ptr(weight), _ptr(bias) if bias is not None else None, _ptr(grad_out),
+                                              _ptr(weight2_t), _ptr(grad_pre_act), m, n // 2, k, dev, _stream(dev))
+    _cabi.check(st, "mlp_swiglu_bwd_bf16")
+
+
 def gelu_bwd_bf16(pre_act, grad_out, grad_pre_act, tanh_form: bool = False) -> None:
     """grad_pre_act = grad_out * gelu'(pre_act), all bf16 of one shape: the exact (error function) form, or the tanh form
     of the GEMM's GELU epilogue.  Not part of the reference's operator module (its GELU backward is torch autograd's)."""

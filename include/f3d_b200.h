@@ -241,6 +241,9 @@ int f3d_row_stats_bf16(const void *x, void *stats, uint32_t rows, uint32_t C, in
 
 /* grad_pre_act [M, N] = gradient of silu(gate) * up with respect to [gate | up] = A W^T + bias (fp32 [N] or NULL) for
  * grad_out [M, N / 2]; bf16, the pre-activation is recomputed inside the product.  N a multiple of 128, K of 8. */
+/* the same where grad_out is the product A2 W2^T (A2 bf16 [M, K], W2 bf16 [hidden, K]), formed in the same kernel */
+int f3d_mlp_swiglu_bwd_bf16(const void *A, const void *W, const void *bias, const void *A2, const void *W2, void *grad_pre_act, int M, int hidden,
+                            int K, int device, void *stream);
 int f3d_linear_swiglu_bwd_bf16(const void *A, const void *W, const void *bias, const void *grad_out, void *grad_pre_act, int M, int N,
                                int K, int device, void *stream);
 

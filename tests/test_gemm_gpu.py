@@ -360,3 +360,22 @@ def test_linear_wgrad_of_split_outputs(cuda_device, m, s, c, k):
     ref_b = g.float().sum(1).reshape(-1)
     assert torch.isfinite(gw).all() and (gw - ref_w).abs().max().item() <= 1e-4 * ref_w.abs().max().item() + 1e-5 * m ** 0.5
     assert (gb - ref_b).abs().max().item() <= 1e-4 * ref_b.abs().max().item() + 1e-5 * m ** 0.5
+
+
+@pytest.mark.parametrize("m,f,k,bias", [(1, 64, 32, True), (127, 64, 16, True), (129, 192, 64, False), (300, 256, 128, True), (20000, 128, 32, True),
+                                        (5000, 1024, 256, False), (700, 2048, 512, True)])
+def test_mlp_swiglu_gradient(cuda_device, m, f, k, bias):
+    """The gradient of [gate | up] with the gradient of the activation formed in the same kernel: one and several k-blocks and
+    column tiles, the bias inside the product and outside."""
+    from flash3dtransformer_b200.lib import pshattn
+    gen = torch.Generator(cuda_device).manual_seed(m + f)
+    x, go = (torch.randn(m, k, device=cuda_device, generator=gen).bfloat16() for _ in range(2))
+    w1, w2t = ((torch.randn(r, k, device=cuda_device, generator=gen) / k ** 0.5).bfloat16() for r in (2 * f, f))
+    b = torch.randn(2 * f, device=cuda_device, generator=gen) if bias else None
+    out = torch.full((m, 2 * f), float("nan"), device=cuda_device, dtype=torch.bfloat16)
+    pshattn.mlp_swiglu_bwd_bf16(x, w1, b, go, w2t, out)
+    pshattn.device_status()
+    y = (x.float() @ w1.float().t() + (b if bias else 0.0)).requires_grad_(True)
+    gate, up = y.chunk(2, dim=1)
+    ref, = torch.autograd.grad(torch.nn.functional.silu(gate) * up, y, go.float() @ w2t.float().t())
+    _check(out, ref)
