@@ -185,11 +185,17 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   const int num_tiles = m_tiles * n_tiles;
   const int kb_per_split = (g.K + BK - 1) / BK;
   const int kb_count = kb_per_split * (BUILD == kMlpBwd ? 2 : g.ksplit);
-  // The bias enters the product itself when the kernel has one column tile: the tile of ones times the columns' bias
+  // Tiles are dealt out round-robin, column tile fastest: where the grid is a multiple of the column tiles a CTA keeps its
+  // columns (and with them its W tiles and its bias) from tile to tile.
+  const bool same_cols = n_tiles == 1 || gridDim.x % (uint32_t)n_tiles == 0;
+  const int own_n0 = n_tiles == 1 ? 0 : (int)(blockIdx.x % (uint32_t)n_tiles) * BN;
+  // The bias enters the product itself when a CTA keeps its columns (with several column tiles: and has many tiles of one
+  // k-block, whose epilogue is the bound): the tile of ones times the columns' bias
   // terms (hi + mid + lo in the element type, exact to 2^-24) adds b[n] to every accumulator in fp32, and the epilogue
   // neither loads nor adds it.  Every 16-byte half of the ones rows is (1, 1, 1, 0, ...), the bias rows carry their terms
   // in the first half and zeros in the second, so the sum does not depend on where the 32-byte swizzle puts the halves.
-  const bool fold_bias = g.bias != nullptr && g.ln_stats == nullptr && n_tiles == 1 && g.ksplit == 1;
+  const bool fold_bias = g.bias != nullptr && g.ln_stats == nullptr && g.ksplit == 1 && same_cols &&
+                         (n_tiles == 1 || (kb_count == 1 && num_tiles >= 4 * (int)gridDim.x));
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) { tc::mbar_init(&full[s], 1); tc::mbar_init(&empty[s], 1); }
     for (int a = 0; a < kAcc; ++a) { tc::mbar_init(&acc_full[a], 1); tc::mbar_init(&acc_empty[a], kEpiWarps); }
@@ -205,9 +211,9 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     for (int c = threadIdx.x; c < BM * 2; c += kGemmThreads) tc::sts128(tc::smem_u32(fold_base) + c * 16, make_uint4(one2, one1, 0u, 0u));
     for (int r = threadIdx.x; r < BN; r += kGemmThreads) {
       // row r of the W tile is output column r, or for SwiGLU gate column r | up column r - BN / 2
-      int col = r;
-      if (swiglu) col = r < BN / 2 ? r : g.N / 2 + (r - BN / 2);
-      const bool live = swiglu ? (r < BN / 2 ? r < g.N / 2 : r - BN / 2 < g.N / 2) : r < g.N;
+      int col = own_n0 + r;
+      if (swiglu) col = own_n0 / 2 + (r < BN / 2 ? r : g.N / 2 + (r - BN / 2));
+      const bool live = swiglu ? own_n0 / 2 + (r < BN / 2 ? r : r - BN / 2) < g.N / 2 : col < g.N;
       const float b = live ? __ldg(g.bias + col + after) : 0.f;
       uint32_t w0, w1;
       if (F16) {
@@ -243,11 +249,11 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     if (tc::elect_one()) {
       uint32_t it = 0;
       bool ok = true;
-      // With a single column tile and a k-block count that divides the ring, stage s always carries k-block
+      // With the same columns from tile to tile and a k-block count that divides the ring, stage s always carries k-block
       // s % kb_count, so its W tile never changes: it is loaded on the stage's first use and stays resident.
       // (A TMA tile load costs about 7 cycles per box row whatever the row length; reloading a 128- or 256-row W
       // tile for every 128 rows of A took a third of the time of the narrow-K shapes.)
-      const bool w_resident = BUILD != kMlpBwd && n_tiles == 1 && kStages % kb_count == 0;
+      const bool w_resident = same_cols && kStages % kb_count == 0 && (BUILD != kMlpBwd || kb_count == 2);
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
         const int mt = n_tiles == 1 ? tile : tile / n_tiles;      // a single column tile is the common case: no division
         const int m0 = mt * BM, n0 = (tile - mt * n_tiles) * BN;
@@ -257,9 +263,10 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
           unsigned char *sa = stage_base + s * S::kStageBytes;
           if (BUILD == kMlpBwd && kb >= kb_per_split) {            // the second product: 128 rows of A2, 64 of W2
             const int x2 = (kb - kb_per_split) * BK;
-            tc::mbar_expect_tx(&full[s], S::kABytes + S::kBBytes / 2);
+            const bool w2 = !w_resident || it < (uint32_t)kStages;
+            tc::mbar_expect_tx(&full[s], S::kABytes + (w2 ? S::kBBytes / 2 : 0));
             tc::tma_load_2d(sa, &map_a2, &full[s], x2, m0);
-            tc::tma_load_2d(sa + S::kABytes, &map_b2, &full[s], x2, n0 / 2);
+            if (w2) tc::tma_load_2d(sa + S::kABytes, &map_b2, &full[s], x2, n0 / 2);
             continue;
           }
           // k-block kb of slice sp starts at column kx of rows [sp * M + m0, ...) of A and [sp * N + n0, ...) of W;
@@ -671,6 +678,12 @@ static int launch_gemm_build(const CUtensorMap &ma, const CUtensorMap &mb, const
   F3D_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(kern), device, GemmSmem<BN, LEAN>::kTotal));
   int tiles = ((g.M + BM - 1) / BM) * ((g.N + BN - 1) / BN);
   int grid = tiles < sm_count(device) ? tiles : sm_count(device);
+  // With several rounds of tiles a grid that is a multiple of the column tiles lets every CTA keep its columns: worth the few
+  // SMs it leaves out (at most 1 in 30 here) for products of one k-block, which then load A only and take the bias in the
+  // product (983,040 rows, K = 64: N = 192 97 -> 83 us, N = 512 with SwiGLU 137 -> 117).  With two k-blocks it measured level
+  // or slower (N = 384, K = 128 90.6 -> 94.4), so those keep every SM.
+  const int n_tiles = (g.N + BN - 1) / BN, k_blocks = (g.K + BK - 1) / BK * (BUILD == kMlpBwd ? 2 : g.ksplit);
+  if (tiles >= 4 * grid && k_blocks == 1 && grid % n_tiles <= grid / 30) grid -= grid % n_tiles;
   launch(kern, grid, gemm_threads(LEAN), GemmSmem<BN, LEAN>::kTotal, st, ma, mb, mc, ma2 ? *ma2 : ma, mb2 ? *mb2 : mb, g);
   return check_launch("gemm_bf16_tcgen05");
 }

@@ -2,7 +2,7 @@
 
 Forward passes run the hand-written kernels (tcgen05 GEMM with fused bias / residual / SwiGLU epilogues, bucketed
 attention, pooling, unpooling).  In the backward passes of the projections the input gradient g W runs on the same
-tcgen05 GEMM; the weight gradient g^T x (a reduction over all rows) is a plain library GEMM.  The backward passes of
+tcgen05 GEMM and the weight gradient g^T x (a reduction over all rows) on a kernel of its own.  The backward passes of
 attention, pooling and unpooling run the native kernels.
 """
 from __future__ import annotations

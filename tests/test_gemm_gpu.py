@@ -379,3 +379,21 @@ def test_mlp_swiglu_gradient(cuda_device, m, f, k, bias):
     gate, up = y.chunk(2, dim=1)
     ref, = torch.autograd.grad(torch.nn.functional.silu(gate) * up, y, go.float() @ w2t.float().t())
     _check(out, ref)
+
+
+@pytest.mark.parametrize("m,n,k,epi", [(76000, 192, 64, 0), (76000, 512, 64, 2), (40000, 768, 32, 0), (128 * 600 - 1, 640, 64, 0), (30000, 1536, 16, 2)])
+def test_many_tiles_of_one_k_block(cuda_device, m, n, k, epi):
+    """Several rounds of tiles over several column tiles with one k-block: every CTA keeps its columns, W and the bias."""
+    from flash3dtransformer_b200.lib import pshattn
+    gen = torch.Generator(cuda_device).manual_seed(n + k)
+    x = torch.randn(m, k, device=cuda_device, generator=gen).bfloat16()
+    w = (torch.randn(n, k, device=cuda_device, generator=gen) / k ** 0.5).bfloat16()
+    b = torch.randn(n, device=cuda_device, generator=gen)
+    out = torch.full((m, n // 2 if epi == 2 else n), float("nan"), device=cuda_device, dtype=torch.bfloat16)
+    pshattn.linear_bf16(x, w, b, out, epilogue=epi)
+    pshattn.device_status()
+    ref = x.float() @ w.float().t() + b
+    if epi == 2:
+        gate, up = ref.chunk(2, dim=1)
+        ref = torch.nn.functional.silu(gate) * up
+    _check(out, ref)
