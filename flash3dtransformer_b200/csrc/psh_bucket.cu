@@ -202,7 +202,7 @@ __device__ __forceinline__ uint32_t scene_tiles(const PshArgs &a, uint32_t scene
 // Direct mode: sums of every column of a tile table over the scene's tiles in front of this one (pre) and over all of them
 // (tot), into shared memory.  A warp takes four columns at a time, a lane up to three of a column's words, so that twelve
 // loads are in flight.
-constexpr uint32_t kDirectTiles = 96, kDirectWords = 8192;
+constexpr uint32_t kDirectTiles = 96, kDirectWords = kDirectTiles * 129;
 __device__ __forceinline__ void column_sums(const PshArgs &a, const TileInfo &t, const uint32_t *tab, uint32_t *pre, uint32_t *tot) {
   const uint32_t tiles = scene_tiles(a, t.scene), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (uint32_t b0 = warp * 4; b0 < a.nbp; b0 += kPshWarps * 4) {
@@ -902,8 +902,9 @@ static int psh_run(PshArgs a, const PshPlan &p, uint32_t *scratch, uint32_t max_
   const unsigned scan_blocks = (unsigned)(((size_t)a.batch * p.nbp + kPshWarps - 1) / kPshWarps);
   // the round A table is fully rewritten by the histogram kernel for live tiles; the round B and C tables are
   // accumulated with atomics and must start at zero (they are adjacent: one memset)
-  // Small tables (a scan of 20,000 points: 79 tiles x 80 columns) cost a tile less to add up by itself, 32 words a thread at
-  // the limit, than a scan launch costs the stream and the host: four launches instead of seven and a memset.
+  // Small tables cost a tile less to add up by itself, 48 words a thread at the limit, than a scan launch costs the stream and
+  // the host: four launches instead of seven and a memset (a scan of 20,000 points, 79 tiles x 129 columns: 25.7 -> 21.8 us
+  // on the device, 18 -> 9 us of host time; from 97 tiles on a lane would need a fourth word of every column).
   a.direct = p.tiles_max <= kDirectTiles && (size_t)p.tiles_max * p.nbp <= kDirectWords;
   if (max_n > 0) {
     if (!a.direct) F3D_CUDA_TRY(cudaMemsetAsync(a.tabB, 0, 2 * rows * p.nbp * sizeof(uint32_t), st));
