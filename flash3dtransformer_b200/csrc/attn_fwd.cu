@@ -43,7 +43,7 @@ int *status_word(int device);
 constexpr int kBQ = 128;      // query rows per tile
 constexpr int kShortWindow = 8;     // query tiles of a scope up to which a CTA takes two (W = 1024)
 
-// How query tiles map to CTAs: one each; two of a scope one after the other (kTwoTiles); one shared by a cluster (kSplit).
+// How query tiles map to CTAs: one each; two of a scope one after the other (kTwoTiles); one shared by several (kSplit).
 // Builds of their own: the issuing thread's code is on the critical path, and what the plain mapping does not need costs it 2 %.
 enum AttnMode : int { kPlain = 0, kTwoTiles = 1, kSplit = 2 };
 
@@ -52,7 +52,9 @@ struct AttnFwdArgs {
   int B, L, H, num_scopes, k, bucket, q_blocks_per_bucket;   // q_blocks_per_bucket = bucket / 128
   float scale_log2;          // log2(e) / sqrt(D)
   int *status;
-  int splits;                // kSplit: CTAs (one cluster) that share the keys of a query tile, 2 or 4
+  int splits;                // kSplit: CTAs that share the keys of a query tile
+  float *parts;              // kSplit without clusters: [query tile][part][D + 2][128] O, reference and sum of every part, and
+  int *parts_done;           // [query tile] parts that have left theirs; zero before and after the launch
 };
 
 __device__ __forceinline__ float fast_exp2(float x) {
@@ -470,7 +472,60 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   if (pass == 1 || !__syncthreads_or(sm.ok && sm.bad)) break;
   }
 
-  if (SPLIT) {
+  if (SPLIT && a.parts) {
+    // The parts of a query tile meet in memory: each leaves its rows there, column by column, and the last one to do so adds
+    // them up, in the order of the parts.
+    __shared__ int last;
+    const size_t tile = (size_t)(blockIdx.z * gridDim.y + blockIdx.y) * (gridDim.x / a.splits) + blockIdx.x / a.splits;
+    float *const all = a.parts + tile * a.splits * kBQ * (D + 2) + row;                // this thread's row of every part
+    constexpr int kPart = kBQ * (D + 2);
+    if (warp != 0) {
+      float *const mine = all + (size_t)part * kPart;
+#pragma unroll
+      for (int c = 0; c < D; c += 16) {
+        uint32_t o[16];
+        tc::tmem_ld_32x32b_x16(sm.tmem_o + c, o);
+        tc::tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 16; ++i) mine[(c + i) * kBQ] = __uint_as_float(o[i]);
+      }
+      mine[D * kBQ] = sm.m_run;
+      mine[(D + 1) * kBQ] = sm.l_run;
+      __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(a.parts_done + tile, 1) == a.splits - 1;
+    __syncthreads();
+    const int q_tok = q_token(qt) + row;
+    if (last && warp != 0 && q_tok < a.L) {
+      __threadfence();
+      float m = -INFINITY, l = 0.f;
+      for (int p = 0; p < a.splits; ++p) m = fmaxf(m, __ldcg(all + (size_t)p * kPart + D * kBQ));
+      for (int p = 0; p < a.splits; ++p)
+        l = fmaf(fast_exp2(__ldcg(all + (size_t)p * kPart + D * kBQ) - m), __ldcg(all + (size_t)p * kPart + (D + 1) * kBQ), l);
+      const float inv = 1.f / l;
+      const size_t tok = (size_t)row0 + q_tok;
+      __nv_bfloat16 *const out = a.O + (tok * a.H + head) * D;
+#pragma unroll
+      for (int c = 0; c < D; c += 16) {
+        float x[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) x[i] = 0.f;
+        for (int p = 0; p < a.splits; ++p) {
+          const float *o = all + (size_t)p * kPart;
+          const float w = fast_exp2(__ldcg(o + D * kBQ) - m);
+#pragma unroll
+          for (int i = 0; i < 16; ++i) x[i] = fmaf(w, __ldcg(o + (c + i) * kBQ), x[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < 16; i += 8)
+          *reinterpret_cast<uint4 *>(out + c + i) = make_uint4(pack_p2<F16>(x[i] * inv, x[i + 1] * inv), pack_p2<F16>(x[i + 2] * inv, x[i + 3] * inv),
+                                                               pack_p2<F16>(x[i + 4] * inv, x[i + 5] * inv), pack_p2<F16>(x[i + 6] * inv, x[i + 7] * inv));
+      }
+      a.lse[tok * a.H + head] = (m + log2f(l)) * 0.6931471805599453f;
+    }
+    if (last && threadIdx.x == 0) a.parts_done[tile] = 0;
+  } else if (SPLIT) {
     // The parts of a query tile meet in shared memory: CTA p of the cluster receives every part's O, reference and sum of
     // `share` of the rows, over the operands nobody needs any more, and writes those rows.
     constexpr int kStride = D + 4;                                // floats per row of a part
@@ -541,11 +596,28 @@ static int launch_attn_fwd(const void *Q, const void *K, const void *V, AttnFwdA
   const long long room = (long long)sm_count(device) * C::kMinCtas;
   // A query tile is a chain of key tiles, 0.4 us each on an SM that has little else to do.  Where the tiles are so few that
   // the SMs would hold less than half of the CTAs they have room for, the keys of a tile are shared out to a cluster of two
-  // or four CTAs (three, and five to eight, measure slower: their clusters pack the SMs badly); a part keeps at least 512
+  // or four CTAs (clusters of three, and five to eight, measure slower: they pack the SMs badly); a part keeps at least 512
   // keys, below which joining the parts costs what the split saves.  One head, D = 32, W = 4096: 12,288 tokens 49 -> 29 us
   // (four), 24,576 tokens 59 -> 45 us (two; four, which no longer fit at once: 48).
   a.splits = 1;
   while (a.splits < 4 && tiles * heads * a.splits * 2 <= room && tiles_per_scope / (2 * a.splits) >= 4) a.splits *= 2;
+  // Where two CTAs a tile leave a third of the room empty and four do not fit at once, three do: packed into clusters they fit
+  // badly, so they are launched by themselves and meet in memory (3-4 us more than a cluster needs).  One head, W = 4096:
+  // 20,480 to 24,576 tokens D = 32 50 -> 39.5 us, 2 heads D = 64 57 -> 46.6; W = 2048: D = 32 28.8 -> 25.4; D = 128 46.4 -> 41.6.
+  if (a.splits == 2 && tiles * heads * 3 <= room && tiles_per_scope / 3 >= 4) {
+    void *parts = nullptr, *done = nullptr;
+    if (workspace(device, 11, (size_t)(tiles * heads) * 3 * kBQ * (D + 2) * sizeof(float), st, &parts) == F3D_OK &&
+        workspace(device, 12, (size_t)(tiles * heads) * sizeof(int), st, &done) == F3D_OK) {
+      a.splits = 3;
+      a.parts = static_cast<float *>(parts);
+      a.parts_done = static_cast<int *>(done);
+      auto kern = attn_fwd_kernel<D, F16, kSplit>;
+      F3D_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(kern), device, C::template smem<kSplit>()));
+      launch(kern, dim3((unsigned)(tiles * 3), a.H, a.B), C::kThreads, C::template smem<kSplit>(), st, mq, mk, mv, a);
+      return check_launch("buck_swin_fwd");
+    }
+    // (no scratch on a stream that captures before it ever ran this: the cluster of two)
+  }
   if (a.splits > 1) {
     auto kern = attn_fwd_kernel<D, F16, kSplit>;
     F3D_TRY(ensure_dynamic_smem(reinterpret_cast<const void *>(kern), device, C::template smem<kSplit>()));

@@ -135,6 +135,35 @@ def test_many_short_scopes(cuda_device, d, dtype, bucket, k, jump):
         assert (sub[4] - ref_lse).abs().max().item() <= 2e-2
 
 
+@pytest.mark.parametrize("l,h,d,bucket,k,dtype", [(24576, 1, 32, 512, 8, torch.bfloat16), (9728, 2, 16, 256, 19, torch.bfloat16), (10240, 2, 64, 512, 4, torch.float16),
+                                                  (12288, 1, 128, 512, 8, torch.bfloat16), (19968, 1, 32, 512, 3, torch.float16)])
+@pytest.mark.parametrize("jump", [False, True])
+def test_three_parts_of_a_tile(cuda_device, l, h, d, bucket, k, dtype, jump):
+    """Tile counts that three CTAs a tile fill the GPU with: parts of unequal length, a row whose scores send one part into the
+    careful pass, the same bits on a second run (the counters are back at zero).  Checked on the last scope."""
+    from flash3dtransformer_b200.lib import pshattn
+    dev = cuda_device
+    g = torch.Generator(dev).manual_seed(5)
+    q, kk, v = (torch.randn(1, l, h, d, generator=g, device=dev).to(dtype) for _ in range(3))
+    if jump:
+        kk[:, bucket * k - 5::bucket * k] *= 12.0
+        q[:, 7::128] *= 4.0
+    sc = torch.arange(l // bucket).reshape(-1, k)
+    runs = []
+    for _ in range(2):
+        o = torch.zeros(1, l, h, d, dtype=dtype, device=dev)
+        lse = torch.zeros(1, l, h, dtype=torch.float32, device=dev)
+        pshattn.buck_swin_fwd(q, kk, v, o, lse, sc.to(torch.uint32).to(dev), bucket)
+        runs.append((o, lse))
+    pshattn.device_status()
+    assert torch.equal(runs[0][0], runs[1][0]) and torch.equal(runs[0][1], runs[1][1])
+    rows = slice(l - bucket * k, l)
+    sub = [t[:, rows].cpu() for t in (q, kk, v, runs[0][0], runs[0][1])]
+    ref_o, ref_lse = ao.buck_swin_fwd(sub[0], sub[1], sub[2], torch.arange(k).reshape(1, k), bucket)
+    assert (sub[3].float() - ref_o).abs().max().item() <= 3e-2
+    assert (sub[4] - ref_lse).abs().max().item() <= 2e-2
+
+
 def test_errors(cuda_device):
     from flash3dtransformer_b200.lib import pshattn
     dev = cuda_device
