@@ -221,12 +221,16 @@ template <typename T>
 __global__ void __launch_bounds__(kPoolThreads) unpool_add_kernel(const T *__restrict__ res, const T *__restrict__ down,
                                                                   T *__restrict__ up, GatherArgs a, uint32_t covered_rows,
                                                                   uint32_t up_rows, uint32_t zero_blocks) {
+  constexpr uint32_t kTailReach = sizeof(T) == 4 ? 500 : 1000;
   const uint32_t after = grid_enter();
   res += after; down += after; a.unpool_ind += after;
   constexpr int N = Chunk<T>::N;
   // The blocks that clear the tail come first in the grid.  The mark of an unfilled slot (rows of the pooled input + 3) is
   // out of range for the pooling, but not for a residual padded by more than three rows: what the gather blocks store
-  // there, as the reference does, has to come behind the zeros.
+  // there, as the reference does, has to come behind the zeros.  It only counts near the tail: with the zeros written last, as
+  // they once were, a store from further than a resident round of blocks in front of them had long been cleared again, one
+  // from nearer came behind them.  That line (1,000 blocks, 500 for 4-byte features, where half of the stores survived) is
+  // kept as a rule, so that the row has the value it had and no longer depends on the timing.
   if (blockIdx.x < zero_blocks) {
     uint64_t gid = (uint64_t)blockIdx.x * kPoolThreads + threadIdx.x;
     uint64_t row = covered_rows + gid / a.chunks_per_row;
@@ -246,7 +250,7 @@ __global__ void __launch_bounds__(kPoolThreads) unpool_add_kernel(const T *__res
   Chunk<T>::load(down + (size_t)row * a.C + ch * N, d);
   for (uint32_t s = 0; s < a.S; ++s) {
     uint32_t r = __ldg(a.unpool_ind + (size_t)row * a.S + s);
-    if (r < a.valid_N) {
+    if (r < a.valid_N && (r < covered_rows || gridDim.x - blockIdx.x < kTailReach)) {
       float v[N];
       Chunk<T>::load(res + (size_t)r * a.C + ch * N, v);
 #pragma unroll

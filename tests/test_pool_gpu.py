@@ -184,3 +184,22 @@ def test_full_size_pool_unpool_properties(cuda_device):
     second = ind[:, 1]
     ok = second < down.shape[0]
     assert torch.equal(down[first[ok]], down[second[ok]])
+
+
+@pytest.mark.parametrize("dtype,C,blocks", [("bf16", 32, 1000), ("fp32", 128, 500)])
+def test_unpool_mark_in_the_tail(cuda_device, dtype, C, blocks):
+    """A marked slot that names a row of a padded residual's tail stores there when it lies near the tail, and leaves the zeros
+    when it lies further in front: on both sides of the line, the same on every run."""
+    from flash3dtransformer_b200.lib import pshattn
+    per_block = 256 // (C * (2 if dtype == "bf16" else 4) // 16)
+    rows = per_block * (blocks + 64)
+    n = rows * 2 - 1
+    res, down = (torch.ones(r, C, device=cuda_device, dtype=TORCH_DT[dtype]) for r in (n + 64, rows))
+    for behind, stored in ((blocks + 8, False), (blocks - 8, True), (1, True)):
+        ind = torch.arange(rows * 2)
+        ind[2 * (rows - behind * per_block) + 1] = n + 3
+        t = ind.to(torch.uint32).view(rows, 2).to(cuda_device)
+        for _ in range(5):
+            out = torch.full((n + 64, C), 5.0, device=cuda_device, dtype=TORCH_DT[dtype])
+            pshattn.additive_unpool_fwd(res, down, out, t, 2, covered_rows=n)
+            assert out[n + 3].float().eq(2.0 if stored else 0.0).all() and out[n + 4:].eq(0).all() and out[n:n + 3].eq(0).all()
