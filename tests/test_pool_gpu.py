@@ -193,7 +193,7 @@ def test_unpool_mark_in_the_tail(cuda_device, dtype, C, blocks):
     from flash3dtransformer_b200.lib import pshattn
     per_block = 256 // (C * (2 if dtype == "bf16" else 4) // 16)
     rows = per_block * (blocks + 64)
-    n = rows * 2 - 1
+    n = rows * 2
     res, down = (torch.ones(r, C, device=cuda_device, dtype=TORCH_DT[dtype]) for r in (n + 64, rows))
     for behind, stored in ((blocks + 8, False), (blocks - 8, True), (1, True)):
         ind = torch.arange(rows * 2)
